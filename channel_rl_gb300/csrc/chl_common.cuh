@@ -118,9 +118,6 @@ struct ChlInst {
   const double *dxf, *dyf, *dzf;  // raw spacings (dt)
   const double *hx2, *hy2, *hz2;  // squared centre widths (x(i)-x(i-1))^2 etc. (Vreman)
   const double *w0x2, *w1x2;      // 2 x weight_y_0/1 by face row jv
-  const double *w0, *w1;          // weight_y_0/1 by face row jv (w1 = 1 - w0)
-  const double *rdxc4, *rdyc4, *rdzc4;   // 4 x rdxc, rdyc, rdzc (centre fluxes, kept 4 x)
-  const double *rdxc2, *rdyc2, *rdzc2;   // 2 x rdxc, rdyc, rdzc (xy and yz edge fluxes, kept 2 x)
   // sqrt(4/216) x rdxc, rdyc, rdzc and rdxf, rdyf, rdzf: the dynamic model's
   // filtered strain, whose M_ij term needs 4/216 x |S| S_ij
   const double *rdxcs, *rdycs, *rdzcs, *rdxfs, *rdyfs, *rdzfs;
@@ -135,7 +132,13 @@ struct ChlInst {
   double *F1[3];                  // stage-1 RHS (kept for stages 2 and 3)
   double *Fp[3];                  // RHS for the actual pressure
   double *nut, *S;                // nu + nu_t (Ny+2 rows), |S| (Ny+2 rows)
-  double *G[9];                   // momentum face fluxes (chl_rhs.cu)
+  long long *G[9];                // momentum face fluxes in fixed point (chl_rhs.cu)
+  long long *X[3];                // U, V, W of the set being worked on, in fixed point (k_fix)
+  // reciprocal spacings and the y-face weight in fixed point: entry r stands
+  // for r 2^e, one exponent per table, r < 2^63 (chl_fix.cuh)
+  const long long *fxrxc, *fxrxf, *fxryc, *fxryf, *fxrzc, *fxrzf, *fxw1;
+  int exc, exf, eyc, eyf, ezc, ezf;
+  int *upd;                       // shifts and exponents of the stage update (chl_rhs.cu: UPD_*)
   double *q[CHL_NQ], *r[CHL_NQ];  // DSM filter ping-pong
   double *E[3];                   // edge fields (S12, S13, S23 numerators)
   double2 *spec;                  // [Ny+2][Nz][Nxh] spectra (rows 1..Ny used)
@@ -179,6 +182,14 @@ struct F64 {
   __device__ __forceinline__ double mul(double a, double b) const { return fma(a, b, mz); }
 };
 __device__ __forceinline__ F64 f64_of(const ChlInst& I) { return F64{I.fk[FK_ONE], I.fk[FK_MZERO]}; }
+
+// -x on the integer pipe (a store of -x would take an FP64 instruction, and
+// in every thread where the compiler predicates it)
+__device__ __forceinline__ double chl_neg(double x) {
+  long long r;
+  asm("xor.b64 %0, %1, 0x8000000000000000;" : "=l"(r) : "l"(__double_as_longlong(x)));
+  return __longlong_as_double(r);
+}
 
 // fmax(x, 0.0) on the integer pipe: x where its bit pattern is that of a
 // positive finite number or +inf, else +0 (negative numbers, zeros and NaN,
@@ -239,7 +250,7 @@ __device__ __forceinline__ double chl_sqrt(double a) {
 // device scalar slots
 enum {
   CHL_S_DT = 0, CHL_S_T, CHL_S_DPDX, CHL_S_Q0, CHL_S_SHIFT, CHL_S_DIVMAX,
-  CHL_S_DC,            // 6 slots: dt c1 / 4, dt c2 / 4 of RK3 stages 0, 1, 2
+  CHL_S_DC,            // 6 slots: dt c1, dt c2 of RK3 stages 0, 1, 2
   CHL_S_NSCAL = 16
 };
 
@@ -248,14 +259,13 @@ enum {
 __host__ __device__ inline double chl_rk_c1(int s) { return s == 0 ? 0.0 : 1.0 / 4.0; }
 __host__ __device__ inline double chl_rk_c2(int s) { return s == 0 ? 8.0 / 15.0 : (s == 1 ? 5.0 / 12.0 : 3.0 / 4.0); }
 
-// Writes dt and the stage products dt c / 4 that the stage update reads
-// (its fluxes are 4 x), so that no grid point forms them.  Every writer of
-// the step size goes through here.
+// Writes dt and the stage products dt c that the stage update reads, so that
+// no grid point forms them.  Every writer of the step size goes through here.
 __host__ __device__ inline void chl_put_dt(double* scal, double dt) {
   scal[CHL_S_DT] = dt;
   for (int s = 0; s < 3; ++s) {
-    scal[CHL_S_DC + 2 * s] = dt * (0.25 * chl_rk_c1(s));
-    scal[CHL_S_DC + 2 * s + 1] = dt * (0.25 * chl_rk_c2(s));
+    scal[CHL_S_DC + 2 * s] = dt * chl_rk_c1(s);
+    scal[CHL_S_DC + 2 * s + 1] = dt * chl_rk_c2(s);
   }
 }
 
@@ -268,7 +278,10 @@ struct ChlField1 {
   double* dev;
   int n1, n2, n3, nrow, kind;
 };
-struct ChlFields3 { ChlField1 f[3]; };
+struct ChlFields3 {
+  ChlField1 f[3];
+  unsigned* vmax;   // where unpacking folds the largest |U|, |V|, |W| (zeroed before)
+};
 
 struct ChlMap {
   const ChlInst* inst;   // device array of instances
@@ -278,6 +291,7 @@ struct ChlMap {
 };
 
 __device__ __forceinline__ int chl_find(const ChlMap& m, int b, int& local) {
+  if (m.n == 1) { local = b; return 0; }   // no table to read ahead of the kernel's first load
   int lo = 0, hi = m.n - 1;
   while (lo < hi) {                 // last instance with off[idx] <= b
     int mid = (lo + hi + 1) >> 1;
@@ -291,6 +305,15 @@ __device__ __forceinline__ int chl_find(const ChlMap& m, int b, int& local) {
 // unsigned arithmetic (an instance has fewer than 2^31 points, checked at
 // creation): the 64-bit divisions this replaces were long integer sequences
 // ahead of every kernel's first load.
+// Planes (consecutive k) per thread of the flux kernel: 4, halved while the
+// instance would have fewer than 4 x 256 threads per SM (at 256x96x192 one,
+// two, four and eight planes take 211, 184, 172 and 174 us).
+#define CHL_FLUX_THREADS 128
+__host__ __device__ inline int chl_planes(int Nx, int Ny, int Nz) {
+  int m = 4;
+  while (m > 1 && (long)Nx * (Ny + 1) * ((Nz + m - 1) / m) < 256L * CHL_MIN_BLOCKS) m >>= 1;
+  return m;
+}
 struct ChlIdx { int i, j, k; };
 __device__ __forceinline__ ChlIdx chl_split(unsigned t, unsigned Nx, unsigned rows) {
   const unsigned q = t / Nx, k = q / rows;
@@ -305,6 +328,12 @@ __device__ __forceinline__ int wrap(int i, int n) { return i < 0 ? i + n : (i >=
 // slot of the status area that counts k_minabs's finished blocks (the last
 // one forms dt); the counters return to 0 after each use
 #define CHL_CNT_DT 4
+// largest |U|, |V|, |W| of velocity sets 0, 1 and 2 and largest |nu + nu_t|
+// (high words of the doubles; chl_fix.cuh).  Set 0's lie behind the status
+// word, so an upload clears both at once.
+#define CHL_ST_VMAX0 1
+#define CHL_ST_VMAX12 5
+#define CHL_ST_NMAX 11
 
 // The bounds-checked build (-DCHL_BOUNDS_CHECK, build.build(variant="bounds"))
 // records an out-of-range index in the status word and clamps it, so the
@@ -320,13 +349,15 @@ __device__ __forceinline__ void chl_clamp(const ChlInst& I, int& i, int& j, int&
 #endif
 }
 
+// element of a centre-like and of a V-like field (an instance has fewer than
+// 2^31 points, so 32-bit arithmetic)
 __device__ __forceinline__ size_t cidx(const ChlInst& I, int i, int jc, int k) {
   chl_clamp(I, i, jc, k, I.Ny + 1);
-  return (size_t)i + (size_t)I.Nx * ((size_t)jc + (size_t)(I.Ny + 2) * (size_t)k);
+  return (unsigned)i + (unsigned)I.Nx * ((unsigned)jc + (unsigned)(I.Ny + 2) * (unsigned)k);
 }
 __device__ __forceinline__ size_t vidx(const ChlInst& I, int i, int jv, int k) {
   chl_clamp(I, i, jv, k, I.Ny);
-  return (size_t)i + (size_t)I.Nx * ((size_t)jv + (size_t)(I.Ny + 1) * (size_t)k);
+  return (unsigned)i + (unsigned)I.Nx * ((unsigned)jv + (unsigned)(I.Ny + 1) * (unsigned)k);
 }
 
 #define LDG(p) __ldg(p)

@@ -19,7 +19,7 @@
 //    the real-row packing are folded; the mode's column is staged in shared
 //    memory by asynchronous copies when it fits;
 //  * the inverse runs the same way back and the x pass writes the pressure.
-#include "chl_common.cuh"
+#include "chl_fix.cuh"
 
 #include <cooperative_groups.h>
 
@@ -228,6 +228,8 @@ __device__ __forceinline__ double2* fft_smem(double2* a, double2* b, int nrows, 
 // mode 0: div of velocity set s_in (compute_pseudo_pressure_rhs, projection.f90:40-55)
 // mode 1: div of the actual-pressure RHS Fp with the wall rows of Fv set to
 //         the pressure BC planes and the BC source terms of pressure.f90:138-139.
+// mode 2: mode 0 without a velocity correction to follow (the tuner).  Mode 0
+//         clears the set's largest velocities, which k_project forms anew.
 __global__ void __launch_bounds__(256)
 k_div_fftx(ChlMap map, int s_in, int mode, int xmb) {
   chl_pdl_wait();
@@ -244,7 +246,8 @@ k_div_fftx(ChlMap map, int s_in, int mode, int xmb) {
   double* T = reinterpret_cast<double*>(sm + 2 * CR * Nx);   // pass table
   stage_twiddles(T, I.twx, chl_tw_len(Nx));
   const double *U, *V, *W;
-  if (mode == 0) { U = I.U[s_in]; V = I.V[s_in]; W = I.W[s_in]; }
+  if (mode == 0 && lb == 0 && threadIdx.x < 3) chl_vmax(I, s_in)[threadIdx.x] = 0u;
+  if (mode != 1) { U = I.U[s_in]; V = I.V[s_in]; W = I.W[s_in]; }
   else { U = I.Fp[0]; V = I.Fp[1]; W = I.Fp[2]; }
   for (int w = threadIdx.x; w < cr_n * Nx; w += blockDim.x) {
     const int cr = w / Nx, i = w - cr * Nx;
@@ -771,7 +774,8 @@ k_fftx_inv(ChlMap map, int dst, int xmb) {
 }
 
 // ------------------------------------------------------------ velocity correction
-// project_velocity (projection.f90:192-214) + Dirichlet ghost rows.
+// project_velocity (projection.f90:192-214) + Dirichlet ghost rows; folds
+// the set's largest velocities (cleared by k_div_fftx) for its fixed-point copies.
 __global__ void __launch_bounds__(256)
 k_project(ChlMap map, int s) {
   chl_pdl_wait();
@@ -779,22 +783,28 @@ k_project(ChlMap map, int s) {
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
   const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  if (t >= (unsigned)(Nx * Ny * Nz)) return;
-  const ChlIdx ix = chl_split(t, Nx, Ny);
-  const int i = ix.i, jc = 1 + ix.j, k = ix.k;
-  const double* p = I.p;
-  const size_t c = cidx(I, i, jc, k);
-  const double p0 = LDG(p + c);
-  double* U = I.U[s]; double* V = I.V[s]; double* W = I.W[s];
-  const double un = U[c] - (LDG(p + cidx(I, wrap(i + 1, Nx), jc, k)) - p0) * LDG(I.rdxf + i);
-  const double wn = W[c] - (LDG(p + cidx(I, i, jc, wrap(k + 1, Nz))) - p0) * LDG(I.rdzf + k);
-  U[c] = un; W[c] = wn;
-  if (jc <= Ny - 1) {
-    const size_t v = vidx(I, i, jc, k);
-    V[v] = V[v] - (LDG(p + cidx(I, i, jc + 1, k)) - p0) * LDG(I.rdyf + jc);
+  unsigned hi[3] = {0u, 0u, 0u};
+  if (t < (unsigned)(Nx * Ny * Nz)) {
+    const ChlIdx ix = chl_split(t, Nx, Ny);
+    const int i = ix.i, jc = 1 + ix.j, k = ix.k;
+    const double* p = I.p;
+    const size_t c = cidx(I, i, jc, k);
+    const double p0 = LDG(p + c);
+    double* U = I.U[s]; double* V = I.V[s]; double* W = I.W[s];
+    const double un = U[c] - (LDG(p + cidx(I, wrap(i + 1, Nx), jc, k)) - p0) * LDG(I.rdxf + i);
+    const double wn = W[c] - (LDG(p + cidx(I, i, jc, wrap(k + 1, Nz))) - p0) * LDG(I.rdzf + k);
+    U[c] = un; W[c] = wn;
+    hi[0] = chl_abshi(un); hi[2] = chl_abshi(wn);
+    if (jc <= Ny - 1) {
+      const size_t v = vidx(I, i, jc, k);
+      const double vn = V[v] - (LDG(p + cidx(I, i, jc + 1, k)) - p0) * LDG(I.rdyf + jc);
+      V[v] = vn;
+      hi[1] = chl_abshi(vn);
+    }
+    if (jc == 1) { U[cidx(I, i, 0, k)] = chl_neg(un); W[cidx(I, i, 0, k)] = chl_neg(wn); }
+    if (jc == Ny) { U[cidx(I, i, Ny + 1, k)] = chl_neg(un); W[cidx(I, i, Ny + 1, k)] = chl_neg(wn); }
   }
-  if (jc == 1) { U[cidx(I, i, 0, k)] = -un; W[cidx(I, i, 0, k)] = -wn; }
-  if (jc == Ny) { U[cidx(I, i, Ny + 1, k)] = -un; W[cidx(I, i, Ny + 1, k)] = -wn; }
+  chl_block_max(chl_vmax(I, s), hi);
 }
 
 // ------------------------------------------------------------ actual pressure: wall BC planes

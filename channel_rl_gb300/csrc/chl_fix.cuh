@@ -1,0 +1,92 @@
+// 64-bit fixed-point arithmetic on the integer pipe.
+//
+// GB300 issues one warp FP64 instruction per 64-67 clocks and SM
+// sub-partition, whatever it is; in the same time the integer pipe issues
+// 13 64-bit additions, 4 of the products below or 2.7 conversions (measured
+// clocks per warp instruction: 5, 16, 24), and the two pipes run side by
+// side.  Sums and products of quantities whose largest magnitude is known
+// are therefore formed here in 64-bit integers F standing for F 2^e, e the
+// exponent of the quantity's last bit, and only the result goes back to
+// double.  A field is scaled by its own largest magnitude (kept with the
+// velocity set, ChlInst::status), so that |F| < 2^61: eight bits finer than
+// a double's last bit at that magnitude, and exact for every double down to
+// 2^-8 of it.  Sums and differences are exact; a product keeps 60 bits or
+// more of its largest possible value.
+#pragma once
+#include "chl_common.cuh"
+
+typedef long long fx;
+
+// exponent of the last bit for a quantity whose largest |x| has the high
+// word `hi` (bits of the double >> 32, sign cleared), such that |F| < 2^BITS;
+// magnitudes below 2^-958 are scaled as that (they round to zero)
+template <int BITS>
+__device__ __forceinline__ int fx_exp(unsigned hi) {
+  const int E = max((int)(hi >> 20), 64);
+  return E - 1022 - BITS;
+}
+__device__ __forceinline__ bool fx_bad(unsigned hi) { return hi >= 0x7FF00000u; }
+
+// x as F 2^e, rounded toward zero
+__device__ __forceinline__ fx fx_from(double x, int e) {
+  const long long b = __double_as_longlong(x);
+  const int r = e + 1086 - (((int)(b >> 52)) & 0x7FF);
+  unsigned long long f;
+  // shr clamps shift amounts above 63, which give 0 (also for x = 0)
+  asm("shr.u64 %0, %1, %2;" : "=l"(f) : "l"(((unsigned long long)b << 11) | 0x8000000000000000ULL), "r"(r));
+  return b < 0 ? -(fx)f : (fx)f;
+}
+
+// F 2^e as a double, rounded to nearest; results below the normal range give
+// zero, above it infinity
+__device__ __forceinline__ double fx_to(fx f, int e) {
+  const unsigned long long a = f < 0 ? 0ULL - (unsigned long long)f : (unsigned long long)f;
+  const int lz = __clzll((long long)a);
+  unsigned long long n;
+  asm("shl.b64 %0, %1, %2;" : "=l"(n) : "l"(a), "r"(lz));
+  int ef = e + 1085 - lz;
+  const unsigned long long m = (n >> 11) + ((n >> 10) & 1ULL);
+  unsigned long long r = m + ((unsigned long long)(unsigned)ef << 52);
+  if (ef < 0 || a == 0) r = 0;
+  if (ef > 0x7FD && a != 0) r = 0x7FF0000000000000ULL;
+  return __longlong_as_double((long long)(r | ((unsigned long long)f & 0x8000000000000000ULL)));
+}
+
+// (a b) >> 64, low by less than three units, for |a| < 2^62 and |b| < 2^63:
+// the product of the high words plus the cross terms, whose low words enter
+// with 31 bits so that they are signed 32-bit factors.
+__device__ __forceinline__ fx fx_mul(fx a, fx b) {
+  const int ah = (int)(a >> 32), bh = (int)(b >> 32);
+  const int al = (int)((unsigned)a >> 1), bl = (int)((unsigned)b >> 1);
+  const long long t = (long long)ah * bl + (long long)bh * al;
+  return (long long)ah * bh + (t >> 31);
+}
+
+// High words of the largest |U|, |V|, |W| of a velocity set, and of the
+// largest |nu + nu_t|.  Written with the fields by every kernel that leaves a
+// velocity set behind (upload, projection, mass-flow shift) or nu + nu_t.
+__device__ __forceinline__ unsigned* chl_vmax(const ChlInst& I, int set) {
+  return reinterpret_cast<unsigned*>(I.status) + (set == 0 ? CHL_ST_VMAX0 : CHL_ST_VMAX12 + 3 * (set - 1));
+}
+__device__ __forceinline__ unsigned* chl_nmax(const ChlInst& I) {
+  return reinterpret_cast<unsigned*>(I.status) + CHL_ST_NMAX;
+}
+__device__ __forceinline__ unsigned chl_abshi(double x) { return (unsigned)__double2hiint(x) & 0x7FFFFFFFu; }
+
+// Folds each thread's N values into g[0..N) (whole block; every thread
+// calls).  The global word is read first: only blocks that raise it issue an
+// atomic, or the tens of thousands of same-address atomics would take longer
+// than the kernels.
+template <int N>
+__device__ __forceinline__ void chl_block_max(unsigned* g, const unsigned (&v)[N]) {
+  __shared__ unsigned sm[N];
+  if (threadIdx.x < N) sm[threadIdx.x] = 0u;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    const unsigned m = __reduce_max_sync(0xffffffffu, v[q]);
+    if ((threadIdx.x & 31) == 0) atomicMax(sm + q, m);
+  }
+  __syncthreads();
+  if (threadIdx.x < N && sm[threadIdx.x] > __ldcg(g + threadIdx.x)) atomicMax(g + threadIdx.x, sm[threadIdx.x]);
+}

@@ -15,6 +15,7 @@
 
 // ------------------------------------------------------------ launchers (other TUs)
 extern "C" {
+void chl_launch_fix(const ChlMap&, int, int, int, cudaStream_t);
 void chl_launch_flux(const ChlMap&, int, int, cudaStream_t);
 void chl_launch_update(const ChlMap&, int, int, int, int, int, cudaStream_t);
 void chl_launch_edges(const ChlMap&, int, int, int, cudaStream_t);
@@ -71,7 +72,7 @@ namespace {
 constexpr double RK_T[3] = {8.0 / 15.0, 2.0 / 3.0, 1.0};
 
 enum { M_PT, M_EDGE, M_FULL, M_DSMF, M_WALL, M_PLANE, M_FFTX, M_FFTZ, M_TRI, M_MINABS, M_ROWS, M_MLP, M_WALLN,
-       M_ZPLANE, M_ZSOLVE, M_EPAIR, M_FULLZ2, M_FULLX2, NMAP };
+       M_ZPLANE, M_ZSOLVE, M_EPAIR, M_FULLZ2, M_FULLX2, M_FLUX, NMAP };
 constexpr int MLP_NPARAM = 4545;
 
 // Grid constants of one instance (host, FP64), in the device index
@@ -339,11 +340,11 @@ static int upload_consts(chl_handle* h, Inst& I) {
   size_t o_rdyc = A.take(8 * (Ny + 2)), o_rdyf = A.take(8 * (Ny + 2)), o_dyf = A.take(8 * (Ny + 2));
   size_t o_hx2 = A.take(8 * (Nx + 3)), o_hz2 = A.take(8 * (Nz + 3)), o_hy2 = A.take(8 * (Ny + 2));
   size_t o_w0 = A.take(8 * (Ny + 2)), o_w1 = A.take(8 * (Ny + 2)), o_ygc = A.take(8 * (Ny + 2));
-  size_t o_rdxc4 = A.take(8 * (Nx + 3)), o_rdyc4 = A.take(8 * (Ny + 2)), o_rdzc4 = A.take(8 * (Nz + 3));
-  size_t o_rdxc2 = A.take(8 * (Nx + 3)), o_rdyc2 = A.take(8 * (Ny + 2)), o_rdzc2 = A.take(8 * (Nz + 3));
+  size_t o_fxrxc = A.take(8 * (Nx + 3)), o_fxryc = A.take(8 * (Ny + 2)), o_fxrzc = A.take(8 * (Nz + 3));
+  size_t o_fxrxf = A.take(8 * (Nx + 3)), o_fxryf = A.take(8 * (Ny + 2)), o_fxrzf = A.take(8 * (Nz + 3));
+  size_t o_fxw1 = A.take(8 * (Ny + 2)), o_upd = A.take(64);
   size_t o_rdxcs = A.take(8 * (Nx + 3)), o_rdycs = A.take(8 * (Ny + 2)), o_rdzcs = A.take(8 * (Nz + 3));
   size_t o_rdxfs = A.take(8 * (Nx + 3)), o_rdyfs = A.take(8 * (Ny + 2)), o_rdzfs = A.take(8 * (Nz + 3));
-  size_t o_w0u = A.take(8 * (Ny + 2)), o_w1u = A.take(8 * (Ny + 2));
   size_t o_csd = A.take(8 * (Ny + 2)), o_dw = A.take(8 * (Ny + 2));
   size_t o_twx = A.take(8 * (size_t)chl_tw_len(Nx)), o_twz = A.take(8 * (size_t)chl_tw_len(Nz));
   size_t o_ti = A.take(8 * ntri), o_tm = A.take(8 * ntri), o_tc = A.take(8 * ntri);
@@ -353,8 +354,9 @@ static int upload_consts(chl_handle* h, Inst& I) {
   for (int s = 0; s < 3; ++s) o_F1[s] = A.take(8 * (s == 1 ? nv : nc));
   for (int s = 0; s < 3; ++s) o_Fp[s] = A.take(8 * (s == 1 ? nv : nc));
   size_t o_nut = A.take(8 * nc), o_S = A.take(8 * nc);
-  size_t o_G[9];
+  size_t o_G[9], o_X[3];
   for (int m = 0; m < 9; ++m) o_G[m] = A.take(8 * nc);
+  for (int m = 0; m < 3; ++m) o_X[m] = A.take(8 * (m == 1 ? nv : nc));
   size_t o_q[CHL_NQ] = {}, o_r[CHL_NQ] = {};
   if (dsm) for (int m = 0; m < CHL_NQ; ++m) { o_q[m] = A.take(8 * nc); o_r[m] = A.take(8 * nc); }
   size_t o_E[3];
@@ -408,17 +410,19 @@ static int upload_consts(chl_handle* h, Inst& I) {
   D.rdzc = P(o_rdzc) + 1; D.rdzf = P(o_rdzf) + 1; D.dzf = P(o_dzf) + 1;
   D.hx2 = P(o_hx2) + 1; D.hz2 = P(o_hz2) + 1; D.hy2 = P(o_hy2);
   D.rdyc = P(o_rdyc); D.rdyf = P(o_rdyf); D.dyf = P(o_dyf); D.w0x2 = P(o_w0); D.w1x2 = P(o_w1); D.ygc = P(o_ygc);
-  D.rdxc4 = P(o_rdxc4) + 1; D.rdyc4 = P(o_rdyc4); D.rdzc4 = P(o_rdzc4) + 1;
-  D.rdxc2 = P(o_rdxc2) + 1; D.rdyc2 = P(o_rdyc2); D.rdzc2 = P(o_rdzc2) + 1;
+  auto L = [&](size_t o) { return (long long*)(base + o); };
+  D.fxrxc = L(o_fxrxc) + 1; D.fxryc = L(o_fxryc); D.fxrzc = L(o_fxrzc) + 1;
+  D.fxrxf = L(o_fxrxf) + 1; D.fxryf = L(o_fxryf); D.fxrzf = L(o_fxrzf) + 1;
+  D.fxw1 = L(o_fxw1); D.upd = (int*)(base + o_upd);
   D.rdxcs = P(o_rdxcs) + 1; D.rdycs = P(o_rdycs); D.rdzcs = P(o_rdzcs) + 1;
   D.rdxfs = P(o_rdxfs) + 1; D.rdyfs = P(o_rdyfs); D.rdzfs = P(o_rdzfs) + 1;
-  D.w0 = P(o_w0u); D.w1 = P(o_w1u);
   D.smag_csdelta = P(o_csd); D.smag_dwall = P(o_dw);
   D.twx = (const double*)(base + o_twx); D.twz = (const double*)(base + o_twz);
   D.tri_inv = P(o_ti); D.tri_m = P(o_tm); D.tri_c = P(o_tc);
   for (int s = 0; s < 3; ++s) { D.U[s] = P(o_U[s]); D.V[s] = P(o_V[s]); D.W[s] = P(o_W[s]); D.F1[s] = P(o_F1[s]); D.Fp[s] = P(o_Fp[s]); }
   D.nut = P(o_nut); D.S = P(o_S);
-  for (int m = 0; m < 9; ++m) D.G[m] = P(o_G[m]);
+  for (int m = 0; m < 9; ++m) D.G[m] = L(o_G[m]);
+  for (int m = 0; m < 3; ++m) D.X[m] = L(o_X[m]);
   for (int m = 0; m < CHL_NQ; ++m) { D.q[m] = dsm ? P(o_q[m]) : nullptr; D.r[m] = dsm ? P(o_r[m]) : nullptr; }
   for (int m = 0; m < 3; ++m) D.E[m] = P(o_E[m]);
   D.spec = (double2*)(base + o_spec); D.p = P(o_p); D.P = P(o_P);
@@ -440,10 +444,7 @@ static int upload_consts(chl_handle* h, Inst& I) {
   CK(put(o_hx2, c.hx2)); CK(put(o_hz2, c.hz2)); CK(put(o_hy2, c.hy2));
   const std::vector<double> ygc(c.yg.begin() + 1, c.yg.begin() + 1 + c.nyg);
   CK(put(o_ygc, ygc));
-  // the flux kernel keeps its centre and xz-edge fluxes 4 x and its xy and
-  // yz edge fluxes 2 x (chl_rhs.cu): doubled y weights, quadrupled and
-  // doubled centre reciprocals, exact power-of-two scalings (kept in
-  // `scaled` for the rest of this function)
+  // scaled copies (kept in `scaled` for the rest of this function)
   std::vector<std::vector<double>> scaled;
   auto times = [&scaled](const std::vector<double>& v, double f) -> const std::vector<double>& {
     scaled.emplace_back(v);
@@ -452,9 +453,27 @@ static int upload_consts(chl_handle* h, Inst& I) {
   };
   scaled.reserve(16);
   CK(put(o_w0, times(c.w0, 2.0))); CK(put(o_w1, times(c.w1, 2.0)));
-  CK(put(o_w0u, c.w0)); CK(put(o_w1u, c.w1));
-  CK(put(o_rdxc4, times(c.rdxc, 4.0))); CK(put(o_rdyc4, times(c.rdyc, 4.0))); CK(put(o_rdzc4, times(c.rdzc, 4.0)));
-  CK(put(o_rdxc2, times(c.rdxc, 2.0))); CK(put(o_rdyc2, times(c.rdyc, 2.0))); CK(put(o_rdzc2, times(c.rdzc, 2.0)));
+  // reciprocal spacings in fixed point, 63 bits at the table's largest
+  std::vector<std::vector<long long>> fixed;
+  fixed.reserve(8);
+  auto fixtab = [&](size_t o, const std::vector<double>& v, int e) {
+    fixed.emplace_back(v.size(), 0LL);
+    for (size_t q = 0; q < v.size(); ++q) if (std::isfinite(v[q])) fixed.back()[q] = std::llrint(std::ldexp(v[q], -e));
+    return cudaMemcpyAsync(base + o, fixed.back().data(), 8 * v.size(), cudaMemcpyHostToDevice, h->st);
+  };
+  auto fixexp = [](const std::vector<double>& v) {
+    double m = 0.0;
+    for (double x : v) if (std::isfinite(x)) m = std::max(m, x);
+    int k;
+    std::frexp(m, &k);
+    return k - 63;
+  };
+  D.exc = fixexp(c.rdxc); D.exf = fixexp(c.rdxf); D.eyc = fixexp(c.rdyc);
+  D.eyf = fixexp(c.rdyf); D.ezc = fixexp(c.rdzc); D.ezf = fixexp(c.rdzf);
+  CK(fixtab(o_fxrxc, c.rdxc, D.exc)); CK(fixtab(o_fxrxf, c.rdxf, D.exf));
+  CK(fixtab(o_fxryc, c.rdyc, D.eyc)); CK(fixtab(o_fxryf, c.rdyf, D.eyf));
+  CK(fixtab(o_fxrzc, c.rdzc, D.ezc)); CK(fixtab(o_fxrzf, c.rdzf, D.ezf));
+  CK(fixtab(o_fxw1, c.w1, -63));
   const double fs = std::sqrt(4.0 / 216.0);
   CK(put(o_rdxcs, times(c.rdxc, fs))); CK(put(o_rdycs, times(c.rdyc, fs))); CK(put(o_rdzcs, times(c.rdzc, fs)));
   CK(put(o_rdxfs, times(c.rdxf, fs))); CK(put(o_rdyfs, times(c.rdyf, fs))); CK(put(o_rdzfs, times(c.rdzf, fs)));
@@ -550,6 +569,7 @@ static int build_maps(chl_handle* h) {
         case M_FULL: b = cdiv((long)Nx * (Ny + 2) * Nz, h->tb_pt); break;
         case M_FULLZ2: b = cdiv((long)Nx * (Ny + 2) * (Nz / 2), h->tb_pt); break;   // z planes in pairs (Nz even)
         case M_FULLX2: b = cdiv((long)(Nx / 2) * (Ny + 2) * Nz, h->tb_pt); break;   // x points in pairs (Nx even)
+        case M_FLUX: b = cdiv((long)Nx * (Ny + 1) * cdiv(Nz, chl_planes(Nx, Ny, Nz)), CHL_FLUX_THREADS); break;
         case M_DSMF: b = Ny * dsm_npart(Nx, Ny, Nz); break;
         case M_WALL: b = cdiv(2L * Nx * Nz, 256); break;
         case M_PLANE: b = cdiv((long)Nx * Nz, 256); break;
@@ -596,6 +616,7 @@ static int enqueue_sgs(chl_handle* h, int s, bool with_wm, int stage = 0) {
     if (with_wm && h->wall_model == CHL_WM_MLP)
       KL("mlp_wallmodel", chl_launch_mlp(h->map(M_MLP), h->nblk[M_MLP], s, stage, h->d_mlp_status, st));
   };
+  KL("fix", chl_launch_fix(h->map(M_FULL), h->nblk[M_FULL], s, 1, st));
   if (fused) wall_stress();
   if (h->LES_model == CHL_LES_DYNAMIC) {
     KL("edges", chl_launch_edges(h->map(h->epair ? M_EPAIR : M_EDGE), h->nblk[h->epair ? M_EPAIR : M_EDGE], s,
@@ -633,7 +654,6 @@ static int enqueue_sgs(chl_handle* h, int s, bool with_wm, int stage = 0) {
 static int enqueue_projection(chl_handle* h, int s, int mode) {
   cudaStream_t st = h->st;
   const bool correct = mode == 0;
-  if (mode == 2) mode = 0;
   KL("div_fft_x", chl_launch_div_fftx(h->map(M_FFTX), h->nblk[M_FFTX], h->tx, h->smem_x, s, mode, h->x_min_blocks, st));
   if (h->zsolve) {
     KL("z_solve", chl_launch_zsolve(h->map(M_ZSOLVE), h->nblk[M_ZSOLVE], h->zlanes, h->smem_zs, st));
@@ -643,10 +663,17 @@ static int enqueue_projection(chl_handle* h, int s, int mode) {
     else KL("tridiag", chl_launch_tri(h->map(M_TRI), h->nblk[M_TRI], h->smem_t, st));
     KL("fft_z", chl_launch_fftz(h->map(M_FFTZ), h->nblk[M_FFTZ], h->tz, h->smem_z, 1, h->zcw, st));
   }
-  KL("ifft_x", chl_launch_fftx_inv(h->map(M_FFTX), h->nblk[M_FFTX], h->tx, h->smem_x, mode == 0 ? 0 : 1, h->x_min_blocks, st));
+  KL("ifft_x", chl_launch_fftx_inv(h->map(M_FFTX), h->nblk[M_FFTX], h->tx, h->smem_x, mode == 1 ? 1 : 0, h->x_min_blocks, st));
   if (correct) KL("project", chl_launch_project(h->map(M_PT), h->nblk[M_PT], s, st));
   LAUNCHED();
   return CHL_OK;
+}
+
+// The momentum RHS of velocity set 0 into Fp (chl_compute_rhs, the actual
+// pressure, the tuner); the set's fixed-point copies are in place.
+static void enqueue_rhs_only(chl_handle* h) {
+  chl_launch_flux(h->map(M_FLUX), h->nblk[M_FLUX], 0, h->st);
+  chl_launch_update(h->map(M_PT), h->nblk[M_PT], 0, 0, 0, 2, h->st);
 }
 
 // compute_dt: one launch.  k_minabs's last block per instance forms dt
@@ -667,7 +694,7 @@ static int enqueue_rk3(chl_handle* h) {
   for (int s = 0; s < 3; ++s) {
     int rc = enqueue_sgs(h, sin[s], h->wall_model != CHL_WM_NONE, s);
     if (rc) return rc;
-    KL("rhs_flux", chl_launch_flux(h->map(M_EDGE), h->nblk[M_EDGE], sin[s], h->st));
+    KL("rhs_flux", chl_launch_flux(h->map(M_FLUX), h->nblk[M_FLUX], sin[s], h->st));
     KL("rhs_update", chl_launch_update(h->map(M_PT), h->nblk[M_PT], 0, sout[s], s, s == 0 ? 0 : 1, h->st));
     LAUNCHED();
     rc = enqueue_projection(h, sout[s], 0);
@@ -888,6 +915,7 @@ static ChlFields3 fields3(Inst* I, bool out = false) {
   f.f[0] = ChlField1{s, I->dev.U[0], c.nx, c.nyg, c.nzg, c.Ny + 2, 0};
   f.f[1] = ChlField1{s + n, I->dev.V[0], c.nxg, c.ny, c.nzg, c.Ny + 1, 1};
   f.f[2] = ChlField1{s + 2 * n, I->dev.W[0], c.nxg, c.nyg, c.nz, c.Ny + 2, 0};
+  f.vmax = (unsigned*)I->dev.status + CHL_ST_VMAX0;
   return f;
 }
 
@@ -902,13 +930,13 @@ int chl_upload(chl_handle* h, int inst, const double* U, const double* V, const 
     const ChlField1& d = f3.f[q];
     CK(cudaMemcpyAsync(d.fort, src[q], 8 * (size_t)d.n1 * d.n2 * d.n3, cudaMemcpyHostToDevice, h->st));
   }
+  CK(cudaMemsetAsync(I->dev.status, 0, sizeof(int) * (CHL_ST_VMAX0 + 3), h->st));   // status word, set 0's maxima
   chl_launch_unpack3(f3, I->c.Nx, I->c.Nz, h->st);
   LAUNCHED();
   const int Nz = I->c.Nz;
   // Qflow_x_0 of this instance (mass_flow.f90:24-61); the kernel runs per instance
   chl_launch_qflow(h->d_inst + inst, Nz, 0, CHL_S_Q0, h->st);
   LAUNCHED();
-  CK(cudaMemsetAsync(I->dev.status, 0, sizeof(int), h->st));
   I->uploaded = true;
   return finish(h);
 }
@@ -1153,8 +1181,7 @@ int chl_rk3_step(chl_handle* h, int nsteps) {
 static int enqueue_stencils(chl_handle* h) {
   int rc = enqueue_sgs(h, 0, false);
   if (rc) return rc;
-  chl_launch_flux(h->map(M_EDGE), h->nblk[M_EDGE], 0, h->st);
-  chl_launch_update(h->map(M_PT), h->nblk[M_PT], 0, 0, 0, 2, h->st);
+  enqueue_rhs_only(h);
   LAUNCHED();
   return CHL_OK;
 }
@@ -1183,9 +1210,9 @@ static int time_group(chl_handle* h, int group, int reps, cudaEvent_t a, cudaEve
 int chl_autotune(chl_handle* h, int reps, char* report, int report_len) {
   int rc = check_ready(h); if (rc) return rc;
   if (reps < 1) reps = 1;
-  // nu + nu_t, the pseudo-pressure, S (the strain or model nu_t that
-  // chl_compute_wall_model rebuilds nu_t from) and the row coefficients of
-  // every instance, restored at the end
+  // nu + nu_t with its largest magnitude, the pseudo-pressure, S (the strain
+  // or model nu_t that chl_compute_wall_model rebuilds nu_t from) and the row
+  // coefficients of every instance, restored at the end
   std::vector<double*> saved;
   cudaEvent_t ea = nullptr, eb = nullptr;
   auto ncent = [](const Inst& I) { return (size_t)I.c.Nx * (I.c.Ny + 2) * I.c.Nz; };   // centre-field length
@@ -1199,6 +1226,7 @@ int chl_autotune(chl_handle* h, int reps, char* report, int report_len) {
       cudaMemcpyAsync(I.dev.p, saved[q] + n, 8 * n, cudaMemcpyDeviceToDevice, h->st);
       cudaMemcpyAsync(I.dev.S, saved[q] + 2 * n, 8 * n, cudaMemcpyDeviceToDevice, h->st);
       cudaMemcpyAsync(I.dev.coef, saved[q] + 3 * n, 8 * ncoef(I), cudaMemcpyDeviceToDevice, h->st);
+      cudaMemcpyAsync(I.dev.status + CHL_ST_NMAX, saved[q] + 3 * n + ncoef(I), sizeof(int), cudaMemcpyDeviceToDevice, h->st);
     }
     cudaStreamSynchronize(h->st);
     for (double* s : saved) cudaFree(s);
@@ -1209,12 +1237,13 @@ int chl_autotune(chl_handle* h, int reps, char* report, int report_len) {
   for (auto& I : h->in) {
     const size_t n = ncent(I);
     double* s = nullptr;
-    cudaError_t e = cudaMalloc(&s, 8 * (3 * n + ncoef(I)));
+    cudaError_t e = cudaMalloc(&s, 8 * (3 * n + ncoef(I) + 1));
     if (e == cudaSuccess) {
       e = cudaMemcpyAsync(s, I.dev.nut, 8 * n, cudaMemcpyDeviceToDevice, h->st);
       if (e == cudaSuccess) e = cudaMemcpyAsync(s + n, I.dev.p, 8 * n, cudaMemcpyDeviceToDevice, h->st);
       if (e == cudaSuccess) e = cudaMemcpyAsync(s + 2 * n, I.dev.S, 8 * n, cudaMemcpyDeviceToDevice, h->st);
       if (e == cudaSuccess) e = cudaMemcpyAsync(s + 3 * n, I.dev.coef, 8 * ncoef(I), cudaMemcpyDeviceToDevice, h->st);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(s + 3 * n + ncoef(I), I.dev.status + CHL_ST_NMAX, sizeof(int), cudaMemcpyDeviceToDevice, h->st);
       if (e != cudaSuccess) cudaFree(s);
       else saved.push_back(s);
     }
@@ -1342,6 +1371,7 @@ int chl_compute_eddy_viscosity(chl_handle* h) {
 
 int chl_compute_wall_model(chl_handle* h) {
   int rc = check_ready(h); if (rc) return rc;
+  chl_launch_fix(h->map(M_FULL), h->nblk[M_FULL], 0, 1, h->st);   // k_nut forms the largest nu + nu_t anew
   if (h->wall_model >= CHL_WM_EQLOG) chl_launch_eqwm(h->map(M_WALLN), h->nblk[M_WALLN], 0, h->st);
   if (h->wall_model == CHL_WM_MLP) chl_launch_mlp(h->map(M_MLP), h->nblk[M_MLP], 0, 0, h->d_mlp_status, h->st);
   chl_launch_nut(h->map(M_FULL), h->nblk[M_FULL], 0, h->wall_model != CHL_WM_NONE ? 1 : 0, h->st);
@@ -1354,8 +1384,8 @@ int chl_compute_rhs(chl_handle* h, int inst, double* Fu, double* Fv, double* Fw)
   Inst* I = get_inst(h, inst);
   if (!I) return CHL_E_ARG;
   if ((rc = drain_copies(h))) return rc;
-  chl_launch_flux(h->map(M_EDGE), h->nblk[M_EDGE], 0, h->st);
-  chl_launch_update(h->map(M_PT), h->nblk[M_PT], 0, 0, 0, 2, h->st);
+  chl_launch_fix(h->map(M_FULL), h->nblk[M_FULL], 0, 0, h->st);
+  enqueue_rhs_only(h);
   LAUNCHED();
   const Consts& c = I->c;
   const int Nx = c.Nx, Ny = c.Ny, Nz = c.Nz;
@@ -1397,8 +1427,8 @@ int chl_compute_dPx_for_constant_mass_flow(chl_handle* h, int inst, double* dPdx
 int chl_compute_pressure(chl_handle* h) {
   int rc = check_ready(h); if (rc) return rc;
   chl_launch_pbc(h->map(M_WALL), h->nblk[M_WALL], 0, h->st);
-  chl_launch_flux(h->map(M_EDGE), h->nblk[M_EDGE], 0, h->st);
-  chl_launch_update(h->map(M_PT), h->nblk[M_PT], 0, 0, 0, 2, h->st);
+  chl_launch_fix(h->map(M_FULL), h->nblk[M_FULL], 0, 0, h->st);
+  enqueue_rhs_only(h);
   LAUNCHED();
   rc = enqueue_projection(h, 0, 1); if (rc) return rc;
   chl_launch_pghost(h->map(M_PLANE), h->nblk[M_PLANE], h->st);
@@ -1453,10 +1483,10 @@ int chl_set_fields(chl_handle* h, int inst, const double* U, const double* V, co
   }
   CK(cudaEventRecord(I->ev_h2d, h->st_h2d));
   CK(cudaStreamWaitEvent(h->st, I->ev_h2d, 0));
+  CK(cudaMemsetAsync(I->dev.status, 0, sizeof(int) * (CHL_ST_VMAX0 + 3), h->st));   // status word, set 0's maxima
   chl_launch_unpack3(f3, I->c.Nx, I->c.Nz, h->st);
   LAUNCHED();
   CK(cudaEventRecord(I->ev_unpacked, h->st));
-  CK(cudaMemsetAsync(I->dev.status, 0, sizeof(int), h->st));
   return CHL_OK;   // stream-ordered; no synchronisation
 }
 

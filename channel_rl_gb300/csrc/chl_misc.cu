@@ -1,5 +1,5 @@
 // Layout conversion, time step, constant mass flow, reductions.
-#include "chl_common.cuh"
+#include "chl_fix.cuh"
 
 // ------------------------------------------------------------ Fortran <-> device layout
 // Fortran array F(n1,n2,n3) (column-major, full ghosted extents of the
@@ -31,26 +31,40 @@ __global__ void k_pack(double* __restrict__ F, const double* __restrict__ src, i
 // long integer sequence) had held them to a fifth of the HBM bandwidth.
 #define CHL_CONV_ROWS 4
 #define CHL_CONV_LANES 64
+// Unpacking also folds the field's largest magnitude into f3.vmax.
 __global__ void __launch_bounds__(CHL_CONV_ROWS * CHL_CONV_LANES)
 k_unpack3(ChlFields3 f3, int Nx, int Nz) {
   const ChlField1& q = f3.f[blockIdx.y];
   const int nrow = q.nrow;
   const int r = blockIdx.x * CHL_CONV_ROWS + threadIdx.y;      // row (j, k) of the device field
-  if (r >= nrow * Nz) return;
-  const int j = r % nrow, k = r / nrow;
-  double* __restrict__ dst = q.dev + (size_t)Nx * r;
-  const int last = nrow - 1;
-  if (q.kind == 1 && (j == 0 || j == last)) {
-    for (int i = threadIdx.x; i < Nx; i += CHL_CONV_LANES) dst[i] = 0.0;
-    return;
+  unsigned hi = 0u;
+  if (r < nrow * Nz) {
+    const int j = r % nrow, k = r / nrow;
+    double* __restrict__ dst = q.dev + (size_t)Nx * r;
+    const int last = nrow - 1;
+    if (q.kind == 1 && (j == 0 || j == last)) {
+      for (int i = threadIdx.x; i < Nx; i += CHL_CONV_LANES) dst[i] = 0.0;
+    } else {
+      int js = j;
+      bool neg = false;
+      if (q.kind == 0 && j == 0) { js = 1; neg = true; }
+      if (q.kind == 0 && j == last) { js = last - 1; neg = true; }
+      const double* __restrict__ src = q.fort + 1 + (size_t)q.n1 * ((size_t)js + (size_t)q.n2 * (size_t)(k + 1));
+      for (int i = threadIdx.x; i < Nx; i += CHL_CONV_LANES) {
+        const double v = src[i];
+        dst[i] = neg ? chl_neg(v) : v;
+        hi = max(hi, chl_abshi(v));
+      }
+    }
   }
-  int js = j;
-  bool neg = false;
-  if (q.kind == 0 && j == 0) { js = 1; neg = true; }
-  if (q.kind == 0 && j == last) { js = last - 1; neg = true; }
-  const double* __restrict__ src = q.fort + 1 + (size_t)q.n1 * ((size_t)js + (size_t)q.n2 * (size_t)(k + 1));
-  if (neg) { for (int i = threadIdx.x; i < Nx; i += CHL_CONV_LANES) dst[i] = -src[i]; }
-  else { for (int i = threadIdx.x; i < Nx; i += CHL_CONV_LANES) dst[i] = src[i]; }
+  __shared__ unsigned sm;
+  const bool first = threadIdx.x == 0 && threadIdx.y == 0;
+  if (first) sm = 0u;
+  __syncthreads();
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if ((threadIdx.x & 31) == 0) atomicMax(&sm, hi);
+  __syncthreads();
+  if (first && sm > __ldcg(f3.vmax + blockIdx.y)) atomicMax(f3.vmax + blockIdx.y, sm);
 }
 
 __global__ void __launch_bounds__(CHL_CONV_ROWS * CHL_CONV_LANES)
@@ -169,6 +183,11 @@ __device__ void dt_from_minima(const ChlInst& I) {
 #define MINABS_ROWS 16
 __device__ __forceinline__ int minabs_chunks(int Ny) { return (Ny + MINABS_ROWS - 1) / MINABS_ROWS; }
 
+// a minimum goes out only where it lowers the value read before
+__device__ __forceinline__ void lower(unsigned long long* g, unsigned long long m) {
+  if (m < __ldcg(g)) atomicMin(g, m);
+}
+
 __global__ void __launch_bounds__(256)
 k_minabs(ChlMap map, int s) {
   chl_pdl_wait();
@@ -211,9 +230,9 @@ k_minabs(ChlMap map, int s) {
       bv = x < bv ? x : bv;
     }
     if (lane == 0) atomicMin(sv + (jc - j0), bv);
-    if (!fixed_x && ok) { atomicMin(g + i, mu); mu = CHL_BIG_BITS; }
+    if (!fixed_x && ok) { lower(g + i, mu); mu = CHL_BIG_BITS; }
   }
-  if (fixed_x && (int)(threadIdx.x % nxr) < Nx && (int)threadIdx.x < nw) atomicMin(g + threadIdx.x % nxr, mu);
+  if (fixed_x && (int)(threadIdx.x % nxr) < Nx && (int)threadIdx.x < nw) lower(g + threadIdx.x % nxr, mu);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const unsigned long long x = __shfl_xor_sync(0xffffffffu, mw, o);
@@ -225,9 +244,9 @@ k_minabs(ChlMap map, int s) {
   if (threadIdx.x == 0) {
     unsigned long long m = swm[0];
     for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = swm[w] < m ? swm[w] : m;
-    atomicMin(g + Nx + Ny + 1 + k, m);
+    lower(g + Nx + Ny + 1 + k, m);
   }
-  if (threadIdx.x <= j1 - j0) atomicMin(g + Nx + j0 + threadIdx.x, sv[threadIdx.x]);
+  if (threadIdx.x <= j1 - j0) lower(g + Nx + j0 + threadIdx.x, sv[threadIdx.x]);
   // the instance's last block to finish forms dt from the minima and
   // resets them for the next step
   __shared__ int last;
@@ -305,6 +324,7 @@ __global__ void k_massflow(ChlMap map, int s, int force) {
   if (threadIdx.x == 0) {
     const double d = I.scal[CHL_S_Q0] - red[0] / (double)(Nx * Nz);
     I.scal[CHL_S_SHIFT] = d;
+    if (!force) chl_vmax(I, s)[0] = 0u;     // k_shift forms the largest |U| anew
     if (!force) I.scal[CHL_S_DPDX] = 0.0;   // dPdx = 0 after the shift (time_integration.f90:92)
   }
 }
@@ -328,15 +348,20 @@ k_shift(ChlMap map, int s) {
     // step counter of the wall-model exploration noise (shared by the batch)
     if (blockIdx.x == 0 && I.mlp_cfg) atomicAdd(I.mlp_cfg + 4, 1u);
   }
-  if (t >= (unsigned)(Nx * Ny * Nz) || !I.x_mass_cte) return;
-  const ChlIdx p = chl_split(t, Nx, Ny);
-  const int i = p.i, jc = 1 + p.j, k = p.k;
-  double* U = I.U[s];
-  const double d = I.scal[CHL_S_SHIFT];
-  const double un = U[cidx(I, i, jc, k)] + d;
-  U[cidx(I, i, jc, k)] = un;
-  if (jc == 1) U[cidx(I, i, 0, k)] = -un;
-  if (jc == Ny) U[cidx(I, i, Ny + 1, k)] = -un;
+  if (!I.x_mass_cte) return;
+  unsigned hi[1] = {0u};
+  if (t < (unsigned)(Nx * Ny * Nz)) {
+    const ChlIdx p = chl_split(t, Nx, Ny);
+    const int i = p.i, jc = 1 + p.j, k = p.k;
+    double* U = I.U[s];
+    const double d = I.scal[CHL_S_SHIFT];
+    const double un = U[cidx(I, i, jc, k)] + d;
+    U[cidx(I, i, jc, k)] = un;
+    if (jc == 1) U[cidx(I, i, 0, k)] = chl_neg(un);
+    if (jc == Ny) U[cidx(I, i, Ny + 1, k)] = chl_neg(un);
+    hi[0] = chl_abshi(un);
+  }
+  chl_block_max(chl_vmax(I, s), hi);
 }
 
 // time advance t += dt (compute_time_step_RK3 leaves t = to + rk_t(3)*dt)

@@ -19,7 +19,7 @@
 // aborts in the reference) is written from its formula.  The stress wall
 // model is compute_wall_model (wallmodel.f90:23-46); the equilibrium log-law
 // wall stress that feeds it is new.
-#include "chl_common.cuh"
+#include "chl_fix.cuh"
 
 // ---------------------------------------------------------------- edges
 // E12 at (x-face a, y-face jv, z-centre k), E13 at (x-face a, centre row jc,
@@ -585,11 +585,24 @@ k_eqwm(ChlMap map, int s_in) {
 }
 
 // ------------------------------------------------------------ nu_t (+ wall model rows)
+// nu + nu_t of every centre but the interior ones of the Smagorinsky models:
+// no model, AMD and Vreman (S holds nu_t itself) and the ghost rows.  A call,
+// so that its FP64 instructions are not predicated into the common path.
+static __device__ __noinline__ double nut_other(const ChlInst& I, int i, int jc, int k) {
+  if (I.LES_model == 0) return I.nu;
+  if (jc == 0 || jc == I.Ny + 1) {         // ghost rows: the rule of Dirichlet_nu_t
+    const int js = jc == 0 ? 1 : I.Ny;
+    const double sv = I.S[cidx(I, i, js, k)];
+    return I.nu + nut_ghost(I, chl_pos(I.LES_model >= 3 ? sv : I.coef[js] * sv));
+  }
+  return I.nu + chl_pos(I.S[cidx(I, i, jc, k)]);
+}
 // One thread per centre (i, jc, k), jc = 0..Ny+1.  On the wall-model rows
 // (jc = 0, 1 and Ny, Ny+1) nu_t is the mean of the face values at x faces
-// i-1 and i: each thread forms face i and takes face i-1 from the lane to
-// its left when that lane is on the same row (i > 0), so no thread returns
-// before the shuffle.
+// i-1 and i, the same in both rows of a wall: the threads of rows 1 and Ny
+// write both.  Each forms face i and takes face i-1 from the lane to its left
+// when that lane is on the same row (i > 0), so no thread returns before the
+// shuffle.
 __global__ void __launch_bounds__(256)
 k_nut(ChlMap map, int s_in, int use_wm) {
   chl_pdl_wait();
@@ -600,31 +613,31 @@ k_nut(ChlMap map, int s_in, int use_wm) {
   const bool valid = t < (unsigned)(Nx * (Ny + 2) * Nz);
   const ChlIdx p = chl_split(valid ? t : 0u, Nx, Ny + 2);
   const int i = p.i, jc = p.j, k = p.k;
-  const bool wmrow = valid && use_wm && I.wall_model != 0 && (jc <= 1 || jc >= Ny);
-  const int wall = jc <= 1 ? 0 : 1;
+  const bool wm = use_wm && I.wall_model != 0 && (jc <= 1 || jc >= Ny);
+  const bool wmrow = valid && wm && (jc == 1 || jc == Ny);
+  const int wall = jc == 1 ? 0 : 1;
   const double* U = I.U[s_in];
   const double f = wmrow ? wm_face(I, U, i, k, wall) : 0.0;
   const double f_left = __shfl_up_sync(0xffffffffu, f, 1);
-  if (!valid) return;
-  // stored as nu + nu_t: every consumer adds nu (equations.f90:139-155)
-  double* out = I.nut + cidx(I, i, jc, k);
-  if (wmrow) {
-    const double fl = ((threadIdx.x & 31) > 0 && i > 0) ? f_left : wm_face(I, U, wrap(i - 1, Nx), k, wall);
-    *out = I.nu + 0.5 * (fl + f);
-  } else if (I.LES_model == 0) {
-    *out = I.nu;
-  } else if (jc == 0 || jc == Ny + 1) {         // ghost rows: the rule of Dirichlet_nu_t
-    const int js = jc == 0 ? 1 : Ny;
-    const double sv = I.S[cidx(I, i, js, k)];
-    *out = I.nu + nut_ghost(I, chl_pos(I.LES_model >= 3 ? sv : I.coef[js] * sv));
-  } else if (I.LES_model >= 3) {                // AMD and Vreman store nu_t itself in S
-    *out = I.nu + chl_pos(I.S[cidx(I, i, jc, k)]);
-  } else {
-    // nu + max(0, c |S|) as one FMA, nu + c |S|, clipped below at nu by the
-    // bit patterns (both positive; a NaN, for which max gives 0, gives nu)
+  double v = 0.0;
+  if (valid && (!wm || wmrow)) {
+    // stored as nu + nu_t: every consumer adds nu (equations.f90:139-155)
     const double nu = I.nu;
-    *out = chl_atleast(fma(I.coef[jc], I.S[cidx(I, i, jc, k)], nu), nu);
+    if (wmrow) {
+      const double fl = ((threadIdx.x & 31) > 0 && i > 0) ? f_left : wm_face(I, U, wrap(i - 1, Nx), k, wall);
+      v = nu + 0.5 * (fl + f);
+      I.nut[cidx(I, i, wall == 0 ? 0 : Ny + 1, k)] = v;
+    } else if (I.LES_model == 0 || I.LES_model >= 3 || jc == 0 || jc == Ny + 1) {
+      v = nut_other(I, i, jc, k);
+    } else {
+      // nu + max(0, c |S|) as one FMA, nu + c |S|, clipped below at nu by the
+      // bit patterns (both positive; a NaN, for which max gives 0, gives nu)
+      v = chl_atleast(fma(I.coef[jc], I.S[cidx(I, i, jc, k)], nu), nu);
+    }
+    I.nut[cidx(I, i, jc, k)] = v;
   }
+  const unsigned hi[1] = {chl_abshi(v)};
+  chl_block_max(chl_nmax(I), hi);
 }
 
 // ------------------------------------------------------------ launchers

@@ -25,7 +25,7 @@
 // where 2:nx, 1:nx-1 are meant (subgrid.f90:930-931,946-947); they start at
 // the same index, so element-wise they read the intended values, which is
 // what is computed here.
-#include "chl_common.cuh"
+#include "chl_fix.cuh"
 
 namespace {
 
@@ -93,14 +93,15 @@ __device__ __forceinline__ Grad gradients(const ChlInst& I, const double* U, con
 // values at x faces i-1 and i (face i-1 from the lane to the left when that
 // lane is on the same row, i > 0).  Every lane of the warp reaches the
 // shuffle; lanes past the instance's last centre carry valid = false.
-__device__ __forceinline__ void write_nut_rows(const ChlInst& I, const double* U, int i, int jc, int k, double v,
-                                               int use_wm, bool valid) {
+// Returns the high word of the largest magnitude written.
+__device__ __forceinline__ unsigned write_nut_rows(const ChlInst& I, const double* U, int i, int jc, int k, double v,
+                                                   int use_wm, bool valid) {
   const int Ny = I.Ny;
   const bool wmrow = valid && use_wm && I.wall_model != 0 && (jc == 1 || jc == Ny);
   const int wall = jc == 1 ? 0 : 1;
   const double f = wmrow ? wm_face(I, U, i, k, wall) : 0.0;
   const double f_left = __shfl_up_sync(0xffffffffu, f, 1);
-  if (!valid) return;
+  if (!valid) return 0u;
   const double nu = I.nu;
   double* nt = I.nut;
   if (wmrow) {
@@ -108,12 +109,18 @@ __device__ __forceinline__ void write_nut_rows(const ChlInst& I, const double* U
     const double w = 0.5 * (fl + f);
     nt[cidx(I, i, jc, k)] = nu + w;
     nt[cidx(I, i, jc == 1 ? 0 : Ny + 1, k)] = nu + w;
-    return;
+    return chl_abshi(nu + w);
   }
   const double vc = chl_pos(v);
   nt[cidx(I, i, jc, k)] = nu + vc;
-  if (jc == 1) nt[cidx(I, i, 0, k)] = nu + nut_ghost(I, vc);
-  if (jc == Ny) nt[cidx(I, i, Ny + 1, k)] = nu + nut_ghost(I, vc);
+  unsigned hi = chl_abshi(nu + vc);
+  if (jc == 1 || jc == Ny) {
+    const double g = nu + nut_ghost(I, vc);
+    if (jc == 1) nt[cidx(I, i, 0, k)] = g;
+    if (jc == Ny) nt[cidx(I, i, Ny + 1, k)] = g;
+    hi = max(hi, chl_abshi(g));
+  }
+  return hi;
 }
 
 }  // namespace
@@ -157,7 +164,8 @@ k_amd(ChlMap map, int s_in, int use_wm) {
   N = fma(a12, t12, N); N = fma(a13, t13, N); N = fma(a23, t23, N);
   const double v = (-0.3 * N) / D;
   if (valid) I.S[cidx(I, i, jc, k)] = v;
-  write_nut_rows(I, I.U[s_in], i, jc, k, v, use_wm, valid);
+  const unsigned hi[1] = {write_nut_rows(I, I.U[s_in], i, jc, k, v, use_wm, valid)};
+  chl_block_max(chl_nmax(I), hi);
 }
 
 __global__ void __launch_bounds__(256)
@@ -193,7 +201,8 @@ k_vreman(ChlMap map, int s_in, int use_wm) {
   Ab = fma(0.0625, Ao, Ab);
   const double v = 2.5 * (0.1 * 0.1) * chl_sqrt(Bb / Ab);
   if (valid) I.S[cidx(I, i, jc, k)] = v;
-  write_nut_rows(I, I.U[s_in], i, jc, k, v, use_wm, valid);
+  const unsigned hi[1] = {write_nut_rows(I, I.U[s_in], i, jc, k, v, use_wm, valid)};
+  chl_block_max(chl_nmax(I), hi);
 }
 
 extern "C" {
