@@ -135,10 +135,13 @@ struct ChlInst {
   long long *G[9];                // momentum face fluxes in fixed point (chl_rhs.cu)
   long long *X[3];                // U, V, W of the set being worked on, in fixed point (k_fix)
   // reciprocal spacings and the y-face weight in fixed point: entry r stands
-  // for r 2^e, one exponent per table, r < 2^63 (chl_fix.cuh)
+  // for r 2^e, r < 2^63, one exponent for a table along x or z and one per
+  // row along y; the weight's is -63 (chl_fix.cuh)
   const long long *fxrxc, *fxrxf, *fxryc, *fxryf, *fxrzc, *fxrzf, *fxw1;
-  int exc, exf, eyc, eyf, ezc, ezf;
-  int *upd;                       // shifts and exponents of the stage update (chl_rhs.cu: UPD_*)
+  const int *eyc, *eyf;
+  int exc, exf, ezc, ezf;
+  int4 *upd;                      // per row, from the flux kernel to the update: exponents (chl_rhs.cu)
+  unsigned *nmax;                 // largest |nu + nu_t| of every centre row (chl_fix.cuh)
   double *q[CHL_NQ], *r[CHL_NQ];  // DSM filter ping-pong
   double *E[3];                   // edge fields (S12, S13, S23 numerators)
   double2 *spec;                  // [Ny+2][Nz][Nxh] spectra (rows 1..Ny used)
@@ -328,12 +331,11 @@ __device__ __forceinline__ int wrap(int i, int n) { return i < 0 ? i + n : (i >=
 // slot of the status area that counts k_minabs's finished blocks (the last
 // one forms dt); the counters return to 0 after each use
 #define CHL_CNT_DT 4
-// largest |U|, |V|, |W| of velocity sets 0, 1 and 2 and largest |nu + nu_t|
-// (high words of the doubles; chl_fix.cuh).  Set 0's lie behind the status
-// word, so an upload clears both at once.
+// largest |U|, |V|, |W| of velocity sets 0, 1 and 2 (high words of the
+// doubles; chl_fix.cuh).  Set 0's lie behind the status word, so an upload
+// clears both at once.
 #define CHL_ST_VMAX0 1
 #define CHL_ST_VMAX12 5
-#define CHL_ST_NMAX 11
 
 // The bounds-checked build (-DCHL_BOUNDS_CHECK, build.build(variant="bounds"))
 // records an out-of-range index in the status word and clamps it, so the

@@ -52,7 +52,8 @@ __device__ __forceinline__ double fx_to(fx f, int e) {
   return __longlong_as_double((long long)(r | ((unsigned long long)f & 0x8000000000000000ULL)));
 }
 
-// (a b) >> 64, low by less than three units, for |a| < 2^62 and |b| < 2^63:
+// (a b) >> 64, low by less than three units, for |a| < 2^62 and |b| < 2^63 (or
+// |a| < 2^63 and 0 <= b < 2^63):
 // the product of the high words plus the cross terms, whose low words enter
 // with 31 bits so that they are signed 32-bit factors.
 __device__ __forceinline__ fx fx_mul(fx a, fx b) {
@@ -62,14 +63,22 @@ __device__ __forceinline__ fx fx_mul(fx a, fx b) {
   return (long long)ah * bh + (t >> 31);
 }
 
+// (a b) >> S for 34 <= S <= 64, |a b| < 2^(62+S): keeps 64 - S more bits of a
+// product whose factors leave room for them.
+template <int S>
+__device__ __forceinline__ fx fx_mul_shr(fx a, fx b) {
+  const int ah = (int)(a >> 32), bh = (int)(b >> 32);
+  const int al = (int)((unsigned)a >> 1), bl = (int)((unsigned)b >> 1);
+  const long long t = (long long)ah * bl + (long long)bh * al;
+  return (fx)((unsigned long long)((long long)ah * bh) << (64 - S)) + (t >> (S - 33));
+}
+
 // High words of the largest |U|, |V|, |W| of a velocity set, and of the
-// largest |nu + nu_t|.  Written with the fields by every kernel that leaves a
-// velocity set behind (upload, projection, mass-flow shift) or nu + nu_t.
+// largest |nu + nu_t| of every centre row.  Written with the fields by every
+// kernel that leaves a velocity set behind (upload, projection, mass-flow
+// shift) or nu + nu_t.
 __device__ __forceinline__ unsigned* chl_vmax(const ChlInst& I, int set) {
   return reinterpret_cast<unsigned*>(I.status) + (set == 0 ? CHL_ST_VMAX0 : CHL_ST_VMAX12 + 3 * (set - 1));
-}
-__device__ __forceinline__ unsigned* chl_nmax(const ChlInst& I) {
-  return reinterpret_cast<unsigned*>(I.status) + CHL_ST_NMAX;
 }
 __device__ __forceinline__ unsigned chl_abshi(double x) { return (unsigned)__double2hiint(x) & 0x7FFFFFFFu; }
 
@@ -89,4 +98,29 @@ __device__ __forceinline__ void chl_block_max(unsigned* g, const unsigned (&v)[N
   }
   __syncthreads();
   if (threadIdx.x < N && sm[threadIdx.x] > __ldcg(g + threadIdx.x)) atomicMax(g + threadIdx.x, sm[threadIdx.x]);
+}
+
+// Folds each thread's v into g[off + j], j = q mod rows the row of its x-line
+// q = k rows + j (whole block, at most 256 threads; x-lines are numbered
+// upwards through the block and hold four points or more).
+#define CHL_BLOCK_LINES 68
+__device__ __forceinline__ void chl_line_max(unsigned* g, unsigned q, int rows, int off, unsigned v) {
+  __shared__ unsigned sm[CHL_BLOCK_LINES];
+  __shared__ unsigned q0;
+  if (threadIdx.x < CHL_BLOCK_LINES) sm[threadIdx.x] = 0u;
+  for (unsigned l = threadIdx.x + blockDim.x; l < CHL_BLOCK_LINES; l += blockDim.x) sm[l] = 0u;
+  if (threadIdx.x == 0) q0 = q;
+  __syncthreads();
+  const unsigned l = min(q - q0, (unsigned)CHL_BLOCK_LINES - 1u);
+  if (__all_sync(0xffffffffu, l == __shfl_sync(0xffffffffu, l, 0))) {
+    v = __reduce_max_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0) atomicMax(sm + l, v);
+  } else {
+    atomicMax(sm + l, v);
+  }
+  __syncthreads();
+  for (unsigned w = threadIdx.x; w < CHL_BLOCK_LINES; w += blockDim.x) {
+    unsigned* d = g + off + (q0 + w) % (unsigned)rows;
+    if (sm[w] && sm[w] > __ldcg(d)) atomicMax(d, sm[w]);
+  }
 }

@@ -342,7 +342,8 @@ static int upload_consts(chl_handle* h, Inst& I) {
   size_t o_w0 = A.take(8 * (Ny + 2)), o_w1 = A.take(8 * (Ny + 2)), o_ygc = A.take(8 * (Ny + 2));
   size_t o_fxrxc = A.take(8 * (Nx + 3)), o_fxryc = A.take(8 * (Ny + 2)), o_fxrzc = A.take(8 * (Nz + 3));
   size_t o_fxrxf = A.take(8 * (Nx + 3)), o_fxryf = A.take(8 * (Ny + 2)), o_fxrzf = A.take(8 * (Nz + 3));
-  size_t o_fxw1 = A.take(8 * (Ny + 2)), o_upd = A.take(64);
+  size_t o_fxw1 = A.take(8 * (Ny + 2)), o_upd = A.take(16 * (Ny + 2));
+  size_t o_eyc = A.take(4 * (Ny + 2)), o_eyf = A.take(4 * (Ny + 2)), o_nmax = A.take(4 * (Ny + 2));
   size_t o_rdxcs = A.take(8 * (Nx + 3)), o_rdycs = A.take(8 * (Ny + 2)), o_rdzcs = A.take(8 * (Nz + 3));
   size_t o_rdxfs = A.take(8 * (Nx + 3)), o_rdyfs = A.take(8 * (Ny + 2)), o_rdzfs = A.take(8 * (Nz + 3));
   size_t o_csd = A.take(8 * (Ny + 2)), o_dw = A.take(8 * (Ny + 2));
@@ -413,7 +414,8 @@ static int upload_consts(chl_handle* h, Inst& I) {
   auto L = [&](size_t o) { return (long long*)(base + o); };
   D.fxrxc = L(o_fxrxc) + 1; D.fxryc = L(o_fxryc); D.fxrzc = L(o_fxrzc) + 1;
   D.fxrxf = L(o_fxrxf) + 1; D.fxryf = L(o_fxryf); D.fxrzf = L(o_fxrzf) + 1;
-  D.fxw1 = L(o_fxw1); D.upd = (int*)(base + o_upd);
+  D.fxw1 = L(o_fxw1); D.upd = (int4*)(base + o_upd);
+  D.eyc = (const int*)(base + o_eyc); D.eyf = (const int*)(base + o_eyf); D.nmax = (unsigned*)(base + o_nmax);
   D.rdxcs = P(o_rdxcs) + 1; D.rdycs = P(o_rdycs); D.rdzcs = P(o_rdzcs) + 1;
   D.rdxfs = P(o_rdxfs) + 1; D.rdyfs = P(o_rdyfs); D.rdzfs = P(o_rdzfs) + 1;
   D.smag_csdelta = P(o_csd); D.smag_dwall = P(o_dw);
@@ -453,27 +455,34 @@ static int upload_consts(chl_handle* h, Inst& I) {
   };
   scaled.reserve(16);
   CK(put(o_w0, times(c.w0, 2.0))); CK(put(o_w1, times(c.w1, 2.0)));
-  // reciprocal spacings in fixed point, 63 bits at the table's largest
+  // reciprocal spacings in fixed point, 63 bits: one exponent per table along
+  // x and z (uniform), one per row along y
   std::vector<std::vector<long long>> fixed;
-  fixed.reserve(8);
-  auto fixtab = [&](size_t o, const std::vector<double>& v, int e) {
+  std::vector<std::vector<int>> fixede;
+  fixed.reserve(8); fixede.reserve(2);
+  auto exponent = [](double m) { int k = 0; std::frexp(m, &k); return k - 63; };   // m 2^-e < 2^63
+  auto fixtab = [&](size_t o, const std::vector<double>& v, const std::vector<int>& e) {
     fixed.emplace_back(v.size(), 0LL);
-    for (size_t q = 0; q < v.size(); ++q) if (std::isfinite(v[q])) fixed.back()[q] = std::llrint(std::ldexp(v[q], -e));
+    for (size_t q = 0; q < v.size(); ++q)
+      if (std::isfinite(v[q])) fixed.back()[q] = std::llrint(std::ldexp(v[q], -e[e.size() == 1 ? 0 : q]));
     return cudaMemcpyAsync(base + o, fixed.back().data(), 8 * v.size(), cudaMemcpyHostToDevice, h->st);
   };
-  auto fixexp = [](const std::vector<double>& v) {
+  auto uniform = [&](size_t o, const std::vector<double>& v, int& e) {
     double m = 0.0;
     for (double x : v) if (std::isfinite(x)) m = std::max(m, x);
-    int k;
-    std::frexp(m, &k);
-    return k - 63;
+    e = exponent(m);
+    return fixtab(o, v, {e});
   };
-  D.exc = fixexp(c.rdxc); D.exf = fixexp(c.rdxf); D.eyc = fixexp(c.rdyc);
-  D.eyf = fixexp(c.rdyf); D.ezc = fixexp(c.rdzc); D.ezf = fixexp(c.rdzf);
-  CK(fixtab(o_fxrxc, c.rdxc, D.exc)); CK(fixtab(o_fxrxf, c.rdxf, D.exf));
-  CK(fixtab(o_fxryc, c.rdyc, D.eyc)); CK(fixtab(o_fxryf, c.rdyf, D.eyf));
-  CK(fixtab(o_fxrzc, c.rdzc, D.ezc)); CK(fixtab(o_fxrzf, c.rdzf, D.ezf));
-  CK(fixtab(o_fxw1, c.w1, -63));
+  auto perrow = [&](size_t o, size_t oe, const std::vector<double>& v) {
+    fixede.emplace_back(v.size(), -4096);   // undefined entries: below every other exponent
+    for (size_t q = 0; q < v.size(); ++q) if (std::isfinite(v[q])) fixede.back()[q] = exponent(v[q]);
+    cudaError_t e = cudaMemcpyAsync(base + oe, fixede.back().data(), 4 * v.size(), cudaMemcpyHostToDevice, h->st);
+    return e == cudaSuccess ? fixtab(o, v, fixede.back()) : e;
+  };
+  CK(uniform(o_fxrxc, c.rdxc, D.exc)); CK(uniform(o_fxrxf, c.rdxf, D.exf));
+  CK(uniform(o_fxrzc, c.rdzc, D.ezc)); CK(uniform(o_fxrzf, c.rdzf, D.ezf));
+  CK(perrow(o_fxryc, o_eyc, c.rdyc)); CK(perrow(o_fxryf, o_eyf, c.rdyf));
+  CK(fixtab(o_fxw1, c.w1, {-63}));
   const double fs = std::sqrt(4.0 / 216.0);
   CK(put(o_rdxcs, times(c.rdxc, fs))); CK(put(o_rdycs, times(c.rdyc, fs))); CK(put(o_rdzcs, times(c.rdzc, fs)));
   CK(put(o_rdxfs, times(c.rdxf, fs))); CK(put(o_rdyfs, times(c.rdyf, fs))); CK(put(o_rdzfs, times(c.rdzf, fs)));
@@ -1210,7 +1219,7 @@ static int time_group(chl_handle* h, int group, int reps, cudaEvent_t a, cudaEve
 int chl_autotune(chl_handle* h, int reps, char* report, int report_len) {
   int rc = check_ready(h); if (rc) return rc;
   if (reps < 1) reps = 1;
-  // nu + nu_t with its largest magnitude, the pseudo-pressure, S (the strain
+  // nu + nu_t with its rows' largest magnitudes, the pseudo-pressure, S (the strain
   // or model nu_t that chl_compute_wall_model rebuilds nu_t from) and the row
   // coefficients of every instance, restored at the end
   std::vector<double*> saved;
@@ -1226,7 +1235,7 @@ int chl_autotune(chl_handle* h, int reps, char* report, int report_len) {
       cudaMemcpyAsync(I.dev.p, saved[q] + n, 8 * n, cudaMemcpyDeviceToDevice, h->st);
       cudaMemcpyAsync(I.dev.S, saved[q] + 2 * n, 8 * n, cudaMemcpyDeviceToDevice, h->st);
       cudaMemcpyAsync(I.dev.coef, saved[q] + 3 * n, 8 * ncoef(I), cudaMemcpyDeviceToDevice, h->st);
-      cudaMemcpyAsync(I.dev.status + CHL_ST_NMAX, saved[q] + 3 * n + ncoef(I), sizeof(int), cudaMemcpyDeviceToDevice, h->st);
+      cudaMemcpyAsync(I.dev.nmax, saved[q] + 3 * n + ncoef(I), sizeof(int) * ncoef(I), cudaMemcpyDeviceToDevice, h->st);
     }
     cudaStreamSynchronize(h->st);
     for (double* s : saved) cudaFree(s);
@@ -1237,13 +1246,13 @@ int chl_autotune(chl_handle* h, int reps, char* report, int report_len) {
   for (auto& I : h->in) {
     const size_t n = ncent(I);
     double* s = nullptr;
-    cudaError_t e = cudaMalloc(&s, 8 * (3 * n + ncoef(I) + 1));
+    cudaError_t e = cudaMalloc(&s, 8 * (3 * n + 2 * ncoef(I)));
     if (e == cudaSuccess) {
       e = cudaMemcpyAsync(s, I.dev.nut, 8 * n, cudaMemcpyDeviceToDevice, h->st);
       if (e == cudaSuccess) e = cudaMemcpyAsync(s + n, I.dev.p, 8 * n, cudaMemcpyDeviceToDevice, h->st);
       if (e == cudaSuccess) e = cudaMemcpyAsync(s + 2 * n, I.dev.S, 8 * n, cudaMemcpyDeviceToDevice, h->st);
       if (e == cudaSuccess) e = cudaMemcpyAsync(s + 3 * n, I.dev.coef, 8 * ncoef(I), cudaMemcpyDeviceToDevice, h->st);
-      if (e == cudaSuccess) e = cudaMemcpyAsync(s + 3 * n + ncoef(I), I.dev.status + CHL_ST_NMAX, sizeof(int), cudaMemcpyDeviceToDevice, h->st);
+      if (e == cudaSuccess) e = cudaMemcpyAsync(s + 3 * n + ncoef(I), I.dev.nmax, sizeof(int) * ncoef(I), cudaMemcpyDeviceToDevice, h->st);
       if (e != cudaSuccess) cudaFree(s);
       else saved.push_back(s);
     }

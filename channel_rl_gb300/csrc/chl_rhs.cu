@@ -32,61 +32,48 @@
 // V-like (rows 0..Ny): 5 GUy, 6 GVx, 7 GVz, 8 GWy
 enum { G_UX = 0, G_VY, G_WZ, G_UZ, G_WX, G_UY, G_VX, G_VZ, G_WY };
 
-// Exponents of a launch, from the largest |U|, |V|, |W|, |nu + nu_t| of its
-// input.  Flux m = viscous - advective part: the advective product has last
-// bit 2^A, the viscous one 2^B, the stored flux 2^G, one above the larger,
-// so that |flux| < 2^60.
-struct FluxExp { int A, B, G; };
-__device__ __forceinline__ FluxExp flux_exp(const ChlInst& I, int sin, int m) {
+// Exponents of the fluxes of row j (y-face j and centre row j), from the
+// largest |U|, |V|, |W| of the launch's input and the largest |nu + nu_t| of
+// the row and the one above.  Flux m = viscous - advective part: the
+// advective product has last bit 2^adv[m], the viscous one 2^vis[m]; the
+// fluxes of one momentum component are stored with last bit 2^G, one above
+// the largest, so that |flux| < 2^62.  Rows have their own exponents because
+// the y spacing and nu + nu_t differ by orders of magnitude between the wall
+// and the core.
+__device__ constexpr int FLUX_A[9] = {0, 1, 2, 0, 2, 0, 1, 1, 2};   // momentum component
+__device__ constexpr int FLUX_B[9] = {0, 1, 2, 2, 0, 1, 0, 2, 1};   // direction
+struct RowExp { int adv[9], vis[9], G[3], n; bool bad; };
+__device__ __forceinline__ RowExp row_exp(const ChlInst& I, int sin, int j) {
   const unsigned* vm = chl_vmax(I, sin);
-  const int a = m == G_UX || m == G_UZ || m == G_UY ? 0 : (m == G_VY || m == G_VX || m == G_VZ ? 1 : 2);
-  const int b = m == G_UX || m == G_VX || m == G_WX ? 0 : (m == G_UY || m == G_VY || m == G_WY ? 1 : 2);
-  const int ea = fx_exp<61>(vm[a]), eb = fx_exp<61>(vm[b]), en = fx_exp<60>(*chl_nmax(I));
-  const int er = m == G_UX ? I.exc : m == G_VY ? I.eyc : m == G_WZ ? I.ezc
-               : b == 0 ? I.exf : b == 1 ? I.eyf : I.ezf;
-  FluxExp q;
-  // factors of the averages: one half in the products on y-face edges, a
-  // quarter in the others; viscosity 1, 4 and 2 x at centres, xz and y-face edges
-  q.A = ea + eb + (m >= G_UY ? 63 : 62);
-  q.B = en + ea + er + (m <= G_WZ ? 128 : m <= G_WX ? 126 : 127);
-  q.G = max(q.A, q.B) + 1;
+  const unsigned nm = max(I.nmax[j], I.nmax[j + 1]);
+  const int ev[3] = {fx_exp<61>(vm[0]), fx_exp<61>(vm[1]), fx_exp<61>(vm[2])};
+  const int ef[3] = {I.exf, I.eyf[j], I.ezf}, ec[3] = {I.exc, I.eyc[j], I.ezc};
+  RowExp q;
+  q.n = fx_exp<60>(nm);
+  q.G[0] = q.G[1] = q.G[2] = -100000;
+#pragma unroll
+  for (int m = 0; m < 9; ++m) {
+    const int a = FLUX_A[m], b = FLUX_B[m];
+    // factors of the averages: one half in the products on y-face edges, a
+    // quarter in the others; viscosity 1, 4 and 2 x at centres, xz and y-face edges
+    q.adv[m] = ev[a] + ev[b] + (m >= G_UY ? 61 : 60);
+    q.vis[m] = q.n + ev[a] + (m <= G_WZ ? ec[b] + 125 : m <= G_WX ? ef[b] + 123 : ef[b] + 124);
+    q.G[a] = max(q.G[a], max(q.adv[m], q.vis[m]) + 1);
+  }
+  q.bad = fx_bad(vm[0]) || fx_bad(vm[1]) || fx_bad(vm[2]) || fx_bad(nm);
   return q;
 }
 
-// Table of the stage update, written by k_flux's first block of the instance
-// for k_rhs_update (so that none of its blocks waits for it): alignment
-// shifts of the nine terms, the three exponents of F, and whether an input
-// was not finite (F is then NaN, as its products would be).
-enum { UPD_SHIFT = 0, UPD_EXP = 9, UPD_BAD = 12, UPD_N = 13 };
-// Component c of F sums three flux differences times a reciprocal spacing,
-// term q from flux field UPD_FLUX[c][q]; the products are aligned to 2^eF.
-__device__ constexpr int UPD_FLUX[3][3] = {{G_UX, G_UY, G_UZ}, {G_VX, G_VY, G_VZ}, {G_WX, G_WY, G_WZ}};
-__device__ __forceinline__ void write_upd(const ChlInst& I, int sin, int c) {   // c = 0..3
-  if (c == 3) {
-    const unsigned* vm = chl_vmax(I, sin);
-    I.upd[UPD_BAD] = fx_bad(vm[0]) || fx_bad(vm[1]) || fx_bad(vm[2]) || fx_bad(*chl_nmax(I));
-    return;
-  }
-  int e[3];
-  for (int q = 0; q < 3; ++q) {
-    const int er = q == 0 ? (c == 0 ? I.exf : I.exc) : q == 1 ? (c == 1 ? I.eyf : I.eyc) : (c == 2 ? I.ezf : I.ezc);
-    e[q] = flux_exp(I, sin, UPD_FLUX[c][q]).G + er + 64;
-  }
-  const int eF = max(max(e[0], e[1]), e[2]) + 2;
-  for (int q = 0; q < 3; ++q) I.upd[UPD_SHIFT + 3 * c + q] = min(63, eF - e[q]);
-  I.upd[UPD_EXP + c] = eF;
-}
-
 // Fixed-point copies of the velocity set that a stage works on (rows as
-// stored, ghosts included); reset_n clears the largest |nu + nu_t| ahead of
-// the kernels that form it.  Moves 48 bytes per point: HBM-bound.
+// stored, ghosts included); reset_n clears the rows' largest |nu + nu_t|
+// ahead of the kernels that form them.  Moves 48 bytes per point: HBM-bound.
 __global__ void __launch_bounds__(256)
 k_fix(ChlMap map, int s, int reset_n) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  if (reset_n && t == 0) *chl_nmax(I) = 0u;
+  if (reset_n && t < (unsigned)(I.Ny + 2)) I.nmax[t] = 0u;
   const unsigned* vm = chl_vmax(I, s);
   const unsigned nc = (unsigned)(I.Nx * (I.Ny + 2) * I.Nz), nv = (unsigned)(I.Nx * (I.Ny + 1) * I.Nz);
   if (t < nc) {
@@ -103,19 +90,9 @@ k_fix(ChlMap map, int s, int reset_n) {
 __global__ void __launch_bounds__(CHL_FLUX_THREADS, 6)
 k_flux(ChlMap map, int sin) {
   chl_pdl_wait();
-  __shared__ int sh[20];      // right shifts of the advective (0..8) and viscous (9..17) parts, exponent of nu
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
   const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
-  if (threadIdx.x < 18) {
-    const int m = threadIdx.x % 9;
-    const FluxExp q = flux_exp(I, sin, m);
-    sh[threadIdx.x] = min(63, q.G - (threadIdx.x < 9 ? q.A : q.B));
-  } else if (threadIdx.x == 18) {
-    sh[18] = fx_exp<60>(*chl_nmax(I));
-  } else if (lb == 0 && threadIdx.x >= 32 && threadIdx.x < 36) {
-    write_upd(I, sin, threadIdx.x - 32);
-  }
   const int M = chl_planes(Nx, Ny, Nz);
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
   const ChlIdx p = chl_split(t, Nx, Ny + 1);
@@ -137,13 +114,24 @@ k_flux(ChlMap map, int sin) {
     w_m = LDG(W + cidx(I, i, j, k0 == 0 ? Nz - 1 : k0 - 1));
     dn_a = LDG(nt + cidx(I, i, j, k0)); dn_b = LDG(nt + cidx(I, i, jp, k0)); dn_p = LDG(nt + cidx(I, ip, j, k0));
   }
-  __syncthreads();
   if (!valid) return;
-  const int en = sh[18];
+  int sa[9], sv_[9];          // right shifts of the advective and viscous parts
+  int en;
+  {
+    const RowExp q = row_exp(I, sin, j);
+    en = q.n;
+#pragma unroll
+    for (int m = 0; m < 9; ++m) {
+      sa[m] = min(63, q.G[FLUX_A[m]] - q.adv[m]);
+      sv_[m] = min(63, q.G[FLUX_A[m]] - q.vis[m]);
+    }
+    if (i == 0 && k0 == 0) I.upd[j] = make_int4(q.G[0], q.G[1], q.G[2], q.bad);   // for k_rhs_update
+  }
   fx n_a = fx_from(dn_a, en), n_b = fx_from(dn_b, en), n_p = fx_from(dn_p, en);
-#define ADV(m, f) ((f) >> sh[m])
-#define VIS(m, f) ((f) >> sh[9 + (m)])
-#define PUT(m, e, adv, vis) I.G[m][e] = VIS(m, vis) - ADV(m, adv)
+#define MUL fx_mul
+#define ADV fx_mul_shr<62>
+#define VIS fx_mul_shr<61>
+#define PUT(m, e, adv, vis) I.G[m][e] = ((vis) >> sv_[m]) - ((adv) >> sa[m])
   for (int k = k0; k < k1; ++k) {
     const int kp = k + 1 == Nz ? 0 : k + 1;
     const size_t c = cidx(I, i, j, k), e = vidx(I, i, j, k);
@@ -156,37 +144,38 @@ k_flux(ChlMap map, int sin) {
     const fx nx_a = n_a + n_p;             // x pair of row j: the xy and xz edges share it
     {  // yz edge (x-centre i, y-face j, z-face k): vw, nu -> GVz, GWy
       const fx dw = w_b - w_a;
-      const fx vw = fx_mul(w_a + 2 * fx_mul(dw, w1), v_0 + v_z);                      // 2 v w
+      const fx vw = ADV(w_a + 2 * MUL(dw, w1), v_0 + v_z);                            // 2 v w
       const fx na = n_a + n_az;
-      const fx nyz = na + 2 * fx_mul(n_b + n_bz - na, w1);                            // 2 nu
-      PUT(G_VZ, e, vw, fx_mul(nyz, fx_mul(v_z - v_0, rzf)));
-      PUT(G_WY, e, vw, fx_mul(nyz, fx_mul(dw, ryf)));
+      const fx nyz = na + 2 * MUL(n_b + n_bz - na, w1);                               // 2 nu
+      PUT(G_VZ, e, vw, VIS(nyz, MUL(v_z - v_0, rzf)));
+      PUT(G_WY, e, vw, VIS(nyz, MUL(dw, ryf)));
     }
     {  // xy edge (x-face i, y-face j, z-centre k): uv, nu -> GUy, GVx
       const fx du = u_b - u_a;
-      const fx uv = fx_mul(u_a + 2 * fx_mul(du, w1), v_0 + v_p);                      // 2 u v
-      const fx nxy = nx_a + 2 * fx_mul(n_b + n_bp - nx_a, w1);                        // 2 nu
-      PUT(G_UY, e, uv, fx_mul(nxy, fx_mul(du, ryf)));
-      PUT(G_VX, e, uv, fx_mul(nxy, fx_mul(v_p - v_0, rxf)));
+      const fx uv = ADV(u_a + 2 * MUL(du, w1), v_0 + v_p);                            // 2 u v
+      const fx nxy = nx_a + 2 * MUL(n_b + n_bp - nx_a, w1);                           // 2 nu
+      PUT(G_UY, e, uv, VIS(nxy, MUL(du, ryf)));
+      PUT(G_VX, e, uv, VIS(nxy, MUL(v_p - v_0, rxf)));
     }
     if (j >= 1) {
       {  // cell centre: diagonal fluxes
         const fx u_m = LDG(U + cidx(I, im, j, k)), v_m = LDG(V + vidx(I, i, jm, k));
         const fx su = u_m + u_a, sv = v_m + v_0, sw = w_m + w_a;
-        PUT(G_UX, c, fx_mul(su, su), fx_mul(n_a, fx_mul(u_a - u_m, rxc)));
-        PUT(G_VY, c, fx_mul(sv, sv), fx_mul(n_a, fx_mul(v_0 - v_m, ryc)));
-        PUT(G_WZ, c, fx_mul(sw, sw), fx_mul(n_a, fx_mul(w_a - w_m, LDG(I.fxrzc + k))));
+        PUT(G_UX, c, ADV(su, su), VIS(n_a, MUL(u_a - u_m, rxc)));
+        PUT(G_VY, c, ADV(sv, sv), VIS(n_a, MUL(v_0 - v_m, ryc)));
+        PUT(G_WZ, c, ADV(sw, sw), VIS(n_a, MUL(w_a - w_m, LDG(I.fxrzc + k))));
       }
-      {  // xz edge (x-face i, y-centre j, z-face k): uw, nu -> GUz, GWx
+      {  // xz edge (x-face i, y-centre jc, z-face k): uw, nu -> GUz, GWx
         const fx w_p = LDG(W + cidx(I, ip, j, k));
-        const fx uw = fx_mul(u_a + u_z, w_a + w_p);                                   // 4 u w
+        const fx uw = ADV(u_a + u_z, w_a + w_p);                                      // 4 u w
         const fx nxz = nx_a + (n_az + n_pz);                                          // 4 nu
-        PUT(G_UZ, c, uw, fx_mul(nxz, fx_mul(u_z - u_a, rzf)));
-        PUT(G_WX, c, uw, fx_mul(nxz, fx_mul(w_p - w_a, rxf)));
+        PUT(G_UZ, c, uw, VIS(nxz, MUL(u_z - u_a, rzf)));
+        PUT(G_WX, c, uw, VIS(nxz, MUL(w_p - w_a, rxf)));
       }
     }
     u_a = u_z; v_0 = v_z; w_m = w_a; n_a = n_az; n_b = n_bz; n_p = n_pz;
   }
+#undef MUL
 #undef ADV
 #undef VIS
 #undef PUT
@@ -198,6 +187,15 @@ struct RhsArgs {
   int mode;               // 0: stage 1 (store F1), 1: stages 2/3, 2: actual-pressure RHS only
 };
 
+// A difference of y fluxes, whose rows have their own exponents.
+__device__ __forceinline__ double row_diff(fx hi, int eh, fx lo, int el) {
+  const int m = max(eh, el);
+  return fx_to((hi >> min(63, m - eh)) - (lo >> min(63, m - el)), m);
+}
+
+// The flux differences are exact integers; each is rounded once to a double
+// and multiplied by its reciprocal spacing there (with the products in
+// integers as well, F lost two to four bits to their common exponent).
 __global__ void __launch_bounds__(256)
 k_rhs_update(ChlMap map, RhsArgs a) {
   chl_pdl_wait();
@@ -211,25 +209,29 @@ k_rhs_update(ChlMap map, RhsArgs a) {
   const int im = wrap(i - 1, Nx), ip = wrap(i + 1, Nx);
   const int km = wrap(k - 1, Nz), kp = wrap(k + 1, Nz);
   const fx* const* G = I.G;
-  const int* u = I.upd;
-  const fx rxc = LDG(I.fxrxc + i), rxf = LDG(I.fxrxf + i);
-  const fx rzc = LDG(I.fxrzc + k), rzf = LDG(I.fxrzf + k);
-  const fx ryc = LDG(I.fxryc + jc);
+  const double rxc = LDG(I.rdxc + i), rxf = LDG(I.rdxf + i), ryc = LDG(I.rdyc + jc);
+  const double rzc = LDG(I.rdzc + k), rzf = LDG(I.rdzf + k);
   const size_t c = cidx(I, i, jc, k), e = vidx(I, i, jc, k), em = vidx(I, i, jc - 1, k);
   const bool hasv = jc <= Ny - 1;
-#define TERM(q, m, hi, lo, r) (fx_mul(LDG(G[m] + (hi)) - LDG(G[m] + (lo)), r) >> LDG(u + UPD_SHIFT + (q)))
+  // exponents of the fluxes of rows jc - 1, jc, jc + 1
+  const int4 e0 = LDG(I.upd + jc), el = LDG(I.upd + jc - 1), eh = LDG(I.upd + min(jc + 1, Ny));
+#define D(m, hi, lo, e) fx_to(LDG(G[m] + (hi)) - LDG(G[m] + (lo)), e)
   // u at (x-face i, row jc, z-centre k), w at (x-centre i, row jc, z-face k),
   // v at (x-centre i, y-face jv = jc, z-centre k)
-  double Fu = fx_to(TERM(0, G_UX, cidx(I, ip, jc, k), c, rxf) + TERM(1, G_UY, e, em, ryc)
-                    + TERM(2, G_UZ, c, cidx(I, i, jc, km), rzc), LDG(u + UPD_EXP)) + I.scal[CHL_S_DPDX];
-  double Fw = fx_to(TERM(6, G_WX, c, cidx(I, im, jc, k), rxc) + TERM(7, G_WY, e, em, ryc)
-                    + TERM(8, G_WZ, cidx(I, i, jc, kp), c, rzf), LDG(u + UPD_EXP + 2));
+  double Fu = fma(D(G_UX, cidx(I, ip, jc, k), c, e0.x), rxf, I.scal[CHL_S_DPDX]);
+  Fu = fma(row_diff(LDG(G[G_UY] + e), e0.x, LDG(G[G_UY] + em), el.x), ryc, Fu);
+  Fu = fma(D(G_UZ, c, cidx(I, i, jc, km), e0.x), rzc, Fu);
+  double Fw = D(G_WX, c, cidx(I, im, jc, k), e0.z) * rxc;
+  Fw = fma(row_diff(LDG(G[G_WY] + e), e0.z, LDG(G[G_WY] + em), el.z), ryc, Fw);
+  Fw = fma(D(G_WZ, cidx(I, i, jc, kp), c, e0.z), rzf, Fw);
   double Fv = 0.0;
-  if (hasv)
-    Fv = fx_to(TERM(3, G_VX, e, vidx(I, im, jc, k), rxc) + TERM(4, G_VY, cidx(I, i, jc + 1, k), c, LDG(I.fxryf + jc))
-               + TERM(5, G_VZ, e, vidx(I, i, jc, km), rzc), LDG(u + UPD_EXP + 1));
-#undef TERM
-  if (LDG(u + UPD_BAD)) Fu = Fv = Fw = __longlong_as_double(0x7FF8000000000000LL);
+  if (hasv) {
+    Fv = D(G_VX, e, vidx(I, im, jc, k), e0.y) * rxc;
+    Fv = fma(row_diff(LDG(G[G_VY] + cidx(I, i, jc + 1, k)), eh.y, LDG(G[G_VY] + c), e0.y), LDG(I.rdyf + jc), Fv);
+    Fv = fma(D(G_VZ, e, vidx(I, i, jc, km), e0.y), rzc, Fv);
+  }
+#undef D
+  if (e0.w | el.w | eh.w) Fu = Fv = Fw = __longlong_as_double(0x7FF8000000000000LL);
   if (a.mode == 2) {           // actual-pressure RHS: keep F only
     I.Fp[0][c] = Fu; I.Fp[2][c] = Fw;
     if (hasv) I.Fp[1][e] = Fv;

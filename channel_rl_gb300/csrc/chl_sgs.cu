@@ -611,7 +611,8 @@ k_nut(ChlMap map, int s_in, int use_wm) {
   const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
   const bool valid = t < (unsigned)(Nx * (Ny + 2) * Nz);
-  const ChlIdx p = chl_split(valid ? t : 0u, Nx, Ny + 2);
+  // lanes past the end repeat the last centre and write nothing
+  const ChlIdx p = chl_split(valid ? t : (unsigned)(Nx * (Ny + 2) * Nz) - 1u, Nx, Ny + 2);
   const int i = p.i, jc = p.j, k = p.k;
   const bool wm = use_wm && I.wall_model != 0 && (jc <= 1 || jc >= Ny);
   const bool wmrow = valid && wm && (jc == 1 || jc == Ny);
@@ -636,8 +637,7 @@ k_nut(ChlMap map, int s_in, int use_wm) {
     }
     I.nut[cidx(I, i, jc, k)] = v;
   }
-  const unsigned hi[1] = {chl_abshi(v)};
-  chl_block_max(chl_nmax(I), hi);
+  chl_line_max(I.nmax, (unsigned)(k * (Ny + 2) + jc), Ny + 2, 0, chl_abshi(v));
 }
 
 // ------------------------------------------------------------ launchers

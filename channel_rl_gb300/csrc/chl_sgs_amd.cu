@@ -93,7 +93,8 @@ __device__ __forceinline__ Grad gradients(const ChlInst& I, const double* U, con
 // values at x faces i-1 and i (face i-1 from the lane to the left when that
 // lane is on the same row, i > 0).  Every lane of the warp reaches the
 // shuffle; lanes past the instance's last centre carry valid = false.
-// Returns the high word of the largest magnitude written.
+// Returns the high word of the largest magnitude written; the ghost row's
+// counts for the row next to it.
 __device__ __forceinline__ unsigned write_nut_rows(const ChlInst& I, const double* U, int i, int jc, int k, double v,
                                                    int use_wm, bool valid) {
   const int Ny = I.Ny;
@@ -133,7 +134,8 @@ k_amd(ChlMap map, int s_in, int use_wm) {
   const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
   const bool valid = t < (unsigned)(Nx * Ny * Nz);
-  const ChlIdx p = chl_split(valid ? t : 0u, Nx, Ny);   // lanes past the end compute point 0 and write nothing
+  // lanes past the end repeat the last centre and write nothing
+  const ChlIdx p = chl_split(valid ? t : (unsigned)(Nx * Ny * Nz) - 1u, Nx, Ny);
   const int i = p.i, jc = 1 + p.j, k = p.k;
   const Grad g = gradients(I, I.U[s_in], I.V[s_in], I.W[s_in], i, jc, k);
   // centre strain: diagonal S_ii; 8 S_ij off the diagonal
@@ -164,8 +166,7 @@ k_amd(ChlMap map, int s_in, int use_wm) {
   N = fma(a12, t12, N); N = fma(a13, t13, N); N = fma(a23, t23, N);
   const double v = (-0.3 * N) / D;
   if (valid) I.S[cidx(I, i, jc, k)] = v;
-  const unsigned hi[1] = {write_nut_rows(I, I.U[s_in], i, jc, k, v, use_wm, valid)};
-  chl_block_max(chl_nmax(I), hi);
+  chl_line_max(I.nmax, (unsigned)(k * Ny + jc - 1), Ny, 1, write_nut_rows(I, I.U[s_in], i, jc, k, v, use_wm, valid));
 }
 
 __global__ void __launch_bounds__(256)
@@ -176,7 +177,7 @@ k_vreman(ChlMap map, int s_in, int use_wm) {
   const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
   const bool valid = t < (unsigned)(Nx * Ny * Nz);
-  const ChlIdx p = chl_split(valid ? t : 0u, Nx, Ny);
+  const ChlIdx p = chl_split(valid ? t : (unsigned)(Nx * Ny * Nz) - 1u, Nx, Ny);
   const int i = p.i, jc = 1 + p.j, k = p.k;
   const Grad g = gradients(I, I.U[s_in], I.V[s_in], I.W[s_in], i, jc, k);
   // a_ij = du_j/dx_i (reference layout 1 4 5 / 7 2 6 / 8 9 3); the
@@ -201,8 +202,7 @@ k_vreman(ChlMap map, int s_in, int use_wm) {
   Ab = fma(0.0625, Ao, Ab);
   const double v = 2.5 * (0.1 * 0.1) * chl_sqrt(Bb / Ab);
   if (valid) I.S[cidx(I, i, jc, k)] = v;
-  const unsigned hi[1] = {write_nut_rows(I, I.U[s_in], i, jc, k, v, use_wm, valid)};
-  chl_block_max(chl_nmax(I), hi);
+  chl_line_max(I.nmax, (unsigned)(k * Ny + jc - 1), Ny, 1, write_nut_rows(I, I.U[s_in], i, jc, k, v, use_wm, valid));
 }
 
 extern "C" {
