@@ -47,21 +47,40 @@ __host__ __device__ inline int chl_tri_lanes(long modes, int Ny) {
 // some SMs and 1 on most.  A function of the instance's own extents only,
 // so an instance sums its planes in the same order alone and in a batch.
 // Stockham FFT passes (chl_fft.cu): radix 4 while the remaining length
-// allows, then 3, then 2.  Each pass with twiddles (sub-transform size
-// Ns > 1) has CHL_TW_F fields of Ns doubles in the length's pass table.
-#define CHL_TW_F 7
-__host__ __device__ inline int chl_fft_radix(int rem) { return rem % 4 == 0 ? 4 : (rem % 3 == 0 ? 3 : 2); }
-__host__ __device__ inline int chl_tw_len(int N) {
+// allows, then 3, then 2.
+inline int chl_fft_radix(int rem) { return rem % 4 == 0 ? 4 : (rem % 3 == 0 ? 3 : 2); }
+// table of a length: one entry per pass, then Ns (R - 1) twiddles per pass
+// after the first
+inline int chl_twf_len(int N) {
   int Ns = 1, rem = N, len = 0;
   while (rem > 1) {
     const int R = chl_fft_radix(rem);
-    if (Ns > 1) len += CHL_TW_F * Ns;
+    len += Ns > 1 ? 1 + Ns * (R - 1) : 1;
     Ns *= R; rem /= R;
   }
   return len;
 }
-// bytes of a pass table in shared memory, kept a multiple of 16
-__host__ __device__ inline size_t chl_tw_bytes(int len) { return ((size_t)len * 8 + 15) & ~(size_t)15; }
+inline int chl_fft_passes(int N) {
+  int n = 0;
+  for (int rem = N; rem > 1; ++n) rem /= chl_fft_radix(rem);
+  return n;
+}
+// Bits of a line's largest component at the start, so that every pass with
+// twiddles reads elements of modulus below 2^61: the modulus is below sqrt(2)
+// times the component and grows by R in the first pass and by R/2 in each
+// later one but the last (log2 in hundredths, rounded up).
+inline int chl_fft_bits(int N) {
+  int grow = 50, rem = N;
+  bool first = true;
+  while (rem > 1) {
+    const int R = chl_fft_radix(rem);
+    rem /= R;
+    if (rem > 1) grow += R == 4 ? 200 : (R == 3 ? 159 : 100);
+    if (rem > 1 && !first) grow -= 100;
+    first = false;
+  }
+  return (6100 - grow) / 100;
+}
 
 #define CHL_DSMF_THREADS 64
 // Points of one plane sum: the Nx x Nz plane, then the reference's
@@ -76,10 +95,11 @@ __host__ __device__ inline int chl_dsm_ppt(int Nx, int Ny, int Nz) {
   return ppt;
 }
 // complex rows (pairs of real x lines) per x-transform block: up to
-// 1024/Nx, halved while the instance's grid would have fewer than
+// 512/Nx (at 256x96x192 the two x transforms take 95 + 54 us per launch with
+// 1024 points, 89 + 51 with 512, 91 + 52 with 256), halved while the instance's grid would have fewer than
 // min_blocks blocks (CHL_FFT_MIN_BLOCKS unless the tuner chose another)
 __host__ __device__ inline int chl_fftx_rows(int Nx, int nrow, int min_blocks) {
-  int cr = 1024 / Nx;
+  int cr = 512 / Nx;
   if (cr < 1) cr = 1;
   while (cr > 1 && (nrow + cr - 1) / cr < min_blocks) cr >>= 1;
   return cr;
@@ -125,7 +145,11 @@ struct ChlInst {
   const double *smag_csdelta;     // Cs*Delta_j by centre row (static Smagorinsky)
   const double *smag_dwall;       // distance of centre row to the nearer wall (van Driest)
   // Fourier / tridiagonal
-  const double *twx, *twz;        // pass tables of the x and z transforms (chl_tw_len doubles)
+  // tables of the x and z transforms (chl_fft.cu, chl_twf_len) with their
+  // lengths, passes and starting bits: loops over a length's factors are
+  // divisions that a thread of a transform would spend half its time on
+  const int4 *twx, *twz;
+  int lenx, lenz, passx, passz, bitsx, bitsz;
   const double *tri_inv, *tri_m, *tri_c;   // [Ny][Nz][Nxh] Thomas factors
   // state: three velocity sets (start-of-step / stage 1 / stage 2)
   double *U[3], *V[3], *W[3];

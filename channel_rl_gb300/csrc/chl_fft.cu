@@ -8,10 +8,10 @@
 // The reference transforms each y-plane with FFTW-MPI and calls LAPACK
 // zgtsv per mode.  Here:
 //  * x: two real rows are packed as one complex row, transformed by a
-//    shared-memory Stockham FFT (radix 4/3/2) and split into two
+//    shared-memory Stockham FFT (radix 4/3/2, fixed point) and split into two
 //    half-spectra (kx = 0..Nx/2) - fused with the divergence that produces
 //    the rows;
-//  * z: complex columns of the half-spectrum, staged 16 kx-columns at a time
+//  * z: complex columns of the half-spectrum, staged up to 8 kx-columns at a time
 //    in shared memory;
 //  * y: one thread per mode runs the Thomas elimination with factors
 //    precomputed once per grid (the matrix of a mode never changes between
@@ -24,205 +24,225 @@
 #include <cooperative_groups.h>
 
 // ------------------------------------------------------------ Stockham passes
-// Data of `nrows` transforms of length N; element e of row r is at
-// r*rs + e*es.  One pass of radix R with sub-transform size Ns.
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-  return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
-}
-__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-
-template <int R>
-__device__ __forceinline__ void dft_small(double2* v, bool inv) {
-  if (R == 2) {
-    const double2 a = v[0], b = v[1];
-    v[0] = cadd(a, b); v[1] = csub(a, b);
-  } else if (R == 4) {
-    const double2 a = cadd(v[0], v[2]), b = csub(v[0], v[2]);
-    const double2 c = cadd(v[1], v[3]), e = csub(v[1], v[3]);
-    // d = e * (-i) forward, e * (+i) inverse
-    const double2 d = inv ? make_double2(-e.y, e.x) : make_double2(e.y, -e.x);
-    v[0] = cadd(a, c); v[2] = csub(a, c);
-    v[1] = cadd(b, d); v[3] = csub(b, d);
-  } else if (R == 3) {
-    const double s3 = 0.86602540378443864676;   // sin(2 pi/3)
-    const double2 s = cadd(v[1], v[2]), d = csub(v[1], v[2]);
-    const double2 t = make_double2(fma(-0.5, s.x, v[0].x), fma(-0.5, s.y, v[0].y));
-    // forward: out1 = t - i s3 d, out2 = t + i s3 d (inverse swaps)
-    const double2 m = inv ? make_double2(-s3 * d.y, s3 * d.x) : make_double2(s3 * d.y, -s3 * d.x);
-    v[0] = cadd(v[0], s);
-    v[1] = cadd(t, m);
-    v[2] = csub(t, m);
-  }
-}
-
-// Twiddle multiplications in tangent form (E. Linzer and E. Feig, Modified
-// FFTs for fused multiply-add architectures, Math. Comp. 60 (1993) 347): a
-// twiddle w = C + iS
-// is kept as a scale sigma and a multiplier m with |m| <= 1 - sigma = C,
-// m = S/C where |C| >= |S|, else sigma = S, m = C/S - so v w = sigma y with
-// y two FMAs away from v, and each sigma is folded into an FMA of the
-// butterfly instead of costing a multiplication.  A radix-4 butterfly with
-// twiddles then takes 22 FP64 instructions instead of 28, a radix-3 one 16
-// instead of 22, a radix-2 one 6 instead of 8.  The choice of form and the
-// sign flips of the inverse transform (conjugate twiddles) are integer
-// operations on bit patterns, which the FP64-bound passes get for free.
+// Autosort Stockham FFT of radix 4, 3, 2 in 64-bit fixed point (chl_fix.cuh),
+// shared memory to shared memory.  On the FP64 pipe a radix-4 butterfly with
+// twiddles took 22 instructions of 64 clocks; here it is 36 32-bit
+// multiply-adds (IMAD.WIDE) and about 70 additions and shifts, which the
+// integer pipes issue in a fifth of that.
 //
-// Pass table of a length N, per pass with twiddles (sub-transform size
-// Ns > 1, radix R), CHL_TW_F fields of Ns entries, entry jm being the
-// butterflies j with j mod Ns = jm (twiddles w_r = exp(-2 pi i jm r/(Ns R)),
-// r = 1..R-1, in the forward direction):
-//   0 m1, 1 m2, 2 m3 (radix 4) or sin(2 pi/3) sigma1 (radix 3), 3 sigma1,
-//   4 sigma2 (radix 4) or sigma1 / 2 (radix 3), 5 sigma3/sigma1 (radix 4)
-//   or sigma2/sigma1 (radix 3), 6 form bits (bit r set: w_r in the S form),
-//   stored as the bit pattern of a double.
-// The sign flips and operand selects are inline PTX: written as C++ the
-// compiler folds "FMA of two selects on one condition" into two FMAs and a
-// select, which doubles the FP64 work these forms exist to save.
-__device__ __forceinline__ double flip(double x, unsigned f) {
-  long long r;
-  asm("{\n\t.reg .b64 t;\n\tcvt.u64.u32 t, %2;\n\tshl.b64 t, t, 63;\n\txor.b64 %0, %1, t;\n\t}"
-      : "=l"(r) : "l"(__double_as_longlong(x)), "r"(f));
-  return __longlong_as_double(r);
-}
-// v w / sigma: (a - b m, b + a m) in the C form, (a m - b, b m + a) =
-// (-(b - a m), a + b m) in the S form.  With (p, q) = (b, a) in the C form
-// and (a, b) in the S form both are (+/- fma(p, -m, q), fma(q, m, p)): two
-// selects and, in the S form, a sign flip of the first component.  The flip
-// XORs a mask chosen between 0 and sgn, the bit pattern of -0.0 read from
-// device memory: were the mask visibly the sign bit, ptxas would turn the
-// flip into a pair of predicated FMAs, one per form, and every warp would
-// issue both.
-__device__ __forceinline__ double2 tw_apply(double2 v, double m, unsigned sform, long long sgn) {
-  long long p, q, t;
-  asm("{\n\t.reg .pred s;\n\t"
-      "setp.ne.u32 s, %5, 0;\n\t"
-      "selp.b64 %0, %3, %4, s;\n\t"     // p = S form ? a : b
-      "selp.b64 %1, %4, %3, s;\n\t"     // q = S form ? b : a
-      "selp.b64 %2, %6, 0, s;\n\t}"     // t = S form ? sgn : 0
-      : "=l"(p), "=l"(q), "=l"(t)
-      : "l"(__double_as_longlong(v.x)), "l"(__double_as_longlong(v.y)), "r"(sform), "l"(sgn));
-  const double P = __longlong_as_double(p), Q = __longlong_as_double(q);
-  return make_double2(__longlong_as_double(__double_as_longlong(fma(P, -m, Q)) ^ t), fma(Q, m, P));
-}
-__device__ __forceinline__ double2 fma2(double s, double2 y, double2 v) {
-  return make_double2(fma(s, y.x, v.x), fma(s, y.y, v.y));
+// Every line is scaled by its own largest component (found while it is
+// loaded), so a line's result does not depend on which lines share its block.
+// The first pass (no twiddles) grows a line by at most its radix R; every
+// later pass is halved, growth R/2, because the halved product is what the
+// multiplication gives.  fft_bits(N) is the number of bits a line may start
+// with so that no pass input exceeds 2^61: 56 for N = 256, three bits finer
+// than a double's last bit at the line's largest component; the rounding of a
+// pass (below one unit per product) stays there too.  Measured error of the
+// projection: chl_fft's callers compare with FP64 in tests/test_fft_fixed_gpu.py.
+//
+// Table of a length: per pass {R, Ns, 2^32/Ns, 2^32/(N/R)}, then the twiddles.
+// Twiddles w = c + is as the words (high, low >> 1) of c 2^63 and s 2^63
+// (2^63 - 1 for 1), per pass with twiddles and radix digit r = 1..R-1: entries
+// jm = 0..Ns-1 for w = exp(-2 pi i jm r/(Ns R)).
+typedef longlong2 fx2;
+__device__ __forceinline__ fx2 add2(fx2 a, fx2 b) { return make_longlong2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ fx2 sub2(fx2 a, fx2 b) { return make_longlong2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ fx2 halve(fx2 a) { return make_longlong2(a.x >> 1, a.y >> 1); }
+
+// v w / 2 (INV: v conj(w) / 2).  The four cross terms of a component, at most
+// 2^62.9 together for |v| < 2^61, are summed before their one shift; the
+// starting value rounds it and makes up for the dropped low products.
+template <bool INV>
+__device__ __forceinline__ fx2 tw_mul(fx2 v, int4 w) {
+  const long long R = 1LL << 31;
+  const fx n = INV ? -v.x : -v.y;
+  const int xh = (int)(v.x >> 32), xl = (int)((unsigned)v.x >> 1);
+  const int yh = (int)(v.y >> 32), yl = (int)((unsigned)v.y >> 1);
+  const int nh = (int)(n >> 32), nl = (int)((unsigned)n >> 1);
+  const int ah = INV ? yh : nh, al = INV ? yl : nl;    // times s into the real part
+  const int bh = INV ? nh : xh, bl = INV ? nl : xl;    // times s into the imaginary part
+  long long t = R + (long long)xh * w.y + (long long)w.x * xl;
+  t += (long long)ah * w.w;
+  t += (long long)w.z * al;
+  long long u = R + (long long)yh * w.y + (long long)w.x * yl;
+  u += (long long)bh * w.w;
+  u += (long long)w.z * bl;
+  return make_longlong2((long long)xh * w.x + (long long)ah * w.z + (t >> 31),
+                        (long long)yh * w.x + (long long)bh * w.z + (u >> 31));
 }
 
-// Work items (row, butterfly j) are numbered so that consecutive threads
-// touch neighbouring shared-memory words: j fastest when a row is contiguous
-// (es = 1, the x lines), the row fastest when rows are interleaved (rs = 1,
-// the z columns), which keeps the 16-byte accesses free of bank conflicts.
-// tab: this pass's table (Ns > 1), staged in shared memory by the caller.
-// TW: the pass has twiddles (Ns > 1) - a template parameter, not a branch
-// on Ns inside the loop: ptxas predicates both sides of such a branch, and
-// a predicated-off FP64 instruction still takes its turn on the FP64 pipe
-// (measured: 2 extra instructions per complex point over a 128-point
-// transform).
-// INV (the inverse transform) likewise: a runtime direction would put
-// predicated sign flips into every butterfly.
-template <int R, bool TW, bool INV>
-__device__ void stockham_pass(const double2* __restrict__ x, double2* __restrict__ y, int nrows, int rs, int es,
-                              int N, int Ns, const double* __restrict__ tab, long long sgn) {
-  const int nb = N / R;
-  const bool rowfast = rs < es;
-  constexpr unsigned iv = INV ? 1u : 0u;
-  for (int w = threadIdx.x; w < nrows * nb; w += blockDim.x) {
-    int row, j;
-    if (rowfast) { j = w / nrows; row = w - j * nrows; }
-    else { row = w / nb; j = w - row * nb; }
-    const double2* xr = x + (size_t)row * rs;
-    double2* yr = y + (size_t)row * rs;
-    const int jm = j % Ns;
-    double2 v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = xr[(j + r * nb) * es];
-    if (!TW) {
-      dft_small<R>(v, INV);
-    } else {
-      const unsigned fb = (unsigned)__double_as_longlong(tab[6 * Ns + jm]);
-      const unsigned f1 = (fb >> 1) & 1u, f2 = (fb >> 2) & 1u;
-      const double s1 = flip(tab[3 * Ns + jm], iv & f1);
-      const double2 y1 = tw_apply(v[1], flip(tab[jm], iv), f1, sgn);
-      if (R == 2) {
-        const double2 v0 = v[0];
-        v[0] = fma2(s1, y1, v0);
-        v[1] = fma2(-s1, y1, v0);
-      } else if (R == 4) {
-        const unsigned f3 = (fb >> 3) & 1u;
-        const double2 y2 = tw_apply(v[2], flip(tab[Ns + jm], iv), f2, sgn);
-        const double2 y3 = tw_apply(v[3], flip(tab[2 * Ns + jm], iv), f3, sgn);
-        const double s2 = flip(tab[4 * Ns + jm], iv & f2);
-        const double rho = flip(tab[5 * Ns + jm], iv & (f1 ^ f3));
-        const double2 a = fma2(s2, y2, v[0]), b = fma2(-s2, y2, v[0]);
-        const double2 c = fma2(rho, y3, y1), e = fma2(-rho, y3, y1);
-        // (v1 w1 - v3 w3) times -i (forward) or +i (inverse) is s1 e times it
-        const double si = flip(s1, iv);
-        v[0] = fma2(s1, c, a);
-        v[2] = fma2(-s1, c, a);
-        v[1] = make_double2(fma(si, e.y, b.x), fma(-si, e.x, b.y));
-        v[3] = make_double2(fma(-si, e.y, b.x), fma(si, e.x, b.y));
-      } else {   // R == 3
-        const double2 y2 = tw_apply(v[2], flip(tab[Ns + jm], iv), f2, sgn);
-        const double h1 = flip(tab[4 * Ns + jm], iv & f1);
-        const double rho = flip(tab[5 * Ns + jm], iv & (f1 ^ f2));
-        // forward: out1,2 = t -/+ i sin(2pi/3) (v1 w1 - v2 w2); inverse +/-
-        const double k1 = flip(tab[2 * Ns + jm], iv & (f1 ^ 1u));
-        const double2 sp = fma2(rho, y2, y1), dp = fma2(-rho, y2, y1);
-        const double2 v0 = v[0];
-        const double2 t = fma2(-h1, sp, v0);
-        v[0] = fma2(s1, sp, v0);
-        v[1] = make_double2(fma(k1, dp.y, t.x), fma(-k1, dp.x, t.y));
-        v[2] = make_double2(fma(-k1, dp.y, t.x), fma(k1, dp.x, t.y));
-      }
-    }
-    const int idxD = (j / Ns) * Ns * R + jm;
-#pragma unroll
-    for (int r = 0; r < R; ++r) yr[(idxD + r * Ns) * es] = v[r];
+#define FX_SIN60 0x6ED9EBA16132A9CFLL   // sin(2 pi/3) 2^63
+// Butterfly of v[0..R): the first input as it is (pass one) or halved by the
+// caller, the others twiddled.
+template <int R, bool INV>
+__device__ __forceinline__ void butterfly(fx2* v) {
+  if (R == 2) {
+    const fx2 a = v[0], b = v[1];
+    v[0] = add2(a, b); v[1] = sub2(a, b);
+  } else if (R == 4) {
+    const fx2 a = add2(v[0], v[2]), b = sub2(v[0], v[2]);
+    const fx2 c = add2(v[1], v[3]), e = sub2(v[1], v[3]);
+    // d = e * (-i) forward, e * (+i) inverse
+    v[0] = add2(a, c); v[2] = sub2(a, c);
+    const fx2 p = make_longlong2(b.x + e.y, b.y - e.x), q = make_longlong2(b.x - e.y, b.y + e.x);
+    v[1] = INV ? q : p; v[3] = INV ? p : q;
+  } else {
+    const fx2 t0 = add2(v[1], v[2]), d = sub2(v[1], v[2]);
+    const fx2 t = sub2(v[0], halve(t0));
+    const fx mx = 2 * fx_mul(d.x, FX_SIN60), my = 2 * fx_mul(d.y, FX_SIN60);
+    v[0] = add2(v[0], t0);
+    const fx2 p = make_longlong2(t.x + my, t.y - mx), q = make_longlong2(t.x - my, t.y + mx);
+    v[1] = INV ? q : p; v[2] = INV ? p : q;
   }
 }
 
-// Copies a length's pass table (len doubles) into shared memory; the first
-// barrier of fft_smem orders it before any use.
-__device__ __forceinline__ void stage_twiddles(double* tws, const double* __restrict__ tab, int len) {
+// Shared memory, in 16-byte units; tiles and tables go by their offset in it
+// (a pointer that alternates between the tiles would be a generic one).
+__device__ __forceinline__ fx2* smem_fx() { extern __shared__ double2 sm[]; return reinterpret_cast<fx2*>(sm); }
+__device__ __forceinline__ double2* smem_d2() { extern __shared__ double2 sm[]; return sm; }
+__device__ __forceinline__ int4* smem_tw() { extern __shared__ double2 sm[]; return reinterpret_cast<int4*>(sm); }
+
+// n / d for n, d < 2^16 by one multiplication with m = 2^32/d rounded up (0
+// stands for d = 1)
+__device__ __forceinline__ int small_div(int n, unsigned m) { return m == 0u ? n : (int)__umulhi((unsigned)n, m); }
+struct SmallDiv {
+  int d; unsigned m;
+  __device__ __forceinline__ explicit SmallDiv(int dd) : d(dd), m(0xFFFFFFFFu / (unsigned)dd + 1u) {}
+  __device__ __forceinline__ int div(int n) const { return small_div(n, m); }
+};
+
+// One pass over nrows lines: butterfly inputs from ld(row, element), results
+// to st(row, element, value).  Work items (row, butterfly j) are numbered so
+// that consecutive threads touch neighbouring words: j fastest when a row is
+// contiguous (the x lines), the row fastest when rows are interleaved (the z
+// columns), which keeps the 16-byte accesses free of bank conflicts.
+template <int R, bool TW, bool INV, class LD, class ST>
+__device__ __forceinline__ void fx_pass(const LD& ld, const ST& st, const SmallDiv& rows, bool rowfast, int N, int4 pass,
+                                        int tab) {
+  const int nb = N / R, Ns = pass.y;
+  const int d = rowfast ? rows.d : nb;
+  const unsigned dm = rowfast ? rows.m : (unsigned)pass.w;
+  for (int w = threadIdx.x; w < rows.d * nb; w += blockDim.x) {
+    const int q = small_div(w, dm), m = w - q * d;
+    const int row = rowfast ? m : q, j = rowfast ? q : m;
+    fx2 v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = ld(row, j + r * nb);
+    int o = j * R, step = 1;
+    if (TW) {
+      const int g = small_div(j, (unsigned)pass.z), jm = j - g * Ns;
+      v[0] = halve(v[0]);
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[r] = tw_mul<INV>(v[r], smem_tw()[tab + (r - 1) * Ns + jm]);
+      o = g * Ns * R + jm;
+      step = Ns;
+    }
+    butterfly<R, INV>(v);
+#pragma unroll
+    for (int r = 0; r < R; ++r) st(row, o + r * step, v[r]);
+  }
+}
+
+template <bool TW, bool INV, class LD, class ST>
+__device__ __forceinline__ void fx_pass_any(const LD& ld, const ST& st, const SmallDiv& rows, bool rowfast, int N,
+                                            int4 pass, int tab) {
+  if (pass.x == 4) fx_pass<4, TW, INV>(ld, st, rows, rowfast, N, pass, tab);
+  else if (pass.x == 3) fx_pass<3, TW, INV>(ld, st, rows, rowfast, N, pass, tab);
+  else fx_pass<2, TW, INV>(ld, st, rows, rowfast, N, pass, tab);
+}
+
+// Conversions of a line.  Doubles come in on the integer pipe; of a result's
+// two components one goes out on each pipe (scaled by the power of two after
+// the hardware's conversion on the FP64 pipe, which nothing else here uses):
+// at 256x96x192 the four transforms of a stage take 275 us with all
+// conversions on the integer pipe, 262 us like this and 332 us with all of
+// them on the FP64 pipe.
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }   // -1022 <= e <= 1023
+struct LineIn {
+  int bits; const unsigned* hi;
+  __device__ __forceinline__ int exponent(int r) const { return fx_line_exp(hi[r], bits); }
+};
+__device__ __forceinline__ fx2 fx2_from(double2 d, int e) { return make_longlong2(fx_from(d.x, e), fx_from(d.y, e)); }
+
+// shared-memory tile of lines: element e of row r at off + r*rs + e*es
+struct TileLd {
+  int off, rs, es;
+  __device__ __forceinline__ fx2 operator()(int r, int e) const { return smem_fx()[off + r * rs + e * es]; }
+};
+struct TileSt {
+  int off, rs, es;
+  __device__ __forceinline__ void operator()(int r, int e, fx2 v) const { smem_fx()[off + r * rs + e * es] = v; }
+};
+// a tile that holds doubles, converted with the exponent of its line
+struct RawLd {
+  int off, rs, es; LineIn in;
+  __device__ __forceinline__ fx2 operator()(int r, int e) const {
+    return fx2_from(smem_d2()[off + r * rs + e * es], in.exponent(r));
+  }
+};
+// a line's result as doubles: the passes with twiddles halved it `halvings`
+// times; a line with a non-finite input is NaN throughout
+struct LineOut {
+  int bits, halvings; const unsigned* hi;
+  __device__ __forceinline__ double2 operator()(int r, fx2 v) const {
+    const int x = fx_line_exp(hi[r], bits) + halvings;
+    const double s = fx_bad(hi[r]) ? __longlong_as_double(0x7FF8000000000000LL) : pow2(x);
+    double a = fx_to(v.x, x);
+    if (fx_bad(hi[r])) a = s;
+    return make_double2(a, __ll2double_rn(v.y) * s);
+  }
+};
+struct DoubleTileSt {
+  int off, rs, es; LineOut out;
+  __device__ __forceinline__ void operator()(int r, int e, fx2 v) const { smem_d2()[off + r * rs + e * es] = out(r, v); }
+};
+
+// Full transform of `passes` passes: the first from `first` into b, the ones
+// between through the tiles b and a, the last to `last`.  tab: the length's
+// table in shared memory.  Ends without a barrier.
+template <bool INV, class LD, class ST>
+__device__ __forceinline__ void fx_fft(const LD& first, const ST& last, int a, int b, int nrows, int rs, int es, int N,
+                                       int passes, int tab) {
+  const bool rowfast = rs < es;
+  const SmallDiv rows(nrows);
+  __syncthreads();
+  if (passes == 1) {
+    fx_pass_any<false, INV>(first, last, rows, rowfast, N, smem_tw()[tab], 0);
+    return;
+  }
+  fx_pass_any<false, INV>(first, TileSt{b, rs, es}, rows, rowfast, N, smem_tw()[tab], 0);
+  int src = b, dst = a, tw = tab + passes;
+  for (int p = 1; p < passes - 1; ++p) {
+    const int4 pass = smem_tw()[tab + p];
+    __syncthreads();
+    fx_pass_any<true, INV>(TileLd{src, rs, es}, TileSt{dst, rs, es}, rows, rowfast, N, pass, tw);
+    tw += pass.y * (pass.x - 1);
+    const int t = src; src = dst; dst = t;
+  }
+  __syncthreads();
+  fx_pass_any<true, INV>(TileLd{src, rs, es}, last, rows, rowfast, N, smem_tw()[tab + passes - 1], tw);
+}
+// the tile that fx_fft's last pass may write (it reads the other one)
+__device__ __forceinline__ int fx_last_tile(int a, int b, int passes) { return passes & 1 ? b : a; }
+
+// Copies a length's twiddles into shared memory; the barrier ahead of the
+// first pass orders it before any use.
+__device__ __forceinline__ void stage_twiddles(int4* tws, const int4* __restrict__ tab, int len) {
   for (int w = threadIdx.x; w < len; w += blockDim.x) tws[w] = LDG(tab + w);
 }
 
-// Full transform; returns the buffer holding the result (a or b).  tab: the
-// length's pass table in shared memory (stage_twiddles); sgn: the bit
-// pattern of -0.0 from the instance's constants (see tw_apply).
-template <bool INV>
-__device__ double2* fft_smem_dir(double2* a, double2* b, int nrows, int rs, int es, int N,
-                                 const double* tab, long long sgn) {
-  int Ns = 1, rem = N, off = 0;
-  double2 *src = a, *dst = b;
-  while (rem > 1) {
-    __syncthreads();
-    const int R = chl_fft_radix(rem);
-    const double* tp = tab + off;
-    if (R == 4) {
-      if (Ns == 1) stockham_pass<4, false, INV>(src, dst, nrows, rs, es, N, Ns, tp, sgn);
-      else stockham_pass<4, true, INV>(src, dst, nrows, rs, es, N, Ns, tp, sgn);
-    } else if (R == 3) {
-      if (Ns == 1) stockham_pass<3, false, INV>(src, dst, nrows, rs, es, N, Ns, tp, sgn);
-      else stockham_pass<3, true, INV>(src, dst, nrows, rs, es, N, Ns, tp, sgn);
-    } else {
-      if (Ns == 1) stockham_pass<2, false, INV>(src, dst, nrows, rs, es, N, Ns, tp, sgn);
-      else stockham_pass<2, true, INV>(src, dst, nrows, rs, es, N, Ns, tp, sgn);
-    }
-    if (Ns > 1) off += CHL_TW_F * Ns;
-    Ns *= R; rem /= R;
-    double2* t = src; src = dst; dst = t;
+// Largest component of line `row` among the values of the calling warp's
+// lanes (high words; all lanes call, those without a value pass 0).
+__device__ __forceinline__ void fold_line(unsigned* hi, int row, unsigned v) {
+  const unsigned full = 0xffffffffu;
+  if (__all_sync(full, row == __shfl_sync(full, row, 0))) {
+    v = __reduce_max_sync(full, v);
+    if ((threadIdx.x & 31) == 0) atomicMax(hi + row, v);
+  } else {
+    atomicMax(hi + row, v);
   }
-  __syncthreads();
-  return src;
 }
-__device__ __forceinline__ double2* fft_smem(double2* a, double2* b, int nrows, int rs, int es, int N,
-                                             const double* tab, bool inv, long long sgn) {
-  return inv ? fft_smem_dir<true>(a, b, nrows, rs, es, N, tab, sgn)
-             : fft_smem_dir<false>(a, b, nrows, rs, es, N, tab, sgn);
-}
-
+__device__ __forceinline__ unsigned abshi2(double2 v) { return max(chl_abshi(v.x), chl_abshi(v.y)); }
 
 // ------------------------------------------------------------ divergence + forward x
 // mode 0: div of velocity set s_in (compute_pseudo_pressure_rhs, projection.f90:40-55)
@@ -241,18 +261,21 @@ k_div_fftx(ChlMap map, int s_in, int mode, int xmb) {
   const int CR = chl_fftx_rows(Nx, nrow, xmb);
   const int g0 = lb * CR;
   const int cr_n = min(CR, nrow - g0);
-  double2* A = sm;
-  double2* B = sm + CR * Nx;
-  double* T = reinterpret_cast<double*>(sm + 2 * CR * Nx);   // pass table
-  stage_twiddles(T, I.twx, chl_tw_len(Nx));
+  const int A = 0, B = CR * (Nx + 2), T = B + CR * Nx;       // tiles, twiddles
+  unsigned* hi = reinterpret_cast<unsigned*>(sm + T + I.lenx);
+  stage_twiddles(smem_tw() + T, I.twx, I.lenx);
+  for (int r = threadIdx.x; r < CR; r += blockDim.x) hi[r] = 0u;
+  __syncthreads();
   const double *U, *V, *W;
   if (mode == 0 && lb == 0 && threadIdx.x < 3) chl_vmax(I, s_in)[threadIdx.x] = 0u;
   if (mode != 1) { U = I.U[s_in]; V = I.V[s_in]; W = I.W[s_in]; }
   else { U = I.Fp[0]; V = I.Fp[1]; W = I.Fp[2]; }
-  for (int w = threadIdx.x; w < cr_n * Nx; w += blockDim.x) {
-    const int cr = w / Nx, i = w - cr * Nx;
-    const int g = g0 + cr;
-    const int jc = 1 + g / (Nz / 2), k0 = 2 * (g % (Nz / 2));
+  const SmallDiv byNx(Nx);
+  for (int w0 = 0; w0 < cr_n * Nx; w0 += blockDim.x) {
+    const int w = min(w0 + (int)threadIdx.x, cr_n * Nx - 1);   // lanes past the end repeat the last point
+    const int cr = byNx.div(w), i = w - cr * Nx;
+    const unsigned g = g0 + cr;
+    const int jz = (int)(g / (unsigned)(Nz / 2)), jc = 1 + jz, k0 = 2 * ((int)g - jz * (Nz / 2));
     const int im = wrap(i - 1, Nx);
     double dv[2];
 #pragma unroll
@@ -272,26 +295,39 @@ k_div_fftx(ChlMap map, int s_in, int mode, int xmb) {
       }
       dv[h] = d;
     }
-    A[cr * Nx + i] = make_double2(dv[0], dv[1]);
+    sm[cr * Nx + i] = make_double2(dv[0], dv[1]);
+    fold_line(hi, cr, abshi2(make_double2(dv[0], dv[1])));
   }
-  double2* res = fft_smem(A, B, cr_n, Nx, 1, Nx, T, false, __double_as_longlong(I.fk[FK_MZERO]));
+  // one bit less than the transform allows: the split below adds two elements
+  const int bits = I.bitsx - 1;
+  const int last = fx_last_tile(A, B, I.passx);
+  fx_fft<false>(RawLd{A, Nx, 1, LineIn{bits, hi}}, TileSt{last, Nx, 1}, A, B, cr_n, Nx, 1, Nx, I.passx, T);
+  const fx2* res = smem_fx() + last;
+  __syncthreads();
   // split the packed spectrum into the two half-spectra (each times 2)
+  const LineOut out{bits, I.passx - 1, hi};
+  const SmallDiv byNxh(Nxh);
   for (int w = threadIdx.x; w < cr_n * Nxh; w += blockDim.x) {
-    const int cr = w / Nxh, kx = w - cr * Nxh;
-    const int g = g0 + cr;
-    const int jc = 1 + g / (Nz / 2), k0 = 2 * (g % (Nz / 2));
-    const double2 z = res[cr * Nx + kx];
-    const double2 zc = res[cr * Nx + (kx == 0 ? 0 : Nx - kx)];   // conj taken below
-    const double2 Aa = make_double2(z.x + zc.x, z.y - zc.y);
-    const double2 Bb = make_double2(z.y + zc.y, zc.x - z.x);
-    I.spec[((size_t)jc * Nz + k0) * Nxh + kx] = Aa;
-    I.spec[((size_t)jc * Nz + k0 + 1) * Nxh + kx] = Bb;
+    const int cr = byNxh.div(w), kx = w - cr * Nxh;
+    const unsigned g = g0 + cr;
+    const int jz = (int)(g / (unsigned)(Nz / 2)), jc = 1 + jz, k0 = 2 * ((int)g - jz * (Nz / 2));
+    const fx2 z = res[cr * Nx + kx];
+    const fx2 zc = res[cr * Nx + (kx == 0 ? 0 : Nx - kx)];   // conj taken below
+    I.spec[((size_t)jc * Nz + k0) * Nxh + kx] = out(cr, make_longlong2(z.x + zc.x, z.y - zc.y));
+    I.spec[((size_t)jc * Nz + k0 + 1) * Nxh + kx] = out(cr, make_longlong2(z.y + zc.y, zc.x - z.x));
   }
 }
 
 // ------------------------------------------------------------ z transform of the half spectrum
+// a column's element k straight to the spectrum
+struct SpecSt {
+  double2* spec; const size_t* coff; int pitch; LineOut out;
+  __device__ __forceinline__ void operator()(int c, int k, fx2 v) const { spec[coff[c] + (size_t)k * pitch] = out(c, v); }
+};
+
+template <bool INV>
 __global__ void __launch_bounds__(256)
-k_fftz(ChlMap map, int inv, int zcw) {
+k_fftz(ChlMap map, int zcw) {
   chl_pdl_wait();
   // The Ny x Nxh columns (jc, kx) of an instance are numbered jc-major and
   // cut into runs of zcw (chl_fftz_cols); a run may cross into the next
@@ -299,6 +335,7 @@ k_fftz(ChlMap map, int inv, int zcw) {
   // block is short.
   extern __shared__ double2 sm[];
   __shared__ size_t coff[16];
+  __shared__ unsigned hi[16];    // the columns' largest components
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
   const int Nz = I.Nz, Nxh = I.Nxh;
@@ -307,22 +344,27 @@ k_fftz(ChlMap map, int inv, int zcw) {
   if (threadIdx.x < cw) {
     const int q = q0 + threadIdx.x;
     coff[threadIdx.x] = (size_t)(1 + q / Nxh) * Nz * Nxh + (q % Nxh);
+    hi[threadIdx.x] = 0u;
   }
   __syncthreads();
-  double2* A = sm;
-  double2* B = sm + Nz * zcw;
-  double* T = reinterpret_cast<double*>(sm + 2 * Nz * zcw);   // pass table
-  stage_twiddles(T, I.twz, chl_tw_len(Nz));
+  const int A = 0, B = Nz * zcw, T = 2 * Nz * zcw;           // tiles, twiddles
+  stage_twiddles(smem_tw() + T, I.twz, I.lenz);
   double2* spec = I.spec;
+  unsigned mine = 0u;
+  const bool fixed_c = blockDim.x % cw == 0;     // a thread stays on one column
+  const SmallDiv bycw(cw);
   for (int w = threadIdx.x; w < Nz * cw; w += blockDim.x) {
-    const int k = w / cw, c = w - k * cw;
-    A[k * zcw + c] = spec[coff[c] + (size_t)k * Nxh];
+    const int k = bycw.div(w), c = w - k * cw;
+    const double2 v = spec[coff[c] + (size_t)k * Nxh];
+    sm[k * zcw + c] = v;
+    mine = max(mine, abshi2(v));
+    if (!fixed_c) { atomicMax(hi + c, mine); mine = 0u; }
   }
-  double2* res = fft_smem(A, B, cw, 1, zcw, Nz, T, inv != 0, __double_as_longlong(I.fk[FK_MZERO]));
-  for (int w = threadIdx.x; w < Nz * cw; w += blockDim.x) {
-    const int k = w / cw, c = w - k * cw;
-    spec[coff[c] + (size_t)k * Nxh] = res[k * zcw + c];
-  }
+  if (fixed_c) atomicMax(hi + threadIdx.x % cw, mine);
+  const int bits = I.bitsz;
+  const RawLd first{A, 1, zcw, LineIn{bits, hi}};
+  const SpecSt last{spec, coff, Nxh, LineOut{bits, I.passz - 1, hi}};
+  fx_fft<INV>(first, last, A, B, cw, 1, zcw, Nz, I.passz, T);
 }
 
 // ------------------------------------------------------------ tridiagonal per mode
@@ -583,6 +625,22 @@ k_tri_scan(ChlMap map) {
 // of the cluster reaches (no early exit).
 namespace cg = cooperative_groups;
 
+// hi[r] of the rows r of a tile (element e at r + e*es), one warp per row
+__device__ __forceinline__ void line_max(const double2* p, int nrows, int es, int N, unsigned* hi) {
+  const int lane = threadIdx.x & 31;
+  for (int r = threadIdx.x >> 5; r < nrows; r += blockDim.x >> 5) {
+    unsigned v = 0u;
+    for (int e = lane; e < N; e += 32) v = max(v, abshi2(p[r + e * es]));
+    v = __reduce_max_sync(0xffffffffu, v);
+    if (lane == 0) hi[r] = v;
+  }
+}
+// row r, wavenumber e of a spectrum column
+struct RowSt {
+  double2* p; size_t rowpitch, pitch; LineOut out;
+  __device__ __forceinline__ void operator()(int r, int e, fx2 v) const { p[(size_t)r * rowpitch + (size_t)e * pitch] = out(r, v); }
+};
+
 __global__ void __launch_bounds__(256)
 k_zsolve(ChlMap map) {
   chl_pdl_wait();
@@ -598,25 +656,30 @@ k_zsolve(ChlMap map) {
   const int lo = min(Ny, r * L), hi = min(Ny, lo + L), nr = hi - lo;
   const size_t ps = (size_t)modes;              // row pitch of spec and factors
   double2* A = sm;
-  double2* B = sm + (size_t)L * Nz;
-  double* T = reinterpret_cast<double*>(sm + (size_t)2 * L * Nz);   // pass table
-  double2* fz = reinterpret_cast<double2*>(reinterpret_cast<char*>(T) + chl_tw_bytes(chl_tw_len(Nz)));
-                                                // forward lane values
+  const int T = 2 * L * Nz;                                     // twiddles
+  double2* fz = sm + T + I.lenz;                       // forward lane values
   double2* bw = fz + Nz;                        // backward lane values
   double2* yin = bw + Nz;
   double2* xin = yin + Nz;
   double* fA = reinterpret_cast<double*>(xin + Nz);
   double* bA = fA + Nz;
+  unsigned* top = reinterpret_cast<unsigned*>(bA + Nz);          // the lines' largest components
   const int t = threadIdx.x, bd = blockDim.x;
-  stage_twiddles(T, I.twz, chl_tw_len(Nz));
+  const int bits = I.bitsz, halvings = I.passz - 1;
+  stage_twiddles(smem_tw() + T, I.twz, I.lenz);
   // rows [lo, hi) of column kx: element (row l, kz) at l + kz*nr
   double2* spec = I.spec + ps + kx;             // row jc = 1
   for (int w = t; w < nr * Nz; w += bd) {
     const int l = w % nr, kz = w / nr;
     A[l + (size_t)kz * nr] = spec[(size_t)(lo + l) * ps + (size_t)kz * Nxh];
   }
-  double2* res = fft_smem(A, B, nr, 1, nr, Nz, T, false, __double_as_longlong(I.fk[FK_MZERO]));
-  double2* other = res == A ? B : A;
+  __syncthreads();
+  line_max(A, nr, nr, Nz, top);
+  const int r0 = fx_last_tile(0, L * Nz, I.passz);
+  double2* res = sm + r0;
+  fx_fft<false>(RawLd{0, 1, nr, LineIn{bits, top}}, DoubleTileSt{r0, 1, nr, LineOut{bits, halvings, top}}, 0, L * Nz, nr, 1,
+                nr, Nz, I.passz, T);
+  __syncthreads();
   const double* __restrict__ fi = I.tri_inv + kx;
   const double* __restrict__ fm = I.tri_m + kx;
   const double* __restrict__ fc = I.tri_c + kx;
@@ -726,15 +789,38 @@ k_zsolve(ChlMap map) {
       res[(j - lo) + (size_t)kz * nr] = d;
     }
   }
-  double2* out = fft_smem(res, other, nr, 1, nr, Nz, T, true, __double_as_longlong(I.fk[FK_MZERO]));
-  for (int w = t; w < nr * Nz; w += bd) {
-    const int l = w % nr, kz = w / nr;
-    spec[(size_t)(lo + l) * ps + (size_t)kz * Nxh] = out[l + (size_t)kz * nr];
-  }
+  __syncthreads();
+  line_max(res, nr, nr, Nz, top);
+  fx_fft<true>(RawLd{r0, 1, nr, LineIn{bits, top}}, RowSt{spec + (size_t)lo * ps, ps, (size_t)Nxh, LineOut{bits, halvings, top}},
+               r0, L * Nz - r0, nr, 1, nr, Nz, I.passz, T);
   cl.sync();   // no CTA leaves while another may still read its lane values
 }
 
 // ------------------------------------------------------------ inverse x -> pressure field
+// the packed line of two real rows from their half-spectra pa, pb (stored at
+// kx and Nxh + kx): element kx is pa + i pb, element Nx - kx conj(pa) + i conj(pb)
+struct PackLd {
+  int pitch, Nx; LineIn in;
+  __device__ __forceinline__ fx2 operator()(int r, int e) const {
+    const bool lo = e <= Nx / 2;
+    const double2* q = smem_d2() + r * pitch + (lo ? e : Nx - e);
+    const int s = in.exponent(r);
+    const fx2 a = fx2_from(q[0], s), b = fx2_from(q[Nx / 2 + 1], s);
+    return lo ? make_longlong2(a.x - b.y, a.y + b.x) : make_longlong2(a.x + b.y, b.x - a.y);
+  }
+};
+// the two real rows (planes k0, k0 + 1) of a packed line
+struct RealSt {
+  const ChlInst* I; double* p; int g0; LineOut out;
+  __device__ __forceinline__ void operator()(int r, int i, fx2 v) const {
+    const unsigned g = g0 + r, h = I->Nz / 2;
+    const int jc = 1 + (int)(g / h), k0 = 2 * (int)(g % h);
+    const double2 z = out(r, v);
+    p[cidx(*I, i, jc, k0)] = z.x;
+    p[cidx(*I, i, jc, k0 + 1)] = z.y;
+  }
+};
+
 __global__ void __launch_bounds__(256)
 k_fftx_inv(ChlMap map, int dst, int xmb) {
   chl_pdl_wait();
@@ -746,31 +832,26 @@ k_fftx_inv(ChlMap map, int dst, int xmb) {
   const int CR = chl_fftx_rows(Nx, nrow, xmb);
   const int g0 = lb * CR;
   const int cr_n = min(CR, nrow - g0);
-  double2* A = sm;
-  double2* B = sm + CR * Nx;
-  double* T = reinterpret_cast<double*>(sm + 2 * CR * Nx);   // pass table
-  stage_twiddles(T, I.twx, chl_tw_len(Nx));
-  for (int w = threadIdx.x; w < cr_n * Nx; w += blockDim.x) {
-    const int cr = w / Nx, kx = w - cr * Nx;
-    const int g = g0 + cr;
-    const int jc = 1 + g / (Nz / 2), k0 = 2 * (g % (Nz / 2));
-    const bool lo = kx <= Nx / 2;
-    const int kk = lo ? kx : Nx - kx;
-    const double2 pa = I.spec[((size_t)jc * Nz + k0) * Nxh + kk];
-    const double2 pb = I.spec[((size_t)jc * Nz + k0 + 1) * Nxh + kk];
-    A[cr * Nx + kx] = lo ? make_double2(pa.x - pb.y, pa.y + pb.x)
-                         : make_double2(pa.x + pb.y, pb.x - pa.y);
+  const int A = 0, B = CR * (Nx + 2), T = B + CR * Nx;       // tiles, twiddles
+  unsigned* hi = reinterpret_cast<unsigned*>(sm + T + I.lenx);
+  stage_twiddles(smem_tw() + T, I.twx, I.lenx);
+  for (int r = threadIdx.x; r < CR; r += blockDim.x) hi[r] = 0u;
+  __syncthreads();
+  const SmallDiv byNxh(Nxh);
+  for (int w0 = 0; w0 < cr_n * Nxh; w0 += blockDim.x) {
+    const int w = min(w0 + (int)threadIdx.x, cr_n * Nxh - 1);
+    const int cr = byNxh.div(w), kx = w - cr * Nxh;
+    const unsigned g = g0 + cr;
+    const int jz = (int)(g / (unsigned)(Nz / 2)), jc = 1 + jz, k0 = 2 * ((int)g - jz * (Nz / 2));
+    const double2 pa = I.spec[((size_t)jc * Nz + k0) * Nxh + kx];
+    const double2 pb = I.spec[((size_t)jc * Nz + k0 + 1) * Nxh + kx];
+    sm[cr * (Nx + 2) + kx] = pa;
+    sm[cr * (Nx + 2) + Nxh + kx] = pb;
+    fold_line(hi, cr, max(abshi2(pa), abshi2(pb)));
   }
-  double2* res = fft_smem(A, B, cr_n, Nx, 1, Nx, T, true, __double_as_longlong(I.fk[FK_MZERO]));
-  double* out = dst == 0 ? I.p : I.P;
-  for (int w = threadIdx.x; w < cr_n * Nx; w += blockDim.x) {
-    const int cr = w / Nx, i = w - cr * Nx;
-    const int g = g0 + cr;
-    const int jc = 1 + g / (Nz / 2), k0 = 2 * (g % (Nz / 2));
-    const double2 z = res[cr * Nx + i];
-    out[cidx(I, i, jc, k0)] = z.x;
-    out[cidx(I, i, jc, k0 + 1)] = z.y;
-  }
+  const int bits = I.bitsx - 1;      // an element is a sum of two components
+  const RealSt last{&I, dst == 0 ? I.p : I.P, g0, LineOut{bits, I.passx - 1, hi}};
+  fx_fft<true>(PackLd{Nx + 2, Nx, LineIn{bits, hi}}, last, A, B, cr_n, Nx, 1, Nx, I.passx, T);
 }
 
 // ------------------------------------------------------------ velocity correction
@@ -855,19 +936,24 @@ __global__ void k_pghost(ChlMap map) {
 }
 
 extern "C" {
-// two ping-pong tiles plus the pass table (twz: the longest z pass table
-// of the launch's instances, in doubles)
+// two ping-pong tiles (an x line's raw half-spectra take Nx + 2 elements), the
+// twiddles (twz: the longest z table of the launch's instances) and, for the
+// x lines, their largest components
 size_t chl_smem_fftx(int Nx, int nrow, int xmb) {
-  return (size_t)2 * chl_fftx_rows(Nx, nrow, xmb) * Nx * sizeof(double2) + chl_tw_bytes(chl_tw_len(Nx));
+  const size_t rows = chl_fftx_rows(Nx, nrow, xmb);
+  return rows * (2 * (size_t)Nx + 2) * sizeof(double2) + (size_t)chl_twf_len(Nx) * sizeof(int4) + rows * sizeof(unsigned);
 }
-size_t chl_smem_fftz(int maxNz, int zcw, int twz) { return (size_t)2 * zcw * maxNz * sizeof(double2) + chl_tw_bytes(twz); }
-// kx columns staged per z-transform block: 16, halved while two Nz x cols
-// complex tiles would exceed the 227 KB a block may use, and halved (down
+size_t chl_smem_fftz(int maxNz, int zcw, int twz) {
+  return (size_t)2 * zcw * maxNz * sizeof(double2) + (size_t)twz * sizeof(int4);
+}
+// kx columns staged per z-transform block: 8 (at 256x96x192 two, four, eight
+// and sixteen columns take 48, 48, 46 and 57 us per launch), halved while two
+// Nz x cols complex tiles would exceed the 227 KB a block may use, and halved (down
 // to 2) while the grid over all `ncols` columns would have fewer than
 // min_blocks blocks (CHL_FFT_MIN_BLOCKS, about four per SM, unless the
 // tuner chose another)
 int chl_fftz_cols(int maxNz, long ncols, int min_blocks, int twz) {
-  int c = 16;
+  int c = 8;
   while (c > 1 && chl_smem_fftz(maxNz, c, twz) > (size_t)227 * 1024) c /= 2;
   while (c > 2 && (ncols + c - 1) / c < min_blocks) c /= 2;
   return c;
@@ -875,13 +961,17 @@ int chl_fftz_cols(int maxNz, long ncols, int min_blocks, int twz) {
 int chl_fft_setup(size_t smx, size_t smz, size_t smt) {
   cudaError_t e1 = cudaFuncSetAttribute(k_div_fftx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx);
   cudaError_t e2 = cudaFuncSetAttribute(k_fftx_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx);
-  cudaError_t e3 = cudaFuncSetAttribute(k_fftz, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz);
+  cudaError_t e3 = cudaFuncSetAttribute(k_fftz<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz);
+  if (e3 == cudaSuccess) e3 = cudaFuncSetAttribute(k_fftz<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz);
   cudaError_t e4 = smt ? cudaFuncSetAttribute(k_tri_staged, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smt)
                        : cudaSuccess;
   return (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess || e4 != cudaSuccess) ? 1 : 0;
 }
 void chl_launch_div_fftx(const ChlMap& m, int nb, int nt, size_t smem, int s_in, int mode, int xmb, cudaStream_t st) { chl_launch_pdl(k_div_fftx, dim3(nb), dim3(nt), smem, st, m, s_in, mode, xmb); }
-void chl_launch_fftz(const ChlMap& m, int nb, int nt, size_t smem, int inv, int zcw, cudaStream_t st) { chl_launch_pdl(k_fftz, dim3(nb), dim3(nt), smem, st, m, inv, zcw); }
+void chl_launch_fftz(const ChlMap& m, int nb, int nt, size_t smem, int inv, int zcw, cudaStream_t st) { 
+  if (inv) chl_launch_pdl(k_fftz<true>, dim3(nb), dim3(nt), smem, st, m, zcw);
+  else chl_launch_pdl(k_fftz<false>, dim3(nb), dim3(nt), smem, st, m, zcw);
+}
 // smem > 0: the staged form with TRI_W-mode blocks (chl_tri_modes_per_block)
 void chl_launch_tri(const ChlMap& m, int nb, size_t smem, cudaStream_t st) {
   if (smem) chl_launch_pdl(k_tri_staged, dim3(nb), dim3(TRI_W), smem, st, m);
@@ -909,8 +999,8 @@ size_t chl_smem_zsolve(int Nx, int Ny, int Nz) {
   const int P = chl_tri_lanes((long)Nz * Nxh, Ny);
   if (P != 1 && P != 2 && P != 4 && P != 8) return 0;
   const int L = (Ny + P - 1) / P;
-  const size_t b = (size_t)2 * L * Nz * sizeof(double2) + chl_tw_bytes(chl_tw_len(Nz)) + (size_t)4 * Nz * sizeof(double2) +
-                   (size_t)2 * Nz * sizeof(double);
+  const size_t b = (size_t)2 * L * Nz * sizeof(double2) + (size_t)chl_twf_len(Nz) * sizeof(int4) +
+                   (size_t)4 * Nz * sizeof(double2) + (size_t)2 * Nz * sizeof(double) + (size_t)L * sizeof(unsigned);
   return b <= (size_t)227 * 1024 ? b : 0;
 }
 int chl_zsolve_setup(size_t smem) {

@@ -25,6 +25,7 @@ __device__ __forceinline__ int fx_exp(unsigned hi) {
   const int E = max((int)(hi >> 20), 64);
   return E - 1022 - BITS;
 }
+__device__ __forceinline__ int fx_line_exp(unsigned hi, int bits) { return max((int)(hi >> 20), 64) - 1022 - bits; }
 __device__ __forceinline__ bool fx_bad(unsigned hi) { return hi >= 0x7FF00000u; }
 
 // x as F 2^e, rounded toward zero

@@ -217,10 +217,54 @@ struct Arena {
   size_t take(size_t bytes) { size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; }
 };
 
-// Pass table of the length-N Stockham FFT (layout in chl_fft.cu): per pass
-// with twiddles and butterfly class jm, the twiddles w_r = C + iS =
-// exp(-2 pi i m/N), m = jm r N/(Ns R), each as sigma (C or S, the larger in
-// magnitude) and m (S/C or C/S), and the butterfly's combined scales.
+// Table of the length-N transforms (layout in chl_fft.cu): per pass {R, Ns,
+// 2^32/Ns, 2^32/(N/R)} (the reciprocals rounded up, 0 for 1), then per pass
+// after the first and r = 1..R-1 the twiddles w = exp(-2 pi i jm r/(Ns R)), jm = 0..Ns-1, as the
+// words (high, low >> 1) of cos 2^63 and of sin 2^63, 2^63 - 1 at most.
+std::vector<int4> fft_table(int N) {
+  std::vector<int4> t;
+  const long double pi2 = 2.0L * acosl(-1.0L);
+  auto fixed = [](long double v) {
+    const long double one = 9223372036854775808.0L;   // 2^63
+    return v >= 1.0L ? 0x7FFFFFFFFFFFFFFFLL : (v <= -1.0L ? -0x7FFFFFFFFFFFFFFFLL : llrintl(v * one));
+  };
+  int Ns = 1, rem = N;
+  auto recip = [](int d) { return (int)(unsigned)(0x100000000ULL / (unsigned)d + (0x100000000ULL % (unsigned)d != 0)); };
+  while (rem > 1) {
+    const int R = chl_fft_radix(rem);
+    t.push_back(make_int4(R, Ns, recip(Ns), recip(N / R)));
+    Ns *= R; rem /= R;
+  }
+  Ns = 1; rem = N;
+  while (rem > 1) {
+    const int R = chl_fft_radix(rem);
+    if (Ns > 1)
+      for (int r = 1; r < R; ++r)
+        for (int jm = 0; jm < Ns; ++jm) {
+          const long double a = pi2 * (long double)((long)jm * r % ((long)Ns * R)) / ((long double)Ns * R);
+          const long long c = fixed(cosl(a)), s = fixed(-sinl(a));
+          t.push_back(make_int4((int)(c >> 32), (int)((unsigned)c >> 1), (int)(s >> 32), (int)((unsigned)s >> 1)));
+        }
+    Ns *= R; rem /= R;
+  }
+  return t;
+}
+
+// FP64 pass table of a length-N Stockham FFT in tangent form
+// (chl_fft_pass_table): per pass with twiddles and butterfly class jm, the
+// twiddles w_r = C + iS = exp(-2 pi i m/N), m = jm r N/(Ns R), each as sigma
+// (C or S, the larger in magnitude) and m (S/C or C/S), and the butterfly's
+// combined scales.
+constexpr int CHL_TW_F = 7;
+int chl_tw_len(int N) {
+  int Ns = 1, rem = N, len = 0;
+  while (rem > 1) {
+    const int R = chl_fft_radix(rem);
+    if (Ns > 1) len += CHL_TW_F * Ns;
+    Ns *= R; rem /= R;
+  }
+  return len;
+}
 std::vector<double> fft_pass_table(int N) {
   std::vector<double> t((size_t)chl_tw_len(N));
   const double pi = 4.0 * std::atan(1.0);
@@ -282,7 +326,7 @@ struct chl_handle {
   int* d_off[NMAP] = {};
   int nblk[NMAP] = {};
   size_t smem_x = 0, smem_z = 0, smem_t = 0;
-  int zcw = 16;                       // kx columns per z-transform block
+  int zcw = 8;                        // kx columns per z-transform block
   int tx = 256, tz = 256;             // threads of the x and z transform blocks
   // projection tile shapes (chl_autotune): block-count targets of the x and
   // z transforms and the tridiagonal form: 0 row-batched, 1 staged, 2 the
@@ -293,10 +337,10 @@ struct chl_handle {
   bool zsolve = false;                // the fused form is in use
   int zlanes = 1;                     // its cluster size
   size_t smem_zs = 0;
-  int twz = 0;                        // longest z pass table of the instances (doubles)
+  int twz = 0;                        // longest z transform table of the instances
   bool epair = false;                 // edges as x-pair sums (k_edges_pair): every Nx <= 256
   int tb_epair = 256;                 // its block: the largest Nx rounded up to a power of two, >= 64
-  int tb_pt = 256;                    // threads per block of the point maps (stencils, updates)
+  int tb_pt = 128;                    // threads per block of the point maps (stencils, updates)
   bool tri_scan = false;              // some instance splits its tridiagonal columns (chl_tri_lanes)
   int LES_model = 0, wall_model = 0, any_mass = 0;
   float* d_mlp_theta = nullptr;       // learned wall model parameters (shared)
@@ -347,7 +391,7 @@ static int upload_consts(chl_handle* h, Inst& I) {
   size_t o_rdxcs = A.take(8 * (Nx + 3)), o_rdycs = A.take(8 * (Ny + 2)), o_rdzcs = A.take(8 * (Nz + 3));
   size_t o_rdxfs = A.take(8 * (Nx + 3)), o_rdyfs = A.take(8 * (Ny + 2)), o_rdzfs = A.take(8 * (Nz + 3));
   size_t o_csd = A.take(8 * (Ny + 2)), o_dw = A.take(8 * (Ny + 2));
-  size_t o_twx = A.take(8 * (size_t)chl_tw_len(Nx)), o_twz = A.take(8 * (size_t)chl_tw_len(Nz));
+  size_t o_twx = A.take(16 * (size_t)chl_twf_len(Nx)), o_twz = A.take(16 * (size_t)chl_twf_len(Nz));
   size_t o_ti = A.take(8 * ntri), o_tm = A.take(8 * ntri), o_tc = A.take(8 * ntri);
   // state
   size_t o_U[3], o_V[3], o_W[3], o_F1[3], o_Fp[3];
@@ -419,7 +463,9 @@ static int upload_consts(chl_handle* h, Inst& I) {
   D.rdxcs = P(o_rdxcs) + 1; D.rdycs = P(o_rdycs); D.rdzcs = P(o_rdzcs) + 1;
   D.rdxfs = P(o_rdxfs) + 1; D.rdyfs = P(o_rdyfs); D.rdzfs = P(o_rdzfs) + 1;
   D.smag_csdelta = P(o_csd); D.smag_dwall = P(o_dw);
-  D.twx = (const double*)(base + o_twx); D.twz = (const double*)(base + o_twz);
+  D.twx = (const int4*)(base + o_twx); D.twz = (const int4*)(base + o_twz);
+  D.lenx = chl_twf_len(Nx); D.lenz = chl_twf_len(Nz); D.passx = chl_fft_passes(Nx); D.passz = chl_fft_passes(Nz);
+  D.bitsx = chl_fft_bits(Nx); D.bitsz = chl_fft_bits(Nz);
   D.tri_inv = P(o_ti); D.tri_m = P(o_tm); D.tri_c = P(o_tc);
   for (int s = 0; s < 3; ++s) { D.U[s] = P(o_U[s]); D.V[s] = P(o_V[s]); D.W[s] = P(o_W[s]); D.F1[s] = P(o_F1[s]); D.Fp[s] = P(o_Fp[s]); }
   D.nut = P(o_nut); D.S = P(o_S);
@@ -488,9 +534,9 @@ static int upload_consts(chl_handle* h, Inst& I) {
   CK(put(o_rdxfs, times(c.rdxf, fs))); CK(put(o_rdyfs, times(c.rdyf, fs))); CK(put(o_rdzfs, times(c.rdzf, fs)));
   CK(put(o_csd, c.csdelta)); CK(put(o_dw, c.dwall));
   {
-    const std::vector<double> tx = fft_pass_table(Nx), tz = fft_pass_table(Nz);
-    if (!tx.empty()) CK(cudaMemcpy(base + o_twx, tx.data(), 8 * tx.size(), cudaMemcpyHostToDevice));
-    if (!tz.empty()) CK(cudaMemcpy(base + o_twz, tz.data(), 8 * tz.size(), cudaMemcpyHostToDevice));
+    const std::vector<int4> tx = fft_table(Nx), tz = fft_table(Nz);
+    if (!tx.empty()) CK(cudaMemcpy(base + o_twx, tx.data(), 16 * tx.size(), cudaMemcpyHostToDevice));
+    if (!tz.empty()) CK(cudaMemcpy(base + o_twz, tz.data(), 16 * tz.size(), cudaMemcpyHostToDevice));
   }
   // Thomas factors per mode: denominators of the elimination of
   // Dyy + kxx + kzz (the zgtsv system of projection.f90:97-110), with the
@@ -537,7 +583,7 @@ static int build_maps(chl_handle* h) {
     modes += (long)I.c.Nz * I.c.Nxh;
   }
   h->twz = 0;
-  for (auto& I : h->in) h->twz = std::max(h->twz, chl_tw_len(I.c.Nz));
+  for (auto& I : h->in) h->twz = std::max(h->twz, chl_twf_len(I.c.Nz));
   h->zcw = chl_fftz_cols(mz, zcols, h->z_min_blocks, h->twz);
   h->tz = chl_fft_threads(h->zcw, mz);
   h->tx = 64;
