@@ -157,7 +157,6 @@ __device__ __forceinline__ void fx_pass_any(const LD& ld, const ST& st, const Sm
 // at 256x96x192 the four transforms of a stage take 275 us with all
 // conversions on the integer pipe, 262 us like this and 332 us with all of
 // them on the FP64 pipe.
-__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }   // -1022 <= e <= 1023
 struct LineIn {
   int bits; const unsigned* hi;
   __device__ __forceinline__ int exponent(int r) const { return fx_line_exp(hi[r], bits); }

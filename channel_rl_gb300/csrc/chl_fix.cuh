@@ -53,6 +53,9 @@ __device__ __forceinline__ double fx_to(fx f, int e) {
   return __longlong_as_double((long long)(r | ((unsigned long long)f & 0x8000000000000000ULL)));
 }
 
+// 2^e as a double, -1022 <= e <= 1023
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+
 // (a b) >> 64, low by less than three units, for |a| < 2^62 and |b| < 2^63 (or
 // |a| < 2^63 and 0 <= b < 2^63):
 // the product of the high words plus the cross terms, whose low words enter

@@ -72,7 +72,7 @@ namespace {
 constexpr double RK_T[3] = {8.0 / 15.0, 2.0 / 3.0, 1.0};
 
 enum { M_PT, M_EDGE, M_FULL, M_DSMF, M_WALL, M_PLANE, M_FFTX, M_FFTZ, M_TRI, M_MINABS, M_ROWS, M_MLP, M_WALLN,
-       M_ZPLANE, M_ZSOLVE, M_EPAIR, M_FULLZ2, M_FULLX2, M_FLUX, NMAP };
+       M_ZPLANE, M_ZSOLVE, M_EPAIR, M_FULLZ2, M_FULLX2, M_FLUX, M_MARCH, NMAP };
 constexpr int MLP_NPARAM = 4545;
 
 // Grid constants of one instance (host, FP64), in the device index
@@ -625,6 +625,7 @@ static int build_maps(chl_handle* h) {
         case M_FULLZ2: b = cdiv((long)Nx * (Ny + 2) * (Nz / 2), h->tb_pt); break;   // z planes in pairs (Nz even)
         case M_FULLX2: b = cdiv((long)(Nx / 2) * (Ny + 2) * Nz, h->tb_pt); break;   // x points in pairs (Nx even)
         case M_FLUX: b = cdiv((long)Nx * (Ny + 1) * cdiv(Nz, chl_planes(Nx, Ny, Nz)), CHL_FLUX_THREADS); break;
+        case M_MARCH: b = cdiv((long)Nx * Ny * cdiv(Nz, chl_planes(Nx, Ny, Nz)), CHL_FLUX_THREADS); break;
         case M_DSMF: b = Ny * dsm_npart(Nx, Ny, Nz); break;
         case M_WALL: b = cdiv(2L * Nx * Nz, 256); break;
         case M_PLANE: b = cdiv((long)Nx * Nz, 256); break;
@@ -688,7 +689,7 @@ static int enqueue_sgs(chl_handle* h, int s, bool with_wm, int stage = 0) {
                                  h->epair ? h->tb_epair : 0, st));
     KL("centre_strain", chl_launch_centre(h->map(M_PT), h->nblk[M_PT], s, 0, h->epair, st));
   } else if (h->LES_model == CHL_LES_AMD) {
-    KL("amd", chl_launch_amd(h->map(M_PT), h->nblk[M_PT], s, with_wm ? 1 : 0, st));
+    KL("amd", chl_launch_amd(h->map(M_MARCH), h->nblk[M_MARCH], s, with_wm ? 1 : 0, st));
   } else if (h->LES_model == CHL_LES_VREMAN) {
     KL("vreman", chl_launch_vreman(h->map(M_PT), h->nblk[M_PT], s, with_wm ? 1 : 0, st));
   }

@@ -126,47 +126,127 @@ __device__ __forceinline__ unsigned write_nut_rows(const ChlInst& I, const doubl
 
 }  // namespace
 
-__global__ void __launch_bounds__(256)
+// One's-complement magnitudes of the high words, or-ed: the bit length of the
+// result is that of the largest of them.
+__device__ __forceinline__ void top_or(unsigned& m, fx a) {
+  const int h = (int)(a >> 32);
+  m |= (unsigned)(h ^ (h >> 31));
+}
+// a 2^s for s of either sign (toward minus infinity)
+__device__ __forceinline__ fx scale2(fx a, int s) { return (a << max(s, 0)) >> max(-s, 0); }
+
+// AMD in fixed point.  As FP64 code this kernel issued 114 FP64 instructions
+// per point (0.97 ms per launch at 256x96x192, the FP64 pipe 90 % busy).  The
+// edge differences are exact integers from the fixed-point copies (k_fix);
+// each point scales its fifteen by their largest, so that the products keep
+// 54 bits or more of the largest product, and forms the derivatives, D and
+// the a_ij there.  N and the division are FP64 (17 instructions).
+// A thread marches through chl_planes planes: what planes share (pair sums of
+// U and V, differences of W) is carried.
+__global__ void __launch_bounds__(CHL_FLUX_THREADS, 4)   // 128 registers: 2, 3, 4, 5 blocks per SM take 417, 321, 299, 307 us
 k_amd(ChlMap map, int s_in, int use_wm) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
-  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
+  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz, M = chl_planes(Nx, Ny, Nz);
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  const bool valid = t < (unsigned)(Nx * Ny * Nz);
-  // lanes past the end repeat the last centre and write nothing
-  const ChlIdx p = chl_split(valid ? t : (unsigned)(Nx * Ny * Nz) - 1u, Nx, Ny);
-  const int i = p.i, jc = 1 + p.j, k = p.k;
-  const Grad g = gradients(I, I.U[s_in], I.V[s_in], I.W[s_in], i, jc, k);
-  // centre strain: diagonal S_ii; 8 S_ij off the diagonal
-  const double s11 = g.dux * g.rxc, s22 = g.dvy * g.ryc, s33 = g.dwz * g.rzc;
-  const double t12 = g.dUy + g.dVx, t13 = g.dUz + g.dWx, t23 = g.dVz + g.dWy;
-  // grid-scaled centre differences, 4 x: Yu, Zu, Xv, Zv, Xw, Yw
-  const double Yu = g.uyL + g.uyH, Zu = g.uzL + g.uzH, Xv = g.vxL + g.vxR;
-  const double Zv = g.vzL + g.vzH, Xw = g.wxL + g.wxR, Yw = g.wyL + g.wyH;
-  // Numerator and denominator are both formed 16 x (their ratio is what
-  // counts), which takes the 1/16 of the 4 x off-diagonal terms out.
-  // denominator: sum of squared centre derivatives (the off-diagonal ones are 4 x)
-  double q = g.dUy * g.dUy;
-  q = fma(g.dUz, g.dUz, q); q = fma(g.dVx, g.dVx, q); q = fma(g.dVz, g.dVz, q);
-  q = fma(g.dWx, g.dWx, q); q = fma(g.dWy, g.dWy, q);
-  double D = s11 * s11; D = fma(s22, s22, D); D = fma(s33, s33, D);
-  D = fma(16.0, D, q);                                   // 16 x
-  // numerator: sum_k (d^_k u_i)(d^_k u_j) S_ij with the reference's product
-  // forms; the third mixed term of each S_ij is the edge product averaged.
-  const double u4 = 4.0 * g.dux, v4 = 4.0 * g.dvy, w4 = 4.0 * g.dwz;
-  const double a11 = fma(u4, u4, fma(Yu, Yu, Zu * Zu));   // 16 x
-  const double a22 = fma(v4, v4, fma(Xv, Xv, Zv * Zv));
-  const double a33 = fma(w4, w4, fma(Xw, Xw, Yw * Yw));
-  const double a12 = fma(0.5, fma(g.uzL, g.vzL, g.uzH * g.vzH), fma(Xv, g.dux, Yu * g.dvy));
-  const double a13 = fma(0.5, fma(g.uyL, g.wyL, g.uyH * g.wyH), fma(Xw, g.dux, Zu * g.dwz));
-  const double a23 = fma(0.5, fma(g.vxL, g.wxL, g.vxR * g.wxR), fma(Yw, g.dvy, Zv * g.dwz));
-  double N = a11 * s11;
-  N = fma(a22, s22, N); N = fma(a33, s33, N);
-  N = fma(a12, t12, N); N = fma(a13, t13, N); N = fma(a23, t23, N);
-  const double v = (-0.3 * N) / D;
-  if (valid) I.S[cidx(I, i, jc, k)] = v;
-  chl_line_max(I.nmax, (unsigned)(k * Ny + jc - 1), Ny, 1, write_nut_rows(I, I.U[s_in], i, jc, k, v, use_wm, valid));
+  const ChlIdx p = chl_split(t, Nx, Ny);
+  const int i = p.i, jc = 1 + p.j, k0 = p.k * M;
+  const int im = wrap(i - 1, Nx), ip = wrap(i + 1, Nx);
+  const fx* __restrict__ U = I.X[0];
+  const fx* __restrict__ V = I.X[1];
+  const fx* __restrict__ W = I.X[2];
+#define UC(ii, jj, kk) LDG(U + cidx(I, ii, jj, kk))
+#define WC(ii, jj, kk) LDG(W + cidx(I, ii, jj, kk))
+#define VV(ii, jj, kk) LDG(V + vidx(I, ii, jj, kk))
+  // reciprocal spacings with one exponent er
+  const int el = I.eyf[jc - 1], eh = I.eyf[jc], ec = I.eyc[jc];
+  const int er = max(max(max(el, eh), max(ec, I.exf)), max(max(I.exc, I.ezf), I.ezc));
+  const fx ryl = LDG(I.fxryf + jc - 1) >> min(63, er - el), ryh = LDG(I.fxryf + jc) >> min(63, er - eh);
+  const fx ryc = LDG(I.fxryc + jc) >> min(63, er - ec);
+  const fx rxf = LDG(I.fxrxf + i - 1) >> min(63, er - I.exf), rxc = LDG(I.fxrxc + i) >> min(63, er - I.exc);
+  const unsigned* vm = chl_vmax(I, s_in);
+  const int eu = fx_exp<61>(vm[0]), ev = fx_exp<61>(vm[1]), ew = fx_exp<61>(vm[2]);
+  const bool bad = fx_bad(vm[0]) || fx_bad(vm[1]) || fx_bad(vm[2]);
+  const int ks = min(k0, Nz - 1), kb = ks == 0 ? Nz - 1 : ks - 1;    // lanes past the last plane repeat it
+  fx um = UC(im, jc, ks), u0 = UC(i, jc, ks);
+  fx vm0 = VV(i, jc - 1, ks), v0 = VV(i, jc, ks);
+  fx wm = WC(i, jc, kb);
+  fx uzL = (um + u0) - (UC(im, jc, kb) + UC(i, jc, kb));
+  fx vzL = (vm0 + v0) - (VV(i, jc - 1, kb) + VV(i, jc, kb));
+  fx wxl = wm - WC(im, jc, kb), wxr = WC(ip, jc, kb) - wm;          // W's x and y differences, plane below
+  fx wyl = wm - WC(i, jc - 1, kb), wyh = WC(i, jc + 1, kb) - wm;
+  unsigned hi = 0u;
+  for (int q = 0; q < M; ++q) {
+    const int k = min(k0 + q, Nz - 1), kp = k + 1 == Nz ? 0 : k + 1;
+    const bool valid = k0 + q < Nz;
+    const fx up_m = UC(im, jc, kp), up_0 = UC(i, jc, kp), vp_m = VV(i, jc - 1, kp), vp_0 = VV(i, jc, kp);
+    const fx w0 = WC(i, jc, k), wim = WC(im, jc, k), wip = WC(ip, jc, k);
+    const fx wjm = WC(i, jc - 1, k), wjp = WC(i, jc + 1, k);
+    const fx us = um + u0, vs = vm0 + v0;
+    fx uyL = us - (UC(im, jc - 1, k) + UC(i, jc - 1, k)), uyH = (UC(im, jc + 1, k) + UC(i, jc + 1, k)) - us;
+    fx vxL = vs - (VV(im, jc - 1, k) + VV(im, jc, k)), vxR = (VV(ip, jc - 1, k) + VV(ip, jc, k)) - vs;
+    const fx uzN = (up_m + up_0) - us, vzN = (vp_m + vp_0) - vs;
+    const fx xl = w0 - wim, xr = wip - w0, yl = w0 - wjm, yh = wjp - w0;
+    fx wxL = wxl + xl, wxR = wxr + xr, wyL = wyl + yl, wyH = wyh + yh;
+    fx dux = u0 - um, dvy = v0 - vm0, dwz = w0 - wm;
+    // scale: |x| < 2^60 in units of 2^et
+    unsigned mu = 0u, mv = 0u, mw = 0u;
+    top_or(mu, dux); top_or(mu, uyL); top_or(mu, uyH); top_or(mu, uzL); top_or(mu, uzN);
+    top_or(mv, dvy); top_or(mv, vxL); top_or(mv, vxR); top_or(mv, vzL); top_or(mv, vzN);
+    top_or(mw, dwz); top_or(mw, wxL); top_or(mw, wxR); top_or(mw, wyL); top_or(mw, wyH);
+    const int et = max(max(eu + 64 - __clz((int)mu), ev + 64 - __clz((int)mv)), ew + 64 - __clz((int)mw)) - 60;
+    const int su = eu - et, sv = ev - et, sw = ew - et;
+    dux = scale2(dux, su); uyL = scale2(uyL, su); uyH = scale2(uyH, su);
+    const fx uL = scale2(uzL, su), uH = scale2(uzN, su);
+    dvy = scale2(dvy, sv); vxL = scale2(vxL, sv); vxR = scale2(vxR, sv);
+    const fx vL = scale2(vzL, sv), vH = scale2(vzN, sv);
+    dwz = scale2(dwz, sw); wxL = scale2(wxL, sw); wxR = scale2(wxR, sw); wyL = scale2(wyL, sw); wyH = scale2(wyH, sw);
+    uzL = uzN; vzL = vzN; wxl = xl; wxr = xr; wyl = yl; wyh = yh;
+    um = up_m; u0 = up_0; vm0 = vp_m; v0 = vp_0; wm = w0;
+    // grid-scaled centre differences, 4 x
+    const fx Yu = uyL + uyH, Zu = uL + uH, Xv = vxL + vxR, Zv = vL + vH, Xw = wxL + wxR, Yw = wyL + wyH;
+    // derivatives, 4 x, scaled anew: the spacings differ by up to the
+    // stretching of the grid (units 2^(et + er + 64 - sd))
+    const fx rzf = LDG(I.fxrzf + k - 1) >> min(63, er - I.ezf), rzc = LDG(I.fxrzc + k) >> min(63, er - I.ezc);
+    fx s11 = 4 * fx_mul(dux, rxc), s22 = 4 * fx_mul(dvy, ryc), s33 = 4 * fx_mul(dwz, rzc);
+    fx dUy = fx_mul(uyL, ryl) + fx_mul(uyH, ryh), dWy = fx_mul(wyL, ryl) + fx_mul(wyH, ryh);
+    fx dUz = fx_mul(Zu, rzf), dVz = fx_mul(Zv, rzf), dVx = fx_mul(Xv, rxf), dWx = fx_mul(Xw, rxf);
+    unsigned md = 0u;
+    top_or(md, s11); top_or(md, s22); top_or(md, s33);
+    top_or(md, dUy); top_or(md, dUz); top_or(md, dVx); top_or(md, dVz); top_or(md, dWx); top_or(md, dWy);
+    const int sd = __clz((int)md) - 3;     // |x| < 2^61; a derivative is below 2^61 already
+    s11 <<= sd; s22 <<= sd; s33 <<= sd;
+    dUy <<= sd; dUz <<= sd; dVx <<= sd; dVz <<= sd; dWx <<= sd; dWy <<= sd;
+    // D, 16 x (2^64 units of the derivatives' square); 12 makes up for nine products
+    const fx D = (fx_mul(s11, s11) + fx_mul(s22, s22) + fx_mul(s33, s33) + 12) +
+                 (fx_mul(dUy, dUy) + fx_mul(dUz, dUz) + fx_mul(dVx, dVx)) +
+                 (fx_mul(dVz, dVz) + fx_mul(dWx, dWx) + fx_mul(dWy, dWy));
+    // a_ii 16 x in 2^63 units, a_ij 4 x in 2^61 units of the differences' square:
+    // sum_k (d^_k u_i)(d^_k u_j) with the reference's product forms; the third
+    // mixed term of each is the edge product averaged
+#define SQ(a) fx_mul_shr<63>(a, a)
+    const fx a11 = SQ(4 * dux) + SQ(Yu) + SQ(Zu), a22 = SQ(4 * dvy) + SQ(Xv) + SQ(Zv), a33 = SQ(4 * dwz) + SQ(Xw) + SQ(Yw);
+#undef SQ
+    const fx a12 = fx_mul_shr<61>(Xv, dux) + fx_mul_shr<61>(Yu, dvy) + fx_mul_shr<62>(uL, vL) + fx_mul_shr<62>(uH, vH);
+    const fx a13 = fx_mul_shr<61>(Xw, dux) + fx_mul_shr<61>(Zu, dwz) + fx_mul_shr<62>(uyL, wyL) + fx_mul_shr<62>(uyH, wyH);
+    const fx a23 = fx_mul_shr<61>(Yw, dvy) + fx_mul_shr<61>(Zv, dwz) + fx_mul_shr<62>(vxL, wxL) + fx_mul_shr<62>(vxR, wxR);
+    // N = sum a_ij S_ij, 64 x (S_ii 4 x, a_ij 4 x with S_ij 8 x in 2^-2 units of a_ii)
+    double Nd = fx_to(a11, 0) * fx_to(s11, 0);
+    Nd = fma(fx_to(a22, 0), fx_to(s22, 0), Nd);
+    Nd = fma(fx_to(a33, 0), fx_to(s33, 0), Nd);
+    Nd = fma(fx_to(a12, 0), fx_to(dUy + dVx, 0), Nd);
+    Nd = fma(fx_to(a13, 0), fx_to(dUz + dWx, 0), Nd);
+    Nd = fma(fx_to(a23, 0), fx_to(dVz + dWy, 0), Nd);
+    double v = (-0.3 * Nd) / fx_to(D, 0) * pow2(min(1023, max(-1022, et - er - 67 + sd)));
+    if (bad) v = __longlong_as_double(0x7FF8000000000000LL);
+    if (valid) I.S[cidx(I, i, jc, k)] = v;
+    hi = max(hi, write_nut_rows(I, I.U[s_in], i, jc, k, v, use_wm, valid));
+  }
+#undef UC
+#undef WC
+#undef VV
+  chl_line_max(I.nmax, (unsigned)(p.k * Ny + p.j), Ny, 1, hi);
 }
 
 __global__ void __launch_bounds__(256)
@@ -206,6 +286,6 @@ k_vreman(ChlMap map, int s_in, int use_wm) {
 }
 
 extern "C" {
-void chl_launch_amd(const ChlMap& m, int nb, int s_in, int use_wm, cudaStream_t st) { chl_launch_pdl(k_amd, dim3(nb), dim3(m.tb), 0, st, m, s_in, use_wm); }
+void chl_launch_amd(const ChlMap& m, int nb, int s_in, int use_wm, cudaStream_t st) { chl_launch_pdl(k_amd, dim3(nb), dim3(CHL_FLUX_THREADS), 0, st, m, s_in, use_wm); }
 void chl_launch_vreman(const ChlMap& m, int nb, int s_in, int use_wm, cudaStream_t st) { chl_launch_pdl(k_vreman, dim3(nb), dim3(m.tb), 0, st, m, s_in, use_wm); }
 }
