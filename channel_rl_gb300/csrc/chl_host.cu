@@ -59,7 +59,8 @@ void chl_launch_shift(const ChlMap&, int, int, cudaStream_t);
 void chl_launch_tadvance(const ChlMap&, cudaStream_t);
 void chl_launch_divmax(const ChlMap&, int, int, double*, cudaStream_t);
 void chl_launch_qflow(const ChlInst*, int, int, int, cudaStream_t);
-void chl_launch_stats(const ChlMap&, int, double*, int, int, cudaStream_t);
+void chl_launch_stats(const ChlMap&, int, double*, double*, int, int, cudaStream_t);
+size_t chl_stats_parts();
 int chl_mlp_setup();
 void chl_launch_mlp(const ChlMap&, int, int, int, int*, cudaStream_t);
 void chl_launch_mlp_test(const float*, const float*, const float*, int, float*, float*, int*, cudaStream_t);
@@ -347,7 +348,7 @@ struct chl_handle {
   unsigned int* d_mlp_cfg = nullptr;  // sigma, train, seed lo/hi, evaluation counter, debug [5..6], shared draws [7]
   int* d_mlp_status = nullptr;
   double* d_divout = nullptr;
-  double* d_stats = nullptr;
+  double* d_stats = nullptr;          // statistics per instance, then the rows' partial sums
   double* d_agent = nullptr;          // wall-agent observations: inputs and outputs
   size_t agent_cap = 0;
   int stats_pitch = 0;
@@ -914,7 +915,9 @@ int chl_batch_create(int n, const chl_grid_desc* descs, chl_handle** out) {
   e = cudaMalloc(&h->d_divout, sizeof(double) * 2 * n);
   if (e != cudaSuccess) { h->err = "device allocation failed"; *out = h; return CHL_E_NOMEM; }
   for (auto& I : h->in) h->stats_pitch = std::max(h->stats_pitch, 7 * (I.c.Ny + 1) + 4);
-  e = cudaMalloc(&h->d_stats, sizeof(double) * (size_t)h->stats_pitch * n);
+  size_t rows = 0;
+  for (auto& I : h->in) rows += I.c.Ny + 1;
+  e = cudaMalloc(&h->d_stats, sizeof(double) * ((size_t)h->stats_pitch * n + rows * chl_stats_parts()));
   if (e != cudaSuccess) { h->err = "device allocation failed"; *out = h; return CHL_E_NOMEM; }
   int rc = build_maps(h);
   if (rc) { *out = h; return rc; }
@@ -1764,7 +1767,8 @@ int chl_sqrt_selftest(const double* a, double* y, long n) {
 static int run_stats(chl_handle* h, int inst, std::vector<double>& buf) {
   int rc = check_ready(h); if (rc) return rc;
   if (!get_inst(h, inst)) return CHL_E_ARG;
-  chl_launch_stats(h->map(M_ROWS), h->nblk[M_ROWS], h->d_stats, h->stats_pitch, 0, h->st);
+  chl_launch_stats(h->map(M_ROWS), h->nblk[M_ROWS], h->d_stats + (size_t)h->stats_pitch * h->in.size(), h->d_stats,
+                   h->stats_pitch, 0, h->st);
   LAUNCHED();
   buf.resize(h->stats_pitch);
   CK(cudaMemcpyAsync(buf.data(), h->d_stats + (size_t)inst * h->stats_pitch, 8 * (size_t)h->stats_pitch,
