@@ -39,13 +39,6 @@ __host__ __device__ inline int chl_tri_lanes(long modes, int Ny) {
   while (P < 8 && modes * P < (long)CHL_MIN_BLOCKS * 32 && Ny >= 4 * P) P *= 2;
   return P;
 }
-// x-z points per thread of the DSM plane sums (k_dsm_final, blocks of
-// CHL_DSMF_THREADS): 4, halved while the instance's Ny x chunks grid would
-// have fewer than CHL_MIN_BLOCKS blocks.  A large instance has chunks of 256
-// points (192 per plane at 256x192); a 32x48x32 channel gets 768 blocks of
-// one point per thread, 5 per SM, where 256-thread blocks left 2 blocks on
-// some SMs and 1 on most.  A function of the instance's own extents only,
-// so an instance sums its planes in the same order alone and in a batch.
 // Stockham FFT passes (chl_fft.cu): radix 4 while the remaining length
 // allows, then 3, then 2.
 inline int chl_fft_radix(int rem) { return rem % 4 == 0 ? 4 : (rem % 3 == 0 ? 3 : 2); }
@@ -82,17 +75,15 @@ inline int chl_fft_bits(int N) {
   return (6100 - grow) / 100;
 }
 
+// Planes per thread of the DSM plane sums (k_dsm_final, blocks of
+// CHL_DSMF_THREADS columns of a row): 8, halved while the instance would have
+// fewer than CHL_MIN_BLOCKS blocks.  A function of the instance's own extents
+// only, so an instance sums its planes in the same order alone and in a batch.
 #define CHL_DSMF_THREADS 64
-// Points of one plane sum: the Nx x Nz plane, then the reference's
-// duplicated periodic column (i = 0, every k) and plane (k = 0, every i) and
-// one more (0, 0) - its weights 2 and 4 as extra points of weight 1.
-__host__ __device__ inline int chl_dsm_points(int Nx, int Nz) { return Nx * Nz + Nx + Nz + 1; }
-__host__ __device__ inline int chl_dsm_ppt(int Nx, int Ny, int Nz) {
-  const int n = chl_dsm_points(Nx, Nz);
-  int ppt = 4;
-  while (ppt > 1 && (long)Ny * ((n + CHL_DSMF_THREADS * ppt - 1) / (CHL_DSMF_THREADS * ppt)) < CHL_MIN_BLOCKS)
-    ppt >>= 1;
-  return ppt;
+__host__ __device__ inline int chl_dsm_planes(int Nx, int Ny, int Nz) {
+  int m = 8;
+  while (m > 1 && (long)Ny * ((Nx * ((Nz + m - 1) / m) + CHL_DSMF_THREADS - 1) / CHL_DSMF_THREADS) < CHL_MIN_BLOCKS) m >>= 1;
+  return m;
 }
 // complex rows (pairs of real x lines) per x-transform block: up to
 // 512/Nx (at 256x96x192 the two x transforms take 95 + 54 us per launch with
@@ -114,12 +105,7 @@ __host__ __device__ inline int chl_fft_threads(int lines, int n) {
 #define CHL_TRI_SMEM_MAX (128 * 1024)   // largest staged tridiagonal column block
 #endif
 
-// Constants that the FP64 kernels take as register operands (F64 below);
-// held in each instance's descriptor in device memory, set by the host.
-enum { FK_ONE = 0, FK_MZERO, FK_FOUR, FK_NSLOT };
-
 struct ChlInst {
-  double fk[FK_NSLOT];          // 1, -0, 4 (FK_*)
   int Nx, Ny, Nz, Nxh;          // unique cells; Nxh = Nx/2+1
   int LES_model, Dirichlet_nu_t, wall_model, x_mass_cte;
   double nu, CFL, Cs;
@@ -138,9 +124,6 @@ struct ChlInst {
   const double *dxf, *dyf, *dzf;  // raw spacings (dt)
   const double *hx2, *hy2, *hz2;  // squared centre widths (x(i)-x(i-1))^2 etc. (Vreman)
   const double *w0x2, *w1x2;      // 2 x weight_y_0/1 by face row jv
-  // sqrt(4/216) x rdxc, rdyc, rdzc and rdxf, rdyf, rdzf: the dynamic model's
-  // filtered strain, whose M_ij term needs 4/216 x |S| S_ij
-  const double *rdxcs, *rdycs, *rdzcs, *rdxfs, *rdyfs, *rdzfs;
   const double *ygc;              // yg(1..nyg), centre y coordinates with the ghost rows
   const double *smag_csdelta;     // Cs*Delta_j by centre row (static Smagorinsky)
   const double *smag_dwall;       // distance of centre row to the nearer wall (van Driest)
@@ -165,16 +148,15 @@ struct ChlInst {
   const int *eyc, *eyf;
   int exc, exf, ezc, ezf;
   int4 *upd;                      // per row, from the flux kernel to the update: exponents (chl_rhs.cu)
-  unsigned *nmax;                 // largest |nu + nu_t| of every centre row (chl_fix.cuh)
-  double *q[CHL_NQ], *r[CHL_NQ];  // DSM filter ping-pong
-  double *E[3];                   // edge fields (S12, S13, S23 numerators)
+  unsigned *nmax, *smax;          // largest |nu + nu_t| and largest of the six |S| S_ij of every centre row (chl_fix.cuh)
+  double *q[CHL_NQ], *r[CHL_NQ];  // DSM: filter inputs 3..14 and filtered fields 0..17 (chl_sgs.cu; products and r are integers)
   double2 *spec;                  // [Ny+2][Nz][Nxh] spectra (rows 1..Ny used)
   double *p;                      // pseudo-pressure (centres)
   double *P;                      // actual pressure (centres)
   double *alpha;                  // wall stress [2][Nz][Nx]
   double *bc;                     // pressure BC planes [2][Nz][Nx]
   double *part;                   // DSM plane partial sums [2][Ny+2][npart][CHL_DSMF_THREADS]
-  int npart, dsm_ppt;             // chunks per plane, points per thread (chl_dsm_ppt)
+  int npart, dsm_planes;          // chunks of a row's columns, planes per column (chl_dsm_planes)
   double *coef;                   // nu_t coefficient per centre row [Ny+2]
   double *scal;                   // device scalars (CHL_S_*)
   unsigned long long *minabs;     // [Nx+1 | Nz] min |u| bit patterns (dt)
@@ -190,25 +172,6 @@ struct ChlInst {
                                   //   shared-exploration flag (chl_mlp_set_exploration)
   float *mlp_rec;                 // [3 stages][2 Nx Nz][8] per-point record (chl_mlp_debug), or null
 };
-
-// FP64 issue forms.  In a throughput loop on GB300 an FP64 FMA whose
-// operands are all registers issues at 1.91 per clock per SM, while DADD,
-// DMUL and any FP64 instruction with a literal operand issue at 1.61.  Sums,
-// differences and products can be issued as register FMAs:
-// a + b = fma(a, 1, b), a - b = fma(a, 1, -b), a b = fma(a, b, -0).  Each is
-// exact (a times 1 is a, adding -0 leaves a product unchanged, signed zeros
-// included), so the results are bit-identical to the plain operators.  The 1,
-// the -0 and the 4 are read from the instance descriptor in device memory, so
-// they reach the instructions as registers.  Used where it measured faster:
-// the filter passes, the edge strains and the stage update; the flux, strain
-// and L:M kernels and the transforms measured no faster (or slower) with it.
-struct F64 {
-  double one, mz;
-  __device__ __forceinline__ double add(double a, double b) const { return fma(a, one, b); }
-  __device__ __forceinline__ double sub(double a, double b) const { return fma(a, one, -b); }
-  __device__ __forceinline__ double mul(double a, double b) const { return fma(a, b, mz); }
-};
-__device__ __forceinline__ F64 f64_of(const ChlInst& I) { return F64{I.fk[FK_ONE], I.fk[FK_MZERO]}; }
 
 // -x on the integer pipe (a store of -x would take an FP64 instruction, and
 // in every thread where the compiler predicates it)

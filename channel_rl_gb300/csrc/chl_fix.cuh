@@ -128,3 +128,12 @@ __device__ __forceinline__ void chl_line_max(unsigned* g, unsigned q, int rows, 
     if (sm[w] && sm[w] > __ldcg(d)) atomicMax(d, sm[w]);
   }
 }
+
+// One's-complement magnitudes of the high words, or-ed: the bit length of the
+// result is that of the largest of them.
+__device__ __forceinline__ void top_or(unsigned& m, fx a) {
+  const int h = (int)(a >> 32);
+  m |= (unsigned)(h ^ (h >> 31));
+}
+// a 2^s for s of either sign (toward minus infinity)
+__device__ __forceinline__ fx scale2(fx a, int s) { return (a << max(s, 0)) >> max(-s, 0); }

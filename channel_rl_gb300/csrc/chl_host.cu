@@ -18,11 +18,9 @@ extern "C" {
 void chl_launch_fix(const ChlMap&, int, int, int, cudaStream_t);
 void chl_launch_flux(const ChlMap&, int, int, cudaStream_t);
 void chl_launch_update(const ChlMap&, int, int, int, int, int, cudaStream_t);
-void chl_launch_edges(const ChlMap&, int, int, int, cudaStream_t);
-void chl_launch_centre(const ChlMap&, int, int, int, int, cudaStream_t);
-void chl_launch_filter_y(const ChlMap&, int, int, cudaStream_t);
-void chl_launch_filter_x(const ChlMap&, int, cudaStream_t);
-void chl_launch_filter_z(const ChlMap&, int, cudaStream_t);
+void chl_launch_strain(const ChlMap&, int, int, int, cudaStream_t);
+int chl_filter_blocks(int, int, int, int);
+void chl_launch_filter(const ChlMap&, int, int, cudaStream_t);
 void chl_launch_dsm_final(const ChlMap&, int, int, cudaStream_t);
 void chl_launch_coef(const ChlMap&, cudaStream_t);
 void chl_launch_eqwm(const ChlMap&, int, int, cudaStream_t);
@@ -72,8 +70,8 @@ namespace {
 
 constexpr double RK_T[3] = {8.0 / 15.0, 2.0 / 3.0, 1.0};
 
-enum { M_PT, M_EDGE, M_FULL, M_DSMF, M_WALL, M_PLANE, M_FFTX, M_FFTZ, M_TRI, M_MINABS, M_ROWS, M_MLP, M_WALLN,
-       M_ZPLANE, M_ZSOLVE, M_EPAIR, M_FULLZ2, M_FULLX2, M_FLUX, M_MARCH, NMAP };
+enum { M_PT, M_FULL, M_DSMF, M_WALL, M_PLANE, M_FFTX, M_FFTZ, M_TRI, M_MINABS, M_ROWS, M_MLP, M_WALLN,
+       M_ZPLANE, M_ZSOLVE, M_FLUX, M_MARCH, M_FILTER, NMAP };
 constexpr int MLP_NPARAM = 4545;
 
 // Grid constants of one instance (host, FP64), in the device index
@@ -303,8 +301,8 @@ std::vector<double> fft_pass_table(int N) {
 }
 
 int dsm_npart(int Nx, int Ny, int Nz) {
-  const int p = chl_dsm_ppt(Nx, Ny, Nz);
-  return (chl_dsm_points(Nx, Nz) + CHL_DSMF_THREADS * p - 1) / (CHL_DSMF_THREADS * p);
+  const int m = chl_dsm_planes(Nx, Ny, Nz);
+  return (Nx * ((Nz + m - 1) / m) + CHL_DSMF_THREADS - 1) / CHL_DSMF_THREADS;
 }
 
 }  // namespace
@@ -339,8 +337,7 @@ struct chl_handle {
   int zlanes = 1;                     // its cluster size
   size_t smem_zs = 0;
   int twz = 0;                        // longest z transform table of the instances
-  bool epair = false;                 // edges as x-pair sums (k_edges_pair): every Nx <= 256
-  int tb_epair = 256;                 // its block: the largest Nx rounded up to a power of two, >= 64
+  int tb_filter = 128;                // threads of the test filter's blocks: a whole x-line of point pairs where it fits
   int tb_pt = 128;                    // threads per block of the point maps (stencils, updates)
   bool tri_scan = false;              // some instance splits its tridiagonal columns (chl_tri_lanes)
   int LES_model = 0, wall_model = 0, any_mass = 0;
@@ -355,7 +352,7 @@ struct chl_handle {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   ChlMap map(int which) const {
-    const bool pt = which == M_PT || which == M_EDGE || which == M_FULL || which == M_FULLZ2 || which == M_FULLX2;
+    const bool pt = which == M_PT || which == M_FULL;
     return ChlMap{d_inst, d_off[which], (int)in.size(), pt ? tb_pt : 256};
   }
 };
@@ -388,9 +385,7 @@ static int upload_consts(chl_handle* h, Inst& I) {
   size_t o_fxrxc = A.take(8 * (Nx + 3)), o_fxryc = A.take(8 * (Ny + 2)), o_fxrzc = A.take(8 * (Nz + 3));
   size_t o_fxrxf = A.take(8 * (Nx + 3)), o_fxryf = A.take(8 * (Ny + 2)), o_fxrzf = A.take(8 * (Nz + 3));
   size_t o_fxw1 = A.take(8 * (Ny + 2)), o_upd = A.take(16 * (Ny + 2));
-  size_t o_eyc = A.take(4 * (Ny + 2)), o_eyf = A.take(4 * (Ny + 2)), o_nmax = A.take(4 * (Ny + 2));
-  size_t o_rdxcs = A.take(8 * (Nx + 3)), o_rdycs = A.take(8 * (Ny + 2)), o_rdzcs = A.take(8 * (Nz + 3));
-  size_t o_rdxfs = A.take(8 * (Nx + 3)), o_rdyfs = A.take(8 * (Ny + 2)), o_rdzfs = A.take(8 * (Nz + 3));
+  size_t o_eyc = A.take(4 * (Ny + 2)), o_eyf = A.take(4 * (Ny + 2)), o_nmax = A.take(4 * (Ny + 2)), o_smax = A.take(4 * (Ny + 2));
   size_t o_csd = A.take(8 * (Ny + 2)), o_dw = A.take(8 * (Ny + 2));
   size_t o_twx = A.take(16 * (size_t)chl_twf_len(Nx)), o_twz = A.take(16 * (size_t)chl_twf_len(Nz));
   size_t o_ti = A.take(8 * ntri), o_tm = A.take(8 * ntri), o_tc = A.take(8 * ntri);
@@ -404,9 +399,7 @@ static int upload_consts(chl_handle* h, Inst& I) {
   for (int m = 0; m < 9; ++m) o_G[m] = A.take(8 * nc);
   for (int m = 0; m < 3; ++m) o_X[m] = A.take(8 * (m == 1 ? nv : nc));
   size_t o_q[CHL_NQ] = {}, o_r[CHL_NQ] = {};
-  if (dsm) for (int m = 0; m < CHL_NQ; ++m) { o_q[m] = A.take(8 * nc); o_r[m] = A.take(8 * nc); }
-  size_t o_E[3];
-  for (int m = 0; m < 3; ++m) o_E[m] = A.take(8 * nc);
+  if (dsm) for (int m = 0; m < CHL_NQ; ++m) { if (m >= 3 && m < 15) o_q[m] = A.take(8 * nc); o_r[m] = A.take(8 * nc); }
   size_t o_spec = A.take(16 * nspec), o_p = A.take(8 * nc), o_P = A.take(8 * nc);
   size_t o_alpha = A.take(8 * 2 * (size_t)Nx * Nz), o_bc = A.take(8 * 2 * (size_t)Nx * Nz);
   size_t o_part = A.take(8 * 2 * (size_t)(Ny + 2) * npart * CHL_DSMF_THREADS);   // one partial per DSM thread
@@ -428,7 +421,6 @@ static int upload_consts(chl_handle* h, Inst& I) {
   D.Nx = Nx; D.Ny = Ny; D.Nz = Nz; D.Nxh = Nxh;
   D.LES_model = I.d.LES_model; D.Dirichlet_nu_t = I.d.Dirichlet_nu_t;
   D.wall_model = I.d.wall_model; D.x_mass_cte = I.d.x_mass_cte;
-  D.fk[FK_ONE] = 1.0; D.fk[FK_MZERO] = -0.0; D.fk[FK_FOUR] = 4.0;
   D.nu = I.d.nu; D.CFL = I.d.CFL; D.Cs = I.d.Cs;
   D.dxmin = c.dxmin; D.dymin = c.dymin; D.dzmin = c.dzmin;
   {
@@ -461,8 +453,7 @@ static int upload_consts(chl_handle* h, Inst& I) {
   D.fxrxf = L(o_fxrxf) + 1; D.fxryf = L(o_fxryf); D.fxrzf = L(o_fxrzf) + 1;
   D.fxw1 = L(o_fxw1); D.upd = (int4*)(base + o_upd);
   D.eyc = (const int*)(base + o_eyc); D.eyf = (const int*)(base + o_eyf); D.nmax = (unsigned*)(base + o_nmax);
-  D.rdxcs = P(o_rdxcs) + 1; D.rdycs = P(o_rdycs); D.rdzcs = P(o_rdzcs) + 1;
-  D.rdxfs = P(o_rdxfs) + 1; D.rdyfs = P(o_rdyfs); D.rdzfs = P(o_rdzfs) + 1;
+  D.smax = (unsigned*)(base + o_smax);
   D.smag_csdelta = P(o_csd); D.smag_dwall = P(o_dw);
   D.twx = (const int4*)(base + o_twx); D.twz = (const int4*)(base + o_twz);
   D.lenx = chl_twf_len(Nx); D.lenz = chl_twf_len(Nz); D.passx = chl_fft_passes(Nx); D.passz = chl_fft_passes(Nz);
@@ -472,10 +463,9 @@ static int upload_consts(chl_handle* h, Inst& I) {
   D.nut = P(o_nut); D.S = P(o_S);
   for (int m = 0; m < 9; ++m) D.G[m] = L(o_G[m]);
   for (int m = 0; m < 3; ++m) D.X[m] = L(o_X[m]);
-  for (int m = 0; m < CHL_NQ; ++m) { D.q[m] = dsm ? P(o_q[m]) : nullptr; D.r[m] = dsm ? P(o_r[m]) : nullptr; }
-  for (int m = 0; m < 3; ++m) D.E[m] = P(o_E[m]);
+  for (int m = 0; m < CHL_NQ; ++m) { D.q[m] = dsm && m >= 3 && m < 15 ? P(o_q[m]) : nullptr; D.r[m] = dsm ? P(o_r[m]) : nullptr; }
   D.spec = (double2*)(base + o_spec); D.p = P(o_p); D.P = P(o_P);
-  D.alpha = P(o_alpha); D.bc = P(o_bc); D.part = P(o_part); D.npart = npart; D.dsm_ppt = chl_dsm_ppt(Nx, Ny, Nz);
+  D.alpha = P(o_alpha); D.bc = P(o_bc); D.part = P(o_part); D.npart = npart; D.dsm_planes = chl_dsm_planes(Nx, Ny, Nz);
   D.coef = P(o_coef); D.scal = P(o_scal);
   D.minabs = (unsigned long long*)(base + o_min); D.red = P(o_red); D.status = (int*)(base + o_status);
   D.dsm_cnt = (int*)(base + o_dcnt);
@@ -530,9 +520,6 @@ static int upload_consts(chl_handle* h, Inst& I) {
   CK(uniform(o_fxrzc, c.rdzc, D.ezc)); CK(uniform(o_fxrzf, c.rdzf, D.ezf));
   CK(perrow(o_fxryc, o_eyc, c.rdyc)); CK(perrow(o_fxryf, o_eyf, c.rdyf));
   CK(fixtab(o_fxw1, c.w1, {-63}));
-  const double fs = std::sqrt(4.0 / 216.0);
-  CK(put(o_rdxcs, times(c.rdxc, fs))); CK(put(o_rdycs, times(c.rdyc, fs))); CK(put(o_rdzcs, times(c.rdzc, fs)));
-  CK(put(o_rdxfs, times(c.rdxf, fs))); CK(put(o_rdyfs, times(c.rdyf, fs))); CK(put(o_rdzfs, times(c.rdzf, fs)));
   CK(put(o_csd, c.csdelta)); CK(put(o_dw, c.dwall));
   {
     const std::vector<int4> tx = fft_table(Nx), tz = fft_table(Nz);
@@ -606,11 +593,8 @@ static int build_maps(chl_handle* h) {
     h->smem_zs = std::max(h->smem_zs, b);
   }
   h->zsolve = h->zsolve_ok && (h->tri_mode == 3 || (h->tri_mode == 2 && h->zlanes > 1));
-  h->epair = true;
-  int mx = 0;
-  for (auto& I : h->in) { h->epair = h->epair && I.c.Nx <= 256; mx = std::max(mx, I.c.Nx); }
-  h->tb_epair = 64;
-  while (h->tb_epair < mx && h->tb_epair < 256) h->tb_epair *= 2;
+  h->tb_filter = 128;
+  for (auto& I : h->in) if (I.c.Nx / 2 > 128) h->tb_filter = 256;
   h->smem_t = h->tri_scan ? 0 : chl_smem_tri(my, modes, h->tri_mode);
   const int tri_w = chl_tri_modes_per_block(h->smem_t);
   for (int m = 0; m < NMAP; ++m) {
@@ -621,10 +605,8 @@ static int build_maps(chl_handle* h) {
       int b = 0;
       switch (m) {
         case M_PT: b = cdiv((long)Nx * Ny * Nz, h->tb_pt); break;
-        case M_EDGE: b = cdiv((long)Nx * (Ny + 1) * Nz, h->tb_pt); break;
         case M_FULL: b = cdiv((long)Nx * (Ny + 2) * Nz, h->tb_pt); break;
-        case M_FULLZ2: b = cdiv((long)Nx * (Ny + 2) * (Nz / 2), h->tb_pt); break;   // z planes in pairs (Nz even)
-        case M_FULLX2: b = cdiv((long)(Nx / 2) * (Ny + 2) * Nz, h->tb_pt); break;   // x points in pairs (Nx even)
+        case M_FILTER: b = chl_filter_blocks(Nx, Ny, Nz, h->tb_filter); break;
         case M_FLUX: b = cdiv((long)Nx * (Ny + 1) * cdiv(Nz, chl_planes(Nx, Ny, Nz)), CHL_FLUX_THREADS); break;
         case M_MARCH: b = cdiv((long)Nx * Ny * cdiv(Nz, chl_planes(Nx, Ny, Nz)), CHL_FLUX_THREADS); break;
         case M_DSMF: b = Ny * dsm_npart(Nx, Ny, Nz); break;
@@ -640,7 +622,6 @@ static int build_maps(chl_handle* h) {
         case M_WALLN: b = cdiv(2L * Nx * Nz, CHL_WALL_THREADS); break;
         case M_ZPLANE: b = Nz; break;
         case M_ZSOLVE: b = Nxh * h->zlanes; break;
-        case M_EPAIR: b = Nx <= h->tb_epair ? cdiv((long)(Ny + 1) * Nz, h->tb_epair / Nx) : 1; break;   // whole x-rows
       }
       off[q + 1] = off[q] + b;
     }
@@ -676,19 +657,11 @@ static int enqueue_sgs(chl_handle* h, int s, bool with_wm, int stage = 0) {
   KL("fix", chl_launch_fix(h->map(M_FULL), h->nblk[M_FULL], s, 1, st));
   if (fused) wall_stress();
   if (h->LES_model == CHL_LES_DYNAMIC) {
-    KL("edges", chl_launch_edges(h->map(h->epair ? M_EPAIR : M_EDGE), h->nblk[h->epair ? M_EPAIR : M_EDGE], s,
-                                 h->epair ? h->tb_epair : 0, st));
-    KL("centre_strain", chl_launch_centre(h->map(M_PT), h->nblk[M_PT], s, 1, h->epair, st));
-    KL("filter_y", chl_launch_filter_y(h->map(M_FULL), h->nblk[M_FULL], s, st));
-    KL("filter_x", chl_launch_filter_x(h->map(M_FULLX2), h->nblk[M_FULLX2], st));
-    KL("filter_z", chl_launch_filter_z(h->map(M_FULLZ2), h->nblk[M_FULLZ2], st));
-    KL("edges", chl_launch_edges(h->map(h->epair ? M_EPAIR : M_EDGE), h->nblk[h->epair ? M_EPAIR : M_EDGE], 3,
-                                 h->epair ? h->tb_epair : 0, st));
-    KL("dsm_LM_MM", chl_launch_dsm_final(h->map(M_DSMF), h->nblk[M_DSMF], h->epair, st));
+    KL("strain", chl_launch_strain(h->map(M_MARCH), h->nblk[M_MARCH], s, 1, st));
+    KL("filter", chl_launch_filter(h->map(M_FILTER), h->nblk[M_FILTER], h->tb_filter, st));
+    KL("dsm_LM_MM", chl_launch_dsm_final(h->map(M_DSMF), h->nblk[M_DSMF], s, st));
   } else if (h->LES_model == CHL_LES_SMAGORINSKY) {
-    KL("edges", chl_launch_edges(h->map(h->epair ? M_EPAIR : M_EDGE), h->nblk[h->epair ? M_EPAIR : M_EDGE], s,
-                                 h->epair ? h->tb_epair : 0, st));
-    KL("centre_strain", chl_launch_centre(h->map(M_PT), h->nblk[M_PT], s, 0, h->epair, st));
+    KL("strain", chl_launch_strain(h->map(M_MARCH), h->nblk[M_MARCH], s, 0, st));
   } else if (h->LES_model == CHL_LES_AMD) {
     KL("amd", chl_launch_amd(h->map(M_MARCH), h->nblk[M_MARCH], s, with_wm ? 1 : 0, st));
   } else if (h->LES_model == CHL_LES_VREMAN) {

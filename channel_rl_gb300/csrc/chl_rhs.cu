@@ -66,14 +66,14 @@ __device__ __forceinline__ RowExp row_exp(const ChlInst& I, int sin, int j) {
 
 // Fixed-point copies of the velocity set that a stage works on (rows as
 // stored, ghosts included); reset_n clears the rows' largest |nu + nu_t|
-// ahead of the kernels that form them.  Moves 48 bytes per point: HBM-bound.
+// and |S| S_ij ahead of the kernels that form them.  Moves 48 bytes per point: HBM-bound.
 __global__ void __launch_bounds__(256)
 k_fix(ChlMap map, int s, int reset_n) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  if (reset_n && t < (unsigned)(I.Ny + 2)) I.nmax[t] = 0u;
+  if (reset_n && t < (unsigned)(I.Ny + 2)) I.nmax[t] = I.smax[t] = 0u;
   const unsigned* vm = chl_vmax(I, s);
   const unsigned nc = (unsigned)(I.Nx * (I.Ny + 2) * I.Nz), nv = (unsigned)(I.Nx * (I.Ny + 1) * I.Nz);
   if (t < nc) {

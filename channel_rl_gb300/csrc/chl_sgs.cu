@@ -8,369 +8,233 @@
 // and plane counted twice, subgrid.f90:492-509), nu_t = max(0,-1/2 <LM>/<MM>|S|)
 // and the ghost-row rule of Dirichlet_nu_t.
 //
-// The filter is applied as three separable passes with unnormalised weights
-// (1,4,1) and (4,2); the 6^3 = 216 scale, the 1/2 of the centre averages
-// and the 1/8 of the edge averages are folded into the final L:M and M:M
-// dot products, which only enter as the ratio <LM>/<MM>.  This keeps the
-// FP64 instruction count per point at its minimum (the GB300 FP64 pipe, not
-// HBM, bounds this code).
+// The strain, the filter and L are formed in fixed point (chl_fix.cuh,
+// chl_strain.cuh): as FP64 code the dynamic model took 212 FP64 instructions
+// per point and stage, which the FP64 pipe bounds; 30 are left.
 //
 // Static Smagorinsky with van Driest damping (subgrid.f90:563-612, which
 // aborts in the reference) is written from its formula.  The stress wall
 // model is compute_wall_model (wallmodel.f90:23-46); the equilibrium log-law
 // wall stress that feeds it is new.
-#include "chl_fix.cuh"
+#include "chl_strain.cuh"
 
-// ---------------------------------------------------------------- edges
-// E12 at (x-face a, y-face jv, z-centre k), E13 at (x-face a, centre row jc,
-// z-face b), E23 at (x-centre i, y-face jv, z-face b): 2 x the edge strain
-// rates of compute_Sij, stored V-like (E12, E23: Ny+1 rows) and centre-like
-// (E13, rows 1..Ny).  Of the filtered faces (src 3) with the reciprocals
-// scaled by sqrt(4/216) (rdxfs ...), for the filtered strain of k_dsm_final.
-__global__ void __launch_bounds__(256)
-k_edges(ChlMap map, int src) {
+// ---------------------------------------------------------------- strain
+// Strain magnitude and the DSM filter inputs at centres (rows 1..Ny): q3..8
+// the products of the centre velocities' face sums in fixed point (last bit
+// 2^(e_i + e_j + 64)), q9..14 = |S|*(S_ii, 8 S_ij) / sqrt(2) and their
+// largest per row.
+template <bool DSM>
+__global__ void __launch_bounds__(CHL_FLUX_THREADS, 4)
+k_strain(ChlMap map, int s_in) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
-  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
+  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz, M = chl_planes(Nx, Ny, Nz);
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  if (t >= (unsigned)(Nx * (Ny + 1) * Nz)) return;
-  const ChlIdx p = chl_split(t, Nx, Ny + 1);
-  const int a = p.i, j = p.j, k = p.k;
-  const double *U, *V, *W;
-  if (src < 3) { U = I.U[src]; V = I.V[src]; W = I.W[src]; }
-  else { U = I.r[15]; V = I.r[16]; W = I.r[17]; }
-  const int ap = wrap(a + 1, Nx), kp = wrap(k + 1, Nz);
-  const bool filt = src == 3;
-  const double rxf = LDG((filt ? I.rdxfs : I.rdxf) + a), rzf = LDG((filt ? I.rdzfs : I.rdzf) + k);
-  const double ryf = LDG((filt ? I.rdyfs : I.rdyf) + j);
-  const F64 f = f64_of(I);   // differences and products as register FMAs
-  // E12 (jv = j): dU/dy + dV/dx
-  const double e12 = fma(f.sub(LDG(U + cidx(I, a, j + 1, k)), LDG(U + cidx(I, a, j, k))), ryf,
-                         f.mul(f.sub(LDG(V + vidx(I, ap, j, k)), LDG(V + vidx(I, a, j, k))), rxf));
-  // E23 (jv = j, b = k): dV/dz + dW/dy
-  const double e23 = fma(f.sub(LDG(V + vidx(I, a, j, kp)), LDG(V + vidx(I, a, j, k))), rzf,
-                         f.mul(f.sub(LDG(W + cidx(I, a, j + 1, k)), LDG(W + cidx(I, a, j, k))), ryf));
-  I.E[0][vidx(I, a, j, k)] = e12;
-  I.E[2][vidx(I, a, j, k)] = e23;
-  if (j >= 1 && j <= Ny) {
-    // E13 (jc = j, b = k): dU/dz + dW/dx
-    const double e13 = fma(f.sub(LDG(U + cidx(I, a, j, kp)), LDG(U + cidx(I, a, j, k))), rzf,
-                           f.mul(f.sub(LDG(W + cidx(I, ap, j, k)), LDG(W + cidx(I, a, j, k))), rxf));
-    I.E[1][cidx(I, a, j, k)] = e13;
+  const ChlIdx p = chl_split(t, Nx, Ny);
+  const int i = p.i, jc = 1 + p.j, k0 = p.k * M, k1 = min(Nz, k0 + M);
+  unsigned hi = 0u;
+  if (k0 < k1) {
+    const unsigned* vm = chl_vmax(I, s_in);
+    const bool bad = fx_bad(vm[0]) || fx_bad(vm[1]) || fx_bad(vm[2]);
+    StrainColumn col(I, I.X[0], I.X[1], I.X[2], fx_exp<61>(vm[0]), fx_exp<61>(vm[1]), fx_exp<61>(vm[2]), i, jc, k0);
+    for (int k = k0; k < k1; ++k) {
+      fx f[3];
+      Strain s = col.point(k, f);
+      if (bad) s.s = __longlong_as_double(0x7FF8000000000000LL);
+      const size_t c = cidx(I, i, jc, k);
+      I.S[c] = s.s;
+      if (!DSM) continue;
+      fx* const* q = reinterpret_cast<fx* const*>(I.q);
+      q[3][c] = fx_mul(f[0], f[0]); q[4][c] = fx_mul(f[1], f[1]); q[5][c] = fx_mul(f[2], f[2]);
+      q[6][c] = fx_mul(f[0], f[1]); q[7][c] = fx_mul(f[0], f[2]); q[8][c] = fx_mul(f[1], f[2]);
+      const double m[6] = {s.s * s.d1, s.s * s.d2, s.s * s.d3, s.s * s.o12, s.s * s.o13, s.s * s.o23};
+#pragma unroll
+      for (int n = 0; n < 6; ++n) { I.q[9 + n][c] = m[n]; hi = max(hi, chl_abshi(m[n])); }
+    }
   }
+  if (DSM) chl_line_max(I.smax, (unsigned)(p.k * Ny + p.j), Ny, 1, hi);
 }
 
-// The same edges, with the x-pair sums that every centre strain needs
-// formed once per edge: P12(a) = E12(a-1) + E12(a) and P13(a) = E13(a-1) +
-// E13(a) are stored in place of E12 and E13 (E23 as it is).  A block (64,
-// 128 or 256 threads: the launch's largest Nx rounded up to a power of two,
-// at least 64) holds blockDim / Nx whole x-rows (j, k) (Nx <= 256), so the
-// left neighbour, periodic, comes from shared memory: one addition per edge
-// instead of two per centre.  The centre strain's sums keep their order,
-// (E(i-1) + E(i)) + (E'(i-1) + E'(i)), so the result is bit-identical.
-__global__ void __launch_bounds__(256)
-k_edges_pair(ChlMap map, int src) {
-  chl_pdl_wait();
-  __shared__ double s12[256], s13[256];
-  int lb;
-  const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
-  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
-  const int RB = blockDim.x / Nx;
-  const int r = threadIdx.x / Nx, a = threadIdx.x - r * Nx;
-  const unsigned g = (unsigned)lb * RB + r;          // the row (j, k), j = 0..Ny
-  const bool valid = r < RB && g < (unsigned)((Ny + 1) * Nz);
-  const unsigned gk = valid ? g / (unsigned)(Ny + 1) : 0u;
-  const int j = valid ? (int)(g - gk * (unsigned)(Ny + 1)) : 0, k = (int)gk;
-  const double *U, *V, *W;
-  if (src < 3) { U = I.U[src]; V = I.V[src]; W = I.W[src]; }
-  else { U = I.r[15]; V = I.r[16]; W = I.r[17]; }
-  const int ap = wrap(a + 1, Nx), kp = wrap(k + 1, Nz);
-  const bool filt = src == 3;
-  const double rxf = LDG((filt ? I.rdxfs : I.rdxf) + a), rzf = LDG((filt ? I.rdzfs : I.rdzf) + k);
-  const double ryf = LDG((filt ? I.rdyfs : I.rdyf) + j);
-  const F64 f = f64_of(I);   // differences and products as register FMAs
-  const double e12 = fma(f.sub(LDG(U + cidx(I, a, j + 1, k)), LDG(U + cidx(I, a, j, k))), ryf,
-                         f.mul(f.sub(LDG(V + vidx(I, ap, j, k)), LDG(V + vidx(I, a, j, k))), rxf));
-  const double e23 = fma(f.sub(LDG(V + vidx(I, a, j, kp)), LDG(V + vidx(I, a, j, k))), rzf,
-                         f.mul(f.sub(LDG(W + cidx(I, a, j + 1, k)), LDG(W + cidx(I, a, j, k))), ryf));
-  // E13 on the centre rows 1..Ny (row 0 computes an unused value from the ghost row)
-  const double e13 = fma(f.sub(LDG(U + cidx(I, a, j, kp)), LDG(U + cidx(I, a, j, k))), rzf,
-                         f.mul(f.sub(LDG(W + cidx(I, ap, j, k)), LDG(W + cidx(I, a, j, k))), rxf));
-  s12[threadIdx.x] = e12;
-  s13[threadIdx.x] = e13;
-  __syncthreads();
-  if (!valid) return;
-  const int left = r * Nx + (a == 0 ? Nx - 1 : a - 1);
-  I.E[0][vidx(I, a, j, k)] = s12[left] + e12;
-  I.E[2][vidx(I, a, j, k)] = e23;
-  if (j >= 1) I.E[1][cidx(I, a, j, k)] = s13[left] + e13;
-}
-
-// Centre strain: diagonal D, 8*S_offdiag O (sum of four edges), and
-// s = |S|/sqrt(2).  The sqrt(2) never needs forming: nu_t = c |S| where the
-// dynamic model's c comes from L:M / M:M with M linear in |S| and |S^| (so
-// keeping both /sqrt(2) scales c by sqrt(2) and c s = c_true |S|), and the
-// static model's row coefficient carries the sqrt(2) itself (k_coef).
-struct Strain { double d1, d2, d3, o12, o13, o23, s; };
-
-// The six face velocities around centre (i, jc, k): u0 = U(i-1), u1 = U(i),
-// v0 = V(jc-1), v1 = V(jc), w0 = W(k-1), w1 = W(k).
-struct Faces { double u0, u1, v0, v1, w0, w1; };
-
-__device__ __forceinline__ Faces centre_faces(const ChlInst& I, const double* U, const double* V,
-                                              const double* W, int i, int jc, int k) {
-  const int im = wrap(i - 1, I.Nx), km = wrap(k - 1, I.Nz);
-  Faces f;
-  f.u0 = LDG(U + cidx(I, im, jc, k)); f.u1 = LDG(U + cidx(I, i, jc, k));
-  f.v0 = LDG(V + vidx(I, i, jc - 1, k)); f.v1 = LDG(V + vidx(I, i, jc, k));
-  f.w0 = LDG(W + cidx(I, i, jc, km)); f.w1 = LDG(W + cidx(I, i, jc, k));
+// ------------------------------------------------------------ test filter
+// filter_xzy of fifteen fields in one pass over memory, in fixed point: the
+// six products of the centre velocities (rows 1..Ny), the six |S| S_ij (rows
+// 1..Ny, scaled by the largest of the group's rows) and the face velocities U
+// and W (rows 0..Ny+1) and V (rows 0..Ny); each with the one-sided rule
+// (4, 2)/6 at its first and last row.  Three separable FP64 passes took 2
+// instructions of 64 clocks per pass, field and point and moved every field
+// three times: 247 us per pass at 256x96x192.  Here a tap is an integer
+// shift and two additions.
+//
+// A pass forms (a + 4 b + c) >> 3, so that a field starts and ends below 2^60
+// and a filtered value is 512/216 times its integer.  A thread holds two
+// points in x of two rows, filters them in y from the four rows it loads,
+// exchanges with its neighbours in x through shared memory and marches in z,
+// carrying the two planes behind.
+//
+// Rows 1 and Ny of the centre velocities need the one-sided rule in y, which
+// the filtered faces next to them do not have: three more "fields" of two
+// rows each hold (4 f_1 + 2 f_2) of U, W (and of the face sum of V), so that
+// the final kernel forms the wall rows' filtered centre velocities from them
+// like the others from the faces.
+//
+// Blocks per instance: for each of the 15 fields row blocks x plane chunks,
+// then for each of the 3 wall fields one row block x plane chunks.
+#define FILT_FIELDS 15
+struct FiltShape { int nxp, RG, segs, rowblocks, M, nz, full; };   // full: blocks of one field
+__host__ __device__ inline FiltShape filt_shape(int Nx, int Ny, int Nz, int T) {
+  FiltShape f;
+  f.nxp = Nx / 2;
+  f.RG = f.nxp <= T ? T / f.nxp : 1;                       // row groups per block
+  f.segs = f.nxp <= T ? 1 : (f.nxp + T - 3) / (T - 2);     // longer rows: overlapping segments
+  const int groups = (Ny + 3) / 2;                         // of U and W, the most
+  f.rowblocks = (groups + f.RG - 1) / f.RG * f.segs;
+  f.M = 16;
+  while (f.M > 4 && (long)f.rowblocks * FILT_FIELDS * ((Nz + f.M - 1) / f.M) < 2 * CHL_MIN_BLOCKS) f.M >>= 1;
+  f.nz = (Nz + f.M - 1) / f.M;
+  f.full = f.rowblocks * f.nz;
   return f;
 }
 
-// FILT: the filtered strain, with the sqrt(4/216)-scaled reciprocals and
-// edges, so that it comes out times sqrt(4/216).  PAIR: E12 and E13 hold the
-// x-pair sums of k_edges_pair.
-template <bool FILT, bool PAIR>
-__device__ __forceinline__ Strain centre_strain(const ChlInst& I, const Faces& f, int i, int jc, int k) {
-  const int im = wrap(i - 1, I.Nx), km = wrap(k - 1, I.Nz);
-  Strain s;
-  s.d1 = (f.u1 - f.u0) * LDG((FILT ? I.rdxcs : I.rdxc) + i);
-  s.d2 = (f.v1 - f.v0) * LDG((FILT ? I.rdycs : I.rdyc) + jc);
-  s.d3 = (f.w1 - f.w0) * LDG((FILT ? I.rdzcs : I.rdzc) + k);
-  const double* E12 = I.E[0]; const double* E13 = I.E[1]; const double* E23 = I.E[2];
-  if (PAIR) {
-    s.o12 = LDG(E12 + vidx(I, i, jc - 1, k)) + LDG(E12 + vidx(I, i, jc, k));
-    s.o13 = LDG(E13 + cidx(I, i, jc, km)) + LDG(E13 + cidx(I, i, jc, k));
+// the exponent of |S| S_ij in the filter of row group g (rows 1 + 2 g, 2 + 2 g)
+__device__ __forceinline__ int filt_exp(const ChlInst& I, int g) {
+  unsigned m = 0u;
+  for (int j = max(1, 2 * g); j <= min(I.Ny, 2 * g + 3); ++j) m = max(m, I.smax[j]);
+  return fx_exp<60>(m);
+}
+
+struct Pair { fx x, y; };
+__device__ __forceinline__ Pair tap(Pair a, Pair b, Pair c) {
+  return Pair{(a.x + 4 * b.x + c.x) >> 3, (a.y + 4 * b.y + c.y) >> 3};
+}
+__device__ __forceinline__ Pair one_sided(Pair a, Pair b) { return Pair{(a.x >> 1) + (b.x >> 2), (a.y >> 1) + (b.y >> 2)}; }
+
+__global__ void __launch_bounds__(256)
+k_filter(ChlMap map) {
+  chl_pdl_wait();
+  __shared__ longlong2 sm[2][2][256];      // [parity][row][thread]
+  int lb;
+  const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
+  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
+  const FiltShape f = filt_shape(Nx, Ny, Nz, blockDim.x);
+  // field, row block, segment, planes
+  int field, rest;
+  if (lb < FILT_FIELDS * f.full) { field = lb / f.full; rest = lb - field * f.full; }
+  else {
+    const int w = lb - FILT_FIELDS * f.full;
+    field = FILT_FIELDS + w / (f.segs * f.nz);
+    rest = w % (f.segs * f.nz);
+  }
+  const bool wall = field >= FILT_FIELDS;
+  const int rb = wall ? rest % f.segs : rest % f.rowblocks, zc = wall ? rest / f.segs : rest / f.rowblocks;
+  const int seg = rb % f.segs;
+  const int tid = threadIdx.x;
+  int rg, pi, left, right;
+  bool out;
+  if (f.segs == 1) {
+    rg = tid / f.nxp;
+    pi = tid - rg * f.nxp;
+    out = rg < f.RG;
+    left = pi == 0 ? tid + f.nxp - 1 : tid - 1;
+    right = pi == f.nxp - 1 ? tid - (f.nxp - 1) : tid + 1;
+    if (!out) { rg = 0; left = right = tid; }
   } else {
-    s.o12 = (LDG(E12 + vidx(I, im, jc - 1, k)) + LDG(E12 + vidx(I, i, jc - 1, k)))
-          + (LDG(E12 + vidx(I, im, jc, k)) + LDG(E12 + vidx(I, i, jc, k)));
-    s.o13 = (LDG(E13 + cidx(I, im, jc, km)) + LDG(E13 + cidx(I, i, jc, km)))
-          + (LDG(E13 + cidx(I, im, jc, k)) + LDG(E13 + cidx(I, i, jc, k)));
+    rg = 0;
+    pi = seg * ((int)blockDim.x - 2) + tid - 1;
+    out = tid >= 1 && tid < (int)blockDim.x - 1 && pi < f.nxp;
+    pi = pi < 0 ? pi + f.nxp : pi % f.nxp;
+    left = max(tid - 1, 0); right = min(tid + 1, (int)blockDim.x - 1);
   }
-  s.o23 = (LDG(E23 + vidx(I, i, jc - 1, km)) + LDG(E23 + vidx(I, i, jc, km)))
-        + (LDG(E23 + vidx(I, i, jc - 1, k)) + LDG(E23 + vidx(I, i, jc, k)));
-  // |S|^2 = 2 (d.d) + 4 (S12^2+S13^2+S23^2) = 2 (d.d + (o.o)/32)
-  double dd = s.d1 * s.d1; dd = fma(s.d2, s.d2, dd); dd = fma(s.d3, s.d3, dd);
-  double oo = s.o12 * s.o12; oo = fma(s.o13, s.o13, oo); oo = fma(s.o23, s.o23, oo);
-  s.s = chl_sqrt(fma(oo, 0.03125, dd));   // |S| / sqrt(2)
-  return s;
-}
-
-// Raw strain and the DSM filter inputs at centres (rows 1..Ny):
-// q0..2 = 2*(centre velocities), q3..8 = their products, q9..14 = |S|*(d, o).
-// q0..2 are stored only in the two rows next to each wall: the filter is
-// linear and shift-invariant, so away from the walls the filtered centre
-// velocity is the centre average of the filtered face velocity (k_dsm_final
-// forms it there); only rows 1 and Ny, where the centre filter takes its
-// one-sided rule and the face filter does not, need the centre velocity
-// filtered in its own right.
-// DSM and PAIR are template parameters: a runtime switch would leave the
-// FP64 work of the other side predicated in every warp.
-template <bool DSM, bool PAIR>
-__global__ void __launch_bounds__(256)
-k_centre(ChlMap map, int s_in) {
-  chl_pdl_wait();
-  int lb;
-  const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
-  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
-  const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  if (t >= (unsigned)(Nx * Ny * Nz)) return;
-  const ChlIdx p = chl_split(t, Nx, Ny);
-  const int i = p.i, jc = 1 + p.j, k = p.k;
-  const Faces f = centre_faces(I, I.U[s_in], I.V[s_in], I.W[s_in], i, jc, k);
-  const Strain s = centre_strain<false, PAIR>(I, f, i, jc, k);
-  const size_t c = cidx(I, i, jc, k);
-  I.S[c] = s.s;
-  if (!DSM) return;
-  const double uc = f.u0 + f.u1, vc = f.v0 + f.v1, wc = f.w0 + f.w1;
-  if (jc <= 2 || jc >= Ny - 1) { I.q[0][c] = uc; I.q[1][c] = vc; I.q[2][c] = wc; }
-  I.q[3][c] = uc * uc; I.q[4][c] = vc * vc; I.q[5][c] = wc * wc;
-  I.q[6][c] = uc * vc; I.q[7][c] = uc * wc; I.q[8][c] = vc * wc;
-  I.q[9][c] = s.s * s.d1; I.q[10][c] = s.s * s.d2; I.q[11][c] = s.s * s.d3;
-  I.q[12][c] = s.s * s.o12; I.q[13][c] = s.s * s.o13; I.q[14][c] = s.s * s.o23;
-}
-
-// ------------------------------------------------------------ filter passes
-// y pass: q (and the velocity set s_in for the three face components) -> r.
-// Centre components use rows 1..Ny, U and W rows 0..Ny+1, V rows 0..Ny, each
-// with the one-sided rule at its first and last row.
-// Branch-free: at the first (last) row the missing neighbour is replaced by
-// the other one, so lo + 4q + hi becomes 4q + 2*hi (4q + 2*lo), the
-// one-sided 2/3-1/3 rule times 6.  Only the addresses are selected.
-__device__ __forceinline__ double fy(const double* f, size_t c, size_t pitch, int j, int j0, int j1, const F64& k,
-                                     double four) {
-  const size_t lo = (j == j0) ? c + pitch : c - pitch;
-  const size_t hi = (j == j1) ? c - pitch : c + pitch;
-  return fma(four, LDG(f + c), k.add(LDG(f + lo), LDG(f + hi)));
-}
-
-// N components from N0 on: out = in(lo) + 4 in(c) + in(hi).  All loads are
-// issued before the stores: the stores may alias the loads as far as the
-// compiler knows, so this is what keeps enough loads in flight.  The sum
-// and the 4 go in as registers (F64): the filter passes are made of nothing
-// else, and that form measured 12 % faster for the y pass.
-template <int N0, int N>
-__device__ __forceinline__ void filter_group(double* const* in, double* const* out, size_t c, size_t lo,
-                                             size_t hi, const F64& k, double four) {
-  double a[N], b[N], d[N];
-#pragma unroll
-  for (int q = 0; q < N; ++q) {
-    const double* f = in[N0 + q];
-    a[q] = LDG(f + c); b[q] = LDG(f + lo); d[q] = LDG(f + hi);
+  const int g = wall ? 0 : rb / f.segs * f.RG + rg;
+  out = out && (!wall || rg == 0);
+  // source, rows and layout
+  const int comp = wall ? field - FILT_FIELDS : field - 12;     // 0, 1, 2: U, V, W
+  const bool vlike = field >= 12 && comp == 1;
+  const bool conv = field >= 6 && field < 12;
+  const int nrow = vlike ? Ny + 1 : Ny + 2;
+  const int first = field < 12 ? 1 : 0, last = field < 12 ? Ny : (vlike ? Ny : Ny + 1);
+  const longlong2* src;
+  longlong2* dst;
+  if (field < 12) { src = reinterpret_cast<const longlong2*>(I.q[3 + field]); dst = reinterpret_cast<longlong2*>(I.r[3 + field]); }
+  else {
+    src = reinterpret_cast<const longlong2*>(I.X[comp]);
+    dst = reinterpret_cast<longlong2*>(wall ? I.r[comp] : I.r[15 + comp]);
   }
-#pragma unroll
-  for (int q = 0; q < N; ++q) out[N0 + q][c] = fma(four, a[q], k.add(b[q], d[q]));
-}
-
-// The centre components: products and |S| S (3..14) on every row, the centre
-// velocities (0..2) on the wall rows 1 and Ny only (see k_centre).
-__device__ __forceinline__ void filter_centre(double* const* in, double* const* out, size_t c, size_t lo,
-                                              size_t hi, bool wall_row, const F64& k, double four) {
-  filter_group<3, 6>(in, out, c, lo, hi, k, four);
-  filter_group<9, 6>(in, out, c, lo, hi, k, four);
-  if (wall_row) filter_group<0, 3>(in, out, c, lo, hi, k, four);
-}
-
-__global__ void __launch_bounds__(256)
-k_filter_y(ChlMap map, int s_in) {
-  chl_pdl_wait();
-  int lb;
-  const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
-  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
-  const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  if (t >= (unsigned)(Nx * (Ny + 2) * Nz)) return;
-  const ChlIdx p = chl_split(t, Nx, Ny + 2);
-  const int i = p.i, j = p.j, k = p.k;
-  const size_t c = cidx(I, i, j, k);
-  const size_t pc = (size_t)Nx;
-  const F64 f = f64_of(I);
-  const double four = I.fk[FK_FOUR];
-  if (j >= 1 && j <= Ny) {
-    const size_t lo = (j == 1) ? c + pc : c - pc, hi = (j == Ny) ? c - pc : c + pc;
-    filter_centre(I.q, I.r, c, lo, hi, j == 1 || j == Ny, f, four);
+  const int j0 = first + 2 * g;
+  out = out && (wall || j0 <= last);
+  const bool two = wall || j0 < last;
+  int row[4];
+  if (wall) {
+    // U, W: f_1, f_2 next to each wall; V: the face sums there are V(1) and
+    // V(1) + V(2) (V is zero on the wall)
+    row[0] = 1; row[1] = 2;
+    row[2] = vlike ? Ny - 1 : Ny; row[3] = row[2] - 1;
+  } else {
+    const int j = min(j0, last);
+    row[1] = j;
+    row[0] = j == first ? j + 1 : j - 1;
+    row[2] = j == last ? j - 1 : j + 1;
+    row[3] = j + 1 >= last ? j : j + 2;
   }
-  I.r[15][c] = fy(I.U[s_in], c, pc, j, 0, Ny + 1, f, four);
-  I.r[17][c] = fy(I.W[s_in], c, pc, j, 0, Ny + 1, f, four);
-  if (j <= Ny) {
-    const size_t v = vidx(I, i, j, k);
-    I.r[16][v] = fy(I.V[s_in], v, pc, j, 0, Ny, f, four);
+  const int e = conv ? filt_exp(I, min(g, (Ny - 1) / 2)) : 0;
+  const int down = field >= 12 ? 1 : 0;        // the velocities' copies are below 2^61
+  const unsigned pitch = (unsigned)f.nxp * (unsigned)nrow;
+  const unsigned off0 = f.nxp * row[0] + pi, off1 = f.nxp * row[1] + pi, off2 = f.nxp * row[2] + pi, off3 = f.nxp * row[3] + pi;
+  auto get = [&](longlong2 v) {
+    if (conv) return Pair{fx_from(__longlong_as_double(v.x), e), fx_from(__longlong_as_double(v.y), e)};
+    return Pair{v.x >> down, v.y >> down};
+  };
+  const int k0 = zc * f.M, k1 = min(Nz, k0 + f.M);
+  int k = k0 == 0 ? Nz - 1 : k0 - 1;
+  const longlong2* s = src + (size_t)pitch * k;
+  longlong2 n0 = __ldg(s + off0), n1 = __ldg(s + off1), n2 = __ldg(s + off2), n3 = __ldg(s + off3);
+  Pair a0 = {0, 0}, a1 = {0, 0}, b0 = {0, 0}, b1 = {0, 0};      // the planes k - 2 and k - 1 of both rows
+  for (int it = 0; it < k1 - k0 + 2; ++it) {
+    const Pair v0 = get(n0), v1 = get(n1), v2 = get(n2), v3 = get(n3);
+    k = k + 1 == Nz ? 0 : k + 1;
+    if (it < k1 - k0 + 1) {
+      s = src + (size_t)pitch * k;
+      n0 = __ldg(s + off0); n1 = __ldg(s + off1); n2 = __ldg(s + off2); n3 = __ldg(s + off3);
+    }
+    Pair y0, y1;
+    if (wall) {
+      y0 = one_sided(v0, vlike ? Pair{v0.x + v1.x, v0.y + v1.y} : v1);
+      y1 = one_sided(v2, vlike ? Pair{v2.x + v3.x, v2.y + v3.y} : v3);
+    } else {
+      y0 = tap(v0, v1, v2);
+      y1 = tap(v1, v2, v3);
+    }
+    longlong2 (*buf)[256] = sm[it & 1];
+    buf[0][tid] = make_longlong2(y0.x, y0.y);
+    buf[1][tid] = make_longlong2(y1.x, y1.y);
+    __syncthreads();
+    const fx l0 = buf[0][left].y, r0 = buf[0][right].x, l1 = buf[1][left].y, r1 = buf[1][right].x;
+    const Pair x0 = {(l0 + 4 * y0.x + y0.y) >> 3, (y0.x + 4 * y0.y + r0) >> 3};
+    const Pair x1 = {(l1 + 4 * y1.x + y1.y) >> 3, (y1.x + 4 * y1.y + r1) >> 3};
+    if (it >= 2 && out) {
+      const Pair z0 = tap(a0, b0, x0), z1 = tap(a1, b1, x1);
+      // wall fields go to rows 1 and Ny of a centre-like field
+      const int nr = wall ? Ny + 2 : nrow, ra = wall ? 1 : j0, rc = wall ? Ny : j0 + 1;
+      longlong2* d = dst + (size_t)f.nxp * ((size_t)nr * (k0 + it - 2)) + pi;
+      d[(size_t)f.nxp * ra] = make_longlong2(z0.x, z0.y);
+      if (two) d[(size_t)f.nxp * rc] = make_longlong2(z1.x, z1.y);
+    }
+    a0 = b0; a1 = b1; b0 = x0; b1 = x1;
   }
-}
-
-// x pass over point pairs: thread (pair, j, k) forms x points i = 2 pair and
-// i + 1 from the 16-byte pairs to its left, at itself and to its right
-// (periodic; Nx is even and every row starts on a pair, so the pairs are
-// 16-byte aligned) and stores its two results as one pair: three vector
-// loads and one vector store per component for two points, instead of six
-// loads and two stores.  Same arithmetic and operand order as the one-point
-// pass, so bit-identical.  r -> q.
-template <int N0, int N>
-__device__ __forceinline__ void filter_x2_group(double* const* in, double* const* out, size_t cl, size_t cc,
-                                                size_t cr, const F64& f, double four) {
-  double2 l[N], c[N], r[N];
-#pragma unroll
-  for (int q = 0; q < N; ++q) {
-    const double2* g = reinterpret_cast<const double2*>(in[N0 + q]);
-    l[q] = __ldg(g + cl); c[q] = __ldg(g + cc); r[q] = __ldg(g + cr);
-  }
-#pragma unroll
-  for (int q = 0; q < N; ++q)
-    reinterpret_cast<double2*>(out[N0 + q])[cc] =
-        make_double2(fma(four, c[q].x, f.add(l[q].y, c[q].y)), fma(four, c[q].y, f.add(c[q].x, r[q].x)));
-}
-
-__global__ void __launch_bounds__(256)
-k_filter_x2(ChlMap map) {
-  chl_pdl_wait();
-  int lb;
-  const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
-  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
-  const int nxp = Nx / 2;
-  const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  if (t >= (unsigned)(nxp * (Ny + 2) * Nz)) return;
-  const ChlIdx p = chl_split(t, nxp, Ny + 2);
-  const int pi = p.i, j = p.j, k = p.k;
-  const int pl = pi == 0 ? nxp - 1 : pi - 1, pr = pi == nxp - 1 ? 0 : pi + 1;
-  const F64 f = f64_of(I);
-  const double four = I.fk[FK_FOUR];
-  double* const* in = I.r;
-  double* const* out = I.q;
-  // pair indices: row (j, k) of the centre-like layout starts at pair nxp (j + (Ny+2) k)
-  const size_t rc = (size_t)nxp * ((size_t)j + (size_t)(Ny + 2) * k);
-  if (j >= 1 && j <= Ny) {
-    filter_x2_group<3, 6>(in, out, rc + pl, rc + pi, rc + pr, f, four);
-    filter_x2_group<9, 6>(in, out, rc + pl, rc + pi, rc + pr, f, four);
-    if (j == 1 || j == Ny) filter_x2_group<0, 3>(in, out, rc + pl, rc + pi, rc + pr, f, four);
-  }
-  filter_x2_group<15, 1>(in, out, rc + pl, rc + pi, rc + pr, f, four);
-  filter_x2_group<17, 1>(in, out, rc + pl, rc + pi, rc + pr, f, four);
-  if (j <= Ny) {
-    const size_t rv = (size_t)nxp * ((size_t)j + (size_t)(Ny + 1) * k);   // the V-like layout
-    filter_x2_group<16, 1>(in, out, rv + pl, rv + pi, rv + pr, f, four);
-  }
-}
-
-// z pass over plane pairs: thread (i, j, pair) forms planes k = 2 pair and
-// k + 1 from planes k - 1 .. k + 2 (periodic), so each output takes two
-// loads instead of three, all of them independent (the neighbours lie a
-// plane apart, mostly in L2).  Same arithmetic and operand order as the
-// one-plane pass, so bit-identical.  Nz is even (chl_create: nz even), so
-// the planes pair up.  q -> r.
-template <int N0, int N>
-__device__ __forceinline__ void filter_z2_group(double* const* in, double* const* out, size_t km, size_t ka,
-                                                size_t kb, size_t kc, const F64& f, double four) {
-  double a[N], b[N], c[N], d[N];
-#pragma unroll
-  for (int q = 0; q < N; ++q) {
-    const double* g = in[N0 + q];
-    a[q] = LDG(g + km); b[q] = LDG(g + ka); c[q] = LDG(g + kb); d[q] = LDG(g + kc);
-  }
-#pragma unroll
-  for (int q = 0; q < N; ++q) {
-    out[N0 + q][ka] = fma(four, b[q], f.add(a[q], c[q]));
-    out[N0 + q][kb] = fma(four, c[q], f.add(b[q], d[q]));
-  }
-}
-
-__global__ void __launch_bounds__(256)
-k_filter_z2(ChlMap map) {
-  chl_pdl_wait();
-  int lb;
-  const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
-  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
-  const int npair = Nz / 2;
-  const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  if (t >= (unsigned)(Nx * (Ny + 2) * npair)) return;
-  const ChlIdx p = chl_split(t, Nx, Ny + 2);
-  const int i = p.i, j = p.j, k0 = 2 * p.k;
-  const int km = k0 == 0 ? Nz - 1 : k0 - 1, kb = k0 + 1, kc = k0 + 2 == Nz ? 0 : k0 + 2;
-  const F64 f = f64_of(I);
-  const double four = I.fk[FK_FOUR];
-  double* const* in = I.q;
-  double* const* out = I.r;
-  const size_t c0 = cidx(I, i, j, km), c1 = cidx(I, i, j, k0), c2 = cidx(I, i, j, kb), c3 = cidx(I, i, j, kc);
-  if (j >= 1 && j <= Ny) {
-    filter_z2_group<3, 6>(in, out, c0, c1, c2, c3, f, four);
-    filter_z2_group<9, 6>(in, out, c0, c1, c2, c3, f, four);
-    if (j == 1 || j == Ny) filter_z2_group<0, 3>(in, out, c0, c1, c2, c3, f, four);
-  }
-  filter_z2_group<15, 1>(in, out, c0, c1, c2, c3, f, four);
-  filter_z2_group<17, 1>(in, out, c0, c1, c2, c3, f, four);
-  if (j <= Ny)
-    filter_z2_group<16, 1>(in, out, vidx(I, i, j, km), vidx(I, i, j, k0), vidx(I, i, j, kb), vidx(I, i, j, kc), f, four);
 }
 
 // ------------------------------------------------------------ L:M, M:M
 // One block of CHL_DSMF_THREADS per (centre row jc, chunk of the row's
-// chl_dsm_points points); each thread sums its points in a fixed order and
-// writes its partials to part[0|1][jc][chunk][thread] (no reduction tree in
-// every block: its mostly idle warps would issue an FP64 instruction per
-// level for a handful of lanes).  Filtered fields live in r after the three
-// passes.  The last block of a row to finish (a counter per row) adds the
-// row's partials - thread t the entries t, t + CHL_DSMF_THREADS, ... in
-// order, then a fixed-order block tree - and writes the row's coefficient
-// -1/2 <LM>/<MM>, then returns the counter to 0.
+// columns); a column is an x position and chl_dsm_planes planes, which its
+// thread marches through (chl_strain.cuh, on the filtered faces).  Each
+// thread writes its partial sums to part[0|1][jc][chunk][thread] (no
+// reduction tree in every block: its mostly idle warps would issue an FP64
+// instruction per level for a handful of lanes).  The last block of a row to
+// finish (a counter per row) adds the row's partials - thread t the entries
+// t, t + CHL_DSMF_THREADS, ... in order, then a fixed-order block tree - and
+// writes the row's coefficient -1/2 <LM>/<MM>, then returns the counter to 0.
+// L_ij is an integer difference (filtered products less products of filtered
+// velocities, which cancel to a hundredth), M_ij and the sums are FP64.
 __device__ __forceinline__ void block_sum2(double* sl, double* sm, double& a, double& b) {
   sl[threadIdx.x] = a; sm[threadIdx.x] = b;
   __syncthreads();
@@ -381,12 +245,10 @@ __device__ __forceinline__ void block_sum2(double* sl, double* sm, double& a, do
   a = sl[0]; b = sm[0];
 }
 
-// -1/2 <LM>/<MM>: the filter and average scales give 1/8 (see the scaling
-// note above); L and M are both stored / 216, so <LM>/<MM> = lm/mm (times
-// the sqrt(2) that the strain leaves out).  Whole block; every thread gets it.
-// Thread t adds the partials of chunks t mod 4 = 0..3 into four chains
-// (their loads in flight together: on a small instance this tail is
-// latency, not throughput), then the chains in a fixed order.
+// -1/2 <LM>/<MM> (L and M both 216/512 of their values).  Whole block; every
+// thread gets it.  Thread t adds the partials of chunks t mod 4 = 0..3 into
+// four chains (their loads in flight together: on a small instance this tail
+// is latency, not throughput), then the chains in a fixed order.
 __device__ __forceinline__ double dsm_row_coef(const ChlInst& I, int jc, double* sl, double* sm) {
   const int np = I.npart;
   const size_t n = (size_t)np * CHL_DSMF_THREADS;
@@ -408,82 +270,75 @@ __device__ __forceinline__ double dsm_row_coef(const ChlInst& I, int jc, double*
   double lm = (l[0] + l[1]) + (l[2] + l[3]), mm = (m[0] + m[1]) + (m[2] + m[3]);
   __syncthreads();
   block_sum2(sl, sm, lm, mm);
-  return -0.125 * (lm / mm);
+  return -0.5 * (lm / mm);
 }
 
-// One thread's points of row jc: the diagonal and off-diagonal parts of L:M
-// and M:M, each a chain of FMAs straight into its accumulator (the
-// off-diagonal scales 1/4 and 1/32 are applied once by the caller).  The
-// point set is the plane followed by the reference's duplicated periodic
-// column and plane (chl_dsm_points), so every point has weight 1.
-// WALL: row 1 or Ny, whose filtered centre velocities were filtered in their
-// own right; a template parameter rather than a per-point select, since the
-// row is the same for the whole block.
-template <bool WALL, bool PAIR>
-__device__ __forceinline__ void dsm_sums(const ChlInst& I, int jc, int chunk, double& ald, double& alo,
-                                         double& amd, double& amo) {
-  const int Nx = I.Nx, Nz = I.Nz;
-  const int plane = Nx * Nz, npts = chl_dsm_points(Nx, Nz);
-  const double* const* R = I.r;
-  const int ppt = I.dsm_ppt;
-  for (int m = 0; m < ppt; ++m) {
-    const int pidx = chunk * (CHL_DSMF_THREADS * ppt) + m * CHL_DSMF_THREADS + threadIdx.x;
-    if (pidx >= npts) break;
-    int i, k;
-    if (pidx < plane) { i = pidx % Nx; k = pidx / Nx; }
-    else {                                   // the duplicated column, plane and (0, 0)
-      const int e = pidx - plane;
-      i = e < Nz ? 0 : (e < Nz + Nx ? e - Nz : 0);
-      k = e < Nz ? e : 0;
-    }
-    const size_t c = cidx(I, i, jc, k);
-    const Faces f = centre_faces(I, R[15], R[16], R[17], i, jc, k);    // 216 x filtered faces
-    const Strain h = centre_strain<true, PAIR>(I, f, i, jc, k);               // sqrt(4/216) x 216 x filtered strain
-    // M_ij / 216: the 216 of the filtered |S| S_ij terms moves into the
-    // strain factor (4/216, as sqrt(4/216) in each of |S| and S_ij, from the
-    // scaled reciprocals); L_ij / 216: the filtered velocities are divided
-    // once, each product is then one FMA; k_coef's constant carries both
-    const double M1 = fma(h.s, h.d1, -LDG(R[9] + c));
-    const double M2 = fma(h.s, h.d2, -LDG(R[10] + c));
-    const double M3 = fma(h.s, h.d3, -LDG(R[11] + c));
-    const double M4 = fma(h.s, h.o12, -LDG(R[12] + c));
-    const double M5 = fma(h.s, h.o13, -LDG(R[13] + c));
-    const double M6 = fma(h.s, h.o23, -LDG(R[14] + c));
-    // 2 x 216 x filtered centre velocities: filtered in their own right on
-    // the wall rows, the centre average of the filtered faces elsewhere
-    const double fu = WALL ? LDG(R[0] + c) : f.u0 + f.u1;
-    const double fv = WALL ? LDG(R[1] + c) : f.v0 + f.v1;
-    const double fw = WALL ? LDG(R[2] + c) : f.w0 + f.w1;
-    const double gu = fu * (1.0 / 216.0), gv = fv * (1.0 / 216.0);
-    const double L1 = fma(-gu, fu, LDG(R[3] + c));
-    const double L2 = fma(-gv, fv, LDG(R[4] + c));
-    const double L3 = fma(-fw * (1.0 / 216.0), fw, LDG(R[5] + c));
-    const double L4 = fma(-gu, fv, LDG(R[6] + c));
-    const double L5 = fma(-gu, fw, LDG(R[7] + c));
-    const double L6 = fma(-gv, fw, LDG(R[8] + c));
-    ald = fma(L1, M1, ald); ald = fma(L2, M2, ald); ald = fma(L3, M3, ald);
-    alo = fma(L4, M4, alo); alo = fma(L5, M5, alo); alo = fma(L6, M6, alo);
-    amd = fma(M1, M1, amd); amd = fma(M2, M2, amd); amd = fma(M3, M3, amd);
-    amo = fma(M4, M4, amo); amo = fma(M5, M5, amo); amo = fma(M6, M6, amo);
-  }
-}
+struct LMSums { double ld, lo, md, mo; };   // diagonal and off-diagonal parts of L:M and M:M
+// Doubles a column's sums so far: the reference counts plane 0 (and x position
+// 0) twice.  A call, so that its FP64 instructions are not predicated into
+// every point.
+static __device__ __noinline__ void twice(LMSums& s) { s.ld *= 2.0; s.lo *= 2.0; s.md *= 2.0; s.mo *= 2.0; }
 
-template <bool PAIR>
+#define DSM_C 0x4BDA12F684BDA12FLL     // 2048/216 / 32 2^64
 __global__ void __launch_bounds__(CHL_DSMF_THREADS)
-k_dsm_final(ChlMap map) {
+k_dsm_final(ChlMap map, int s_in) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
-  const int Ny = I.Ny;
+  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
   const int np = I.npart;
   const int jc = 1 + lb / np, chunk = lb % np;
-  double ald = 0.0, alo = 0.0, amd = 0.0, amo = 0.0;
-  if (jc == 1 || jc == Ny) dsm_sums<true, PAIR>(I, jc, chunk, ald, alo, amd, amo);
-  else dsm_sums<false, PAIR>(I, jc, chunk, ald, alo, amd, amo);
+  const unsigned col = (unsigned)chunk * CHL_DSMF_THREADS + threadIdx.x;
+  const unsigned kc = col / (unsigned)Nx;
+  const int i = (int)(col - kc * (unsigned)Nx), k0 = (int)kc * I.dsm_planes, k1 = min(Nz, k0 + I.dsm_planes);
+  const bool wall = jc == 1 || jc == Ny;
+  LMSums a = {0.0, 0.0, 0.0, 0.0};
+  if (k0 < k1) {
+    const unsigned* vm = chl_vmax(I, s_in);
+    const int eu = fx_exp<60>(vm[0]), ev = fx_exp<60>(vm[1]), ew = fx_exp<60>(vm[2]);
+    const int es = filt_exp(I, (jc - 1) / 2);
+    const fx* const* R = reinterpret_cast<const fx* const*>(I.r);
+    StrainColumn c(I, R[15], R[16], R[17], eu, ev, ew, i, jc, k0);
+    for (int k = k0; k < k1; ++k) {
+      fx f[3];
+      const Strain h = c.point(k, f);
+      const size_t o = cidx(I, i, jc, k);
+      if (wall) {          // the centre velocities filtered in their own right
+        f[0] = LDG(R[0] + cidx(I, c.im, jc, k)) + LDG(R[0] + o);
+        f[1] = LDG(R[1] + o);
+        f[2] = LDG(R[2] + cidx(I, i, jc, k == 0 ? Nz - 1 : k - 1)) + LDG(R[2] + o);
+      }
+      // M_ij: 4 |S^| S^_ij less the filtered |S| S_ij, the strain 216/512 of its value
+      const double hs = h.s * (4.0 * 512.0 / 216.0);
+      const double M1 = fma(hs, h.d1, -fx_to(LDG(R[9] + o), es));
+      const double M2 = fma(hs, h.d2, -fx_to(LDG(R[10] + o), es));
+      const double M3 = fma(hs, h.d3, -fx_to(LDG(R[11] + o), es));
+      const double M4 = fma(hs, h.o12, -fx_to(LDG(R[12] + o), es));
+      const double M5 = fma(hs, h.o13, -fx_to(LDG(R[13] + o), es));
+      const double M6 = fma(hs, h.o23, -fx_to(LDG(R[14] + o), es));
+      // L_ij: f are the filtered face sums, 216/512 of their value and in
+      // units twice the copies'; g = 512/216 f / 8
+      const fx g0 = fx_mul(2 * f[0], DSM_C), g1 = fx_mul(2 * f[1], DSM_C), g2 = fx_mul(2 * f[2], DSM_C);
+#define PROD(g, h) fx_mul_shr<62>(2 * (g), 2 * (h))
+      const double L1 = fx_to(LDG(R[3] + o) - PROD(g0, f[0]), eu + eu + 60);
+      const double L2 = fx_to(LDG(R[4] + o) - PROD(g1, f[1]), ev + ev + 60);
+      const double L3 = fx_to(LDG(R[5] + o) - PROD(g2, f[2]), ew + ew + 60);
+      const double L4 = fx_to(LDG(R[6] + o) - PROD(g0, f[1]), eu + ev + 60);
+      const double L5 = fx_to(LDG(R[7] + o) - PROD(g0, f[2]), eu + ew + 60);
+      const double L6 = fx_to(LDG(R[8] + o) - PROD(g1, f[2]), ev + ew + 60);
+#undef PROD
+      a.ld = fma(L1, M1, a.ld); a.ld = fma(L2, M2, a.ld); a.ld = fma(L3, M3, a.ld);
+      a.lo = fma(L4, M4, a.lo); a.lo = fma(L5, M5, a.lo); a.lo = fma(L6, M6, a.lo);
+      a.md = fma(M1, M1, a.md); a.md = fma(M2, M2, a.md); a.md = fma(M3, M3, a.md);
+      a.mo = fma(M4, M4, a.mo); a.mo = fma(M5, M5, a.mo); a.mo = fma(M6, M6, a.mo);
+      if (k == 0) twice(a);
+    }
+    if (i == 0) twice(a);
+  }
   const size_t n = (size_t)np * CHL_DSMF_THREADS;
   const size_t q = (size_t)jc * n + (size_t)chunk * CHL_DSMF_THREADS + threadIdx.x;
-  I.part[q] = fma(0.25, alo, ald);
-  I.part[(size_t)(Ny + 2) * n + q] = fma(0.03125, amo, amd);
+  I.part[q] = fma(0.25, a.lo, a.ld);
+  I.part[(size_t)(Ny + 2) * n + q] = fma(0.03125, a.mo, a.md);
   __threadfence();
   __shared__ double sl[CHL_DSMF_THREADS], sm[CHL_DSMF_THREADS];
   __shared__ int last;
@@ -642,23 +497,17 @@ k_nut(ChlMap map, int s_in, int use_wm) {
 
 // ------------------------------------------------------------ launchers
 extern "C" {
-// pair: the x-pair form (k_edges_pair on its row map, blocks of pair threads)
-void chl_launch_edges(const ChlMap& m, int nb, int src, int pair, cudaStream_t st) {
-  if (pair) chl_launch_pdl(k_edges_pair, dim3(nb), dim3(pair), 0, st, m, src);
-  else chl_launch_pdl(k_edges, dim3(nb), dim3(m.tb), 0, st, m, src);
+void chl_launch_strain(const ChlMap& m, int nb, int s_in, int dsm, cudaStream_t st) {
+  if (dsm) chl_launch_pdl(k_strain<true>, dim3(nb), dim3(CHL_FLUX_THREADS), 0, st, m, s_in);
+  else chl_launch_pdl(k_strain<false>, dim3(nb), dim3(CHL_FLUX_THREADS), 0, st, m, s_in);
 }
-void chl_launch_centre(const ChlMap& m, int nb, int s_in, int dsm, int pair, cudaStream_t st) {
-  if (dsm && pair) chl_launch_pdl(k_centre<true, true>, dim3(nb), dim3(m.tb), 0, st, m, s_in);
-  else if (dsm) chl_launch_pdl(k_centre<true, false>, dim3(nb), dim3(m.tb), 0, st, m, s_in);
-  else if (pair) chl_launch_pdl(k_centre<false, true>, dim3(nb), dim3(m.tb), 0, st, m, s_in);
-  else chl_launch_pdl(k_centre<false, false>, dim3(nb), dim3(m.tb), 0, st, m, s_in);
+int chl_filter_blocks(int Nx, int Ny, int Nz, int T) {
+  const FiltShape f = filt_shape(Nx, Ny, Nz, T);
+  return FILT_FIELDS * f.full + 3 * f.segs * f.nz;
 }
-void chl_launch_filter_y(const ChlMap& m, int nb, int s_in, cudaStream_t st) { chl_launch_pdl(k_filter_y, dim3(nb), dim3(m.tb), 0, st, m, s_in); }
-void chl_launch_filter_x(const ChlMap& m, int nb, cudaStream_t st) { chl_launch_pdl(k_filter_x2, dim3(nb), dim3(m.tb), 0, st, m); }
-void chl_launch_filter_z(const ChlMap& m, int nb, cudaStream_t st) { chl_launch_pdl(k_filter_z2, dim3(nb), dim3(m.tb), 0, st, m); }
-void chl_launch_dsm_final(const ChlMap& m, int nb, int pair, cudaStream_t st) {
-  if (pair) chl_launch_pdl(k_dsm_final<true>, dim3(nb), dim3(CHL_DSMF_THREADS), 0, st, m);
-  else chl_launch_pdl(k_dsm_final<false>, dim3(nb), dim3(CHL_DSMF_THREADS), 0, st, m);
+void chl_launch_filter(const ChlMap& m, int nb, int T, cudaStream_t st) { chl_launch_pdl(k_filter, dim3(nb), dim3(T), 0, st, m); }
+void chl_launch_dsm_final(const ChlMap& m, int nb, int s_in, cudaStream_t st) {
+  chl_launch_pdl(k_dsm_final, dim3(nb), dim3(CHL_DSMF_THREADS), 0, st, m, s_in);
 }
 void chl_launch_coef(const ChlMap& m, cudaStream_t st) { chl_launch_pdl(k_coef, dim3(m.n), dim3(128), 0, st, m); }
 void chl_launch_eqwm(const ChlMap& m, int nb, int s_in, cudaStream_t st) { chl_launch_pdl(k_eqwm, dim3(nb), dim3(CHL_WALL_THREADS), 0, st, m, s_in); }

@@ -126,15 +126,6 @@ __device__ __forceinline__ unsigned write_nut_rows(const ChlInst& I, const doubl
 
 }  // namespace
 
-// One's-complement magnitudes of the high words, or-ed: the bit length of the
-// result is that of the largest of them.
-__device__ __forceinline__ void top_or(unsigned& m, fx a) {
-  const int h = (int)(a >> 32);
-  m |= (unsigned)(h ^ (h >> 31));
-}
-// a 2^s for s of either sign (toward minus infinity)
-__device__ __forceinline__ fx scale2(fx a, int s) { return (a << max(s, 0)) >> max(-s, 0); }
-
 // AMD in fixed point.  As FP64 code this kernel issued 114 FP64 instructions
 // per point (0.97 ms per launch at 256x96x192, the FP64 pipe 90 % busy).  The
 // edge differences are exact integers from the fixed-point copies (k_fix);

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from channel_rl_gb300 import cases as C
-from tests.helpers import FIELD_RTOL, oracle_for, regions, rel
+from tests.helpers import FIELD_RTOL, NUT_RTOL, oracle_for, regions, rel
 
 pytestmark = pytest.mark.gpu
 
@@ -34,6 +34,25 @@ def test_projection_of_every_radix_mix(Nx, Nz):
         r = reg[f][0], slice(1, -1), reg[f][2]      # the oracle leaves the ghost rows to the boundary conditions
         assert rel(d[f][r], getattr(o, f)[1:, 1:, 1:][r]) < FIELD_RTOL, f
     ch.close()
+
+
+# the test filter's blocks: several x-lines, one line, a line cut into
+# segments (more than 256 point pairs); one and two rows in the last group
+@pytest.mark.parametrize("Nx,Ny,Nz", ((4, 8, 6), (6, 9, 4), (18, 6, 32), (256, 7, 6), (512, 6, 4), (576, 7, 4), (1024, 5, 4)))
+def test_dynamic_model_over_line_lengths(Nx, Ny, Nz):
+    from channel_rl_gb300.host import Channel
+    case = C.smaller(C.c1_small(), Nx, Ny, Nz)
+    U, V, W = C.initial_fields(case)
+    o = oracle_for(case)
+    o.set_fields(U, V, W)
+    o.compute_eddy_viscosity()
+    ch = Channel(case)
+    ch.upload(U, V, W)
+    ch.compute_eddy_viscosity()
+    nt = ch.download(fields=("nu_t",))["nu_t"]
+    ch.close()
+    reg = regions(o.g)["C"]
+    assert rel(nt[reg], o.nu_t[1:, 1:, 1:][reg]) < NUT_RTOL
 
 
 def _rhs(case, U, V, W):
