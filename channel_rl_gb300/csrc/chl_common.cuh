@@ -113,6 +113,7 @@ struct ChlInst {
   double dt_vis;                // viscous limit of compute_dt, min(CFL d^2/nu) over x, y, z (host-formed)
   double dyw;                   // yg(2)-yg(1), used for both walls (wallmodel.f90:32-35)
   double hb, ht;                // matching heights of the log-law wall model
+  double hnb, hnt;              // hb/nu, ht/nu
   double cbc1, cbc2;            // coef_bc_1*(yg(2)-yg(1)), coef_bc_2*(yg(nyg)-yg(nyg-1))
   double ybot, ytop;            // y(1), y(ny)
   double dy1;                   // y(2)-y(1) (nu_t ghost rule 2 of AMD and Vreman)
@@ -295,9 +296,10 @@ __device__ __forceinline__ int chl_find(const ChlMap& m, int b, int& local) {
 // unsigned arithmetic (an instance has fewer than 2^31 points, checked at
 // creation): the 64-bit divisions this replaces were long integer sequences
 // ahead of every kernel's first load.
-// Planes (consecutive k) per thread of the flux kernel: 4, halved while the
-// instance would have fewer than 4 x 256 threads per SM (at 256x96x192 one,
-// two, four and eight planes take 211, 184, 172 and 174 us).
+// Planes (consecutive k) per thread of the kernels that march (flux, strain,
+// AMD): 4, halved while the instance would have fewer than 4 x 256 threads
+// per SM (at 256x96x192 one, two, four, eight and sixteen planes: k_flux 211,
+// 181, 172, 174, 181 us, k_strain -, 238, 200, 202, 204 us).
 #define CHL_FLUX_THREADS 128
 __host__ __device__ inline int chl_planes(int Nx, int Ny, int Nz) {
   int m = 4;
@@ -375,7 +377,9 @@ __device__ __forceinline__ double nut_ghost(const ChlInst& I, double v) {
 // launched with programmatic stream serialisation, so its blocks may be
 // scheduled while the previous kernel drains, and waits here, first thing,
 // until that kernel has finished and its writes are visible.  Without the
-// launch attribute the wait returns at once.
+// launch attribute the wait returns at once.  (No kernel triggers its
+// successor early: with a trigger ahead of or behind the wait the 32x48x32
+// step took 324 or 296 us instead of 252, the 256x96x192 one 1-5 % more.)
 __device__ __forceinline__ void chl_pdl_wait() {
 #if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ >= 900)
   cudaGridDependencySynchronize();

@@ -38,19 +38,27 @@ __device__ __forceinline__ fx fx_from(double x, int e) {
   return b < 0 ? -(fx)f : (fx)f;
 }
 
-// F 2^e as a double, rounded to nearest; results below the normal range give
-// zero, above it infinity
+// F 2^e as a double, rounded to nearest (the magnitude of a negative F is
+// taken one unit short, which saves the carry); exponents beyond a double's
+// give its smallest and largest magnitudes
 __device__ __forceinline__ double fx_to(fx f, int e) {
-  const unsigned long long a = f < 0 ? 0ULL - (unsigned long long)f : (unsigned long long)f;
-  const int lz = __clzll((long long)a);
+  const int sign = (int)(f >> 63);
+  const unsigned hi = (unsigned)(f >> 32) ^ (unsigned)sign, lo = (unsigned)f ^ (unsigned)sign;
+  const int lz = hi ? __clz((int)hi) : 32 + __clz((int)lo);
   unsigned long long n;
-  asm("shl.b64 %0, %1, %2;" : "=l"(n) : "l"(a), "r"(lz));
-  int ef = e + 1085 - lz;
-  const unsigned long long m = (n >> 11) + ((n >> 10) & 1ULL);
-  unsigned long long r = m + ((unsigned long long)(unsigned)ef << 52);
-  if (ef < 0 || a == 0) r = 0;
-  if (ef > 0x7FD && a != 0) r = 0x7FF0000000000000ULL;
-  return __longlong_as_double((long long)(r | ((unsigned long long)f & 0x8000000000000000ULL)));
+  asm("shl.b64 %0, %1, %2;" : "=l"(n) : "l"(((unsigned long long)hi << 32) | lo), "r"(lz));
+  const int ef = min(max(e + 1085 - lz, 0), 2045);
+  unsigned long long r = (n >> 11) + ((n >> 10) & 1ULL) + ((unsigned long long)(unsigned)ef << 52);
+  unsigned rh = (unsigned)(r >> 32);
+  if (lz == 64) rh = 0u;
+  return __hiloint2double((int)(rh | ((unsigned)sign & 0x80000000u)), (int)(unsigned)r);
+}
+// F as a double, on the FP64 pipe (64 clocks, no other) or the integer pipe
+template <bool HW>
+__device__ __forceinline__ double fx_raw(fx f) { return HW ? __ll2double_rn(f) : fx_to(f, 0); }
+// x 2^e for a normal x and result (an addition to the exponent)
+__device__ __forceinline__ double scale_exp(double x, int e) {
+  return __hiloint2double(__double2hiint(x) + (e << 20), __double2loint(x));
 }
 
 // 2^e as a double, -1022 <= e <= 1023

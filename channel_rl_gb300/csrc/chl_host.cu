@@ -433,6 +433,7 @@ static int upload_consts(chl_handle* h, Inst& I) {
   D.dyw = c.yg[2] - c.yg[1];
   D.hb = c.yg[4] - c.yf[1];
   D.ht = c.yf[c.ny] - c.yg[c.nyg - 3];
+  D.hnb = D.hb / D.nu; D.hnt = D.ht / D.nu;
   D.cbc1 = c.coef_bc_1 * (c.yg[2] - c.yg[1]);
   D.cbc2 = c.coef_bc_2 * (c.yg[c.nyg] - c.yg[c.nyg - 1]);
   D.ybot = c.yf[1]; D.ytop = c.yf[c.ny];

@@ -21,10 +21,10 @@
 // ---------------------------------------------------------------- strain
 // Strain magnitude and the DSM filter inputs at centres (rows 1..Ny): q3..8
 // the products of the centre velocities' face sums in fixed point (last bit
-// 2^(e_i + e_j + 64)), q9..14 = |S|*(S_ii, 8 S_ij) / sqrt(2) and their
+// 2^(e_i + e_j + 64)), q9..14 = |S|*(S_ii, 2 S_ij) / sqrt(2) and their
 // largest per row.
 template <bool DSM>
-__global__ void __launch_bounds__(CHL_FLUX_THREADS, 4)
+__global__ void __launch_bounds__(CHL_FLUX_THREADS, 7)
 k_strain(ChlMap map, int s_in) {
   chl_pdl_wait();
   int lb;
@@ -48,7 +48,10 @@ k_strain(ChlMap map, int s_in) {
       fx* const* q = reinterpret_cast<fx* const*>(I.q);
       q[3][c] = fx_mul(f[0], f[0]); q[4][c] = fx_mul(f[1], f[1]); q[5][c] = fx_mul(f[2], f[2]);
       q[6][c] = fx_mul(f[0], f[1]); q[7][c] = fx_mul(f[0], f[2]); q[8][c] = fx_mul(f[1], f[2]);
-      const double m[6] = {s.s * s.d1, s.s * s.d2, s.s * s.d3, s.s * s.o12, s.s * s.o13, s.s * s.o23};
+      const double se = s.s * pow2(min(1023, max(-1022, s.e)));
+      // two of the six conversions on the FP64 pipe, which is the less busy
+      const double m[6] = {se * fx_raw<true>(s.t[0]), se * fx_raw<true>(s.t[1]), se * fx_raw<false>(s.t[2]),
+                           se * fx_raw<false>(s.t[3]), se * fx_raw<false>(s.t[4]), se * fx_raw<false>(s.t[5])};
 #pragma unroll
       for (int n = 0; n < 6; ++n) { I.q[9 + n][c] = m[n]; hi = max(hi, chl_abshi(m[n])); }
     }
@@ -245,7 +248,8 @@ __device__ __forceinline__ void block_sum2(double* sl, double* sm, double& a, do
   a = sl[0]; b = sm[0];
 }
 
-// -1/2 <LM>/<MM> (L and M both 216/512 of their values).  Whole block; every
+// -1/2 <LM>/<MM> (L and M both 216/512 of their values, M in units of
+// 2^filt_exp).  Whole block; every
 // thread gets it.  Thread t adds the partials of chunks t mod 4 = 0..3 into
 // four chains (their loads in flight together: on a small instance this tail
 // is latency, not throughput), then the chains in a fixed order.
@@ -270,7 +274,8 @@ __device__ __forceinline__ double dsm_row_coef(const ChlInst& I, int jc, double*
   double lm = (l[0] + l[1]) + (l[2] + l[3]), mm = (m[0] + m[1]) + (m[2] + m[3]);
   __syncthreads();
   block_sum2(sl, sm, lm, mm);
-  return -0.5 * (lm / mm);
+  const int es = filt_exp(I, (jc - 1) / 2);
+  return -0.5 * (lm / mm) * pow2(min(1023, max(-1022, -es)));
 }
 
 struct LMSums { double ld, lo, md, mo; };   // diagonal and off-diagonal parts of L:M and M:M
@@ -280,7 +285,7 @@ struct LMSums { double ld, lo, md, mo; };   // diagonal and off-diagonal parts o
 static __device__ __noinline__ void twice(LMSums& s) { s.ld *= 2.0; s.lo *= 2.0; s.md *= 2.0; s.mo *= 2.0; }
 
 #define DSM_C 0x4BDA12F684BDA12FLL     // 2048/216 / 32 2^64
-__global__ void __launch_bounds__(CHL_DSMF_THREADS)
+__global__ void __launch_bounds__(CHL_DSMF_THREADS, 14)
 k_dsm_final(ChlMap map, int s_in) {
   chl_pdl_wait();
   int lb;
@@ -308,14 +313,12 @@ k_dsm_final(ChlMap map, int s_in) {
         f[1] = LDG(R[1] + o);
         f[2] = LDG(R[2] + cidx(I, i, jc, k == 0 ? Nz - 1 : k - 1)) + LDG(R[2] + o);
       }
-      // M_ij: 4 |S^| S^_ij less the filtered |S| S_ij, the strain 216/512 of its value
-      const double hs = h.s * (4.0 * 512.0 / 216.0);
-      const double M1 = fma(hs, h.d1, -fx_to(LDG(R[9] + o), es));
-      const double M2 = fma(hs, h.d2, -fx_to(LDG(R[10] + o), es));
-      const double M3 = fma(hs, h.d3, -fx_to(LDG(R[11] + o), es));
-      const double M4 = fma(hs, h.o12, -fx_to(LDG(R[12] + o), es));
-      const double M5 = fma(hs, h.o13, -fx_to(LDG(R[13] + o), es));
-      const double M6 = fma(hs, h.o23, -fx_to(LDG(R[14] + o), es));
+      // M_ij: 4 |S^| S^_ij less the filtered |S| S_ij (off the diagonal twice
+      // that), 216/512 of its value and in units of the filtered fields
+      const double hs = h.s * scale_exp(4.0 * 512.0 / 216.0, min(900, max(-900, h.e - es)));
+#define MIJ(n) fma(hs, fx_raw<false>(h.t[n]), -fx_raw<(n) < 3>(LDG(R[9 + (n)] + o)))
+      const double M1 = MIJ(0), M2 = MIJ(1), M3 = MIJ(2), M4 = MIJ(3), M5 = MIJ(4), M6 = MIJ(5);
+#undef MIJ
       // L_ij: f are the filtered face sums, 216/512 of their value and in
       // units twice the copies'; g = 512/216 f / 8
       const fx g0 = fx_mul(2 * f[0], DSM_C), g1 = fx_mul(2 * f[1], DSM_C), g2 = fx_mul(2 * f[2], DSM_C);
@@ -337,8 +340,8 @@ k_dsm_final(ChlMap map, int s_in) {
   }
   const size_t n = (size_t)np * CHL_DSMF_THREADS;
   const size_t q = (size_t)jc * n + (size_t)chunk * CHL_DSMF_THREADS + threadIdx.x;
-  I.part[q] = fma(0.25, a.lo, a.ld);
-  I.part[(size_t)(Ny + 2) * n + q] = fma(0.03125, a.mo, a.md);
+  I.part[q] = a.lo + a.ld;
+  I.part[(size_t)(Ny + 2) * n + q] = fma(0.5, a.mo, a.md);
   __threadfence();
   __shared__ double sl[CHL_DSMF_THREADS], sm[CHL_DSMF_THREADS];
   __shared__ int last;
@@ -385,36 +388,64 @@ __global__ void k_coef(ChlMap map) {
 // Newton on f(ut) = ut (ln(h ut/nu)/kappa + B) - |u|.  f is convex and
 // increasing, so Newton converges from either side of the root (from the
 // left the first step lands right of it, then the iterates decrease).  The
-// start is `guess` (the previous stage's u_tau) when it lies above the
-// laminar estimate, which the root always does.  Convergence is quadratic
-// with relative constant 1/(2 kappa f') < 0.1 (f' = u+ + 1/kappa > 11 where
-// the log law applies), so once a correction is below 3e-8 of ut the error
-// left after it is below 0.09 * (3e-8)^2 < 1e-16, under half an ulp: the
-// iteration stops there and the root agrees with a fixed-count solve to
-// rounding.  The log of the
-// branch test is reused as the first iterate's when the start is laminar.
-// FP64 is the scarce pipe here: h/nu is formed once, 1/kappa is a constant
-// multiplier, and each iteration holds one log and one division.
-__device__ double eqlog_tau(double u, double h, double nu, double guess) {
+// log law applies only above its upper crossing with u+ = y+ (y+ ~ 11), i.e.
+// where ln(y+)/kappa + B < y+ at the laminar y+ = sqrt(|u| h/nu); below it
+// tau is the laminar |u| nu/h.
+//
+// The iteration in FP64 throughout, with a log and a division per step: for
+// points next to the crossing and magnitudes outside FP32.  hn = h/nu.
+static __device__ __noinline__ double eqlog_ut_fp64(double au, double hn) {
   const double inv_k = 1.0 / EQWM_KAPPA;   // folded at compile time
-  const double au = fabs(u);
-  const double hn = h / nu;
   const double ut_lam = sqrt(au / hn);
   const double yp_lam = hn * ut_lam;
-  const double l0 = log(yp_lam);
-  const double f0 = ut_lam * fma(l0, inv_k, EQWM_B) - au;
+  const double f0 = ut_lam * fma(log(yp_lam), inv_k, EQWM_B) - au;
   double ut = ut_lam;
-  // log law only above its upper crossing with u+ = y+ (y+ ~ 11)
   if (f0 < 0.0 && yp_lam >= 1.0) {
-    const bool warm = guess > ut_lam;
-    if (warm) ut = guess;
     for (int it = 0; it < 2 * EQWM_ITERS; ++it) {
-      const double lg = (it == 0 && !warm) ? l0 : log(hn * ut);
-      const double g = fma(lg, inv_k, EQWM_B);          // u+ at ut
-      const double d = fma(ut, g, -au) / (g + inv_k);   // f / f'
+      const double g = fma(log(hn * ut), inv_k, EQWM_B);          // u+ at ut
+      const double d = fma(ut, g, -au) / (g + inv_k);             // f / f'
       ut = ut - d;
       if (fabs(d) <= 3e-8 * ut) break;
     }
+  }
+  return ut;
+}
+// The same root from FP32 iterates, which the idle FP32 pipe gives for
+// nothing, and one FP64 step from them: with the iterate within 1e-6 of the
+// root, Halley's step (Newton's with the f'' f/(2 f'^2) term, needed to 1e-10
+// of itself only) leaves 1e-18.  One FP64 log per point instead of one per
+// iteration, and no FP64 division.
+__device__ __forceinline__ double eqlog_tau(double u, double hn, double prev) {
+  const double inv_k = 1.0 / EQWM_KAPPA;
+  const float ik = (float)(1.0 / EQWM_KAPPA), B = (float)EQWM_B;
+  const double au = fabs(u);
+  const float af = (float)au, hf = (float)hn;
+  const float yp = sqrtf(af * hf);
+  const float gap = yp - (logf(yp) * ik + B);          // > 0: log law (for yp >= 1)
+  double ut;
+  if (!(yp > 1e-12f && yp < 1e12f && hf > 1e-12f && hf < 1e12f && fabsf(gap) > 1e-4f * (yp + B))) {
+    ut = eqlog_ut_fp64(au, hn);
+  } else if (gap < 0.0f || yp < 1.0f) {
+    const double tau = au / hn;
+    return u < 0.0 ? -tau : tau;
+  } else {
+    const float lam = yp / hf, warm = sqrtf(fabsf((float)prev));
+    float x = warm > lam ? warm : lam;
+    for (int it = 0; it < 2 * EQWM_ITERS; ++it) {
+      const float g = logf(hf * x) * ik + B;
+      const float d = (x * g - af) / (g + ik);
+      x -= d;
+      if (fabsf(d) <= 1e-6f * x) break;
+    }
+    const double x0 = x;
+    const double g = fma(log(hn * x0), inv_k, EQWM_B);   // u+
+    const double r = fma(x0, g, -au), fp = g + inv_k;     // f and f'
+    double q;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(q) : "d"(fp));
+    double d = r * q;
+    d = fma(fma(-d, fp, r), q, d);
+    const double c = (0.5 * inv_k) * q * d;                        // f'' f / (2 f'^2) times ut
+    ut = x0 - fma(d, c * (double)(1.0f / x), d);
   }
   const double tau = ut * ut;
   return u < 0.0 ? -tau : (u > 0.0 ? tau : 0.0);
@@ -435,8 +466,7 @@ k_eqwm(ChlMap map, int s_in) {
   const int a = p.i, k = p.j, wall = p.k;
   const double* U = I.U[s_in];
   const double u = wall == 0 ? U[cidx(I, a, 3, k)] : U[cidx(I, a, Ny - 2, k)];
-  const double prev = I.alpha[t];
-  I.alpha[t] = eqlog_tau(u, wall == 0 ? I.hb : I.ht, I.nu, sqrt(fabs(prev)));
+  I.alpha[t] = eqlog_tau(u, wall == 0 ? I.hnb : I.hnt, I.alpha[t]);
 }
 
 // ------------------------------------------------------------ nu_t (+ wall model rows)

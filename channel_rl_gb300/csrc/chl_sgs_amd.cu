@@ -134,7 +134,7 @@ __device__ __forceinline__ unsigned write_nut_rows(const ChlInst& I, const doubl
 // the a_ij there.  N and the division are FP64 (17 instructions).
 // A thread marches through chl_planes planes: what planes share (pair sums of
 // U and V, differences of W) is carried.
-__global__ void __launch_bounds__(CHL_FLUX_THREADS, 4)   // 128 registers: 2, 3, 4, 5 blocks per SM take 417, 321, 299, 307 us
+__global__ void __launch_bounds__(CHL_FLUX_THREADS, 5)   // 102 registers: 2, 3, 4, 5, 6 blocks per SM take 417, 321, 289, 288, 290 us
 k_amd(ChlMap map, int s_in, int use_wm) {
   chl_pdl_wait();
   int lb;
@@ -223,12 +223,12 @@ k_amd(ChlMap map, int s_in, int use_wm) {
     const fx a13 = fx_mul_shr<61>(Xw, dux) + fx_mul_shr<61>(Zu, dwz) + fx_mul_shr<62>(uyL, wyL) + fx_mul_shr<62>(uyH, wyH);
     const fx a23 = fx_mul_shr<61>(Yw, dvy) + fx_mul_shr<61>(Zv, dwz) + fx_mul_shr<62>(vxL, wxL) + fx_mul_shr<62>(vxR, wxR);
     // N = sum a_ij S_ij, 64 x (S_ii 4 x, a_ij 4 x with S_ij 8 x in 2^-2 units of a_ii)
-    double Nd = fx_to(a11, 0) * fx_to(s11, 0);
-    Nd = fma(fx_to(a22, 0), fx_to(s22, 0), Nd);
-    Nd = fma(fx_to(a33, 0), fx_to(s33, 0), Nd);
-    Nd = fma(fx_to(a12, 0), fx_to(dUy + dVx, 0), Nd);
-    Nd = fma(fx_to(a13, 0), fx_to(dUz + dWx, 0), Nd);
-    Nd = fma(fx_to(a23, 0), fx_to(dVz + dWy, 0), Nd);
+    double Nd = fx_raw<true>(a11) * fx_raw<false>(s11);
+    Nd = fma(fx_raw<true>(a22), fx_raw<false>(s22), Nd);
+    Nd = fma(fx_raw<false>(a33), fx_raw<false>(s33), Nd);
+    Nd = fma(fx_raw<false>(a12), fx_raw<false>(dUy + dVx), Nd);
+    Nd = fma(fx_raw<false>(a13), fx_raw<false>(dUz + dWx), Nd);
+    Nd = fma(fx_raw<false>(a23), fx_raw<false>(dVz + dWy), Nd);
     double v = (-0.3 * Nd) / fx_to(D, 0) * pow2(min(1023, max(-1022, et - er - 67 + sd)));
     if (bad) v = __longlong_as_double(0x7FF8000000000000LL);
     if (valid) I.S[cidx(I, i, jc, k)] = v;

@@ -15,8 +15,8 @@
 #pragma once
 #include "chl_fix.cuh"
 
-// S_ii, 8 S_ij and |S| / sqrt(2)
-struct Strain { double d1, d2, d3, o12, o13, o23, s; };
+// t: S_11, S_22, S_33 and 2 S_12, 2 S_13, 2 S_23 in units of 2^e; s: |S| / sqrt(2)
+struct Strain { fx t[6]; int e; double s; };
 
 struct StrainColumn {
   const ChlInst& I;
@@ -92,8 +92,8 @@ struct StrainColumn {
     const int e = et + er + 64 - sd;
     Strain r;
     r.s = chl_sqrt(fx_to(q, 2 * e + 60));
-    r.d1 = fx_to(s1, e - 2); r.d2 = fx_to(s2, e - 2); r.d3 = fx_to(s3, e - 2);
-    r.o12 = fx_to(t1, e); r.o13 = fx_to(t2, e); r.o23 = fx_to(t3, e);
+    r.t[0] = s1; r.t[1] = s2; r.t[2] = s3; r.t[3] = t1; r.t[4] = t2; r.t[5] = t3;
+    r.e = e - 2;
     return r;
   }
 };
