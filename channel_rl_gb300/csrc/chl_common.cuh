@@ -279,6 +279,9 @@ struct ChlMap {
   const int* off;        // prefix sum of blocks per instance, off[n] = total
   int n;
   int tb;                // threads per block of the one-thread-per-point maps (tuned)
+  // planes (consecutive k) per thread of the marching kernels and of the test
+  // filter: choices of the launch that move no result
+  int planes, fplanes;
 };
 
 __device__ __forceinline__ int chl_find(const ChlMap& m, int b, int& local) {
@@ -296,16 +299,7 @@ __device__ __forceinline__ int chl_find(const ChlMap& m, int b, int& local) {
 // unsigned arithmetic (an instance has fewer than 2^31 points, checked at
 // creation): the 64-bit divisions this replaces were long integer sequences
 // ahead of every kernel's first load.
-// Planes (consecutive k) per thread of the kernels that march (flux, strain,
-// AMD): 4, halved while the instance would have fewer than 4 x 256 threads
-// per SM (at 256x96x192 one, two, four, eight and sixteen planes: k_flux 211,
-// 181, 172, 174, 181 us, k_strain -, 238, 200, 202, 204 us).
-#define CHL_FLUX_THREADS 128
-__host__ __device__ inline int chl_planes(int Nx, int Ny, int Nz) {
-  int m = 4;
-  while (m > 1 && (long)Nx * (Ny + 1) * ((Nz + m - 1) / m) < 256L * CHL_MIN_BLOCKS) m >>= 1;
-  return m;
-}
+#define CHL_FLUX_THREADS 128   // block of the kernels that march (flux, strain, AMD)
 struct ChlIdx { int i, j, k; };
 __device__ __forceinline__ ChlIdx chl_split(unsigned t, unsigned Nx, unsigned rows) {
   const unsigned q = t / Nx, k = q / rows;

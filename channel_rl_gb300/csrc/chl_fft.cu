@@ -864,25 +864,33 @@ k_project(ChlMap map, int s) {
   const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
   unsigned hi[3] = {0u, 0u, 0u};
-  if (t < (unsigned)(Nx * Ny * Nz)) {
-    const ChlIdx ix = chl_split(t, Nx, Ny);
-    const int i = ix.i, jc = 1 + ix.j, k = ix.k;
+  if (t < (unsigned)(Nx / 2 * Ny * Nz)) {     // pairs of points
+    const ChlIdx ix = chl_split(t, Nx / 2, Ny);
+    const int i = 2 * ix.i, jc = 1 + ix.j, k = ix.k;
+    const bool hasv = jc <= Ny - 1;
+    auto at = [](const double* f, size_t c) { return *reinterpret_cast<const double2*>(f + c); };
+    auto put = [](double* f, size_t c, double2 v) { *reinterpret_cast<double2*>(f + c) = v; };
+    auto top = [](double2 v) { return max(chl_abshi(v.x), chl_abshi(v.y)); };
+    auto neg = [](double2 v) { return make_double2(chl_neg(v.x), chl_neg(v.y)); };
     const double* p = I.p;
-    const size_t c = cidx(I, i, jc, k);
-    const double p0 = LDG(p + c);
     double* U = I.U[s]; double* V = I.V[s]; double* W = I.W[s];
-    const double un = U[c] - (LDG(p + cidx(I, wrap(i + 1, Nx), jc, k)) - p0) * LDG(I.rdxf + i);
-    const double wn = W[c] - (LDG(p + cidx(I, i, jc, wrap(k + 1, Nz))) - p0) * LDG(I.rdzf + k);
-    U[c] = un; W[c] = wn;
-    hi[0] = chl_abshi(un); hi[2] = chl_abshi(wn);
-    if (jc <= Ny - 1) {
-      const size_t v = vidx(I, i, jc, k);
-      const double vn = V[v] - (LDG(p + cidx(I, i, jc + 1, k)) - p0) * LDG(I.rdyf + jc);
-      V[v] = vn;
-      hi[1] = chl_abshi(vn);
+    const size_t c = cidx(I, i, jc, k), e = vidx(I, i, jc, k);
+    const double2 p0 = at(p, c), pz = at(p, cidx(I, i, jc, wrap(k + 1, Nz)));
+    const double2 py = hasv ? at(p, cidx(I, i, jc + 1, k)) : p0;
+    const double px = LDG(p + cidx(I, wrap(i + 2, Nx), jc, k));
+    const double2 u = at(U, c), w = at(W, c), v = at(V, e);
+    const double rx0 = LDG(I.rdxf + i), rx1 = LDG(I.rdxf + i + 1), ry = LDG(I.rdyf + jc), rz = LDG(I.rdzf + k);
+    const double2 un = make_double2(u.x - (p0.y - p0.x) * rx0, u.y - (px - p0.y) * rx1);
+    const double2 wn = make_double2(w.x - (pz.x - p0.x) * rz, w.y - (pz.y - p0.y) * rz);
+    put(U, c, un); put(W, c, wn);
+    hi[0] = top(un); hi[2] = top(wn);
+    if (hasv) {
+      const double2 vn = make_double2(v.x - (py.x - p0.x) * ry, v.y - (py.y - p0.y) * ry);
+      put(V, e, vn);
+      hi[1] = top(vn);
     }
-    if (jc == 1) { U[cidx(I, i, 0, k)] = chl_neg(un); W[cidx(I, i, 0, k)] = chl_neg(wn); }
-    if (jc == Ny) { U[cidx(I, i, Ny + 1, k)] = chl_neg(un); W[cidx(I, i, Ny + 1, k)] = chl_neg(wn); }
+    if (jc == 1) { put(U, cidx(I, i, 0, k), neg(un)); put(W, cidx(I, i, 0, k), neg(wn)); }
+    if (jc == Ny) { put(U, cidx(I, i, Ny + 1, k), neg(un)); put(W, cidx(I, i, Ny + 1, k), neg(wn)); }
   }
   chl_block_max(chl_vmax(I, s), hi);
 }

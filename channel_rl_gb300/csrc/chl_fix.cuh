@@ -114,13 +114,12 @@ __device__ __forceinline__ void chl_block_max(unsigned* g, const unsigned (&v)[N
 
 // Folds each thread's v into g[off + j], j = q mod rows the row of its x-line
 // q = k rows + j (whole block, at most 256 threads; x-lines are numbered
-// upwards through the block and hold four points or more).
-#define CHL_BLOCK_LINES 68
+// upwards through the block and hold two threads or more).
+#define CHL_BLOCK_LINES 130
 __device__ __forceinline__ void chl_line_max(unsigned* g, unsigned q, int rows, int off, unsigned v) {
   __shared__ unsigned sm[CHL_BLOCK_LINES];
   __shared__ unsigned q0;
-  if (threadIdx.x < CHL_BLOCK_LINES) sm[threadIdx.x] = 0u;
-  for (unsigned l = threadIdx.x + blockDim.x; l < CHL_BLOCK_LINES; l += blockDim.x) sm[l] = 0u;
+  for (unsigned l = threadIdx.x; l < CHL_BLOCK_LINES; l += blockDim.x) sm[l] = 0u;
   if (threadIdx.x == 0) q0 = q;
   __syncthreads();
   const unsigned l = min(q - q0, (unsigned)CHL_BLOCK_LINES - 1u);

@@ -19,7 +19,7 @@ void chl_launch_fix(const ChlMap&, int, int, int, cudaStream_t);
 void chl_launch_flux(const ChlMap&, int, int, cudaStream_t);
 void chl_launch_update(const ChlMap&, int, int, int, int, int, cudaStream_t);
 void chl_launch_strain(const ChlMap&, int, int, int, cudaStream_t);
-int chl_filter_blocks(int, int, int, int);
+int chl_filter_blocks(int, int, int, int, int);
 void chl_launch_filter(const ChlMap&, int, int, cudaStream_t);
 void chl_launch_dsm_final(const ChlMap&, int, int, cudaStream_t);
 void chl_launch_coef(const ChlMap&, cudaStream_t);
@@ -70,7 +70,7 @@ namespace {
 
 constexpr double RK_T[3] = {8.0 / 15.0, 2.0 / 3.0, 1.0};
 
-enum { M_PT, M_FULL, M_DSMF, M_WALL, M_PLANE, M_FFTX, M_FFTZ, M_TRI, M_MINABS, M_ROWS, M_MLP, M_WALLN,
+enum { M_PT, M_PT2, M_FULL2, M_DSMF, M_WALL, M_PLANE, M_FFTX, M_FFTZ, M_TRI, M_MINABS, M_ROWS, M_MLP, M_WALLN,
        M_ZPLANE, M_ZSOLVE, M_FLUX, M_MARCH, M_FILTER, NMAP };
 constexpr int MLP_NPARAM = 4545;
 
@@ -332,11 +332,18 @@ struct chl_handle {
   // default rule, 3 the fused z solve (z transform, tridiagonal and inverse
   // z transform in one cluster launch; bit-identical to the others)
   int x_min_blocks = CHL_FFT_MIN_BLOCKS, z_min_blocks = CHL_FFT_MIN_BLOCKS, tri_mode = 2;
+  int xmb() const { return std::max(1, x_min_blocks / (int)in.size()); }   // an instance's share of the x target
   bool zsolve_ok = false;             // every instance has the same lane count and fits (chl_smem_zsolve)
   bool zsolve = false;                // the fused form is in use
   int zlanes = 1;                     // its cluster size
   size_t smem_zs = 0;
   int twz = 0;                        // longest z transform table of the instances
+  // planes per thread of the marching kernels: 4, halved while the batch has
+  // fewer than 4 x 256 threads per SM (at 256x96x192 one, two, four, eight and
+  // sixteen planes: k_flux 211, 181, 172, 174, 181 us, k_strain -, 238, 200,
+  // 202, 204 us); of the test filter: 16, halved while it has fewer than 8
+  // blocks per SM
+  int planes = 4, fplanes = 16;
   int tb_filter = 128;                // threads of the test filter's blocks: a whole x-line of point pairs where it fits
   int tb_pt = 128;                    // threads per block of the point maps (stencils, updates)
   bool tri_scan = false;              // some instance splits its tridiagonal columns (chl_tri_lanes)
@@ -352,8 +359,8 @@ struct chl_handle {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   ChlMap map(int which) const {
-    const bool pt = which == M_PT || which == M_FULL;
-    return ChlMap{d_inst, d_off[which], (int)in.size(), pt ? tb_pt : 256};
+    const bool pt = which == M_PT || which == M_PT2 || which == M_FULL2;
+    return ChlMap{d_inst, d_off[which], (int)in.size(), pt ? tb_pt : 256, planes, fplanes};
   }
 };
 
@@ -578,7 +585,7 @@ static int build_maps(chl_handle* h) {
   h->tx = 64;
   for (auto& I : h->in) {
     const int nrow = I.c.Ny * (I.c.Nz / 2);
-    h->tx = std::max(h->tx, chl_fft_threads(chl_fftx_rows(I.c.Nx, nrow, h->x_min_blocks), I.c.Nx));
+    h->tx = std::max(h->tx, chl_fft_threads(chl_fftx_rows(I.c.Nx, nrow, h->xmb()), I.c.Nx));
   }
   h->tri_scan = false;
   for (auto& I : h->in) h->tri_scan = h->tri_scan || chl_tri_lanes((long)I.c.Nz * I.c.Nxh, I.c.Ny) > 1;
@@ -596,6 +603,12 @@ static int build_maps(chl_handle* h) {
   h->zsolve = h->zsolve_ok && (h->tri_mode == 3 || (h->tri_mode == 2 && h->zlanes > 1));
   h->tb_filter = 128;
   for (auto& I : h->in) if (I.c.Nx / 2 > 128) h->tb_filter = 256;
+  auto threads = [&](int m) { long t = 0; for (auto& I : h->in) t += (long)I.c.Nx * (I.c.Ny + 1) * cdiv(I.c.Nz, m); return t; };
+  h->planes = 4;
+  while (h->planes > 1 && threads(h->planes) < 256L * CHL_MIN_BLOCKS) h->planes >>= 1;
+  auto fblocks = [&](int m) { long b = 0; for (auto& I : h->in) b += chl_filter_blocks(I.c.Nx, I.c.Ny, I.c.Nz, h->tb_filter, m); return b; };
+  h->fplanes = 16;
+  while (h->fplanes > 4 && fblocks(h->fplanes) < 2 * CHL_MIN_BLOCKS) h->fplanes >>= 1;
   h->smem_t = h->tri_scan ? 0 : chl_smem_tri(my, modes, h->tri_mode);
   const int tri_w = chl_tri_modes_per_block(h->smem_t);
   for (int m = 0; m < NMAP; ++m) {
@@ -606,14 +619,15 @@ static int build_maps(chl_handle* h) {
       int b = 0;
       switch (m) {
         case M_PT: b = cdiv((long)Nx * Ny * Nz, h->tb_pt); break;
-        case M_FULL: b = cdiv((long)Nx * (Ny + 2) * Nz, h->tb_pt); break;
-        case M_FILTER: b = chl_filter_blocks(Nx, Ny, Nz, h->tb_filter); break;
-        case M_FLUX: b = cdiv((long)Nx * (Ny + 1) * cdiv(Nz, chl_planes(Nx, Ny, Nz)), CHL_FLUX_THREADS); break;
-        case M_MARCH: b = cdiv((long)Nx * Ny * cdiv(Nz, chl_planes(Nx, Ny, Nz)), CHL_FLUX_THREADS); break;
+        case M_PT2: b = cdiv((long)(Nx / 2) * Ny * Nz, h->tb_pt); break;         // pairs of x points (Nx even)
+        case M_FULL2: b = cdiv((long)(Nx / 2) * (Ny + 2) * Nz, h->tb_pt); break;
+        case M_FILTER: b = chl_filter_blocks(Nx, Ny, Nz, h->tb_filter, h->fplanes); break;
+        case M_FLUX: b = cdiv((long)Nx * (Ny + 1) * cdiv(Nz, h->planes), CHL_FLUX_THREADS); break;
+        case M_MARCH: b = cdiv((long)Nx * Ny * cdiv(Nz, h->planes), CHL_FLUX_THREADS); break;
         case M_DSMF: b = Ny * dsm_npart(Nx, Ny, Nz); break;
         case M_WALL: b = cdiv(2L * Nx * Nz, 256); break;
         case M_PLANE: b = cdiv((long)Nx * Nz, 256); break;
-        case M_FFTX: b = cdiv((long)Ny * (Nz / 2), chl_fftx_rows(Nx, Ny * (Nz / 2), h->x_min_blocks)); break;
+        case M_FFTX: b = cdiv((long)Ny * (Nz / 2), chl_fftx_rows(Nx, Ny * (Nz / 2), h->xmb())); break;
         case M_FFTZ: b = cdiv((long)Ny * Nxh, h->zcw); break;
         case M_TRI: b = h->tri_scan ? cdiv((long)Nz * Nxh * chl_tri_lanes((long)Nz * Nxh, Ny), 128)
                                     : cdiv((long)Nz * Nxh, tri_w); break;
@@ -634,7 +648,7 @@ static int build_maps(chl_handle* h) {
   // per-instance need: the x transform of an instance stages
   // chl_fftx_rows rows of Nx, which is not monotonic in Nx
   size_t sx = 0;
-  for (auto& I : h->in) sx = std::max(sx, chl_smem_fftx(I.c.Nx, I.c.Ny * (I.c.Nz / 2), h->x_min_blocks));
+  for (auto& I : h->in) sx = std::max(sx, chl_smem_fftx(I.c.Nx, I.c.Ny * (I.c.Nz / 2), h->xmb()));
   h->smem_x = sx;
   h->smem_z = chl_smem_fftz(mz, h->zcw, h->twz);
   if (chl_fft_setup(h->smem_x, h->smem_z, h->smem_t)) { h->err = "FFT shared-memory size not supported"; return CHL_E_ARG; }
@@ -655,7 +669,7 @@ static int enqueue_sgs(chl_handle* h, int s, bool with_wm, int stage = 0) {
     if (with_wm && h->wall_model == CHL_WM_MLP)
       KL("mlp_wallmodel", chl_launch_mlp(h->map(M_MLP), h->nblk[M_MLP], s, stage, h->d_mlp_status, st));
   };
-  KL("fix", chl_launch_fix(h->map(M_FULL), h->nblk[M_FULL], s, 1, st));
+  KL("fix", chl_launch_fix(h->map(M_FULL2), h->nblk[M_FULL2], s, 1, st));
   if (fused) wall_stress();
   if (h->LES_model == CHL_LES_DYNAMIC) {
     KL("strain", chl_launch_strain(h->map(M_MARCH), h->nblk[M_MARCH], s, 1, st));
@@ -673,7 +687,7 @@ static int enqueue_sgs(chl_handle* h, int s, bool with_wm, int stage = 0) {
   if (h->LES_model == CHL_LES_SMAGORINSKY) KL("nut_coef", chl_launch_coef(h->map(M_PT), st));
   if (!fused) {
     wall_stress();
-    KL("nut", chl_launch_nut(h->map(M_FULL), h->nblk[M_FULL], s, with_wm ? 1 : 0, st));
+    KL("nut", chl_launch_nut(h->map(M_FULL2), h->nblk[M_FULL2], s, with_wm ? 1 : 0, st));
   }
   LAUNCHED();
   return CHL_OK;
@@ -685,7 +699,7 @@ static int enqueue_sgs(chl_handle* h, int s, bool with_wm, int stage = 0) {
 static int enqueue_projection(chl_handle* h, int s, int mode) {
   cudaStream_t st = h->st;
   const bool correct = mode == 0;
-  KL("div_fft_x", chl_launch_div_fftx(h->map(M_FFTX), h->nblk[M_FFTX], h->tx, h->smem_x, s, mode, h->x_min_blocks, st));
+  KL("div_fft_x", chl_launch_div_fftx(h->map(M_FFTX), h->nblk[M_FFTX], h->tx, h->smem_x, s, mode, h->xmb(), st));
   if (h->zsolve) {
     KL("z_solve", chl_launch_zsolve(h->map(M_ZSOLVE), h->nblk[M_ZSOLVE], h->zlanes, h->smem_zs, st));
   } else {
@@ -694,8 +708,8 @@ static int enqueue_projection(chl_handle* h, int s, int mode) {
     else KL("tridiag", chl_launch_tri(h->map(M_TRI), h->nblk[M_TRI], h->smem_t, st));
     KL("fft_z", chl_launch_fftz(h->map(M_FFTZ), h->nblk[M_FFTZ], h->tz, h->smem_z, 1, h->zcw, st));
   }
-  KL("ifft_x", chl_launch_fftx_inv(h->map(M_FFTX), h->nblk[M_FFTX], h->tx, h->smem_x, mode == 1 ? 1 : 0, h->x_min_blocks, st));
-  if (correct) KL("project", chl_launch_project(h->map(M_PT), h->nblk[M_PT], s, st));
+  KL("ifft_x", chl_launch_fftx_inv(h->map(M_FFTX), h->nblk[M_FFTX], h->tx, h->smem_x, mode == 1 ? 1 : 0, h->xmb(), st));
+  if (correct) KL("project", chl_launch_project(h->map(M_PT2), h->nblk[M_PT2], s, st));
   LAUNCHED();
   return CHL_OK;
 }
@@ -1404,10 +1418,10 @@ int chl_compute_eddy_viscosity(chl_handle* h) {
 
 int chl_compute_wall_model(chl_handle* h) {
   int rc = check_ready(h); if (rc) return rc;
-  chl_launch_fix(h->map(M_FULL), h->nblk[M_FULL], 0, 1, h->st);   // k_nut forms the largest nu + nu_t anew
+  chl_launch_fix(h->map(M_FULL2), h->nblk[M_FULL2], 0, 1, h->st);   // k_nut forms the largest nu + nu_t anew
   if (h->wall_model >= CHL_WM_EQLOG) chl_launch_eqwm(h->map(M_WALLN), h->nblk[M_WALLN], 0, h->st);
   if (h->wall_model == CHL_WM_MLP) chl_launch_mlp(h->map(M_MLP), h->nblk[M_MLP], 0, 0, h->d_mlp_status, h->st);
-  chl_launch_nut(h->map(M_FULL), h->nblk[M_FULL], 0, h->wall_model != CHL_WM_NONE ? 1 : 0, h->st);
+  chl_launch_nut(h->map(M_FULL2), h->nblk[M_FULL2], 0, h->wall_model != CHL_WM_NONE ? 1 : 0, h->st);
   LAUNCHED();
   return finish(h);
 }
@@ -1417,7 +1431,7 @@ int chl_compute_rhs(chl_handle* h, int inst, double* Fu, double* Fv, double* Fw)
   Inst* I = get_inst(h, inst);
   if (!I) return CHL_E_ARG;
   if ((rc = drain_copies(h))) return rc;
-  chl_launch_fix(h->map(M_FULL), h->nblk[M_FULL], 0, 0, h->st);
+  chl_launch_fix(h->map(M_FULL2), h->nblk[M_FULL2], 0, 0, h->st);
   enqueue_rhs_only(h);
   LAUNCHED();
   const Consts& c = I->c;
@@ -1460,7 +1474,7 @@ int chl_compute_dPx_for_constant_mass_flow(chl_handle* h, int inst, double* dPdx
 int chl_compute_pressure(chl_handle* h) {
   int rc = check_ready(h); if (rc) return rc;
   chl_launch_pbc(h->map(M_WALL), h->nblk[M_WALL], 0, h->st);
-  chl_launch_fix(h->map(M_FULL), h->nblk[M_FULL], 0, 0, h->st);
+  chl_launch_fix(h->map(M_FULL2), h->nblk[M_FULL2], 0, 0, h->st);
   enqueue_rhs_only(h);
   LAUNCHED();
   rc = enqueue_projection(h, 0, 1); if (rc) return rc;

@@ -75,17 +75,21 @@ k_fix(ChlMap map, int s, int reset_n) {
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
   if (reset_n && t < (unsigned)(I.Ny + 2)) I.nmax[t] = I.smax[t] = 0u;
   const unsigned* vm = chl_vmax(I, s);
-  const unsigned nc = (unsigned)(I.Nx * (I.Ny + 2) * I.Nz), nv = (unsigned)(I.Nx * (I.Ny + 1) * I.Nz);
-  if (t < nc) {
-    I.X[0][t] = fx_from(LDG(I.U[s] + t), fx_exp<61>(vm[0]));
-    I.X[2][t] = fx_from(LDG(I.W[s] + t), fx_exp<61>(vm[2]));
-  }
-  if (t < nv) I.X[1][t] = fx_from(LDG(I.V[s] + t), fx_exp<61>(vm[1]));
+  // pairs of points (Nx is even)
+  const unsigned nc = (unsigned)(I.Nx * (I.Ny + 2) * I.Nz) / 2, nv = (unsigned)(I.Nx * (I.Ny + 1) * I.Nz) / 2;
+  const int eu = fx_exp<61>(vm[0]), ev = fx_exp<61>(vm[1]), ew = fx_exp<61>(vm[2]);
+  auto put = [t](fx* x, double2 v, int e) { reinterpret_cast<longlong2*>(x)[t] = make_longlong2(fx_from(v.x, e), fx_from(v.y, e)); };
+  auto get = [t](const double* x) { return __ldg(reinterpret_cast<const double2*>(x) + t); };
+  double2 u, v, w;
+  if (t < nc) { u = get(I.U[s]); w = get(I.W[s]); }
+  if (t < nv) v = get(I.V[s]);
+  if (t < nc) { put(I.X[0], u, eu); put(I.X[2], w, ew); }
+  if (t < nv) put(I.X[1], v, ev);
 }
 
 // 28 products and 4 conversions of nu + nu_t per point on the integer pipe,
 // no FP64 instruction; 104 bytes per point.  A thread marches through
-// chl_planes planes at its (i, j), so that what the next plane shares (U, V,
+// a few planes at its (i, j), so that what the next plane shares (U, V,
 // nu + nu_t one plane up, W one down) is loaded and converted once.
 __global__ void __launch_bounds__(CHL_FLUX_THREADS, 6)
 k_flux(ChlMap map, int sin) {
@@ -93,7 +97,7 @@ k_flux(ChlMap map, int sin) {
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
   const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
-  const int M = chl_planes(Nx, Ny, Nz);
+  const int M = map.planes;
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
   const ChlIdx p = chl_split(t, Nx, Ny + 1);
   const int i = p.i, j = p.j, k0 = p.k * M, k1 = min(Nz, k0 + M);

@@ -29,7 +29,7 @@ k_strain(ChlMap map, int s_in) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
-  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz, M = chl_planes(Nx, Ny, Nz);
+  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz, M = map.planes;
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
   const ChlIdx p = chl_split(t, Nx, Ny);
   const int i = p.i, jc = 1 + p.j, k0 = p.k * M, k1 = min(Nz, k0 + M);
@@ -85,15 +85,14 @@ k_strain(ChlMap map, int s_in) {
 // then for each of the 3 wall fields one row block x plane chunks.
 #define FILT_FIELDS 15
 struct FiltShape { int nxp, RG, segs, rowblocks, M, nz, full; };   // full: blocks of one field
-__host__ __device__ inline FiltShape filt_shape(int Nx, int Ny, int Nz, int T) {
+__host__ __device__ inline FiltShape filt_shape(int Nx, int Ny, int Nz, int T, int M) {
   FiltShape f;
   f.nxp = Nx / 2;
   f.RG = f.nxp <= T ? T / f.nxp : 1;                       // row groups per block
   f.segs = f.nxp <= T ? 1 : (f.nxp + T - 3) / (T - 2);     // longer rows: overlapping segments
   const int groups = (Ny + 3) / 2;                         // of U and W, the most
   f.rowblocks = (groups + f.RG - 1) / f.RG * f.segs;
-  f.M = 16;
-  while (f.M > 4 && (long)f.rowblocks * FILT_FIELDS * ((Nz + f.M - 1) / f.M) < 2 * CHL_MIN_BLOCKS) f.M >>= 1;
+  f.M = M;
   f.nz = (Nz + f.M - 1) / f.M;
   f.full = f.rowblocks * f.nz;
   return f;
@@ -119,7 +118,7 @@ k_filter(ChlMap map) {
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
   const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
-  const FiltShape f = filt_shape(Nx, Ny, Nz, blockDim.x);
+  const FiltShape f = filt_shape(Nx, Ny, Nz, blockDim.x, map.fplanes);
   // field, row block, segment, planes
   int field, rest;
   if (lb < FILT_FIELDS * f.full) { field = lb / f.full; rest = lb - field * f.full; }
@@ -482,47 +481,54 @@ static __device__ __noinline__ double nut_other(const ChlInst& I, int i, int jc,
   }
   return I.nu + chl_pos(I.S[cidx(I, i, jc, k)]);
 }
-// One thread per centre (i, jc, k), jc = 0..Ny+1.  On the wall-model rows
-// (jc = 0, 1 and Ny, Ny+1) nu_t is the mean of the face values at x faces
+// One thread per pair of x points of a row (jc, k), jc = 0..Ny+1 (with one
+// point per thread this kernel took 52 us at 256x96x192 for 11 us of HBM
+// traffic: blocks too short-lived for their start-up).  On the wall-model
+// rows (jc = 0, 1 and Ny, Ny+1) nu_t is the mean of the face values at x faces
 // i-1 and i, the same in both rows of a wall: the threads of rows 1 and Ny
-// write both.  Each forms face i and takes face i-1 from the lane to its left
-// when that lane is on the same row (i > 0), so no thread returns before the
-// shuffle.
+// write both.  Each forms its two faces and takes the one before from the
+// lane to its left when that lane is on the same row (i > 0), so no thread
+// returns before the shuffle.
 __global__ void __launch_bounds__(256)
 k_nut(ChlMap map, int s_in, int use_wm) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
-  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
+  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz, nxp = Nx / 2;
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  const bool valid = t < (unsigned)(Nx * (Ny + 2) * Nz);
-  // lanes past the end repeat the last centre and write nothing
-  const ChlIdx p = chl_split(valid ? t : (unsigned)(Nx * (Ny + 2) * Nz) - 1u, Nx, Ny + 2);
-  const int i = p.i, jc = p.j, k = p.k;
+  const bool valid = t < (unsigned)(nxp * (Ny + 2) * Nz);
+  // lanes past the end repeat the last pair and write nothing
+  const ChlIdx p = chl_split(valid ? t : (unsigned)(nxp * (Ny + 2) * Nz) - 1u, nxp, Ny + 2);
+  const int i = 2 * p.i, jc = p.j, k = p.k;
   const bool wm = use_wm && I.wall_model != 0 && (jc <= 1 || jc >= Ny);
   const bool wmrow = valid && wm && (jc == 1 || jc == Ny);
   const int wall = jc == 1 ? 0 : 1;
   const double* U = I.U[s_in];
-  const double f = wmrow ? wm_face(I, U, i, k, wall) : 0.0;
-  const double f_left = __shfl_up_sync(0xffffffffu, f, 1);
-  double v = 0.0;
+  double f0 = 0.0, f1 = 0.0;
+  if (wmrow) { f0 = wm_face(I, U, i, k, wall); f1 = wm_face(I, U, i + 1, k, wall); }
+  const double f_left = __shfl_up_sync(0xffffffffu, f1, 1);
+  double2 v = make_double2(0.0, 0.0);
   if (valid && (!wm || wmrow)) {
     // stored as nu + nu_t: every consumer adds nu (equations.f90:139-155)
     const double nu = I.nu;
+    double2* nut = reinterpret_cast<double2*>(I.nut);
+    const size_t c = cidx(I, i, jc, k) / 2;
     if (wmrow) {
       const double fl = ((threadIdx.x & 31) > 0 && i > 0) ? f_left : wm_face(I, U, wrap(i - 1, Nx), k, wall);
-      v = nu + 0.5 * (fl + f);
-      I.nut[cidx(I, i, wall == 0 ? 0 : Ny + 1, k)] = v;
+      v = make_double2(nu + 0.5 * (fl + f0), nu + 0.5 * (f0 + f1));
+      nut[cidx(I, i, wall == 0 ? 0 : Ny + 1, k) / 2] = v;
     } else if (I.LES_model == 0 || I.LES_model >= 3 || jc == 0 || jc == Ny + 1) {
-      v = nut_other(I, i, jc, k);
+      v = make_double2(nut_other(I, i, jc, k), nut_other(I, i + 1, jc, k));
     } else {
       // nu + max(0, c |S|) as one FMA, nu + c |S|, clipped below at nu by the
       // bit patterns (both positive; a NaN, for which max gives 0, gives nu)
-      v = chl_atleast(fma(I.coef[jc], I.S[cidx(I, i, jc, k)], nu), nu);
+      const double cj = I.coef[jc];
+      const double2 S = __ldg(reinterpret_cast<const double2*>(I.S) + c);
+      v = make_double2(chl_atleast(fma(cj, S.x, nu), nu), chl_atleast(fma(cj, S.y, nu), nu));
     }
-    I.nut[cidx(I, i, jc, k)] = v;
+    nut[c] = v;
   }
-  chl_line_max(I.nmax, (unsigned)(k * (Ny + 2) + jc), Ny + 2, 0, chl_abshi(v));
+  chl_line_max(I.nmax, (unsigned)(k * (Ny + 2) + jc), Ny + 2, 0, max(chl_abshi(v.x), chl_abshi(v.y)));
 }
 
 // ------------------------------------------------------------ launchers
@@ -531,8 +537,8 @@ void chl_launch_strain(const ChlMap& m, int nb, int s_in, int dsm, cudaStream_t 
   if (dsm) chl_launch_pdl(k_strain<true>, dim3(nb), dim3(CHL_FLUX_THREADS), 0, st, m, s_in);
   else chl_launch_pdl(k_strain<false>, dim3(nb), dim3(CHL_FLUX_THREADS), 0, st, m, s_in);
 }
-int chl_filter_blocks(int Nx, int Ny, int Nz, int T) {
-  const FiltShape f = filt_shape(Nx, Ny, Nz, T);
+int chl_filter_blocks(int Nx, int Ny, int Nz, int T, int M) {
+  const FiltShape f = filt_shape(Nx, Ny, Nz, T, M);
   return FILT_FIELDS * f.full + 3 * f.segs * f.nz;
 }
 void chl_launch_filter(const ChlMap& m, int nb, int T, cudaStream_t st) { chl_launch_pdl(k_filter, dim3(nb), dim3(T), 0, st, m); }

@@ -132,14 +132,14 @@ __device__ __forceinline__ unsigned write_nut_rows(const ChlInst& I, const doubl
 // each point scales its fifteen by their largest, so that the products keep
 // 54 bits or more of the largest product, and forms the derivatives, D and
 // the a_ij there.  N and the division are FP64 (17 instructions).
-// A thread marches through chl_planes planes: what planes share (pair sums of
+// A thread marches through a few planes: what planes share (pair sums of
 // U and V, differences of W) is carried.
 __global__ void __launch_bounds__(CHL_FLUX_THREADS, 5)   // 102 registers: 2, 3, 4, 5, 6 blocks per SM take 417, 321, 289, 288, 290 us
 k_amd(ChlMap map, int s_in, int use_wm) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
-  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz, M = chl_planes(Nx, Ny, Nz);
+  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz, M = map.planes;
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
   const ChlIdx p = chl_split(t, Nx, Ny);
   const int i = p.i, jc = 1 + p.j, k0 = p.k * M;
