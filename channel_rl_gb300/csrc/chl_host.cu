@@ -718,7 +718,7 @@ static int enqueue_projection(chl_handle* h, int s, int mode) {
 // pressure, the tuner); the set's fixed-point copies are in place.
 static void enqueue_rhs_only(chl_handle* h) {
   chl_launch_flux(h->map(M_FLUX), h->nblk[M_FLUX], 0, h->st);
-  chl_launch_update(h->map(M_PT), h->nblk[M_PT], 0, 0, 0, 2, h->st);
+  chl_launch_update(h->map(M_PT2), h->nblk[M_PT2], 0, 0, 0, 2, h->st);
 }
 
 // compute_dt: one launch.  k_minabs's last block per instance forms dt
@@ -740,7 +740,7 @@ static int enqueue_rk3(chl_handle* h) {
     int rc = enqueue_sgs(h, sin[s], h->wall_model != CHL_WM_NONE, s);
     if (rc) return rc;
     KL("rhs_flux", chl_launch_flux(h->map(M_FLUX), h->nblk[M_FLUX], sin[s], h->st));
-    KL("rhs_update", chl_launch_update(h->map(M_PT), h->nblk[M_PT], 0, sout[s], s, s == 0 ? 0 : 1, h->st));
+    KL("rhs_update", chl_launch_update(h->map(M_PT2), h->nblk[M_PT2], 0, sout[s], s, s == 0 ? 0 : 1, h->st));
     LAUNCHED();
     rc = enqueue_projection(h, sout[s], 0);
     if (rc) return rc;

@@ -199,7 +199,9 @@ __device__ __forceinline__ double row_diff(fx hi, int eh, fx lo, int el) {
 
 // The flux differences are exact integers; each is rounded once to a double
 // and multiplied by its reciprocal spacing there (with the products in
-// integers as well, F lost two to four bits to their common exponent).
+// integers as well, F lost two to four bits to their common exponent).  One
+// thread per pair of x points: 16-byte loads, and the pair shares the fluxes
+// between its points.
 __global__ void __launch_bounds__(256)
 k_rhs_update(ChlMap map, RhsArgs a) {
   chl_pdl_wait();
@@ -207,58 +209,85 @@ k_rhs_update(ChlMap map, RhsArgs a) {
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
   const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  if (t >= (unsigned)(Nx * Ny * Nz)) return;
-  const ChlIdx p = chl_split(t, Nx, Ny);
-  const int i = p.i, jc = 1 + p.j, k = p.k;
-  const int im = wrap(i - 1, Nx), ip = wrap(i + 1, Nx);
+  if (t >= (unsigned)(Nx / 2 * Ny * Nz)) return;
+  const ChlIdx p = chl_split(t, Nx / 2, Ny);
+  const int i = 2 * p.i, jc = 1 + p.j, k = p.k;
+  const int im = wrap(i - 1, Nx), ip = wrap(i + 2, Nx);
   const int km = wrap(k - 1, Nz), kp = wrap(k + 1, Nz);
   const fx* const* G = I.G;
-  const double rxc = LDG(I.rdxc + i), rxf = LDG(I.rdxf + i), ryc = LDG(I.rdyc + jc);
-  const double rzc = LDG(I.rdzc + k), rzf = LDG(I.rdzf + k);
-  const size_t c = cidx(I, i, jc, k), e = vidx(I, i, jc, k), em = vidx(I, i, jc - 1, k);
   const bool hasv = jc <= Ny - 1;
+  const size_t c = cidx(I, i, jc, k), e = vidx(I, i, jc, k), em = vidx(I, i, jc - 1, k);
+  auto g2 = [](const fx* f, size_t q) { return __ldg(reinterpret_cast<const longlong2*>(f + q)); };
+  auto d2 = [](const double* f, size_t q) { return *reinterpret_cast<const double2*>(f + q); };
+  auto put = [](double* f, size_t q, double2 v) { *reinterpret_cast<double2*>(f + q) = v; };
+  auto neg = [](double2 v) { return make_double2(chl_neg(v.x), chl_neg(v.y)); };
+  const double rxc0 = LDG(I.rdxc + i), rxc1 = LDG(I.rdxc + i + 1), rxf0 = LDG(I.rdxf + i), rxf1 = LDG(I.rdxf + i + 1);
+  const double ryc = LDG(I.rdyc + jc), ryf = LDG(I.rdyf + jc);
+  const double rzc = LDG(I.rdzc + k), rzf = LDG(I.rdzf + k), dpdx = I.scal[CHL_S_DPDX];
   // exponents of the fluxes of rows jc - 1, jc, jc + 1
   const int4 e0 = LDG(I.upd + jc), el = LDG(I.upd + jc - 1), eh = LDG(I.upd + min(jc + 1, Ny));
-#define D(m, hi, lo, e) fx_to(LDG(G[m] + (hi)) - LDG(G[m] + (lo)), e)
-  // u at (x-face i, row jc, z-centre k), w at (x-centre i, row jc, z-face k),
-  // v at (x-centre i, y-face jv = jc, z-centre k)
-  double Fu = fma(D(G_UX, cidx(I, ip, jc, k), c, e0.x), rxf, I.scal[CHL_S_DPDX]);
-  Fu = fma(row_diff(LDG(G[G_UY] + e), e0.x, LDG(G[G_UY] + em), el.x), ryc, Fu);
-  Fu = fma(D(G_UZ, c, cidx(I, i, jc, km), e0.x), rzc, Fu);
-  double Fw = D(G_WX, c, cidx(I, im, jc, k), e0.z) * rxc;
-  Fw = fma(row_diff(LDG(G[G_WY] + e), e0.z, LDG(G[G_WY] + em), el.z), ryc, Fw);
-  Fw = fma(D(G_WZ, cidx(I, i, jc, kp), c, e0.z), rzf, Fw);
-  double Fv = 0.0;
-  if (hasv) {
-    Fv = D(G_VX, e, vidx(I, im, jc, k), e0.y) * rxc;
-    Fv = fma(row_diff(LDG(G[G_VY] + cidx(I, i, jc + 1, k)), eh.y, LDG(G[G_VY] + c), e0.y), LDG(I.rdyf + jc), Fv);
-    Fv = fma(D(G_VZ, e, vidx(I, i, jc, km), e0.y), rzc, Fv);
+  double2 Fu, Fv = make_double2(0.0, 0.0), Fw;
+  {  // u at (x-face i, row jc, z-centre k)
+    const longlong2 x = g2(G[G_UX], c), yh = g2(G[G_UY], e), yl = g2(G[G_UY], em);
+    const longlong2 zh = g2(G[G_UZ], c), zl = g2(G[G_UZ], cidx(I, i, jc, km));
+    const fx xp = LDG(G[G_UX] + cidx(I, ip, jc, k));
+    Fu.x = fma(fx_to(x.y - x.x, e0.x), rxf0, dpdx);
+    Fu.y = fma(fx_to(xp - x.y, e0.x), rxf1, dpdx);
+    Fu.x = fma(row_diff(yh.x, e0.x, yl.x, el.x), ryc, Fu.x);
+    Fu.y = fma(row_diff(yh.y, e0.x, yl.y, el.x), ryc, Fu.y);
+    Fu.x = fma(fx_to(zh.x - zl.x, e0.x), rzc, Fu.x);
+    Fu.y = fma(fx_to(zh.y - zl.y, e0.x), rzc, Fu.y);
   }
-#undef D
-  if (e0.w | el.w | eh.w) Fu = Fv = Fw = __longlong_as_double(0x7FF8000000000000LL);
+  {  // w at (x-centre i, row jc, z-face k)
+    const longlong2 x = g2(G[G_WX], c), yh = g2(G[G_WY], e), yl = g2(G[G_WY], em);
+    const longlong2 zl = g2(G[G_WZ], c), zh = g2(G[G_WZ], cidx(I, i, jc, kp));
+    const fx xm = LDG(G[G_WX] + cidx(I, im, jc, k));
+    Fw.x = fx_to(x.x - xm, e0.z) * rxc0;
+    Fw.y = fx_to(x.y - x.x, e0.z) * rxc1;
+    Fw.x = fma(row_diff(yh.x, e0.z, yl.x, el.z), ryc, Fw.x);
+    Fw.y = fma(row_diff(yh.y, e0.z, yl.y, el.z), ryc, Fw.y);
+    Fw.x = fma(fx_to(zh.x - zl.x, e0.z), rzf, Fw.x);
+    Fw.y = fma(fx_to(zh.y - zl.y, e0.z), rzf, Fw.y);
+  }
+  if (hasv) {  // v at (x-centre i, y-face jv = jc, z-centre k)
+    const longlong2 x = g2(G[G_VX], e), yl = g2(G[G_VY], c), yh = g2(G[G_VY], cidx(I, i, jc + 1, k));
+    const longlong2 zh = g2(G[G_VZ], e), zl = g2(G[G_VZ], vidx(I, i, jc, km));
+    const fx xm = LDG(G[G_VX] + vidx(I, im, jc, k));
+    Fv.x = fx_to(x.x - xm, e0.y) * rxc0;
+    Fv.y = fx_to(x.y - x.x, e0.y) * rxc1;
+    Fv.x = fma(row_diff(yh.x, eh.y, yl.x, e0.y), ryf, Fv.x);
+    Fv.y = fma(row_diff(yh.y, eh.y, yl.y, e0.y), ryf, Fv.y);
+    Fv.x = fma(fx_to(zh.x - zl.x, e0.y), rzc, Fv.x);
+    Fv.y = fma(fx_to(zh.y - zl.y, e0.y), rzc, Fv.y);
+  }
+  if (e0.w | el.w | eh.w) {
+    const double q = __longlong_as_double(0x7FF8000000000000LL);
+    Fu = Fv = Fw = make_double2(q, q);
+  }
   if (a.mode == 2) {           // actual-pressure RHS: keep F only
-    I.Fp[0][c] = Fu; I.Fp[2][c] = Fw;
-    if (hasv) I.Fp[1][e] = Fv;
+    put(I.Fp[0], c, Fu); put(I.Fp[2], c, Fw);
+    if (hasv) put(I.Fp[1], e, Fv);
     return;
   }
   // out = base + dt (c1 F1 + c2 F) as two FMAs per component; the products
   // dt c are formed once per step where dt is set
   const double dc1 = I.scal[CHL_S_DC + 2 * a.stage], dc2 = I.scal[CHL_S_DC + 2 * a.stage + 1];
   double* Uo = I.U[a.sout]; double* Vo = I.V[a.sout]; double* Wo = I.W[a.sout];
-  const double* Ub = I.U[a.sbase]; const double* Vb = I.V[a.sbase]; const double* Wb = I.W[a.sbase];
-  double un = fma(dc2, Fu, Ub[c]), wn = fma(dc2, Fw, Wb[c]), vn = hasv ? fma(dc2, Fv, Vb[e]) : 0.0;
+  auto axpy = [](double s, double2 x, double2 y) { return make_double2(fma(s, x.x, y.x), fma(s, x.y, y.y)); };
+  double2 un = axpy(dc2, Fu, d2(I.U[a.sbase], c)), wn = axpy(dc2, Fw, d2(I.W[a.sbase], c)), vn;
+  if (hasv) vn = axpy(dc2, Fv, d2(I.V[a.sbase], e));
   if (a.mode == 0) {
-    I.F1[0][c] = Fu; I.F1[2][c] = Fw;
-    if (hasv) I.F1[1][e] = Fv;
+    put(I.F1[0], c, Fu); put(I.F1[2], c, Fw);
+    if (hasv) put(I.F1[1], e, Fv);
   } else {
-    un = fma(dc1, I.F1[0][c], un);
-    wn = fma(dc1, I.F1[2][c], wn);
-    if (hasv) vn = fma(dc1, I.F1[1][e], vn);
+    un = axpy(dc1, d2(I.F1[0], c), un);
+    wn = axpy(dc1, d2(I.F1[2], c), wn);
+    if (hasv) vn = axpy(dc1, d2(I.F1[1], e), vn);
   }
-  Uo[c] = un; Wo[c] = wn;
-  if (hasv) Vo[e] = vn;
-  if (jc == 1) { Uo[cidx(I, i, 0, k)] = chl_neg(un); Wo[cidx(I, i, 0, k)] = chl_neg(wn); }
-  if (jc == Ny) { Uo[cidx(I, i, Ny + 1, k)] = chl_neg(un); Wo[cidx(I, i, Ny + 1, k)] = chl_neg(wn); }
+  put(Uo, c, un); put(Wo, c, wn);
+  if (hasv) put(Vo, e, vn);
+  if (jc == 1) { put(Uo, cidx(I, i, 0, k), neg(un)); put(Wo, cidx(I, i, 0, k), neg(wn)); }
+  if (jc == Ny) { put(Uo, cidx(I, i, Ny + 1, k), neg(un)); put(Wo, cidx(I, i, Ny + 1, k), neg(wn)); }
 }
 
 extern "C" {
