@@ -123,7 +123,6 @@ struct ChlInst {
   // geometry (reciprocal spacings; see chl_host.cpp for the exact list)
   const double *rdxc, *rdxf, *rdyc, *rdyf, *rdzc, *rdzf;
   const double *dxf, *dyf, *dzf;  // raw spacings (dt)
-  const double *hx2, *hy2, *hz2;  // squared centre widths (x(i)-x(i-1))^2 etc. (Vreman)
   const double *w0x2, *w1x2;      // 2 x weight_y_0/1 by face row jv
   const double *ygc;              // yg(1..nyg), centre y coordinates with the ghost rows
   const double *smag_csdelta;     // Cs*Delta_j by centre row (static Smagorinsky)
@@ -146,6 +145,7 @@ struct ChlInst {
   // for r 2^e, r < 2^63, one exponent for a table along x or z and one per
   // row along y; the weight's is -63 (chl_fix.cuh)
   const long long *fxrxc, *fxrxf, *fxryc, *fxryf, *fxrzc, *fxrzf, *fxw1;
+  const long long *fxhyl, *fxhyh; // h_y/dy of the y spacings below and above a centre row, 2^-62 (Vreman)
   const int *eyc, *eyf;
   int exc, exf, ezc, ezf;
   int4 *upd;                      // per row, from the flux kernel to the update: exponents (chl_rhs.cu)

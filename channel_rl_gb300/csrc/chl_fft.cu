@@ -51,10 +51,13 @@ __device__ __forceinline__ fx2 halve(fx2 a) { return make_longlong2(a.x >> 1, a.
 
 // v w / 2 (INV: v conj(w) / 2).  The four cross terms of a component, at most
 // 2^62.9 together for |v| < 2^61, are summed before their one shift; the
-// starting value rounds it and makes up for the dropped low products.
-template <bool INV>
+// starting value rounds it, makes up for the dropped low products and, over
+// the R - 1 products of a butterfly, for the quarter of a unit that halving
+// the first input loses on average: the sum of a line, which the mean pressure
+// hangs on, keeps no bias.
+template <int RADIX, bool INV>
 __device__ __forceinline__ fx2 tw_mul(fx2 v, int4 w) {
-  const long long R = 1LL << 31;
+  const long long R = (1LL << 31) + (1LL << 29) / (RADIX - 1);
   const fx n = INV ? -v.x : -v.y;
   const int xh = (int)(v.x >> 32), xl = (int)((unsigned)v.x >> 1);
   const int yh = (int)(v.y >> 32), yl = (int)((unsigned)v.y >> 1);
@@ -133,7 +136,7 @@ __device__ __forceinline__ void fx_pass(const LD& ld, const ST& st, const SmallD
       const int g = small_div(j, (unsigned)pass.z), jm = j - g * Ns;
       v[0] = halve(v[0]);
 #pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = tw_mul<INV>(v[r], smem_tw()[tab + (r - 1) * Ns + jm]);
+      for (int r = 1; r < R; ++r) v[r] = tw_mul<R, INV>(v[r], smem_tw()[tab + (r - 1) * Ns + jm]);
       o = g * Ns * R + jm;
       step = Ns;
     }

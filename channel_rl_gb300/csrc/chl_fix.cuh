@@ -38,11 +38,14 @@ __device__ __forceinline__ fx fx_from(double x, int e) {
   return b < 0 ? -(fx)f : (fx)f;
 }
 
-// F 2^e as a double, rounded to nearest (the magnitude of a negative F is
-// taken one unit short, which saves the carry); exponents beyond a double's
-// give its smallest and largest magnitudes
+// F 2^e as a double, rounded to nearest; exponents beyond a double's give its
+// smallest and largest magnitudes.  EXACT = false takes the magnitude of a
+// negative F one unit short, which saves the carry, for values whose last bits
+// are rounding anyway.
+template <bool EXACT = false>
 __device__ __forceinline__ double fx_to(fx f, int e) {
   const int sign = (int)(f >> 63);
+  if (EXACT) f -= (fx)((unsigned)sign & 1u);
   const unsigned hi = (unsigned)(f >> 32) ^ (unsigned)sign, lo = (unsigned)f ^ (unsigned)sign;
   const int lz = hi ? __clz((int)hi) : 32 + __clz((int)lo);
   unsigned long long n;

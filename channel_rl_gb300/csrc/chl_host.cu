@@ -81,7 +81,6 @@ struct Consts {
   int nx, ny, nz, nxg, nyg, nzg, Nx, Ny, Nz, Nxh;
   std::vector<double> xf, yf, zf, xg, yg, zg;   // 1-based Fortran copies (index 0 unused)
   std::vector<double> rdxc, rdxf, dxf, rdzc, rdzf, dzf;   // offset 1, length N+3
-  std::vector<double> hx2, hz2, hy2;                       // squared centre widths (x, z offset 1)
   std::vector<double> rdyc, rdyf, dyf, w0, w1;            // length Ny+2
   std::vector<double> csdelta, dwall;                     // length Ny+2
   std::vector<double> kxx, kzz;
@@ -153,14 +152,6 @@ int make_consts(const chl_grid_desc& d, Consts& c, std::string& err) {
   };
   periodic(c.xf, c.xg, c.Nx, c.rdxc, c.rdxf, c.dxf);
   periodic(c.zf, c.zg, c.Nz, c.rdzc, c.rdzf, c.dzf);
-  auto widths2 = [&](const std::vector<double>& f, int N, std::vector<double>& w) {
-    w.assign(N + 3, NaN);
-    for (int i = 0; i <= N; ++i) { const double d = f[i + 2] - f[i + 1]; w[i + 1] = d * d; }
-  };
-  widths2(c.xf, c.Nx, c.hx2);
-  widths2(c.zf, c.Nz, c.hz2);
-  c.hy2.assign(c.Ny + 2, NaN);
-  for (int jc = 1; jc <= c.Ny; ++jc) { const double d = c.yf[jc + 1] - c.yf[jc]; c.hy2[jc] = d * d; }
   const int Ny = c.Ny;
   c.rdyc.assign(Ny + 2, NaN); c.rdyf.assign(Ny + 2, NaN); c.dyf.assign(Ny + 2, NaN);
   c.w0.assign(Ny + 2, NaN); c.w1.assign(Ny + 2, NaN);
@@ -387,7 +378,7 @@ static int upload_consts(chl_handle* h, Inst& I) {
   size_t o_rdxc = A.take(8 * (Nx + 3)), o_rdxf = A.take(8 * (Nx + 3)), o_dxf = A.take(8 * (Nx + 3));
   size_t o_rdzc = A.take(8 * (Nz + 3)), o_rdzf = A.take(8 * (Nz + 3)), o_dzf = A.take(8 * (Nz + 3));
   size_t o_rdyc = A.take(8 * (Ny + 2)), o_rdyf = A.take(8 * (Ny + 2)), o_dyf = A.take(8 * (Ny + 2));
-  size_t o_hx2 = A.take(8 * (Nx + 3)), o_hz2 = A.take(8 * (Nz + 3)), o_hy2 = A.take(8 * (Ny + 2));
+  size_t o_hyl = A.take(8 * (Ny + 2)), o_hyh = A.take(8 * (Ny + 2));
   size_t o_w0 = A.take(8 * (Ny + 2)), o_w1 = A.take(8 * (Ny + 2)), o_ygc = A.take(8 * (Ny + 2));
   size_t o_fxrxc = A.take(8 * (Nx + 3)), o_fxryc = A.take(8 * (Ny + 2)), o_fxrzc = A.take(8 * (Nz + 3));
   size_t o_fxrxf = A.take(8 * (Nx + 3)), o_fxryf = A.take(8 * (Ny + 2)), o_fxrzf = A.take(8 * (Nz + 3));
@@ -454,12 +445,11 @@ static int upload_consts(chl_handle* h, Inst& I) {
   D.mass_norm = 1.0 / ((double)Nx * Nz);
   D.rdxc = P(o_rdxc) + 1; D.rdxf = P(o_rdxf) + 1; D.dxf = P(o_dxf) + 1;
   D.rdzc = P(o_rdzc) + 1; D.rdzf = P(o_rdzf) + 1; D.dzf = P(o_dzf) + 1;
-  D.hx2 = P(o_hx2) + 1; D.hz2 = P(o_hz2) + 1; D.hy2 = P(o_hy2);
   D.rdyc = P(o_rdyc); D.rdyf = P(o_rdyf); D.dyf = P(o_dyf); D.w0x2 = P(o_w0); D.w1x2 = P(o_w1); D.ygc = P(o_ygc);
   auto L = [&](size_t o) { return (long long*)(base + o); };
   D.fxrxc = L(o_fxrxc) + 1; D.fxryc = L(o_fxryc); D.fxrzc = L(o_fxrzc) + 1;
   D.fxrxf = L(o_fxrxf) + 1; D.fxryf = L(o_fxryf); D.fxrzf = L(o_fxrzf) + 1;
-  D.fxw1 = L(o_fxw1); D.upd = (int4*)(base + o_upd);
+  D.fxw1 = L(o_fxw1); D.fxhyl = L(o_hyl); D.fxhyh = L(o_hyh); D.upd = (int4*)(base + o_upd);
   D.eyc = (const int*)(base + o_eyc); D.eyf = (const int*)(base + o_eyf); D.nmax = (unsigned*)(base + o_nmax);
   D.smax = (unsigned*)(base + o_smax);
   D.smag_csdelta = P(o_csd); D.smag_dwall = P(o_dw);
@@ -488,7 +478,6 @@ static int upload_consts(chl_handle* h, Inst& I) {
   CK(put(o_rdxc, c.rdxc)); CK(put(o_rdxf, c.rdxf)); CK(put(o_dxf, c.dxf));
   CK(put(o_rdzc, c.rdzc)); CK(put(o_rdzf, c.rdzf)); CK(put(o_dzf, c.dzf));
   CK(put(o_rdyc, c.rdyc)); CK(put(o_rdyf, c.rdyf)); CK(put(o_dyf, c.dyf));
-  CK(put(o_hx2, c.hx2)); CK(put(o_hz2, c.hz2)); CK(put(o_hy2, c.hy2));
   const std::vector<double> ygc(c.yg.begin() + 1, c.yg.begin() + 1 + c.nyg);
   CK(put(o_ygc, ygc));
   // scaled copies (kept in `scaled` for the rest of this function)
@@ -528,6 +517,12 @@ static int upload_consts(chl_handle* h, Inst& I) {
   CK(uniform(o_fxrzc, c.rdzc, D.ezc)); CK(uniform(o_fxrzf, c.rdzf, D.ezf));
   CK(perrow(o_fxryc, o_eyc, c.rdyc)); CK(perrow(o_fxryf, o_eyf, c.rdyf));
   CK(fixtab(o_fxw1, c.w1, {-63}));
+  {
+    // both below 2: a centre row is at most twice its distance to the next centre
+    std::vector<double> hl(Ny + 2, NaN), hh(Ny + 2, NaN);
+    for (int j = 1; j <= Ny; ++j) { hl[j] = c.rdyf[j - 1] / c.rdyc[j]; hh[j] = c.rdyf[j] / c.rdyc[j]; }
+    CK(fixtab(o_hyl, hl, {-62})); CK(fixtab(o_hyh, hh, {-62}));
+  }
   CK(put(o_csd, c.csdelta)); CK(put(o_dw, c.dwall));
   {
     const std::vector<int4> tx = fft_table(Nx), tz = fft_table(Nz);
@@ -680,7 +675,7 @@ static int enqueue_sgs(chl_handle* h, int s, bool with_wm, int stage = 0) {
   } else if (h->LES_model == CHL_LES_AMD) {
     KL("amd", chl_launch_amd(h->map(M_MARCH), h->nblk[M_MARCH], s, with_wm ? 1 : 0, st));
   } else if (h->LES_model == CHL_LES_VREMAN) {
-    KL("vreman", chl_launch_vreman(h->map(M_PT), h->nblk[M_PT], s, with_wm ? 1 : 0, st));
+    KL("vreman", chl_launch_vreman(h->map(M_MARCH), h->nblk[M_MARCH], s, with_wm ? 1 : 0, st));
   }
   // the static model's row coefficient (the dynamic model's is formed by
   // the last block of each row of its plane sums)

@@ -194,7 +194,7 @@ struct RhsArgs {
 // A difference of y fluxes, whose rows have their own exponents.
 __device__ __forceinline__ double row_diff(fx hi, int eh, fx lo, int el) {
   const int m = max(eh, el);
-  return fx_to((hi >> min(63, m - eh)) - (lo >> min(63, m - el)), m);
+  return fx_to<true>((hi >> min(63, m - eh)) - (lo >> min(63, m - el)), m);
 }
 
 // The flux differences are exact integers; each is rounded once to a double
@@ -231,34 +231,34 @@ k_rhs_update(ChlMap map, RhsArgs a) {
     const longlong2 x = g2(G[G_UX], c), yh = g2(G[G_UY], e), yl = g2(G[G_UY], em);
     const longlong2 zh = g2(G[G_UZ], c), zl = g2(G[G_UZ], cidx(I, i, jc, km));
     const fx xp = LDG(G[G_UX] + cidx(I, ip, jc, k));
-    Fu.x = fma(fx_to(x.y - x.x, e0.x), rxf0, dpdx);
-    Fu.y = fma(fx_to(xp - x.y, e0.x), rxf1, dpdx);
+    Fu.x = fma(fx_to<true>(x.y - x.x, e0.x), rxf0, dpdx);
+    Fu.y = fma(fx_to<true>(xp - x.y, e0.x), rxf1, dpdx);
     Fu.x = fma(row_diff(yh.x, e0.x, yl.x, el.x), ryc, Fu.x);
     Fu.y = fma(row_diff(yh.y, e0.x, yl.y, el.x), ryc, Fu.y);
-    Fu.x = fma(fx_to(zh.x - zl.x, e0.x), rzc, Fu.x);
-    Fu.y = fma(fx_to(zh.y - zl.y, e0.x), rzc, Fu.y);
+    Fu.x = fma(fx_to<true>(zh.x - zl.x, e0.x), rzc, Fu.x);
+    Fu.y = fma(fx_to<true>(zh.y - zl.y, e0.x), rzc, Fu.y);
   }
   {  // w at (x-centre i, row jc, z-face k)
     const longlong2 x = g2(G[G_WX], c), yh = g2(G[G_WY], e), yl = g2(G[G_WY], em);
     const longlong2 zl = g2(G[G_WZ], c), zh = g2(G[G_WZ], cidx(I, i, jc, kp));
     const fx xm = LDG(G[G_WX] + cidx(I, im, jc, k));
-    Fw.x = fx_to(x.x - xm, e0.z) * rxc0;
-    Fw.y = fx_to(x.y - x.x, e0.z) * rxc1;
+    Fw.x = fx_to<true>(x.x - xm, e0.z) * rxc0;
+    Fw.y = fx_to<true>(x.y - x.x, e0.z) * rxc1;
     Fw.x = fma(row_diff(yh.x, e0.z, yl.x, el.z), ryc, Fw.x);
     Fw.y = fma(row_diff(yh.y, e0.z, yl.y, el.z), ryc, Fw.y);
-    Fw.x = fma(fx_to(zh.x - zl.x, e0.z), rzf, Fw.x);
-    Fw.y = fma(fx_to(zh.y - zl.y, e0.z), rzf, Fw.y);
+    Fw.x = fma(fx_to<true>(zh.x - zl.x, e0.z), rzf, Fw.x);
+    Fw.y = fma(fx_to<true>(zh.y - zl.y, e0.z), rzf, Fw.y);
   }
   if (hasv) {  // v at (x-centre i, y-face jv = jc, z-centre k)
     const longlong2 x = g2(G[G_VX], e), yl = g2(G[G_VY], c), yh = g2(G[G_VY], cidx(I, i, jc + 1, k));
     const longlong2 zh = g2(G[G_VZ], e), zl = g2(G[G_VZ], vidx(I, i, jc, km));
     const fx xm = LDG(G[G_VX] + vidx(I, im, jc, k));
-    Fv.x = fx_to(x.x - xm, e0.y) * rxc0;
-    Fv.y = fx_to(x.y - x.x, e0.y) * rxc1;
+    Fv.x = fx_to<true>(x.x - xm, e0.y) * rxc0;
+    Fv.y = fx_to<true>(x.y - x.x, e0.y) * rxc1;
     Fv.x = fma(row_diff(yh.x, eh.y, yl.x, e0.y), ryf, Fv.x);
     Fv.y = fma(row_diff(yh.y, eh.y, yl.y, e0.y), ryf, Fv.y);
-    Fv.x = fma(fx_to(zh.x - zl.x, e0.y), rzc, Fv.x);
-    Fv.y = fma(fx_to(zh.y - zl.y, e0.y), rzc, Fv.y);
+    Fv.x = fma(fx_to<true>(zh.x - zl.x, e0.y), rzc, Fv.x);
+    Fv.y = fma(fx_to<true>(zh.y - zl.y, e0.y), rzc, Fv.y);
   }
   if (e0.w | el.w | eh.w) {
     const double q = __longlong_as_double(0x7FF8000000000000LL);

@@ -29,63 +29,71 @@
 
 namespace {
 
-// Edge differences around a centre (device indices i, jc, k).  For each
-// off-diagonal velocity gradient the four edge differences are summed in
-// two pairs: s?L/s?H are the two-point sums on the near/far edge in the
-// derivative direction (2 x the reference's first interpolation), s = sL+sH
-// (4 x the centre value) and d = rl sL + rr sH (4 x the centre derivative,
-// the edge differences divided by their centre-to-centre spacings first;
-// along the uniform x and z that is r (sL + sH)).
-// The centre strain of compute_Sij (subgrid.f90:1014-1072) is the same sums:
-// S12 = (dUy + dVx)/8 from the four edges, etc.
-struct Grad {
-  double dux, dvy, dwz;                  // diagonal differences
-  double uyL, uyH, uzL, uzH;             // U: y and z edge pair sums
-  double vxL, vxR, vzL, vzH;             // V: x and z
-  double wxL, wxR, wyL, wyH;             // W: x and y
-  double dUy, dUz, dVx, dVz, dWx, dWy;   // 4 x centre derivatives
-  double rxc, ryc, rzc;
+// Edge differences around the centres of a column of planes, exact integers
+// from the fixed-point copies (k_fix).  For each off-diagonal velocity gradient
+// the four edge differences are summed in two pairs: ?L/?H are the two-point
+// sums on the near/far edge in the derivative direction (2 x the reference's
+// first interpolation), their sum 4 x the centre difference.  The centre
+// strain of compute_Sij (subgrid.f90:1014-1072) is the same sums.  A thread
+// marches through a few planes and carries what they share (pair sums of U
+// and V, differences of W): 17 loads per centre.
+struct Diffs {
+  fx dux, dvy, dwz;                      // diagonal differences
+  fx uyL, uyH, uzL, uzH;                 // U: y and z edge pair sums
+  fx vxL, vxR, vzL, vzH;                 // V: x and z
+  fx wxL, wxR, wyL, wyH;                 // W: x and y
 };
 
-__device__ __forceinline__ Grad gradients(const ChlInst& I, const double* U, const double* V, const double* W,
-                                          int i, int jc, int k) {
-  const int im = wrap(i - 1, I.Nx), ip = wrap(i + 1, I.Nx), km = wrap(k - 1, I.Nz), kp = wrap(k + 1, I.Nz);
-  auto u = [&](int a, int j, int kk) { return LDG(U + cidx(I, a, j, kk)); };
-  auto v = [&](int a, int j, int kk) { return LDG(V + vidx(I, a, j, kk)); };
-  auto w = [&](int a, int j, int kk) { return LDG(W + cidx(I, a, j, kk)); };
-  const double rxl = LDG(I.rdxf + i - 1), rxr = LDG(I.rdxf + i);
-  const double ryl = LDG(I.rdyf + jc - 1), ryr = LDG(I.rdyf + jc);
-  const double rzl = LDG(I.rdzf + k - 1), rzr = LDG(I.rdzf + k);
-  Grad g;
-  g.rxc = LDG(I.rdxc + i); g.ryc = LDG(I.rdyc + jc); g.rzc = LDG(I.rdzc + k);
-  const double u0 = u(i, jc, k), um = u(im, jc, k);
-  const double v0 = v(i, jc, k), vm = v(i, jc - 1, k);
-  const double w0 = w(i, jc, k), wm = w(i, jc, km);
-  g.dux = u0 - um; g.dvy = v0 - vm; g.dwz = w0 - wm;
-  // U at x-faces im, i
-  g.uyL = (um - u(im, jc - 1, k)) + (u0 - u(i, jc - 1, k));
-  g.uyH = (u(im, jc + 1, k) - um) + (u(i, jc + 1, k) - u0);
-  g.uzL = (um - u(im, jc, km)) + (u0 - u(i, jc, km));
-  g.uzH = (u(im, jc, kp) - um) + (u(i, jc, kp) - u0);
-  // V at y-faces jc-1, jc
-  const double vmm = v(im, jc - 1, k), vm0 = v(im, jc, k);
-  g.vxL = (vm - vmm) + (v0 - vm0);
-  g.vxR = (v(ip, jc - 1, k) - vm) + (v(ip, jc, k) - v0);
-  g.vzL = (vm - v(i, jc - 1, km)) + (v0 - v(i, jc, km));
-  g.vzH = (v(i, jc - 1, kp) - vm) + (v(i, jc, kp) - v0);
-  // W at z-faces km, k
-  g.wxL = (wm - w(im, jc, km)) + (w0 - w(im, jc, k));
-  g.wxR = (w(ip, jc, km) - wm) + (w(ip, jc, k) - w0);
-  g.wyL = (wm - w(i, jc - 1, km)) + (w0 - w(i, jc - 1, k));
-  g.wyH = (w(i, jc + 1, km) - wm) + (w(i, jc + 1, k) - w0);
-  // y is stretched: each edge pair by its own spacing; x and z are uniform
-  // (checked at creation), so one spacing times the pair sum
-  (void)rxr; (void)rzr;
-  g.dUy = fma(ryl, g.uyL, ryr * g.uyH); g.dUz = rzl * (g.uzL + g.uzH);
-  g.dVx = rxl * (g.vxL + g.vxR); g.dVz = rzl * (g.vzL + g.vzH);
-  g.dWx = rxl * (g.wxL + g.wxR); g.dWy = fma(ryl, g.wyL, ryr * g.wyH);
-  return g;
-}
+struct GradColumn {
+  const ChlInst& I;
+  int i, im, ip, jc, er;
+  fx rxf, rxc, ryl, ryh, ryc;            // reciprocal spacings, last bit 2^er
+  fx um, u0, uzL, vm, v0, vzL;           // plane k: U and V faces, their z differences to the plane below
+  fx wm, wxl, wxr, wyl, wyh;             // plane k-1: W and its x and y differences
+
+  __device__ __forceinline__ fx u(int a, int j, int k) const { return LDG(I.X[0] + cidx(I, a, j, k)); }
+  __device__ __forceinline__ fx v(int a, int j, int k) const { return LDG(I.X[1] + vidx(I, a, j, k)); }
+  __device__ __forceinline__ fx w(int a, int j, int k) const { return LDG(I.X[2] + cidx(I, a, j, k)); }
+
+  __device__ __forceinline__ GradColumn(const ChlInst& I_, int i_, int jc_, int k) : I(I_), i(i_), jc(jc_) {
+    im = wrap(i - 1, I.Nx); ip = wrap(i + 1, I.Nx);
+    const int el = I.eyf[jc - 1], eh = I.eyf[jc], ec = I.eyc[jc];
+    er = max(max(max(el, eh), max(ec, I.exf)), max(max(I.exc, I.ezf), I.ezc));
+    ryl = LDG(I.fxryf + jc - 1) >> min(63, er - el);
+    ryh = LDG(I.fxryf + jc) >> min(63, er - eh);
+    ryc = LDG(I.fxryc + jc) >> min(63, er - ec);
+    rxf = LDG(I.fxrxf + i - 1) >> min(63, er - I.exf);
+    rxc = LDG(I.fxrxc + i) >> min(63, er - I.exc);
+    const int kb = k == 0 ? I.Nz - 1 : k - 1;
+    um = u(im, jc, k); u0 = u(i, jc, k);
+    vm = v(i, jc - 1, k); v0 = v(i, jc, k);
+    wm = w(i, jc, kb);
+    uzL = (um + u0) - (u(im, jc, kb) + u(i, jc, kb));
+    vzL = (vm + v0) - (v(i, jc - 1, kb) + v(i, jc, kb));
+    wxl = wm - w(im, jc, kb); wxr = w(ip, jc, kb) - wm;
+    wyl = wm - w(i, jc - 1, kb); wyh = w(i, jc + 1, kb) - wm;
+  }
+  __device__ __forceinline__ fx rzf(int k) const { return LDG(I.fxrzf + k - 1) >> min(63, er - I.ezf); }
+  __device__ __forceinline__ fx rzc(int k) const { return LDG(I.fxrzc + k) >> min(63, er - I.ezc); }
+
+  __device__ __forceinline__ Diffs point(int k) {
+    const int kp = k + 1 == I.Nz ? 0 : k + 1;
+    const fx ump = u(im, jc, kp), u0p = u(i, jc, kp), vmp = v(i, jc - 1, kp), v0p = v(i, jc, kp);
+    const fx w0 = w(i, jc, k);
+    const fx us = um + u0, vs = vm + v0;
+    const fx xl = w0 - w(im, jc, k), xr = w(ip, jc, k) - w0, yl = w0 - w(i, jc - 1, k), yh = w(i, jc + 1, k) - w0;
+    Diffs d;
+    d.uyL = us - (u(im, jc - 1, k) + u(i, jc - 1, k)); d.uyH = (u(im, jc + 1, k) + u(i, jc + 1, k)) - us;
+    d.vxL = vs - (v(im, jc - 1, k) + v(im, jc, k)); d.vxR = (v(ip, jc - 1, k) + v(ip, jc, k)) - vs;
+    d.uzL = uzL; d.uzH = (ump + u0p) - us;
+    d.vzL = vzL; d.vzH = (vmp + v0p) - vs;
+    d.wxL = wxl + xl; d.wxR = wxr + xr; d.wyL = wyl + yl; d.wyH = wyh + yh;
+    d.dux = u0 - um; d.dvy = v0 - vm; d.dwz = w0 - wm;
+    uzL = d.uzH; vzL = d.vzH; wxl = xl; wxr = xr; wyl = yl; wyh = yh;
+    um = ump; u0 = u0p; vm = vmp; v0 = v0p; wm = w0;
+    return d;
+  }
+};
 
 // nu + nu_t for the interior centre (i, jc, k) from its unclipped value v,
 // plus the ghost row next to the first and last interior rows; with the
@@ -132,8 +140,6 @@ __device__ __forceinline__ unsigned write_nut_rows(const ChlInst& I, const doubl
 // each point scales its fifteen by their largest, so that the products keep
 // 54 bits or more of the largest product, and forms the derivatives, D and
 // the a_ij there.  N and the division are FP64 (17 instructions).
-// A thread marches through a few planes: what planes share (pair sums of
-// U and V, differences of W) is carried.
 __global__ void __launch_bounds__(CHL_FLUX_THREADS, 5)   // 102 registers: 2, 3, 4, 5, 6 blocks per SM take 417, 321, 289, 288, 290 us
 k_amd(ChlMap map, int s_in, int use_wm) {
   chl_pdl_wait();
@@ -143,64 +149,36 @@ k_amd(ChlMap map, int s_in, int use_wm) {
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
   const ChlIdx p = chl_split(t, Nx, Ny);
   const int i = p.i, jc = 1 + p.j, k0 = p.k * M;
-  const int im = wrap(i - 1, Nx), ip = wrap(i + 1, Nx);
-  const fx* __restrict__ U = I.X[0];
-  const fx* __restrict__ V = I.X[1];
-  const fx* __restrict__ W = I.X[2];
-#define UC(ii, jj, kk) LDG(U + cidx(I, ii, jj, kk))
-#define WC(ii, jj, kk) LDG(W + cidx(I, ii, jj, kk))
-#define VV(ii, jj, kk) LDG(V + vidx(I, ii, jj, kk))
-  // reciprocal spacings with one exponent er
-  const int el = I.eyf[jc - 1], eh = I.eyf[jc], ec = I.eyc[jc];
-  const int er = max(max(max(el, eh), max(ec, I.exf)), max(max(I.exc, I.ezf), I.ezc));
-  const fx ryl = LDG(I.fxryf + jc - 1) >> min(63, er - el), ryh = LDG(I.fxryf + jc) >> min(63, er - eh);
-  const fx ryc = LDG(I.fxryc + jc) >> min(63, er - ec);
-  const fx rxf = LDG(I.fxrxf + i - 1) >> min(63, er - I.exf), rxc = LDG(I.fxrxc + i) >> min(63, er - I.exc);
   const unsigned* vm = chl_vmax(I, s_in);
   const int eu = fx_exp<61>(vm[0]), ev = fx_exp<61>(vm[1]), ew = fx_exp<61>(vm[2]);
   const bool bad = fx_bad(vm[0]) || fx_bad(vm[1]) || fx_bad(vm[2]);
-  const int ks = min(k0, Nz - 1), kb = ks == 0 ? Nz - 1 : ks - 1;    // lanes past the last plane repeat it
-  fx um = UC(im, jc, ks), u0 = UC(i, jc, ks);
-  fx vm0 = VV(i, jc - 1, ks), v0 = VV(i, jc, ks);
-  fx wm = WC(i, jc, kb);
-  fx uzL = (um + u0) - (UC(im, jc, kb) + UC(i, jc, kb));
-  fx vzL = (vm0 + v0) - (VV(i, jc - 1, kb) + VV(i, jc, kb));
-  fx wxl = wm - WC(im, jc, kb), wxr = WC(ip, jc, kb) - wm;          // W's x and y differences, plane below
-  fx wyl = wm - WC(i, jc - 1, kb), wyh = WC(i, jc + 1, kb) - wm;
+  GradColumn col(I, i, jc, min(k0, Nz - 1));       // lanes past the last plane repeat it
+  const int er = col.er;
   unsigned hi = 0u;
   for (int q = 0; q < M; ++q) {
-    const int k = min(k0 + q, Nz - 1), kp = k + 1 == Nz ? 0 : k + 1;
+    const int k = min(k0 + q, Nz - 1);
     const bool valid = k0 + q < Nz;
-    const fx up_m = UC(im, jc, kp), up_0 = UC(i, jc, kp), vp_m = VV(i, jc - 1, kp), vp_0 = VV(i, jc, kp);
-    const fx w0 = WC(i, jc, k), wim = WC(im, jc, k), wip = WC(ip, jc, k);
-    const fx wjm = WC(i, jc - 1, k), wjp = WC(i, jc + 1, k);
-    const fx us = um + u0, vs = vm0 + v0;
-    fx uyL = us - (UC(im, jc - 1, k) + UC(i, jc - 1, k)), uyH = (UC(im, jc + 1, k) + UC(i, jc + 1, k)) - us;
-    fx vxL = vs - (VV(im, jc - 1, k) + VV(im, jc, k)), vxR = (VV(ip, jc - 1, k) + VV(ip, jc, k)) - vs;
-    const fx uzN = (up_m + up_0) - us, vzN = (vp_m + vp_0) - vs;
-    const fx xl = w0 - wim, xr = wip - w0, yl = w0 - wjm, yh = wjp - w0;
-    fx wxL = wxl + xl, wxR = wxr + xr, wyL = wyl + yl, wyH = wyh + yh;
-    fx dux = u0 - um, dvy = v0 - vm0, dwz = w0 - wm;
+    const Diffs d = col.point(k);
+    fx dux = d.dux, dvy = d.dvy, dwz = d.dwz, uyL = d.uyL, uyH = d.uyH, vxL = d.vxL, vxR = d.vxR;
+    fx wxL = d.wxL, wxR = d.wxR, wyL = d.wyL, wyH = d.wyH;
     // scale: |x| < 2^60 in units of 2^et
     unsigned mu = 0u, mv = 0u, mw = 0u;
-    top_or(mu, dux); top_or(mu, uyL); top_or(mu, uyH); top_or(mu, uzL); top_or(mu, uzN);
-    top_or(mv, dvy); top_or(mv, vxL); top_or(mv, vxR); top_or(mv, vzL); top_or(mv, vzN);
+    top_or(mu, dux); top_or(mu, uyL); top_or(mu, uyH); top_or(mu, d.uzL); top_or(mu, d.uzH);
+    top_or(mv, dvy); top_or(mv, vxL); top_or(mv, vxR); top_or(mv, d.vzL); top_or(mv, d.vzH);
     top_or(mw, dwz); top_or(mw, wxL); top_or(mw, wxR); top_or(mw, wyL); top_or(mw, wyH);
     const int et = max(max(eu + 64 - __clz((int)mu), ev + 64 - __clz((int)mv)), ew + 64 - __clz((int)mw)) - 60;
     const int su = eu - et, sv = ev - et, sw = ew - et;
     dux = scale2(dux, su); uyL = scale2(uyL, su); uyH = scale2(uyH, su);
-    const fx uL = scale2(uzL, su), uH = scale2(uzN, su);
+    const fx uL = scale2(d.uzL, su), uH = scale2(d.uzH, su);
     dvy = scale2(dvy, sv); vxL = scale2(vxL, sv); vxR = scale2(vxR, sv);
-    const fx vL = scale2(vzL, sv), vH = scale2(vzN, sv);
+    const fx vL = scale2(d.vzL, sv), vH = scale2(d.vzH, sv);
     dwz = scale2(dwz, sw); wxL = scale2(wxL, sw); wxR = scale2(wxR, sw); wyL = scale2(wyL, sw); wyH = scale2(wyH, sw);
-    uzL = uzN; vzL = vzN; wxl = xl; wxr = xr; wyl = yl; wyh = yh;
-    um = up_m; u0 = up_0; vm0 = vp_m; v0 = vp_0; wm = w0;
     // grid-scaled centre differences, 4 x
     const fx Yu = uyL + uyH, Zu = uL + uH, Xv = vxL + vxR, Zv = vL + vH, Xw = wxL + wxR, Yw = wyL + wyH;
     // derivatives, 4 x, scaled anew: the spacings differ by up to the
     // stretching of the grid (units 2^(et + er + 64 - sd))
-    const fx rzf = LDG(I.fxrzf + k - 1) >> min(63, er - I.ezf), rzc = LDG(I.fxrzc + k) >> min(63, er - I.ezc);
-    fx s11 = 4 * fx_mul(dux, rxc), s22 = 4 * fx_mul(dvy, ryc), s33 = 4 * fx_mul(dwz, rzc);
+    const fx rzf = col.rzf(k), rxf = col.rxf, ryl = col.ryl, ryh = col.ryh;
+    fx s11 = 4 * fx_mul(dux, col.rxc), s22 = 4 * fx_mul(dvy, col.ryc), s33 = 4 * fx_mul(dwz, col.rzc(k));
     fx dUy = fx_mul(uyL, ryl) + fx_mul(uyH, ryh), dWy = fx_mul(wyL, ryl) + fx_mul(wyH, ryh);
     fx dUz = fx_mul(Zu, rzf), dVz = fx_mul(Zv, rzf), dVx = fx_mul(Xv, rxf), dWx = fx_mul(Xw, rxf);
     unsigned md = 0u;
@@ -234,49 +212,87 @@ k_amd(ChlMap map, int s_in, int use_wm) {
     if (valid) I.S[cidx(I, i, jc, k)] = v;
     hi = max(hi, write_nut_rows(I, I.U[s_in], i, jc, k, v, use_wm, valid));
   }
-#undef UC
-#undef WC
-#undef VV
   chl_line_max(I.nmax, (unsigned)(p.k * Ny + p.j), Ny, 1, hi);
 }
 
-__global__ void __launch_bounds__(256)
+// Vreman in fixed point (124 FP64 instructions per point before, 25 now).
+// b_ij sums products of the grid-scaled differences h_m a_mi and h_m a_mj of
+// components i and j, so each component is scaled by its own largest: b_22 of
+// a weak V keeps its digits beside b_11.  Along the uniform x and z the
+// grid-scaled difference is the mean edge difference itself, along y the edge
+// differences times h_y/dy of their spacings.  B_b, which cancels, and the
+// quotient are FP64.
+__global__ void __launch_bounds__(CHL_FLUX_THREADS, 5)
 k_vreman(ChlMap map, int s_in, int use_wm) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
-  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
+  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz, M = map.planes;
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  const bool valid = t < (unsigned)(Nx * Ny * Nz);
-  const ChlIdx p = chl_split(valid ? t : (unsigned)(Nx * Ny * Nz) - 1u, Nx, Ny);
-  const int i = p.i, jc = 1 + p.j, k = p.k;
-  const Grad g = gradients(I, I.U[s_in], I.V[s_in], I.W[s_in], i, jc, k);
-  // a_ij = du_j/dx_i (reference layout 1 4 5 / 7 2 6 / 8 9 3); the
-  // off-diagonal entries are kept 4 x (the 1/16 is folded below)
-  const double a1 = g.dux * g.rxc, a2 = g.dvy * g.ryc, a3 = g.dwz * g.rzc;
-  const double a4 = g.dVx, a5 = g.dWx, a7 = g.dUy, a6 = g.dWy, a8 = g.dUz, a9 = g.dVz;
-  const double hx = LDG(I.hx2 + i), hy = LDG(I.hy2 + jc), hz = LDG(I.hz2 + k);
-  const double qx = 0.0625 * hx, qy = 0.0625 * hy, qz = 0.0625 * hz;
-  // b_ij = sum_m dx_m^2 a_mi a_mj
-  const double b11 = fma(hx * a1, a1, fma(qy * a7, a7, qz * a8 * a8));
-  const double b22 = fma(qx * a4, a4, fma(hy * a2, a2, qz * a9 * a9));
-  const double b33 = fma(qx * a5, a5, fma(qy * a6, a6, hz * a3 * a3));
-  const double hx4 = 0.25 * hx, hy4 = 0.25 * hy, hz4 = 0.25 * hz;
-  const double b12 = fma(hx4 * a1, a4, fma(hy4 * a7, a2, qz * a8 * a9));
-  const double b13 = fma(hx4 * a1, a5, fma(qy * a7, a6, hz4 * a8 * a3));
-  const double b23 = fma(qx * a4, a5, fma(hy4 * a2, a6, hz4 * a9 * a3));
-  const double Bb = b11 * b22 - b12 * b12 + b11 * b33 - b13 * b13 + b22 * b33 - b23 * b23;
-  double Ab = a1 * a1;
-  Ab = fma(a2, a2, Ab); Ab = fma(a3, a3, Ab);
-  double Ao = a4 * a4;
-  Ao = fma(a5, a5, Ao); Ao = fma(a6, a6, Ao); Ao = fma(a7, a7, Ao); Ao = fma(a8, a8, Ao); Ao = fma(a9, a9, Ao);
-  Ab = fma(0.0625, Ao, Ab);
-  const double v = 2.5 * (0.1 * 0.1) * chl_sqrt(Bb / Ab);
-  if (valid) I.S[cidx(I, i, jc, k)] = v;
-  chl_line_max(I.nmax, (unsigned)(k * Ny + jc - 1), Ny, 1, write_nut_rows(I, I.U[s_in], i, jc, k, v, use_wm, valid));
+  const ChlIdx p = chl_split(t, Nx, Ny);
+  const int i = p.i, jc = 1 + p.j, k0 = p.k * M;
+  const unsigned* vm = chl_vmax(I, s_in);
+  const int eu = fx_exp<61>(vm[0]), ev = fx_exp<61>(vm[1]), ew = fx_exp<61>(vm[2]);
+  const bool bad = fx_bad(vm[0]) || fx_bad(vm[1]) || fx_bad(vm[2]);
+  GradColumn col(I, i, jc, min(k0, Nz - 1));
+  const fx wl = LDG(I.fxhyl + jc), wh = LDG(I.fxhyh + jc);      // h_y / dy below and above, 2^-62
+  unsigned hi = 0u;
+  for (int q = 0; q < M; ++q) {
+    const int k = min(k0 + q, Nz - 1);
+    const bool valid = k0 + q < Nz;
+    const Diffs d = col.point(k);
+    // differences of each component below 2^59 in units of 2^eU, 2^eV, 2^eW
+    unsigned mu = 0u, mv = 0u, mw = 0u;
+    top_or(mu, d.dux); top_or(mu, d.uyL); top_or(mu, d.uyH); top_or(mu, d.uzL); top_or(mu, d.uzH);
+    top_or(mv, d.dvy); top_or(mv, d.vxL); top_or(mv, d.vxR); top_or(mv, d.vzL); top_or(mv, d.vzH);
+    top_or(mw, d.dwz); top_or(mw, d.wxL); top_or(mw, d.wxR); top_or(mw, d.wyL); top_or(mw, d.wyH);
+    const int su = __clz((int)mu) - 5, sv = __clz((int)mv) - 5, sw = __clz((int)mw) - 5;
+    const int eU = eu - su, eV = ev - sv, eW = ew - sw;
+    // grid-scaled differences, 4 x, below 2^61: rows x, y, z of u, v, w
+    const fx xu = 4 * scale2(d.dux, su), yv = 4 * scale2(d.dvy, sv), zw = 4 * scale2(d.dwz, sw);
+    const fx yu = 4 * (fx_mul(scale2(d.uyL, su), wl) + fx_mul(scale2(d.uyH, su), wh));
+    const fx yw = 4 * (fx_mul(scale2(d.wyL, sw), wl) + fx_mul(scale2(d.wyH, sw), wh));
+    const fx zu = scale2(d.uzL, su) + scale2(d.uzH, su), zv = scale2(d.vzL, sv) + scale2(d.vzH, sv);
+    const fx xv = scale2(d.vxL, sv) + scale2(d.vxR, sv), xw = scale2(d.wxL, sw) + scale2(d.wxR, sw);
+    // b_ij, 16 x, 2^64 units
+    const double b11 = fx_to(fx_mul(xu, xu) + fx_mul(yu, yu) + fx_mul(zu, zu) + 4, 0);
+    const double b22 = fx_to(fx_mul(xv, xv) + fx_mul(yv, yv) + fx_mul(zv, zv) + 4, 0);
+    const double b33 = fx_to(fx_mul(xw, xw) + fx_mul(yw, yw) + fx_mul(zw, zw) + 4, 0);
+    const double b12 = fx_to(fx_mul(xu, xv) + fx_mul(yu, yv) + fx_mul(zu, zv) + 4, 0);
+    const double b13 = fx_to(fx_mul(xu, xw) + fx_mul(yu, yw) + fx_mul(zu, zw) + 4, 0);
+    const double b23 = fx_to(fx_mul(xv, xw) + fx_mul(yv, yw) + fx_mul(zv, zw) + 4, 0);
+    // B_b, 256 x: pairs of components with their own units
+    const double q12 = b11 * b22 - b12 * b12, q13 = b11 * b33 - b13 * b13, q23 = b22 * b33 - b23 * b23;
+    const int em = max(eU, max(eV, eW));
+    const int n12 = max(-900, 2 * (eU + eV - 2 * em)), n13 = max(-900, 2 * (eU + eW - 2 * em)), n23 = max(-900, 2 * (eV + eW - 2 * em));
+    const double Bb = fma(q12, pow2(n12), fma(q13, pow2(n13), q23 * pow2(n23)));
+    // derivatives, 4 x, in units of 2^(em + er + 64), then scaled by their largest
+    const fx rzf = col.rzf(k), rxf = col.rxf;
+    const int du = eU - em, dv = eV - em, dw = eW - em;
+    fx a1 = fx_mul(xu, col.rxc) >> min(63, -du), a7 = fx_mul(yu, col.ryc) >> min(63, -du), a8 = fx_mul(zu, rzf) >> min(63, -du);
+    fx a4 = fx_mul(xv, rxf) >> min(63, -dv), a2 = fx_mul(yv, col.ryc) >> min(63, -dv), a9 = fx_mul(zv, rzf) >> min(63, -dv);
+    fx a5 = fx_mul(xw, rxf) >> min(63, -dw), a6 = fx_mul(yw, col.ryc) >> min(63, -dw), a3 = fx_mul(zw, col.rzc(k)) >> min(63, -dw);
+    unsigned md = 0u;
+    top_or(md, a1); top_or(md, a2); top_or(md, a3); top_or(md, a4); top_or(md, a5);
+    top_or(md, a6); top_or(md, a7); top_or(md, a8); top_or(md, a9);
+    const int sd = __clz((int)md) - 3;
+    a1 <<= sd; a2 <<= sd; a3 <<= sd; a4 <<= sd; a5 <<= sd; a6 <<= sd; a7 <<= sd; a8 <<= sd; a9 <<= sd;
+    // a_ij a_ij, 16 x, 2^64 units; 12 makes up for nine products
+    const fx A = (fx_mul(a1, a1) + fx_mul(a2, a2) + fx_mul(a3, a3) + 12) +
+                 (fx_mul(a4, a4) + fx_mul(a5, a5) + fx_mul(a6, a6)) +
+                 (fx_mul(a7, a7) + fx_mul(a8, a8) + fx_mul(a9, a9));
+    // C sqrt(B_b / a_ij a_ij): the quotient is 16 x and in units of
+    // 2^(4 em + 128) / 2^(2 (em + er + 64 - sd) + 64)
+    const double x = chl_sqrt(Bb / fx_to(A, 0));
+    double v = (2.5 * (0.1 * 0.1) * 0.25) * x * pow2(min(1023, max(-1022, em - col.er - 32 + sd)));
+    if (bad) v = __longlong_as_double(0x7FF8000000000000LL);
+    if (valid) I.S[cidx(I, i, jc, k)] = v;
+    hi = max(hi, write_nut_rows(I, I.U[s_in], i, jc, k, v, use_wm, valid));
+  }
+  chl_line_max(I.nmax, (unsigned)(p.k * Ny + p.j), Ny, 1, hi);
 }
 
 extern "C" {
 void chl_launch_amd(const ChlMap& m, int nb, int s_in, int use_wm, cudaStream_t st) { chl_launch_pdl(k_amd, dim3(nb), dim3(CHL_FLUX_THREADS), 0, st, m, s_in, use_wm); }
-void chl_launch_vreman(const ChlMap& m, int nb, int s_in, int use_wm, cudaStream_t st) { chl_launch_pdl(k_vreman, dim3(nb), dim3(m.tb), 0, st, m, s_in, use_wm); }
+void chl_launch_vreman(const ChlMap& m, int nb, int s_in, int use_wm, cudaStream_t st) { chl_launch_pdl(k_vreman, dim3(nb), dim3(CHL_FLUX_THREADS), 0, st, m, s_in, use_wm); }
 }
