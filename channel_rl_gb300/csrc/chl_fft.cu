@@ -38,7 +38,7 @@
 // with so that no pass input exceeds 2^61: 56 for N = 256, three bits finer
 // than a double's last bit at the line's largest component; the rounding of a
 // pass (below one unit per product) stays there too.  Measured error of the
-// projection: chl_fft's callers compare with FP64 in tests/test_fft_fixed_gpu.py.
+// projection: chl_fft's callers compare with FP64 in tests/test_fixed_point_gpu.py.
 //
 // Table of a length: per pass {R, Ns, 2^32/Ns, 2^32/(N/R)}, then the twiddles.
 // Twiddles w = c + is as the words (high, low >> 1) of c 2^63 and s 2^63
@@ -47,34 +47,44 @@
 typedef longlong2 fx2;
 __device__ __forceinline__ fx2 add2(fx2 a, fx2 b) { return make_longlong2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ fx2 sub2(fx2 a, fx2 b) { return make_longlong2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ fx2 halve(fx2 a) { return make_longlong2(a.x >> 1, a.y >> 1); }
+// a / 2, ties to even: a constant bias of a quarter of a unit would add up over
+// the rows of the low modes, which the Poisson solve amplifies most
+__device__ __forceinline__ fx half_even(fx a) { return (a + (fx)(((unsigned)a >> 1) & 1u)) >> 1; }
+__device__ __forceinline__ fx2 halve(fx2 a) { return make_longlong2(half_even(a.x), half_even(a.y)); }
 
 // v w / 2 (INV: v conj(w) / 2).  The four cross terms of a component, at most
-// 2^62.9 together for |v| < 2^61, are summed before their one shift; the
-// starting value rounds it, makes up for the dropped low products and, over
-// the R - 1 products of a butterfly, for the quarter of a unit that halving
-// the first input loses on average: the sum of a line, which the mean pressure
-// hangs on, keeps no bias.
-template <int RADIX, bool INV>
+// 2^62.9 together for |v| < 2^61, are summed before their one shift.  The
+// starting value r takes out the mean of what is dropped: half a unit each for
+// the shift and the low products (2^31) and (c + s)/4 for the last bit of v's
+// components, which the signed 32-bit factors have no room for.
+template <bool INV>
 __device__ __forceinline__ fx2 tw_mul(fx2 v, int4 w) {
-  const long long R = (1LL << 31) + (1LL << 29) / (RADIX - 1);
+  const long long r = (long long)(0x80000000u + (unsigned)((w.x >> 2) + (w.z >> 2)));
   const fx n = INV ? -v.x : -v.y;
   const int xh = (int)(v.x >> 32), xl = (int)((unsigned)v.x >> 1);
   const int yh = (int)(v.y >> 32), yl = (int)((unsigned)v.y >> 1);
   const int nh = (int)(n >> 32), nl = (int)((unsigned)n >> 1);
   const int ah = INV ? yh : nh, al = INV ? yl : nl;    // times s into the real part
   const int bh = INV ? nh : xh, bl = INV ? nl : xl;    // times s into the imaginary part
-  long long t = R + (long long)xh * w.y + (long long)w.x * xl;
+  long long t = r + (long long)xh * w.y + (long long)w.x * xl;
   t += (long long)ah * w.w;
   t += (long long)w.z * al;
-  long long u = R + (long long)yh * w.y + (long long)w.x * yl;
+  long long u = r + (long long)yh * w.y + (long long)w.x * yl;
   u += (long long)bh * w.w;
   u += (long long)w.z * bl;
   return make_longlong2((long long)xh * w.x + (long long)ah * w.z + (t >> 31),
                         (long long)yh * w.x + (long long)bh * w.z + (u >> 31));
 }
 
-#define FX_SIN60 0x6ED9EBA16132A9CFLL   // sin(2 pi/3) 2^63
+// a sin(2 pi/3), |a| < 2^62.  The means of the dropped low product (0.380 of a
+// unit), last bit of a (0.433) and shift (0.5) come back with the start of t.
+__device__ __forceinline__ fx sin60_mul(fx a) {
+  const fx w = 0x6ED9EBA16132A9CFLL;   // sin(2 pi/3) 2^63
+  const int ah = (int)(a >> 32), wh = (int)(w >> 32);
+  const int al = (int)((unsigned)a >> 1), wl = (int)((unsigned)w >> 1);
+  const long long t = 1409783857LL + (long long)ah * wl + (long long)wh * al;
+  return (fx)((unsigned long long)((long long)ah * wh) << 1) + (t >> 30);
+}
 // Butterfly of v[0..R): the first input as it is (pass one) or halved by the
 // caller, the others twiddled.
 template <int R, bool INV>
@@ -92,7 +102,7 @@ __device__ __forceinline__ void butterfly(fx2* v) {
   } else {
     const fx2 t0 = add2(v[1], v[2]), d = sub2(v[1], v[2]);
     const fx2 t = sub2(v[0], halve(t0));
-    const fx mx = 2 * fx_mul(d.x, FX_SIN60), my = 2 * fx_mul(d.y, FX_SIN60);
+    const fx mx = sin60_mul(d.x), my = sin60_mul(d.y);
     v[0] = add2(v[0], t0);
     const fx2 p = make_longlong2(t.x + my, t.y - mx), q = make_longlong2(t.x - my, t.y + mx);
     v[1] = INV ? q : p; v[2] = INV ? p : q;
@@ -136,7 +146,7 @@ __device__ __forceinline__ void fx_pass(const LD& ld, const ST& st, const SmallD
       const int g = small_div(j, (unsigned)pass.z), jm = j - g * Ns;
       v[0] = halve(v[0]);
 #pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = tw_mul<R, INV>(v[r], smem_tw()[tab + (r - 1) * Ns + jm]);
+      for (int r = 1; r < R; ++r) v[r] = tw_mul<INV>(v[r], smem_tw()[tab + (r - 1) * Ns + jm]);
       o = g * Ns * R + jm;
       step = Ns;
     }
@@ -800,14 +810,17 @@ k_zsolve(ChlMap map) {
 
 // ------------------------------------------------------------ inverse x -> pressure field
 // the packed line of two real rows from their half-spectra pa, pb (stored at
-// kx and Nxh + kx): element kx is pa + i pb, element Nx - kx conj(pa) + i conj(pb)
+// kx and Nxh + kx): element kx is pa + i pb, element Nx - kx conj(pa) + i
+// conj(pb).  At kx = 0 and Nx/2 both are real; the rounding that the z passes
+// leave in their imaginary parts would go into the other row.
 struct PackLd {
   int pitch, Nx; LineIn in;
   __device__ __forceinline__ fx2 operator()(int r, int e) const {
     const bool lo = e <= Nx / 2;
     const double2* q = smem_d2() + r * pitch + (lo ? e : Nx - e);
     const int s = in.exponent(r);
-    const fx2 a = fx2_from(q[0], s), b = fx2_from(q[Nx / 2 + 1], s);
+    fx2 a = fx2_from(q[0], s), b = fx2_from(q[Nx / 2 + 1], s);
+    if (e == 0 || 2 * e == Nx) a.y = b.y = 0;
     return lo ? make_longlong2(a.x - b.y, a.y + b.x) : make_longlong2(a.x + b.y, b.x - a.y);
   }
 };
