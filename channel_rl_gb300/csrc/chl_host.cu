@@ -300,12 +300,29 @@ int dsm_npart(int Nx, int Ny, int Nz) {
 
 struct ProfRec { const char* name; int ev; };
 
+// The second stream of a step's capture and the events that fork and join it;
+// they end with the capture, the graph keeps only the dependencies.
+struct SideBranch {
+  struct Handles { cudaStream_t st = nullptr; cudaEvent_t fork = nullptr, wall = nullptr, dt = nullptr; } b;
+  cudaError_t open() {
+    cudaError_t e = cudaStreamCreateWithFlags(&b.st, cudaStreamNonBlocking);
+    for (cudaEvent_t* v : {&b.fork, &b.wall, &b.dt})
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(v, cudaEventDisableTiming);
+    return e;
+  }
+  ~SideBranch() {
+    for (cudaEvent_t v : {b.fork, b.wall, b.dt}) if (v) cudaEventDestroy(v);
+    if (b.st) cudaStreamDestroy(b.st);
+  }
+};
+
 struct chl_handle {
   std::vector<Inst> in;
   // per-launch event profiling (chl_profile_step)
   bool prof = false;
   std::vector<cudaEvent_t> ev;
   std::vector<ProfRec> rec;
+  SideBranch::Handles side;           // set while a step is captured
   ChlInst* d_inst = nullptr;
   cudaStream_t st = nullptr;
   // copy streams of the host-buffer round trip: the next step's upload and
@@ -653,19 +670,29 @@ static int build_maps(chl_handle* h) {
 }
 
 // ------------------------------------------------------------ schedules
-static int enqueue_sgs(chl_handle* h, int s, bool with_wm, int stage = 0) {
+static void enqueue_dt(chl_handle* h, cudaStream_t st);
+// with_dt: the time step's reduction (set 0 only) goes with it.
+static int enqueue_sgs(chl_handle* h, int s, bool with_wm, int stage = 0, bool with_dt = false) {
   cudaStream_t st = h->st;
   // AMD and Vreman write nu + nu_t in their own kernel, whose wall-model
   // rows need the wall stress first; the other models leave it to k_nut
   const bool fused = h->LES_model == CHL_LES_AMD || h->LES_model == CHL_LES_VREMAN;
-  auto wall_stress = [&]() {
-    if (with_wm && (h->wall_model == CHL_WM_EQLOG || h->wall_model == CHL_WM_MLP))
-      KL("eq_wallmodel", chl_launch_eqwm(h->map(M_WALLN), h->nblk[M_WALLN], s, st));
-    if (with_wm && h->wall_model == CHL_WM_MLP)
-      KL("mlp_wallmodel", chl_launch_mlp(h->map(M_MLP), h->nblk[M_MLP], s, stage, h->d_mlp_status, st));
-  };
+  // What needs only the velocities goes on the step graph's side branch
+  // where it has one: the wall stress, which nu + nu_t takes, and the time
+  // step, which the stage update takes (and the learned model's stress).
+  const bool wall = with_wm && h->wall_model >= CHL_WM_EQLOG, mlp = wall && h->wall_model == CHL_WM_MLP;
+  const bool fork = h->side.st && (wall || with_dt);
+  cudaStream_t sd = fork ? h->side.st : st;
+  if (fork) { CK(cudaEventRecord(h->side.fork, st)); CK(cudaStreamWaitEvent(sd, h->side.fork, 0)); }
+  if (with_dt && (mlp || !wall || !fork)) enqueue_dt(h, sd);
+  if (wall) KL("eq_wallmodel", chl_launch_eqwm(h->map(M_WALLN), h->nblk[M_WALLN], s, sd));
+  if (mlp) KL("mlp_wallmodel", chl_launch_mlp(h->map(M_MLP), h->nblk[M_MLP], s, stage, h->d_mlp_status, sd));
+  if (fork && wall) CK(cudaEventRecord(h->side.wall, sd));
+  if (with_dt && wall && !mlp && fork) enqueue_dt(h, sd);
+  if (fork) CK(cudaEventRecord(h->side.dt, sd));
+  auto wall_stress = [&]() -> cudaError_t { return fork && wall ? cudaStreamWaitEvent(st, h->side.wall, 0) : cudaSuccess; };
   KL("fix", chl_launch_fix(h->map(M_FULL2), h->nblk[M_FULL2], s, 1, st));
-  if (fused) wall_stress();
+  if (fused) CK(wall_stress());
   if (h->LES_model == CHL_LES_DYNAMIC) {
     KL("strain", chl_launch_strain(h->map(M_MARCH), h->nblk[M_MARCH], s, 1, st));
     KL("filter", chl_launch_filter(h->map(M_FILTER), h->nblk[M_FILTER], h->tb_filter, st));
@@ -681,7 +708,7 @@ static int enqueue_sgs(chl_handle* h, int s, bool with_wm, int stage = 0) {
   // the last block of each row of its plane sums)
   if (h->LES_model == CHL_LES_SMAGORINSKY) KL("nut_coef", chl_launch_coef(h->map(M_PT), st));
   if (!fused) {
-    wall_stress();
+    CK(wall_stress());
     KL("nut", chl_launch_nut(h->map(M_FULL2), h->nblk[M_FULL2], s, with_wm ? 1 : 0, st));
   }
   LAUNCHED();
@@ -719,22 +746,21 @@ static void enqueue_rhs_only(chl_handle* h) {
 // compute_dt: one launch.  k_minabs's last block per instance forms dt
 // (and resets the minima); with every instance on a fixed step only the
 // non-finite check runs, and it stores dt = -CFL.
-static int enqueue_dt(chl_handle* h) {
+static void enqueue_dt(chl_handle* h, cudaStream_t st) {
   bool fixed = true;   // every instance on a fixed step: only the non-finite check
   for (auto& I : h->in) fixed = fixed && I.d.CFL < 0.0;
-  if (fixed) KL("dt_minabs", chl_launch_nonfinite(h->map(M_PT), h->nblk[M_PT], 0, h->st));
-  else KL("dt_minabs", chl_launch_minabs(h->map(M_MINABS), h->nblk[M_MINABS], 0, h->st));
-  LAUNCHED();
-  return CHL_OK;
+  if (fixed) KL("dt_minabs", chl_launch_nonfinite(h->map(M_PT), h->nblk[M_PT], 0, st));
+  else KL("dt_minabs", chl_launch_minabs(h->map(M_MINABS), h->nblk[M_MINABS], 0, st));
 }
 
-static int enqueue_rk3(chl_handle* h) {
+static int enqueue_rk3(chl_handle* h, bool with_dt) {
   // set in -> out per stage: 0 -> 1, 1 -> 2, 2 -> 0 (base is always set 0)
   const int sin[3] = {0, 1, 2}, sout[3] = {1, 2, 0};
   for (int s = 0; s < 3; ++s) {
-    int rc = enqueue_sgs(h, sin[s], h->wall_model != CHL_WM_NONE, s);
+    int rc = enqueue_sgs(h, sin[s], h->wall_model != CHL_WM_NONE, s, with_dt && s == 0);
     if (rc) return rc;
     KL("rhs_flux", chl_launch_flux(h->map(M_FLUX), h->nblk[M_FLUX], sin[s], h->st));
+    if (with_dt && s == 0 && h->side.st) CK(cudaStreamWaitEvent(h->st, h->side.dt, 0));
     KL("rhs_update", chl_launch_update(h->map(M_PT2), h->nblk[M_PT2], 0, sout[s], s, s == 0 ? 0 : 1, h->st));
     LAUNCHED();
     rc = enqueue_projection(h, sout[s], 0);
@@ -1178,13 +1204,14 @@ int chl_set_scalars(chl_handle* h, int inst, const double* in4) {
 
 int chl_compute_dt(chl_handle* h) {
   int rc = check_ready(h); if (rc) return rc;
-  rc = enqueue_dt(h); if (rc) return rc;
+  enqueue_dt(h, h->st);
+  LAUNCHED();
   return finish(h);
 }
 
 int chl_compute_time_step_RK3(chl_handle* h) {
   int rc = check_ready(h); if (rc) return rc;
-  rc = enqueue_rk3(h); if (rc) return rc;
+  rc = enqueue_rk3(h, false); if (rc) return rc;
   return finish(h);
 }
 
@@ -1192,9 +1219,12 @@ int chl_rk3_step(chl_handle* h, int nsteps) {
   int rc = check_ready(h); if (rc) return rc;
   if (nsteps < 0) { h->err = "nsteps < 0"; return CHL_E_ARG; }
   if (!h->gexec) {
+    SideBranch side;
+    CK(side.open());
     CK(cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
-    rc = enqueue_dt(h);
-    if (!rc) rc = enqueue_rk3(h);
+    h->side = side.b;
+    rc = enqueue_rk3(h, true);
+    h->side = SideBranch::Handles{};
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(h->st, &g);
     if (rc) { if (g) cudaGraphDestroy(g); return rc; }
@@ -1595,8 +1625,7 @@ int chl_profile_step(chl_handle* h, int reps, int maxk, char* names, double* ms_
   for (int r = 0; r < reps; ++r) {
     h->rec.clear();
     h->prof = true;
-    rc = enqueue_dt(h);
-    if (!rc) rc = enqueue_rk3(h);
+    rc = enqueue_rk3(h, true);
     h->prof = false;
     if (rc) return rc;
     CK(cudaStreamSynchronize(h->st));
