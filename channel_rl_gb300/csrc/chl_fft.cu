@@ -380,244 +380,209 @@ k_fftz(ChlMap map, int zcw) {
 }
 
 // ------------------------------------------------------------ tridiagonal per mode
-__global__ void __launch_bounds__(128)
+// The solves are serial chains of FP64 instructions, one of which holds a
+// warp's scheduler for 64 clocks; a channel has few chains, so they are cut
+// as fine as they go: the real and the imaginary part of a mode are columns
+// of their own, in neighbouring lanes (column t = 2 mode + part, rows 2 ps
+// doubles apart; the factors are shared).  With a mode per thread a warp
+// issued 6 FP64 instructions per row where it now issues 3, and the last wave
+// of 774 warps at 256x96x192 left 442 of the 608 schedulers with half the
+// work: 57 us per launch there, now 40 (HBM floor 20); 23 and 17 us for the
+// staged form at 64^3 (5 of them the launch between events).
+// Forward, the product with inv is formed apart from the chain, which is one
+// FMA per row.
+// rows [j0, j0 + TB) of [lo, hi): v[q] = p[j stride]
+template <int TB>
+__device__ __forceinline__ void tri_up(double (&v)[TB], const double* p, size_t stride, int j0, int hi) {
+#pragma unroll
+  for (int q = 0; q < TB; ++q) if (j0 + q < hi) v[q] = p[(size_t)(j0 + q) * stride];
+}
+// rows j1, j1 - 1, ... down to lo
+template <int TB>
+__device__ __forceinline__ void tri_down(double (&v)[TB], const double* p, size_t stride, int j1, int lo) {
+#pragma unroll
+  for (int q = 0; q < TB; ++q) if (j1 - q >= lo) v[q] = p[(size_t)(j1 - q) * stride];
+}
+// Forward elimination y_j = inv_j d_j - m_j y_{j-1} over rows [lo, hi) of a
+// column from y = prev (d: column and row stride; fi, fm: the mode's factors,
+// rows ps apart); STORE: into d, else forms the affine map y_in -> y of the
+// rows, A the product of the -m_j.  The recurrence is serial in j; the loads
+// are not: TB rows are fetched together, and from global memory (GLOBAL) while
+// the TB rows before them are in the chain (47 -> 40 us at 256x96x192; from
+// shared memory it only costs registers).  Short columns leave the last TB
+// early: a predicated-off FP64 instruction takes its 64 clocks all the same.
+template <int TB, bool GLOBAL, bool STORE>
+__device__ __forceinline__ double tri_forward(double* d, size_t ds, const double* __restrict__ fi,
+                                              const double* __restrict__ fm, size_t ps, int lo, int hi, double prev,
+                                              double& A) {
+  double nx[TB], ni[TB], nm[TB];
+  auto fetch = [&](int j) { tri_up(nx, d, ds, j, hi); tri_up(ni, fi, ps, j, hi); tri_up(nm, fm, ps, j, hi); };
+  if (GLOBAL) fetch(lo);
+  for (int j0 = lo; j0 < hi; j0 += TB) {
+    if (!GLOBAL) fetch(j0);
+    double x[TB], m[TB];
+#pragma unroll
+    for (int q = 0; q < TB; ++q) { if (GLOBAL) x[q] = nx[q] * ni[q]; m[q] = nm[q]; }
+    if (GLOBAL) fetch(j0 + TB);
+#pragma unroll
+    for (int q = 0; q < TB; ++q) {
+      if (!GLOBAL && j0 + q >= hi) break;
+      if (j0 + q < hi) {
+        prev = fma(-m[q], prev, GLOBAL ? x[q] : nx[q] * ni[q]);   // m = 0 on the first row
+        if (STORE) d[(size_t)(j0 + q) * ds] = prev;
+        else A = -m[q] * A;
+      }
+    }
+  }
+  return prev;
+}
+// back substitution x_j = y_j - c_j x_{j+1} from the top (c = 0 on the last row)
+template <int TB, bool GLOBAL, bool STORE>
+__device__ __forceinline__ double tri_backward(const double* y, size_t ys, double* d, size_t ds, const double* __restrict__ fc,
+                                               size_t ps, int lo, int hi, double prev, double& A) {
+  double nx[TB], nc[TB];
+  auto fetch = [&](int j) { tri_down(nx, y, ys, j, lo); tri_down(nc, fc, ps, j, lo); };
+  if (GLOBAL) fetch(hi - 1);
+  for (int j1 = hi - 1; j1 >= lo; j1 -= TB) {
+    if (!GLOBAL) fetch(j1);
+    double x[TB], c[TB];
+#pragma unroll
+    for (int q = 0; q < TB; ++q) { x[q] = nx[q]; c[q] = nc[q]; }
+    if (GLOBAL) fetch(j1 - TB);
+#pragma unroll
+    for (int q = 0; q < TB; ++q) {
+      if (!GLOBAL && j1 - q < lo) break;
+      if (j1 - q >= lo) {
+        prev = fma(-c[q], prev, x[q]);
+        if (STORE) d[(size_t)(j1 - q) * ds] = prev;
+        else A = -c[q] * A;
+      }
+    }
+  }
+  return prev;
+}
+
+__global__ void __launch_bounds__(128, 4)
 k_tri(ChlMap map) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
-  const int Ny = I.Ny, Nz = I.Nz, Nxh = I.Nxh;
-  const int mode = lb * blockDim.x + threadIdx.x;
-  if (mode >= Nz * Nxh) return;
-  const size_t ps = (size_t)Nz * Nxh;           // row pitch of spec and factors
-  double2* __restrict__ s = I.spec + ps + mode;  // row jc = 1
-  const double* __restrict__ fi = I.tri_inv + mode;
-  const double* __restrict__ fm = I.tri_m + mode;
-  const double* __restrict__ fc = I.tri_c + mode;
-  // The recurrence is serial in j; the loads are not.  Rows are fetched
-  // TB at a time ahead of the chain so their latency overlaps.
-  constexpr int TB = 8;
-  double2 prev = make_double2(0.0, 0.0);
-  for (int j0 = 0; j0 < Ny; j0 += TB) {
-    double2 d[TB]; double iv[TB], m[TB];
-#pragma unroll
-    for (int q = 0; q < TB; ++q) {
-      const int j = j0 + q;
-      if (j < Ny) { d[q] = s[(size_t)j * ps]; iv[q] = LDG(fi + (size_t)j * ps); m[q] = LDG(fm + (size_t)j * ps); }
-    }
-#pragma unroll
-    for (int q = 0; q < TB; ++q) {
-      const int j = j0 + q;
-      if (j < Ny) {
-        d[q].x = fma(d[q].x, iv[q], -m[q] * prev.x);   // m = 0 on the first row
-        d[q].y = fma(d[q].y, iv[q], -m[q] * prev.y);
-        prev = d[q];
-        s[(size_t)j * ps] = d[q];
-      }
-    }
-  }
-  // back substitution from the last row (prev holds it)
-  for (int j1 = Ny - 2; j1 >= 0; j1 -= TB) {
-    double2 d[TB]; double c[TB];
-#pragma unroll
-    for (int q = 0; q < TB; ++q) {
-      const int j = j1 - q;
-      if (j >= 0) { d[q] = s[(size_t)j * ps]; c[q] = LDG(fc + (size_t)j * ps); }
-    }
-#pragma unroll
-    for (int q = 0; q < TB; ++q) {
-      const int j = j1 - q;
-      if (j >= 0) {
-        d[q].x = fma(-c[q], prev.x, d[q].x);
-        d[q].y = fma(-c[q], prev.y, d[q].y);
-        prev = d[q];
-        s[(size_t)j * ps] = d[q];
-      }
-    }
-  }
+  const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x, mode = t >> 1;
+  const size_t ps = (size_t)I.Nz * I.Nxh;       // row pitch of spec and factors
+  if (mode >= ps) return;
+  double* d = reinterpret_cast<double*>(I.spec + ps) + t;   // row jc = 1
+  double A = 1.0;
+  tri_forward<8, true, true>(d, 2 * ps, I.tri_inv + mode, I.tri_m + mode, ps, 0, I.Ny, 0.0, A);
+  tri_backward<8, true, true>(d, 2 * ps, d, 2 * ps, I.tri_c + mode, ps, 0, I.Ny, 0.0, A);
 }
 
-// Staged form, for columns that fit in shared memory.  One warp of TRI_W
-// modes per block.  Each thread copies its own mode's Ny rows of right side
-// and factors into shared memory with cp.async (all rows in flight at once,
-// where the form above waits once per TB rows), runs both sweeps there and
-// writes only the solution.  A thread reads back only what it copied
+// Staged form, for columns that fit in shared memory: TRI_W modes, 2 TRI_W
+// threads per block.  Each thread copies its column and, with its neighbour,
+// the mode's factors into shared memory with cp.async (all rows in flight at
+// once, where the form above waits once per TB rows), runs both sweeps there
+// and writes only the solution.  A warp reads back only what it copied
 // itself, so the copies need a wait but no block barrier.  The arithmetic
 // and its order are those of k_tri.
 #define TRI_W 32
-__device__ __forceinline__ void cp_async16(void* sdst, const void* gsrc) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" :: "r"(s), "l"(gsrc) : "memory");
-}
 __device__ __forceinline__ void cp_async8(void* sdst, const void* gsrc) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" :: "r"(s), "l"(gsrc) : "memory");
 }
 
-__global__ void __launch_bounds__(TRI_W)
+__global__ void __launch_bounds__(2 * TRI_W)
 k_tri_staged(ChlMap map) {
   chl_pdl_wait();
   extern __shared__ double2 smt[];
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
-  const int Ny = I.Ny, Nz = I.Nz, Nxh = I.Nxh;
-  const int t = threadIdx.x;
-  const int mode = lb * TRI_W + t;
-  if (mode >= Nz * Nxh) return;
-  const size_t ps = (size_t)Nz * Nxh;
-  double2* __restrict__ s = I.spec + ps + mode;  // row jc = 1
-  // [Ny][TRI_W] right side, then [Ny][TRI_W] x (inv, m, c) as doubles
-  double2* sd = smt;
-  double* sf = reinterpret_cast<double*>(smt + (size_t)Ny * TRI_W);
-  double* si = sf;
-  double* sm = sf + (size_t)Ny * TRI_W;
-  double* sc = sf + (size_t)2 * Ny * TRI_W;
-  for (int j = 0; j < Ny; ++j) {
-    const size_t g = (size_t)j * ps, l = (size_t)j * TRI_W + t;
-    cp_async16(sd + l, s + g);
-    cp_async8(si + l, I.tri_inv + mode + g);
-    cp_async8(sm + l, I.tri_m + mode + g);
-    cp_async8(sc + l, I.tri_c + mode + g);
+  const int Ny = I.Ny;
+  const size_t ps = (size_t)I.Nz * I.Nxh;       // row pitch of spec and factors
+  const int t = threadIdx.x, m = t >> 1;
+  const size_t mode = (size_t)lb * TRI_W + m;
+  const bool valid = mode < ps;                 // lanes past the last mode copy nothing
+  double* d = reinterpret_cast<double*>(I.spec + ps + mode) + (t & 1);   // row jc = 1
+  // [Ny][2 TRI_W] right side, then [Ny][TRI_W] inv, m and c
+  double* sd = reinterpret_cast<double*>(smt);
+  double* si = sd + (size_t)Ny * 2 * TRI_W;
+  double* sm = si + (size_t)Ny * TRI_W;
+  double* sc = sm + (size_t)Ny * TRI_W;
+  for (int j = 0; valid && j < Ny; ++j) {
+    const size_t g = (size_t)j * ps + mode, l = (size_t)j * TRI_W + m;
+    cp_async8(sd + (size_t)j * 2 * TRI_W + t, d + (size_t)j * 2 * ps);
+    if (t & 1) {
+      cp_async8(sc + l, I.tri_c + g);
+    } else {
+      cp_async8(si + l, I.tri_inv + g);
+      cp_async8(sm + l, I.tri_m + g);
+    }
   }
   asm volatile("cp.async.commit_group;\n" ::: "memory");
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  double2 prev = make_double2(0.0, 0.0);
-  for (int j = 0; j < Ny; ++j) {
-    const size_t l = (size_t)j * TRI_W + t;
-    double2 d = sd[l];
-    const double iv = si[l], m = sm[l];
-    d.x = fma(d.x, iv, -m * prev.x);   // m = 0 on the first row
-    d.y = fma(d.y, iv, -m * prev.y);
-    prev = d;
-    sd[l] = d;
-  }
-  s[(size_t)(Ny - 1) * ps] = prev;
-  for (int j = Ny - 2; j >= 0; --j) {
-    const size_t l = (size_t)j * TRI_W + t;
-    double2 d = sd[l];
-    const double c = sc[l];
-    d.x = fma(-c, prev.x, d.x);
-    d.y = fma(-c, prev.y, d.y);
-    prev = d;
-    s[(size_t)j * ps] = d;
-  }
+  __syncwarp();
+  if (!valid) return;
+  double A = 1.0;
+  tri_forward<8, false, true>(sd + t, 2 * TRI_W, si + m, sm + m, TRI_W, 0, Ny, 0.0, A);
+  tri_backward<8, false, true>(sd + t, 2 * TRI_W, d, 2 * ps, sc + m, TRI_W, 0, Ny, 0.0, A);
 }
 
 // Lane-split form, for instances with few modes: chl_tri_lanes(modes, Ny) =
-// P lanes per mode (P = 1 for the larger instances of the same launch).
+// P lanes per column (P = 1 for the larger instances of the same launch).
 // Lane p owns rows [p L, (p+1) L), L = ceil(Ny / P).  Forward, the
-// elimination y_j = iv_j d_j - m_j y_{j-1} maps the value entering a lane's
-// rows affinely to the value leaving them: A y_in + B, A the product of the
-// -m_j.  Each lane forms (A, B) from y_in = 0, an inclusive scan of these
-// maps over the P lanes (warp shuffles within the lane group) gives every
-// lane its y_in, and the lane reruns its rows from it, storing them.  The
-// back substitution x_j = y_j - c_j x_{j+1} (c = 0 on the last row) is split
-// the same way from the top.  With P = 1 the arithmetic is k_tri's; with
-// P > 1 the scan rounds differently from the serial sweep (the multipliers
-// are below 1 in magnitude, so the maps are contractions).  Every lane of a
-// warp reaches the shuffles: a lane group belongs to one mode, and lanes
-// past the last mode carry no rows.
-// Rows of a lane are streamed TB at a time, their loads issued ahead of the
-// serial arithmetic as in k_tri.
-#define TSB 8
+// elimination maps the value entering a lane's rows affinely to the value
+// leaving them: A y_in + B.  Each lane forms (A, B) from y_in = 0, an
+// inclusive scan of these maps over the P lanes (warp shuffles within the lane
+// group) gives every lane its y_in, and the lane reruns its rows from it,
+// storing them.  The back substitution is split the same way from the top.
+// With P = 1 the arithmetic is k_tri's; with P > 1 the scan rounds
+// differently from the serial sweep (the multipliers are below 1 in
+// magnitude, so the maps are contractions).  Every lane of a warp reaches the
+// shuffles: a lane group belongs to one column, and lanes past the last
+// carry no rows.
+//
+// The scan: the map (A, z) of lane p's rows in, the value entering them out
+// (0 for the first lane).  UP: lane 0 first, else lane P - 1.
+template <bool UP>
+__device__ __forceinline__ double tri_lane_scan(double A, double z, int p, int P) {
+  const unsigned full = 0xffffffffu;
+  for (int off = 1; off < P; off <<= 1) {
+    const double Ao = UP ? __shfl_up_sync(full, A, off, P) : __shfl_down_sync(full, A, off, P);
+    const double b = UP ? __shfl_up_sync(full, z, off, P) : __shfl_down_sync(full, z, off, P);
+    if (UP ? p >= off : p + off < P) { z = fma(A, b, z); A *= Ao; }
+  }
+  const double in = UP ? __shfl_up_sync(full, z, 1, P) : __shfl_down_sync(full, z, 1, P);
+  return p == (UP ? 0 : P - 1) ? 0.0 : in;
+}
 __global__ void __launch_bounds__(128)
 k_tri_scan(ChlMap map) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
   const int Ny = I.Ny;
-  const long modes = (long)I.Nz * I.Nxh;
-  const int P = chl_tri_lanes(modes, Ny);
-  const long g = (long)lb * blockDim.x + threadIdx.x;
-  const long mode = g / P;
+  const size_t ps = (size_t)I.Nz * I.Nxh;           // row pitch of spec and factors
+  const int P = chl_tri_lanes((long)ps, Ny);
+  const unsigned g = (unsigned)lb * blockDim.x + threadIdx.x, col = g / P;
   const int p = (int)(g % P);
-  const bool valid = mode < modes;
+  const bool valid = col < 2 * ps;
   const int L = (Ny + P - 1) / P;
   const int lo = min(Ny, p * L);
   const int hi = valid ? min(Ny, lo + L) : lo;      // rows [lo, hi) of this lane
-  const size_t ps = (size_t)modes;                  // row pitch of spec and factors
-  const long mm = valid ? mode : 0;
-  double2* __restrict__ s = I.spec + ps + mm;       // row jc = 1
-  const double* __restrict__ fi = I.tri_inv + mm;
-  const double* __restrict__ fm = I.tri_m + mm;
-  const double* __restrict__ fc = I.tri_c + mm;
-  const unsigned full = 0xffffffffu;
-  // forward sweep over [lo, hi) from `prev`; store = false only forms the
-  // lane's affine map (prev from 0, A the product of the -m_j)
-  auto forward = [&](double2 prev, bool store, double& A) {
-    for (int j0 = lo; j0 < hi; j0 += TSB) {
-      double2 d[TSB]; double iv[TSB], m[TSB];
-#pragma unroll
-      for (int q = 0; q < TSB; ++q) {
-        const int j = j0 + q;
-        if (j < hi) { d[q] = s[(size_t)j * ps]; iv[q] = LDG(fi + (size_t)j * ps); m[q] = LDG(fm + (size_t)j * ps); }
-      }
-#pragma unroll
-      for (int q = 0; q < TSB; ++q) {
-        const int j = j0 + q;
-        if (j < hi) {
-          d[q].x = fma(d[q].x, iv[q], -m[q] * prev.x);   // m = 0 on the first row
-          d[q].y = fma(d[q].y, iv[q], -m[q] * prev.y);
-          prev = d[q];
-          if (store) s[(size_t)j * ps] = d[q];
-          else A = -m[q] * A;
-        }
-      }
-    }
-    return prev;
-  };
-  auto backward = [&](double2 prev, bool store, double& A) {
-    for (int j1 = hi - 1; j1 >= lo; j1 -= TSB) {
-      double2 d[TSB]; double c[TSB];
-#pragma unroll
-      for (int q = 0; q < TSB; ++q) {
-        const int j = j1 - q;
-        if (j >= lo) { d[q] = s[(size_t)j * ps]; c[q] = LDG(fc + (size_t)j * ps); }
-      }
-#pragma unroll
-      for (int q = 0; q < TSB; ++q) {
-        const int j = j1 - q;
-        if (j >= lo) {
-          d[q].x = fma(-c[q], prev.x, d[q].x);        // c = 0 on the last row
-          d[q].y = fma(-c[q], prev.y, d[q].y);
-          prev = d[q];
-          if (store) s[(size_t)j * ps] = d[q];
-          else A = -c[q] * A;
-        }
-      }
-    }
-    return prev;
-  };
-  // ---- forward elimination
-  double2 yin = make_double2(0.0, 0.0);
+  const size_t c = valid ? col : 0, mode = c >> 1;
+  double* d = reinterpret_cast<double*>(I.spec + ps) + c;       // row jc = 1
+  const double* fi = I.tri_inv + mode;
+  const double* fm = I.tri_m + mode;
+  const double* fc = I.tri_c + mode;
+  double A = 1.0, in = 0.0;
   if (P > 1) {
-    double A = 1.0;
-    double2 z = forward(make_double2(0.0, 0.0), false, A);
-    for (int off = 1; off < P; off <<= 1) {
-      const double Ao = __shfl_up_sync(full, A, off, P);
-      const double bx = __shfl_up_sync(full, z.x, off, P), by = __shfl_up_sync(full, z.y, off, P);
-      if (p >= off) { z.x = fma(A, bx, z.x); z.y = fma(A, by, z.y); A *= Ao; }
-    }
-    yin.x = __shfl_up_sync(full, z.x, 1, P);
-    yin.y = __shfl_up_sync(full, z.y, 1, P);
-    if (p == 0) yin = make_double2(0.0, 0.0);
+    const double z = tri_forward<8, true, false>(d, 2 * ps, fi, fm, ps, lo, hi, 0.0, A);
+    in = tri_lane_scan<true>(A, z, p, P);
   }
-  double unused = 1.0;
-  forward(yin, true, unused);
-  // ---- back substitution from the top
-  double2 xin = make_double2(0.0, 0.0);   // x of the row above the lane's rows
+  tri_forward<8, true, true>(d, 2 * ps, fi, fm, ps, lo, hi, in, A);
+  A = 1.0; in = 0.0;
   if (P > 1) {
-    double A = 1.0;
-    double2 w = backward(make_double2(0.0, 0.0), false, A);
-    for (int off = 1; off < P; off <<= 1) {
-      const double Ao = __shfl_down_sync(full, A, off, P);
-      const double bx = __shfl_down_sync(full, w.x, off, P), by = __shfl_down_sync(full, w.y, off, P);
-      if (p + off < P) { w.x = fma(A, bx, w.x); w.y = fma(A, by, w.y); A *= Ao; }
-    }
-    xin.x = __shfl_down_sync(full, w.x, 1, P);
-    xin.y = __shfl_down_sync(full, w.y, 1, P);
-    if (p == P - 1) xin = make_double2(0.0, 0.0);
+    const double z = tri_backward<8, true, false>(d, 2 * ps, d, 2 * ps, fc, ps, lo, hi, 0.0, A);
+    in = tri_lane_scan<false>(A, z, p, P);
   }
-  backward(xin, true, unused);
+  tri_backward<8, true, true>(d, 2 * ps, d, 2 * ps, fc, ps, lo, hi, in, A);
 }
 
 // ------------------------------------------------------------ fused z transform + tridiagonal + inverse z
@@ -653,7 +618,9 @@ struct RowSt {
   __device__ __forceinline__ void operator()(int r, int e, fx2 v) const { p[(size_t)r * rowpitch + (size_t)e * pitch] = out(r, v); }
 };
 
-__global__ void __launch_bounds__(256)
+// 64 registers: with 128 (eight rows fetched together) a step of 32x48x32 takes
+// 241 us instead of 236, the block finding no room beside its predecessor's.
+__global__ void __launch_bounds__(256, 4)
 k_zsolve(ChlMap map) {
   chl_pdl_wait();
   extern __shared__ double2 sm[];
@@ -669,13 +636,12 @@ k_zsolve(ChlMap map) {
   const size_t ps = (size_t)modes;              // row pitch of spec and factors
   double2* A = sm;
   const int T = 2 * L * Nz;                                     // twiddles
-  double2* fz = sm + T + I.lenz;                       // forward lane values
-  double2* bw = fz + Nz;                        // backward lane values
-  double2* yin = bw + Nz;
-  double2* xin = yin + Nz;
-  double* fA = reinterpret_cast<double*>(xin + Nz);
-  double* bA = fA + Nz;
-  unsigned* top = reinterpret_cast<unsigned*>(bA + Nz);          // the lines' largest components
+  double* fz = reinterpret_cast<double*>(sm + T + I.lenz);   // per column: forward lane values
+  double* bw = fz + 2 * Nz;                     // backward lane values
+  double* in = bw + 2 * Nz;                     // values entering the rows, first upwards, then downwards
+  double* fA = in + 2 * Nz;
+  double* bA = fA + 2 * Nz;
+  unsigned* top = reinterpret_cast<unsigned*>(bA + 2 * Nz);          // the lines' largest components
   const int t = threadIdx.x, bd = blockDim.x;
   const int bits = I.bitsz, halvings = I.passz - 1;
   stage_twiddles(smem_tw() + T, I.twz, I.lenz);
@@ -692,115 +658,54 @@ k_zsolve(ChlMap map) {
   fx_fft<false>(RawLd{0, 1, nr, LineIn{bits, top}}, DoubleTileSt{r0, 1, nr, LineOut{bits, halvings, top}}, 0, L * Nz, nr, 1,
                 nr, Nz, I.passz, T);
   __syncthreads();
-  const double* __restrict__ fi = I.tri_inv + kx;
-  const double* __restrict__ fm = I.tri_m + kx;
-  const double* __restrict__ fc = I.tri_c + kx;
-  const unsigned full = 0xffffffffu;
+  // column w = 2 kz + part of this CTA's rows: element l at rows + 2 l (kz nr of them before)
+  double* const rows = reinterpret_cast<double*>(res);
+  auto column = [&](int w) { return rows + (size_t)(w >> 1) * 2 * nr + (w & 1); };
+  auto factor = [&](const double* f, int w) { return f + (size_t)lo * ps + kx + (size_t)(w >> 1) * Nxh; };
   // ---- forward elimination: this CTA's lane maps
+  double none = 1.0;
   if (P > 1) {
-    for (int kz = t; kz < Nz; kz += bd) {
-      const size_t mo = (size_t)kz * Nxh;
+    for (int w = t; w < 2 * Nz; w += bd) {
       double Am = 1.0;
-      double2 prev = make_double2(0.0, 0.0);
-      for (int j = lo; j < hi; ++j) {
-        double2 d = res[(j - lo) + (size_t)kz * nr];
-        const double iv = LDG(fi + (size_t)j * ps + mo), m = LDG(fm + (size_t)j * ps + mo);
-        d.x = fma(d.x, iv, -m * prev.x);
-        d.y = fma(d.y, iv, -m * prev.y);
-        prev = d;
-        Am = -m * Am;
-      }
-      fA[kz] = Am;
-      fz[kz] = prev;
+      fz[w] = tri_forward<4, false, false>(column(w), 2, factor(I.tri_inv, w), factor(I.tri_m, w), ps, 0, nr, 0.0, Am);
+      fA[w] = Am;
     }
   }
   cl.sync();
   if (P > 1) {
-    // one thread per (kz, lane p): the inclusive scan of k_tri_scan
-    for (int base = 0; base < Nz * P; base += bd) {
-      const int w = base + t, kz = w / P, p = w % P;
-      const bool ok = kz < Nz;
-      const double* rA = cl.map_shared_rank(fA, p);
-      const double2* rz = cl.map_shared_rank(fz, p);
-      double Av = ok ? rA[kz] : 1.0;
-      double2 z = ok ? rz[kz] : make_double2(0.0, 0.0);
-      for (int off = 1; off < P; off <<= 1) {
-        const double Ao = __shfl_up_sync(full, Av, off, P);
-        const double bx = __shfl_up_sync(full, z.x, off, P), by = __shfl_up_sync(full, z.y, off, P);
-        if (p >= off) { z.x = fma(Av, bx, z.x); z.y = fma(Av, by, z.y); Av *= Ao; }
-      }
-      double2 y;
-      y.x = __shfl_up_sync(full, z.x, 1, P);
-      y.y = __shfl_up_sync(full, z.y, 1, P);
-      if (p == 0) y = make_double2(0.0, 0.0);
-      if (ok && p == r) yin[kz] = y;
+    // one thread per (column, lane p): the inclusive scan of k_tri_scan
+    for (int base = 0; base < 2 * Nz * P; base += bd) {
+      const int w = (base + t) / P, p = (base + t) % P;
+      const bool ok = w < 2 * Nz;
+      const double A0 = ok ? cl.map_shared_rank(fA, p)[w] : 1.0, z = ok ? cl.map_shared_rank(fz, p)[w] : 0.0;
+      const double y = tri_lane_scan<true>(A0, z, p, P);
+      if (ok && p == r) in[w] = y;
     }
   }
   __syncthreads();
-  for (int kz = t; kz < Nz; kz += bd) {
-    const size_t mo = (size_t)kz * Nxh;
-    double2 prev = P > 1 ? yin[kz] : make_double2(0.0, 0.0);
-    for (int j = lo; j < hi; ++j) {
-      double2 d = res[(j - lo) + (size_t)kz * nr];
-      const double iv = LDG(fi + (size_t)j * ps + mo), m = LDG(fm + (size_t)j * ps + mo);
-      d.x = fma(d.x, iv, -m * prev.x);   // m = 0 on the first row
-      d.y = fma(d.y, iv, -m * prev.y);
-      prev = d;
-      res[(j - lo) + (size_t)kz * nr] = d;
-    }
-  }
-  // ---- back substitution from the top
+  for (int w = t; w < 2 * Nz; w += bd)
+    tri_forward<4, false, true>(column(w), 2, factor(I.tri_inv, w), factor(I.tri_m, w), ps, 0, nr, P > 1 ? in[w] : 0.0, none);
+  // ---- back substitution from the top (each thread on its own columns)
   if (P > 1) {
-    for (int kz = t; kz < Nz; kz += bd) {
-      const size_t mo = (size_t)kz * Nxh;
+    for (int w = t; w < 2 * Nz; w += bd) {
       double Am = 1.0;
-      double2 prev = make_double2(0.0, 0.0);
-      for (int j = hi - 1; j >= lo; --j) {
-        double2 d = res[(j - lo) + (size_t)kz * nr];
-        const double c = LDG(fc + (size_t)j * ps + mo);
-        d.x = fma(-c, prev.x, d.x);
-        d.y = fma(-c, prev.y, d.y);
-        prev = d;
-        Am = -c * Am;
-      }
-      bA[kz] = Am;
-      bw[kz] = prev;
+      bw[w] = tri_backward<4, false, false>(column(w), 2, nullptr, 0, factor(I.tri_c, w), ps, 0, nr, 0.0, Am);
+      bA[w] = Am;
     }
   }
   cl.sync();
   if (P > 1) {
-    for (int base = 0; base < Nz * P; base += bd) {
-      const int w = base + t, kz = w / P, p = w % P;
-      const bool ok = kz < Nz;
-      const double* rA = cl.map_shared_rank(bA, p);
-      const double2* rw = cl.map_shared_rank(bw, p);
-      double Av = ok ? rA[kz] : 1.0;
-      double2 v = ok ? rw[kz] : make_double2(0.0, 0.0);
-      for (int off = 1; off < P; off <<= 1) {
-        const double Ao = __shfl_down_sync(full, Av, off, P);
-        const double bx = __shfl_down_sync(full, v.x, off, P), by = __shfl_down_sync(full, v.y, off, P);
-        if (p + off < P) { v.x = fma(Av, bx, v.x); v.y = fma(Av, by, v.y); Av *= Ao; }
-      }
-      double2 x;
-      x.x = __shfl_down_sync(full, v.x, 1, P);
-      x.y = __shfl_down_sync(full, v.y, 1, P);
-      if (p == P - 1) x = make_double2(0.0, 0.0);
-      if (ok && p == r) xin[kz] = x;
+    for (int base = 0; base < 2 * Nz * P; base += bd) {
+      const int w = (base + t) / P, p = (base + t) % P;
+      const bool ok = w < 2 * Nz;
+      const double A0 = ok ? cl.map_shared_rank(bA, p)[w] : 1.0, z = ok ? cl.map_shared_rank(bw, p)[w] : 0.0;
+      const double x = tri_lane_scan<false>(A0, z, p, P);
+      if (ok && p == r) in[w] = x;
     }
   }
   __syncthreads();
-  for (int kz = t; kz < Nz; kz += bd) {
-    const size_t mo = (size_t)kz * Nxh;
-    double2 prev = P > 1 ? xin[kz] : make_double2(0.0, 0.0);
-    for (int j = hi - 1; j >= lo; --j) {
-      double2 d = res[(j - lo) + (size_t)kz * nr];
-      const double c = LDG(fc + (size_t)j * ps + mo);
-      d.x = fma(-c, prev.x, d.x);        // c = 0 on the last row
-      d.y = fma(-c, prev.y, d.y);
-      prev = d;
-      res[(j - lo) + (size_t)kz * nr] = d;
-    }
-  }
+  for (int w = t; w < 2 * Nz; w += bd)
+    tri_backward<4, false, true>(column(w), 2, column(w), 2, factor(I.tri_c, w), ps, 0, nr, P > 1 ? in[w] : 0.0, none);
   __syncthreads();
   line_max(res, nr, nr, Nz, top);
   fx_fft<true>(RawLd{r0, 1, nr, LineIn{bits, top}}, RowSt{spec + (size_t)lo * ps, ps, (size_t)Nxh, LineOut{bits, halvings, top}},
@@ -997,7 +902,7 @@ void chl_launch_fftz(const ChlMap& m, int nb, int nt, size_t smem, int inv, int 
 }
 // smem > 0: the staged form with TRI_W-mode blocks (chl_tri_modes_per_block)
 void chl_launch_tri(const ChlMap& m, int nb, size_t smem, cudaStream_t st) {
-  if (smem) chl_launch_pdl(k_tri_staged, dim3(nb), dim3(TRI_W), smem, st, m);
+  if (smem) chl_launch_pdl(k_tri_staged, dim3(nb), dim3(2 * TRI_W), smem, st, m);
   else chl_launch_pdl(k_tri, dim3(nb), dim3(128), 0, st, m);
 }
 // Shared memory of the staged form for the tallest column (40 bytes per
@@ -1013,7 +918,7 @@ size_t chl_smem_tri(int maxNy, long modes, int mode) {
   const long blocks = (modes + TRI_W - 1) / TRI_W;
   return blocks <= per_sm * CHL_SMS ? b : 0;
 }
-int chl_tri_modes_per_block(size_t smem) { return smem ? TRI_W : 128; }
+int chl_tri_modes_per_block(size_t smem) { return smem ? TRI_W : 64; }
 // Fused z solve: shared memory of a CTA for an instance (0 if its block does
 // not fit, or its lane count is not a cluster size of 1, 2, 4 or 8), and its
 // launch: cluster (P, 1, 1), Nxh x P CTAs per instance.
@@ -1023,7 +928,7 @@ size_t chl_smem_zsolve(int Nx, int Ny, int Nz) {
   if (P != 1 && P != 2 && P != 4 && P != 8) return 0;
   const int L = (Ny + P - 1) / P;
   const size_t b = (size_t)2 * L * Nz * sizeof(double2) + (size_t)chl_twf_len(Nz) * sizeof(int4) +
-                   (size_t)4 * Nz * sizeof(double2) + (size_t)2 * Nz * sizeof(double) + (size_t)L * sizeof(unsigned);
+                   (size_t)10 * Nz * sizeof(double) + (size_t)L * sizeof(unsigned);
   return b <= (size_t)227 * 1024 ? b : 0;
 }
 int chl_zsolve_setup(size_t smem) {

@@ -641,7 +641,7 @@ static int build_maps(chl_handle* h) {
         case M_PLANE: b = cdiv((long)Nx * Nz, 256); break;
         case M_FFTX: b = cdiv((long)Ny * (Nz / 2), chl_fftx_rows(Nx, Ny * (Nz / 2), h->xmb())); break;
         case M_FFTZ: b = cdiv((long)Ny * Nxh, h->zcw); break;
-        case M_TRI: b = h->tri_scan ? cdiv((long)Nz * Nxh * chl_tri_lanes((long)Nz * Nxh, Ny), 128)
+        case M_TRI: b = h->tri_scan ? cdiv(2L * Nz * Nxh * chl_tri_lanes((long)Nz * Nxh, Ny), 128)
                                     : cdiv((long)Nz * Nxh, tri_w); break;
         case M_MINABS: b = Nz * ((Ny + 15) / 16); break;   // planes x 16-row chunks (chl_misc.cu)
         case M_ROWS: b = Ny + 1; break;
