@@ -18,13 +18,13 @@ extern "C" {
 void chl_launch_fix(const ChlMap&, int, int, int, cudaStream_t);
 void chl_launch_flux(const ChlMap&, int, int, cudaStream_t);
 void chl_launch_update(const ChlMap&, int, int, int, int, int, cudaStream_t);
-void chl_launch_strain(const ChlMap&, int, int, int, cudaStream_t);
+void chl_launch_strain(const ChlMap&, int, int, int, int, cudaStream_t);
 int chl_filter_blocks(int, int, int, int, int);
 void chl_launch_filter(const ChlMap&, int, int, cudaStream_t);
 void chl_launch_dsm_final(const ChlMap&, int, int, cudaStream_t);
-void chl_launch_coef(const ChlMap&, cudaStream_t);
 void chl_launch_eqwm(const ChlMap&, int, int, cudaStream_t);
-void chl_launch_nut(const ChlMap&, int, int, int, cudaStream_t);
+void chl_launch_nut(const ChlMap&, int, int, cudaStream_t);
+void chl_launch_wall_rows(const ChlMap&, int, int, cudaStream_t);
 void chl_launch_amd(const ChlMap&, int, int, int, cudaStream_t);
 void chl_launch_vreman(const ChlMap&, int, int, int, cudaStream_t);
 void chl_launch_agent_obs(const ChlInst*, int, int, double, const int*, const double*, double*, double*, cudaStream_t);
@@ -674,43 +674,48 @@ static void enqueue_dt(chl_handle* h, cudaStream_t st);
 // with_dt: the time step's reduction (set 0 only) goes with it.
 static int enqueue_sgs(chl_handle* h, int s, bool with_wm, int stage = 0, bool with_dt = false) {
   cudaStream_t st = h->st;
-  // AMD and Vreman write nu + nu_t in their own kernel, whose wall-model
-  // rows need the wall stress first; the other models leave it to k_nut
-  const bool fused = h->LES_model == CHL_LES_AMD || h->LES_model == CHL_LES_VREMAN;
-  // What needs only the velocities goes on the step graph's side branch
-  // where it has one: the wall stress, which nu + nu_t takes, and the time
-  // step, which the stage update takes (and the learned model's stress).
-  const bool wall = with_wm && h->wall_model >= CHL_WM_EQLOG, mlp = wall && h->wall_model == CHL_WM_MLP;
-  const bool fork = h->side.st && (wall || with_dt);
+  const bool smag = h->LES_model == CHL_LES_SMAGORINSKY;
+  const bool wm = with_wm && h->wall_model != CHL_WM_NONE, mlp = wm && h->wall_model == CHL_WM_MLP;
+  KL("fix", chl_launch_fix(h->map(M_FULL2), h->nblk[M_FULL2], s, smag ? 3 : 1, st));
+  // What needs only the velocities goes on the step graph's side branch where
+  // it has one: the wall stress with the wall rows of nu + nu_t, which the
+  // fluxes take, and the time step, which the stage update takes (and the
+  // learned model's stress).
+  const bool fork = h->side.st && (wm || with_dt);
   cudaStream_t sd = fork ? h->side.st : st;
   if (fork) { CK(cudaEventRecord(h->side.fork, st)); CK(cudaStreamWaitEvent(sd, h->side.fork, 0)); }
-  if (with_dt && (mlp || !wall || !fork)) enqueue_dt(h, sd);
-  if (wall) KL("eq_wallmodel", chl_launch_eqwm(h->map(M_WALLN), h->nblk[M_WALLN], s, sd));
-  if (mlp) KL("mlp_wallmodel", chl_launch_mlp(h->map(M_MLP), h->nblk[M_MLP], s, stage, h->d_mlp_status, sd));
-  if (fork && wall) CK(cudaEventRecord(h->side.wall, sd));
-  if (with_dt && wall && !mlp && fork) enqueue_dt(h, sd);
+  const bool dt_last = wm && !mlp && fork;
+  if (with_dt && !dt_last) enqueue_dt(h, sd);
+  if (wm) {
+    if (h->wall_model >= CHL_WM_EQLOG) KL("eq_wallmodel", chl_launch_eqwm(h->map(M_WALLN), h->nblk[M_WALLN], s, sd));
+    if (mlp) KL("mlp_wallmodel", chl_launch_mlp(h->map(M_MLP), h->nblk[M_MLP], s, stage, h->d_mlp_status, sd));
+    KL("wall_rows", chl_launch_wall_rows(h->map(M_WALL), h->nblk[M_WALL], s, sd));
+    if (fork) CK(cudaEventRecord(h->side.wall, sd));
+  }
+  if (with_dt && dt_last) enqueue_dt(h, sd);
   if (fork) CK(cudaEventRecord(h->side.dt, sd));
-  auto wall_stress = [&]() -> cudaError_t { return fork && wall ? cudaStreamWaitEvent(st, h->side.wall, 0) : cudaSuccess; };
-  KL("fix", chl_launch_fix(h->map(M_FULL2), h->nblk[M_FULL2], s, 1, st));
-  if (fused) CK(wall_stress());
+  // the learned model reads the nu + nu_t of the stage before: its writers wait
+  auto join_mlp = [&]() -> cudaError_t { return fork && mlp ? cudaStreamWaitEvent(st, h->side.wall, 0) : cudaSuccess; };
+  // the static model, AMD and Vreman write nu + nu_t in their own kernel; the
+  // dynamic model and none leave it to k_nut
+  const bool fused = smag || h->LES_model == CHL_LES_AMD || h->LES_model == CHL_LES_VREMAN;
+  if (fused) CK(join_mlp());
   if (h->LES_model == CHL_LES_DYNAMIC) {
-    KL("strain", chl_launch_strain(h->map(M_MARCH), h->nblk[M_MARCH], s, 1, st));
+    KL("strain", chl_launch_strain(h->map(M_MARCH), h->nblk[M_MARCH], s, 1, 0, st));
     KL("filter", chl_launch_filter(h->map(M_FILTER), h->nblk[M_FILTER], h->tb_filter, st));
     KL("dsm_LM_MM", chl_launch_dsm_final(h->map(M_DSMF), h->nblk[M_DSMF], s, st));
-  } else if (h->LES_model == CHL_LES_SMAGORINSKY) {
-    KL("strain", chl_launch_strain(h->map(M_MARCH), h->nblk[M_MARCH], s, 0, st));
+  } else if (smag) {
+    KL("strain", chl_launch_strain(h->map(M_MARCH), h->nblk[M_MARCH], s, 0, wm ? 1 : 0, st));
   } else if (h->LES_model == CHL_LES_AMD) {
-    KL("amd", chl_launch_amd(h->map(M_MARCH), h->nblk[M_MARCH], s, with_wm ? 1 : 0, st));
+    KL("amd", chl_launch_amd(h->map(M_MARCH), h->nblk[M_MARCH], s, wm ? 1 : 0, st));
   } else if (h->LES_model == CHL_LES_VREMAN) {
-    KL("vreman", chl_launch_vreman(h->map(M_MARCH), h->nblk[M_MARCH], s, with_wm ? 1 : 0, st));
+    KL("vreman", chl_launch_vreman(h->map(M_MARCH), h->nblk[M_MARCH], s, wm ? 1 : 0, st));
   }
-  // the static model's row coefficient (the dynamic model's is formed by
-  // the last block of each row of its plane sums)
-  if (h->LES_model == CHL_LES_SMAGORINSKY) KL("nut_coef", chl_launch_coef(h->map(M_PT), st));
   if (!fused) {
-    CK(wall_stress());
-    KL("nut", chl_launch_nut(h->map(M_FULL2), h->nblk[M_FULL2], s, with_wm ? 1 : 0, st));
+    CK(join_mlp());
+    KL("nut", chl_launch_nut(h->map(M_FULL2), h->nblk[M_FULL2], wm ? 1 : 0, st));
   }
+  if (fork && wm && !mlp) CK(cudaStreamWaitEvent(st, h->side.wall, 0));
   LAUNCHED();
   return CHL_OK;
 }
@@ -1446,7 +1451,8 @@ int chl_compute_wall_model(chl_handle* h) {
   chl_launch_fix(h->map(M_FULL2), h->nblk[M_FULL2], 0, 1, h->st);   // k_nut forms the largest nu + nu_t anew
   if (h->wall_model >= CHL_WM_EQLOG) chl_launch_eqwm(h->map(M_WALLN), h->nblk[M_WALLN], 0, h->st);
   if (h->wall_model == CHL_WM_MLP) chl_launch_mlp(h->map(M_MLP), h->nblk[M_MLP], 0, 0, h->d_mlp_status, h->st);
-  chl_launch_nut(h->map(M_FULL2), h->nblk[M_FULL2], 0, h->wall_model != CHL_WM_NONE ? 1 : 0, h->st);
+  if (h->wall_model != CHL_WM_NONE) chl_launch_wall_rows(h->map(M_WALL), h->nblk[M_WALL], 0, h->st);
+  chl_launch_nut(h->map(M_FULL2), h->nblk[M_FULL2], h->wall_model != CHL_WM_NONE ? 1 : 0, h->st);
   LAUNCHED();
   return finish(h);
 }

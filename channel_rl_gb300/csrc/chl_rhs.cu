@@ -64,16 +64,30 @@ __device__ __forceinline__ RowExp row_exp(const ChlInst& I, int sin, int j) {
   return q;
 }
 
+// Row coefficient of the static model, nu_t = coef |S|/sqrt(2): van Driest
+// damping f = 1 - exp(-d/25/(nu/utau)), utau = dPdx^0.5 (subgrid.f90:581-599).
+static __device__ __noinline__ double smag_coef(const ChlInst& I, int jc) {
+  const double ut = sqrt(I.scal[CHL_S_DPDX]);
+  double f = 1.0 - exp(-I.smag_dwall[jc] / 25.0 / (I.nu / ut));
+  if (I.Dirichlet_nu_t == 0) f = 1.0;
+  const double cd = I.smag_csdelta[jc] * f;   // Cs*Delta_j*f
+  return cd * cd * 1.41421356237309504880;    // (Cs Delta f)^2 |S| with S holding |S|/sqrt(2)
+}
+
 // Fixed-point copies of the velocity set that a stage works on (rows as
-// stored, ghosts included); reset_n clears the rows' largest |nu + nu_t|
-// and |S| S_ij ahead of the kernels that form them.  Moves 48 bytes per point: HBM-bound.
+// stored, ghosts included).  prep: 1 clears the rows' largest |nu + nu_t|
+// and |S| S_ij ahead of the kernels that form them, + 2 forms the static
+// model's row coefficients.  Moves 48 bytes per point: HBM-bound.
 __global__ void __launch_bounds__(256)
-k_fix(ChlMap map, int s, int reset_n) {
+k_fix(ChlMap map, int s, int prep) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  if (reset_n && t < (unsigned)(I.Ny + 2)) I.nmax[t] = I.smax[t] = 0u;
+  if (prep && t < (unsigned)(I.Ny + 2)) {
+    I.nmax[t] = I.smax[t] = 0u;
+    if (prep & 2) I.coef[t] = t >= 1 && (int)t <= I.Ny ? smag_coef(I, t) : 0.0;
+  }
   const unsigned* vm = chl_vmax(I, s);
   // pairs of points (Nx is even)
   const unsigned nc = (unsigned)(I.Nx * (I.Ny + 2) * I.Nz) / 2, nv = (unsigned)(I.Nx * (I.Ny + 1) * I.Nz) / 2;
@@ -291,8 +305,8 @@ k_rhs_update(ChlMap map, RhsArgs a) {
 }
 
 extern "C" {
-void chl_launch_fix(const ChlMap& map, int nb_full, int s, int reset_n, cudaStream_t st) {
-  chl_launch_pdl(k_fix, dim3(nb_full), dim3(map.tb), 0, st, map, s, reset_n);
+void chl_launch_fix(const ChlMap& map, int nb_full, int s, int prep, cudaStream_t st) {
+  chl_launch_pdl(k_fix, dim3(nb_full), dim3(map.tb), 0, st, map, s, prep);
 }
 void chl_launch_flux(const ChlMap& map, int nb_edge, int sin, cudaStream_t st) {
   chl_launch_pdl(k_flux, dim3(nb_edge), dim3(CHL_FLUX_THREADS), 0, st, map, sin);

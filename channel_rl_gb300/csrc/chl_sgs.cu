@@ -17,46 +17,56 @@
 // model is compute_wall_model (wallmodel.f90:23-46); the equilibrium log-law
 // wall stress that feeds it is new.
 #include "chl_strain.cuh"
+#include "chl_nut.cuh"
 
 // ---------------------------------------------------------------- strain
 // Strain magnitude and the DSM filter inputs at centres (rows 1..Ny): q3..8
 // the products of the centre velocities' face sums in fixed point (last bit
 // 2^(e_i + e_j + 64)), q9..14 = |S|*(S_ii, 2 S_ij) / sqrt(2) and their
 // largest per row.
+// With DSM = false (the static model, whose row coefficients do not depend on
+// the strain) nu + nu_t instead, so that no pass reads |S| back: 143 -> 157 us
+// at 256x96x192 for the 37 of k_nut and the launch of the coefficients' own
+// kernel.
 template <bool DSM>
 __global__ void __launch_bounds__(CHL_FLUX_THREADS, 7)
-k_strain(ChlMap map, int s_in) {
+k_strain(ChlMap map, int s_in, int use_wm) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
   const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz, M = map.planes;
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
   const ChlIdx p = chl_split(t, Nx, Ny);
-  const int i = p.i, jc = 1 + p.j, k0 = p.k * M, k1 = min(Nz, k0 + M);
+  const int i = p.i, jc = 1 + p.j, k0 = p.k * M;
   unsigned hi = 0u;
-  if (k0 < k1) {
-    const unsigned* vm = chl_vmax(I, s_in);
-    const bool bad = fx_bad(vm[0]) || fx_bad(vm[1]) || fx_bad(vm[2]);
-    StrainColumn col(I, I.X[0], I.X[1], I.X[2], fx_exp<61>(vm[0]), fx_exp<61>(vm[1]), fx_exp<61>(vm[2]), i, jc, k0);
-    for (int k = k0; k < k1; ++k) {
-      fx f[3];
-      Strain s = col.point(k, f);
-      if (bad) s.s = __longlong_as_double(0x7FF8000000000000LL);
-      const size_t c = cidx(I, i, jc, k);
-      I.S[c] = s.s;
-      if (!DSM) continue;
-      fx* const* q = reinterpret_cast<fx* const*>(I.q);
-      q[3][c] = fx_mul(f[0], f[0]); q[4][c] = fx_mul(f[1], f[1]); q[5][c] = fx_mul(f[2], f[2]);
-      q[6][c] = fx_mul(f[0], f[1]); q[7][c] = fx_mul(f[0], f[2]); q[8][c] = fx_mul(f[1], f[2]);
-      const double se = s.s * pow2(min(1023, max(-1022, s.e)));
-      // two of the six conversions on the FP64 pipe, which is the less busy
-      const double m[6] = {se * fx_raw<true>(s.t[0]), se * fx_raw<true>(s.t[1]), se * fx_raw<false>(s.t[2]),
-                           se * fx_raw<false>(s.t[3]), se * fx_raw<false>(s.t[4]), se * fx_raw<false>(s.t[5])};
-#pragma unroll
-      for (int n = 0; n < 6; ++n) { I.q[9 + n][c] = m[n]; hi = max(hi, chl_abshi(m[n])); }
+  const unsigned* vm = chl_vmax(I, s_in);
+  const bool bad = fx_bad(vm[0]) || fx_bad(vm[1]) || fx_bad(vm[2]);
+  StrainColumn col(I, I.X[0], I.X[1], I.X[2], fx_exp<61>(vm[0]), fx_exp<61>(vm[1]), fx_exp<61>(vm[2]), i, jc,
+                   min(k0, Nz - 1));
+  const double cj = DSM ? 0.0 : I.coef[jc], nu = I.nu;
+  for (int k = k0; k < min(Nz, k0 + M); ++k) {
+    fx f[3];
+    Strain s = col.point(k, f);
+    if (bad) s.s = __longlong_as_double(0x7FF8000000000000LL);
+    const size_t c = cidx(I, i, jc, k);
+    I.S[c] = s.s;
+    if (!DSM) {
+      // nu + max(0, c |S|) as in k_nut
+      const double v = chl_atleast(fma(cj, s.s, nu), nu);
+      hi = max(hi, write_nut_rows(I, i, jc, k, v, [&] { return chl_pos(cj * s.s); }, use_wm));
+      continue;
     }
+    fx* const* q = reinterpret_cast<fx* const*>(I.q);
+    q[3][c] = fx_mul(f[0], f[0]); q[4][c] = fx_mul(f[1], f[1]); q[5][c] = fx_mul(f[2], f[2]);
+    q[6][c] = fx_mul(f[0], f[1]); q[7][c] = fx_mul(f[0], f[2]); q[8][c] = fx_mul(f[1], f[2]);
+    const double se = s.s * pow2(min(1023, max(-1022, s.e)));
+    // two of the six conversions on the FP64 pipe, which is the less busy
+    const double d[6] = {se * fx_raw<true>(s.t[0]), se * fx_raw<true>(s.t[1]), se * fx_raw<false>(s.t[2]),
+                         se * fx_raw<false>(s.t[3]), se * fx_raw<false>(s.t[4]), se * fx_raw<false>(s.t[5])};
+#pragma unroll
+    for (int n = 0; n < 6; ++n) { I.q[9 + n][c] = d[n]; hi = max(hi, chl_abshi(d[n])); }
   }
-  if (DSM) chl_line_max(I.smax, (unsigned)(p.k * Ny + p.j), Ny, 1, hi);
+  chl_line_max(DSM ? I.smax : I.nmax, (unsigned)(p.k * Ny + p.j), Ny, 1, hi);
 }
 
 // ------------------------------------------------------------ test filter
@@ -354,32 +364,6 @@ k_dsm_final(ChlMap map, int s_in) {
   }
 }
 
-// ------------------------------------------------------------ nu_t coefficient per row
-// The static model's row coefficient (the dynamic model's is written by
-// k_dsm_final, and this kernel leaves it alone).
-__global__ void k_coef(ChlMap map) {
-  chl_pdl_wait();
-  const ChlInst& I = map.inst[blockIdx.x];
-  const int Ny = I.Ny;
-  if (I.LES_model == 2) return;
-  for (int jc = threadIdx.x; jc < Ny + 2; jc += blockDim.x) {
-    double c = 0.0;
-    if (jc >= 1 && jc <= Ny) {
-      if (I.LES_model == 1) {
-        // van Driest: f = 1 - exp(-d/25/(nu/utau)), utau = dPdx^0.5 (subgrid.f90:581-599)
-        const double ut = sqrt(I.scal[CHL_S_DPDX]);
-        double f = 1.0 - exp(-I.smag_dwall[jc] / 25.0 / (I.nu / ut));
-        if (I.Dirichlet_nu_t == 0) f = 1.0;
-        const double cd = I.smag_csdelta[jc] * f;   // Cs*Delta_j*f
-        c = cd * cd * 1.41421356237309504880;      // (Cs Delta f)^2 |S| with S holding |S|/sqrt(2)
-      } else if (I.LES_model >= 3) {
-        c = 1.0;                           // AMD, Vreman: S holds nu_t itself (not launched for them)
-      }
-    }
-    I.coef[jc] = c;
-  }
-}
-
 // ------------------------------------------------------------ equilibrium log-law wall stress
 #define EQWM_KAPPA 0.41
 #define EQWM_B 5.2
@@ -483,14 +467,10 @@ static __device__ __noinline__ double nut_other(const ChlInst& I, int i, int jc,
 }
 // One thread per pair of x points of a row (jc, k), jc = 0..Ny+1 (with one
 // point per thread this kernel took 52 us at 256x96x192 for 11 us of HBM
-// traffic: blocks too short-lived for their start-up).  On the wall-model
-// rows (jc = 0, 1 and Ny, Ny+1) nu_t is the mean of the face values at x faces
-// i-1 and i, the same in both rows of a wall: the threads of rows 1 and Ny
-// write both.  Each forms its two faces and takes the one before from the
-// lane to its left when that lane is on the same row (i > 0), so no thread
-// returns before the shuffle.
+// traffic: blocks too short-lived for their start-up).  With the wall model on,
+// rows 0, 1 and Ny, Ny+1 are k_wall_rows's.
 __global__ void __launch_bounds__(256)
-k_nut(ChlMap map, int s_in, int use_wm) {
+k_nut(ChlMap map, int use_wm) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
@@ -501,23 +481,12 @@ k_nut(ChlMap map, int s_in, int use_wm) {
   const ChlIdx p = chl_split(valid ? t : (unsigned)(nxp * (Ny + 2) * Nz) - 1u, nxp, Ny + 2);
   const int i = 2 * p.i, jc = p.j, k = p.k;
   const bool wm = use_wm && I.wall_model != 0 && (jc <= 1 || jc >= Ny);
-  const bool wmrow = valid && wm && (jc == 1 || jc == Ny);
-  const int wall = jc == 1 ? 0 : 1;
-  const double* U = I.U[s_in];
-  double f0 = 0.0, f1 = 0.0;
-  if (wmrow) { f0 = wm_face(I, U, i, k, wall); f1 = wm_face(I, U, i + 1, k, wall); }
-  const double f_left = __shfl_up_sync(0xffffffffu, f1, 1);
   double2 v = make_double2(0.0, 0.0);
-  if (valid && (!wm || wmrow)) {
+  if (valid && !wm) {
     // stored as nu + nu_t: every consumer adds nu (equations.f90:139-155)
     const double nu = I.nu;
-    double2* nut = reinterpret_cast<double2*>(I.nut);
     const size_t c = cidx(I, i, jc, k) / 2;
-    if (wmrow) {
-      const double fl = ((threadIdx.x & 31) > 0 && i > 0) ? f_left : wm_face(I, U, wrap(i - 1, Nx), k, wall);
-      v = make_double2(nu + 0.5 * (fl + f0), nu + 0.5 * (f0 + f1));
-      nut[cidx(I, i, wall == 0 ? 0 : Ny + 1, k) / 2] = v;
-    } else if (I.LES_model == 0 || I.LES_model >= 3 || jc == 0 || jc == Ny + 1) {
+    if (I.LES_model == 0 || I.LES_model >= 3 || jc == 0 || jc == Ny + 1) {
       v = make_double2(nut_other(I, i, jc, k), nut_other(I, i + 1, jc, k));
     } else {
       // nu + max(0, c |S|) as one FMA, nu + c |S|, clipped below at nu by the
@@ -526,16 +495,46 @@ k_nut(ChlMap map, int s_in, int use_wm) {
       const double2 S = __ldg(reinterpret_cast<const double2*>(I.S) + c);
       v = make_double2(chl_atleast(fma(cj, S.x, nu), nu), chl_atleast(fma(cj, S.y, nu), nu));
     }
-    nut[c] = v;
+    reinterpret_cast<double2*>(I.nut)[c] = v;
   }
   chl_line_max(I.nmax, (unsigned)(k * (Ny + 2) + jc), Ny + 2, 0, max(chl_abshi(v.x), chl_abshi(v.y)));
 }
 
+// nu + nu_t on the wall-model rows, jc = 0, 1 and Ny, Ny+1: nu_t is the mean
+// of the face values at x faces i-1 and i, the same in both rows of a wall.
+// One thread per wall point; face i-1 comes from the lane to the left when
+// that lane is on the same row, so no thread returns before the shuffle.  A
+// kernel of its own, beside the model's (300 -> 283 us of k_amd and 166 -> 157
+// of k_strain<false> at 256x96x192 where they did these rows, whose divisions
+// the whole block waits for).
+__global__ void __launch_bounds__(256)
+k_wall_rows(ChlMap map, int s_in) {
+  chl_pdl_wait();
+  int lb;
+  const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
+  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
+  const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x, n = (unsigned)(2 * Nx * Nz);
+  const bool valid = t < n;                        // lanes past the end repeat the last point and write nothing
+  const ChlIdx p = chl_split(valid ? t : n - 1u, Nx, Nz);
+  const int i = p.i, k = p.j, wall = p.k;
+  const double* U = I.U[s_in];
+  const double f = wm_face(I, U, i, k, wall);
+  const double f_left = __shfl_up_sync(0xffffffffu, f, 1);
+  const double fl = ((threadIdx.x & 31) > 0 && i > 0) ? f_left : wm_face(I, U, wrap(i - 1, Nx), k, wall);
+  const double v = I.nu + 0.5 * (fl + f);
+  if (valid) I.nut[cidx(I, i, wall == 0 ? 0 : Ny, k)] = I.nut[cidx(I, i, wall == 0 ? 1 : Ny + 1, k)] = v;
+  const unsigned hi = valid ? chl_abshi(v) : 0u;
+  const unsigned m0 = __reduce_max_sync(0xffffffffu, wall == 0 ? hi : 0u), m1 = __reduce_max_sync(0xffffffffu, wall == 0 ? 0u : hi);
+  if ((threadIdx.x & 31) == 0) {
+    if (m0 > __ldcg(I.nmax + 1)) atomicMax(I.nmax + 1, m0);
+    if (m1 > __ldcg(I.nmax + Ny)) atomicMax(I.nmax + Ny, m1);
+  }
+}
+
 // ------------------------------------------------------------ launchers
 extern "C" {
-void chl_launch_strain(const ChlMap& m, int nb, int s_in, int dsm, cudaStream_t st) {
-  if (dsm) chl_launch_pdl(k_strain<true>, dim3(nb), dim3(CHL_FLUX_THREADS), 0, st, m, s_in);
-  else chl_launch_pdl(k_strain<false>, dim3(nb), dim3(CHL_FLUX_THREADS), 0, st, m, s_in);
+void chl_launch_strain(const ChlMap& m, int nb, int s_in, int dsm, int use_wm, cudaStream_t st) {
+  chl_launch_pdl(dsm ? k_strain<true> : k_strain<false>, dim3(nb), dim3(CHL_FLUX_THREADS), 0, st, m, s_in, use_wm);
 }
 int chl_filter_blocks(int Nx, int Ny, int Nz, int T, int M) {
   const FiltShape f = filt_shape(Nx, Ny, Nz, T, M);
@@ -545,7 +544,7 @@ void chl_launch_filter(const ChlMap& m, int nb, int T, cudaStream_t st) { chl_la
 void chl_launch_dsm_final(const ChlMap& m, int nb, int s_in, cudaStream_t st) {
   chl_launch_pdl(k_dsm_final, dim3(nb), dim3(CHL_DSMF_THREADS), 0, st, m, s_in);
 }
-void chl_launch_coef(const ChlMap& m, cudaStream_t st) { chl_launch_pdl(k_coef, dim3(m.n), dim3(128), 0, st, m); }
 void chl_launch_eqwm(const ChlMap& m, int nb, int s_in, cudaStream_t st) { chl_launch_pdl(k_eqwm, dim3(nb), dim3(CHL_WALL_THREADS), 0, st, m, s_in); }
-void chl_launch_nut(const ChlMap& m, int nb, int s_in, int use_wm, cudaStream_t st) { chl_launch_pdl(k_nut, dim3(nb), dim3(m.tb), 0, st, m, s_in, use_wm); }
+void chl_launch_nut(const ChlMap& m, int nb, int use_wm, cudaStream_t st) { chl_launch_pdl(k_nut, dim3(nb), dim3(m.tb), 0, st, m, use_wm); }
+void chl_launch_wall_rows(const ChlMap& m, int nb, int s_in, cudaStream_t st) { chl_launch_pdl(k_wall_rows, dim3(nb), dim3(256), 0, st, m, s_in); }
 }

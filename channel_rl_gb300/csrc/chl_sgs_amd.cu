@@ -1,9 +1,8 @@
 // Anisotropic minimum-dissipation (AMD) and Vreman eddy viscosities, one
 // fused kernel each, one thread per interior centre (rows 1..Ny).  Both write
 // the unclipped nu_t into S and, in the same pass, nu + nu_t with k_nut's
-// rules for these models (write_nut_rows): max(., 0), the ghost-row rule of
-// Dirichlet_nu_t and, when use_wm, the wall-model rows - so the step runs the
-// wall-stress kernels first and no separate nu_t pass.
+// rules for these models (write_nut_rows): max(., 0) and the ghost-row rule of
+// Dirichlet_nu_t - so there is no separate nu_t pass.
 //
 // AMD (subgrid.f90:632-874):
 //   nu_t = max(0, -C N / D),  C = 0.3,
@@ -25,7 +24,7 @@
 // where 2:nx, 1:nx-1 are meant (subgrid.f90:930-931,946-947); they start at
 // the same index, so element-wise they read the intended values, which is
 // what is computed here.
-#include "chl_fix.cuh"
+#include "chl_nut.cuh"
 
 namespace {
 
@@ -94,43 +93,6 @@ struct GradColumn {
     return d;
   }
 };
-
-// nu + nu_t for the interior centre (i, jc, k) from its unclipped value v,
-// plus the ghost row next to the first and last interior rows; with the
-// wall model on, rows 0, 1 and Ny, Ny+1 take the mean of the wall-model face
-// values at x faces i-1 and i (face i-1 from the lane to the left when that
-// lane is on the same row, i > 0).  Every lane of the warp reaches the
-// shuffle; lanes past the instance's last centre carry valid = false.
-// Returns the high word of the largest magnitude written; the ghost row's
-// counts for the row next to it.
-__device__ __forceinline__ unsigned write_nut_rows(const ChlInst& I, const double* U, int i, int jc, int k, double v,
-                                                   int use_wm, bool valid) {
-  const int Ny = I.Ny;
-  const bool wmrow = valid && use_wm && I.wall_model != 0 && (jc == 1 || jc == Ny);
-  const int wall = jc == 1 ? 0 : 1;
-  const double f = wmrow ? wm_face(I, U, i, k, wall) : 0.0;
-  const double f_left = __shfl_up_sync(0xffffffffu, f, 1);
-  if (!valid) return 0u;
-  const double nu = I.nu;
-  double* nt = I.nut;
-  if (wmrow) {
-    const double fl = ((threadIdx.x & 31) > 0 && i > 0) ? f_left : wm_face(I, U, wrap(i - 1, I.Nx), k, wall);
-    const double w = 0.5 * (fl + f);
-    nt[cidx(I, i, jc, k)] = nu + w;
-    nt[cidx(I, i, jc == 1 ? 0 : Ny + 1, k)] = nu + w;
-    return chl_abshi(nu + w);
-  }
-  const double vc = chl_pos(v);
-  nt[cidx(I, i, jc, k)] = nu + vc;
-  unsigned hi = chl_abshi(nu + vc);
-  if (jc == 1 || jc == Ny) {
-    const double g = nu + nut_ghost(I, vc);
-    if (jc == 1) nt[cidx(I, i, 0, k)] = g;
-    if (jc == Ny) nt[cidx(I, i, Ny + 1, k)] = g;
-    hi = max(hi, chl_abshi(g));
-  }
-  return hi;
-}
 
 }  // namespace
 
@@ -210,7 +172,7 @@ k_amd(ChlMap map, int s_in, int use_wm) {
     double v = (-0.3 * Nd) / fx_to(D, 0) * pow2(min(1023, max(-1022, et - er - 67 + sd)));
     if (bad) v = __longlong_as_double(0x7FF8000000000000LL);
     if (valid) I.S[cidx(I, i, jc, k)] = v;
-    hi = max(hi, write_nut_rows(I, I.U[s_in], i, jc, k, v, use_wm, valid));
+    if (valid) hi = max(hi, write_nut_rows(I, i, jc, k, I.nu + chl_pos(v), [v] { return chl_pos(v); }, use_wm));
   }
   chl_line_max(I.nmax, (unsigned)(p.k * Ny + p.j), Ny, 1, hi);
 }
@@ -287,7 +249,7 @@ k_vreman(ChlMap map, int s_in, int use_wm) {
     double v = (2.5 * (0.1 * 0.1) * 0.25) * x * pow2(min(1023, max(-1022, em - col.er - 32 + sd)));
     if (bad) v = __longlong_as_double(0x7FF8000000000000LL);
     if (valid) I.S[cidx(I, i, jc, k)] = v;
-    hi = max(hi, write_nut_rows(I, I.U[s_in], i, jc, k, v, use_wm, valid));
+    if (valid) hi = max(hi, write_nut_rows(I, i, jc, k, I.nu + chl_pos(v), [v] { return chl_pos(v); }, use_wm));
   }
   chl_line_max(I.nmax, (unsigned)(p.k * Ny + p.j), Ny, 1, hi);
 }
