@@ -101,6 +101,12 @@ __host__ __device__ inline int chl_fft_threads(int lines, int n) {
   int t = (lines * n / 4 + 31) & ~31;
   return t < 64 ? 64 : (t > 256 ? 256 : t);
 }
+// blocks of the mass-flow sum of an Nx x Nz plane (partials in red, 2 Nz long)
+#define CHL_MASS_POINTS 1024
+__host__ __device__ inline int chl_mass_blocks(int Nx, int Nz) {
+  const long b = (long)Nx * Nz / CHL_MASS_POINTS;
+  return b < 1 ? 1 : (b > 2 * Nz ? 2 * Nz : (int)b);
+}
 #ifndef CHL_TRI_SMEM_MAX
 #define CHL_TRI_SMEM_MAX (128 * 1024)   // largest staged tridiagonal column block
 #endif
@@ -163,7 +169,7 @@ struct ChlInst {
   unsigned long long *minabs;     // [Nx+1 | Nz] min |u| bit patterns (dt)
   double *red;                    // plane partials [2][Nz]: bulk flow (upload), divergence check
   int *status;                    // device status word (0 ok); [CHL_CNT_DT] block counter of k_minabs
-  int *dsm_cnt;                   // [Ny+2] block counters of the DSM plane sums per centre row
+  int *dsm_cnt;                   // [Ny+2] block counters of the DSM plane sums per centre row; [0] of the mass-flow sum
   // learned wall model (chl_mlp.cu)
   double retau;                   // nominal Re_tau of the instance (feature ln(h Re_tau))
   float *mlp_trace;               // policy-gradient trace of this instance (4545)

@@ -52,7 +52,7 @@ void chl_launch_pack_unique(double*, const double*, int, int, int, int, int, cud
 void chl_launch_minabs(const ChlMap&, int, int, cudaStream_t);
 void chl_launch_minabs_init(const ChlMap&, cudaStream_t);
 void chl_launch_nonfinite(const ChlMap&, int, int, cudaStream_t);
-void chl_launch_massflow(const ChlMap&, cudaStream_t, int, int);
+void chl_launch_massflow(const ChlMap&, int, cudaStream_t, int, int);
 void chl_launch_shift(const ChlMap&, int, int, cudaStream_t);
 void chl_launch_tadvance(const ChlMap&, cudaStream_t);
 void chl_launch_divmax(const ChlMap&, int, int, double*, cudaStream_t);
@@ -71,7 +71,7 @@ namespace {
 constexpr double RK_T[3] = {8.0 / 15.0, 2.0 / 3.0, 1.0};
 
 enum { M_PT, M_PT2, M_FULL2, M_DSMF, M_WALL, M_PLANE, M_FFTX, M_FFTZ, M_TRI, M_MINABS, M_ROWS, M_MLP, M_WALLN,
-       M_ZPLANE, M_ZSOLVE, M_FLUX, M_MARCH, M_FILTER, NMAP };
+       M_ZPLANE, M_ZSOLVE, M_FLUX, M_MARCH, M_FILTER, M_MASS, NMAP };
 constexpr int MLP_NPARAM = 4545;
 
 // Grid constants of one instance (host, FP64), in the device index
@@ -648,6 +648,7 @@ static int build_maps(chl_handle* h) {
         case M_MLP: b = cdiv(2L * Nx * Nz, 128); break;
         case M_WALLN: b = cdiv(2L * Nx * Nz, CHL_WALL_THREADS); break;
         case M_ZPLANE: b = Nz; break;
+        case M_MASS: b = chl_mass_blocks(Nx, Nz); break;
         case M_ZSOLVE: b = Nxh * h->zlanes; break;
       }
       off[q + 1] = off[q] + b;
@@ -772,8 +773,8 @@ static int enqueue_rk3(chl_handle* h, bool with_dt) {
     if (rc) return rc;
   }
   if (h->any_mass) {
-    KL("massflow", chl_launch_massflow(h->map(M_PT), h->st, 0, 0));
-    KL("massflow_shift", chl_launch_shift(h->map(M_PT), h->nblk[M_PT], 0, h->st));   // and t += dt
+    KL("massflow", chl_launch_massflow(h->map(M_MASS), h->nblk[M_MASS], h->st, 0, 0));
+    KL("massflow_shift", chl_launch_shift(h->map(M_PT2), h->nblk[M_PT2], 0, h->st));   // and t += dt
   } else {
     KL("t_advance", chl_launch_tadvance(h->map(M_PT), h->st));
   }
@@ -1491,7 +1492,7 @@ int chl_compute_dPx_for_constant_mass_flow(chl_handle* h, int inst, double* dPdx
   double s[CHL_S_NSCAL];
   CK(cudaMemcpyAsync(s, I->dev.scal, sizeof(s), cudaMemcpyDeviceToHost, h->st));
   if ((rc = finish(h))) return rc;
-  chl_launch_massflow(h->map(M_PT), h->st, 0, 1);
+  chl_launch_massflow(h->map(M_MASS), h->nblk[M_MASS], h->st, 0, 1);
   LAUNCHED();
   double s2[CHL_S_NSCAL];
   CK(cudaMemcpyAsync(s2, I->dev.scal, sizeof(s2), cudaMemcpyDeviceToHost, h->st));

@@ -299,30 +299,56 @@ __global__ void k_minabs_init(ChlMap map) {
 // ------------------------------------------------------------ constant mass flow
 // compute_dPx_for_constant_mass_flow (mass_flow.f90:113-166) over the unique
 // x-z points of rows j_f = 3 and nyg-2, then U += dPdx on the interior
-// (time_integration.f90:89-94); one block per instance for the sum.
-__global__ void k_massflow(ChlMap map, int s, int force) {
-  chl_pdl_wait();
-  const ChlInst& I = map.inst[blockIdx.x];
-  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
-  if (!I.x_mass_cte && !force) {                 // pressure-gradient forcing: no shift
-    if (threadIdx.x == 0) I.scal[CHL_S_SHIFT] = 0.0;
-    return;
-  }
-  const double* U = I.U[s];
-  double acc = 0.0;
-  for (int w = threadIdx.x; w < Nx * Nz; w += blockDim.x) {
-    const int i = w % Nx, k = w / Nx;
-    acc += 0.5 * (U[cidx(I, i, 2, k)] + U[cidx(I, i, Ny - 1, k)]);
-  }
-  __shared__ double red[256];
-  red[threadIdx.x] = acc;
+// (time_integration.f90:89-94).  A block per CHL_MASS_POINTS points of a plane
+// writes its sum to red, the instance's last block to finish (counter
+// dsm_cnt[0]; rows count from 1) adds them in order.  One block for the whole
+// plane is bound by its loads' latency: 94 us at 256x192, 12 like this; k_shift over pairs of
+// points 27 -> 18.
+__device__ __forceinline__ double block_sum256(double v, double* red) {
+  red[threadIdx.x] = v;
   __syncthreads();
   for (int h = 128; h > 0; h >>= 1) {
     if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
     __syncthreads();
   }
+  return red[0];
+}
+__global__ void __launch_bounds__(256)
+k_massflow(ChlMap map, int s, int force) {
+  chl_pdl_wait();
+  int lb;
+  const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
+  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz, nb = chl_mass_blocks(Nx, Nz);
+  if (!I.x_mass_cte && !force) {                 // pressure-gradient forcing: no shift
+    if (lb == 0 && threadIdx.x == 0) I.scal[CHL_S_SHIFT] = 0.0;
+    return;
+  }
+  const double* U = I.U[s];
+  double acc = 0.0;
+#pragma unroll 4
+  for (int w = lb * 256 + threadIdx.x; w < Nx * Nz; w += nb * 256) {
+    const int k = w / Nx, i = w - k * Nx;
+    acc += 0.5 * (U[cidx(I, i, 2, k)] + U[cidx(I, i, Ny - 1, k)]);
+  }
+  __shared__ double red[256];
+  double sum = block_sum256(acc, red);
+  if (nb > 1) {
+    __shared__ int last;
+    if (threadIdx.x == 0) {
+      I.red[lb] = sum;
+      __threadfence();
+      last = atomicAdd(I.dsm_cnt, 1) == nb - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    acc = 0.0;
+    for (int w = threadIdx.x; w < nb; w += 256) acc += __ldcg(I.red + w);
+    sum = block_sum256(acc, red);
+    if (threadIdx.x == 0) I.dsm_cnt[0] = 0;
+  }
   if (threadIdx.x == 0) {
-    const double d = I.scal[CHL_S_Q0] - red[0] / (double)(Nx * Nz);
+    const double d = I.scal[CHL_S_Q0] - sum / (double)(Nx * Nz);
     I.scal[CHL_S_SHIFT] = d;
     if (!force) chl_vmax(I, s)[0] = 0u;     // k_shift forms the largest |U| anew
     if (!force) I.scal[CHL_S_DPDX] = 0.0;   // dPdx = 0 after the shift (time_integration.f90:92)
@@ -350,16 +376,17 @@ k_shift(ChlMap map, int s) {
   }
   if (!I.x_mass_cte) return;
   unsigned hi[1] = {0u};
-  if (t < (unsigned)(Nx * Ny * Nz)) {
-    const ChlIdx p = chl_split(t, Nx, Ny);
-    const int i = p.i, jc = 1 + p.j, k = p.k;
-    double* U = I.U[s];
+  if (t < (unsigned)(Nx / 2 * Ny * Nz)) {     // pairs of points
+    const ChlIdx p = chl_split(t, Nx / 2, Ny);
+    const int i = 2 * p.i, jc = 1 + p.j, k = p.k;
+    auto U = [&](int j) -> double2& { return *reinterpret_cast<double2*>(I.U[s] + cidx(I, i, j, k)); };
     const double d = I.scal[CHL_S_SHIFT];
-    const double un = U[cidx(I, i, jc, k)] + d;
-    U[cidx(I, i, jc, k)] = un;
-    if (jc == 1) U[cidx(I, i, 0, k)] = chl_neg(un);
-    if (jc == Ny) U[cidx(I, i, Ny + 1, k)] = chl_neg(un);
-    hi[0] = chl_abshi(un);
+    double2 u = U(jc);
+    u.x += d; u.y += d;
+    U(jc) = u;
+    if (jc == 1) U(0) = make_double2(chl_neg(u.x), chl_neg(u.y));
+    if (jc == Ny) U(Ny + 1) = make_double2(chl_neg(u.x), chl_neg(u.y));
+    hi[0] = max(chl_abshi(u.x), chl_abshi(u.y));
   }
   chl_block_max(chl_vmax(I, s), hi);
 }
@@ -481,7 +508,7 @@ void chl_launch_minabs(const ChlMap& m, int nb, int s, cudaStream_t st) {
 void chl_launch_nonfinite(const ChlMap& m, int nb, int s, cudaStream_t st) {
   chl_launch_pdl(k_nonfinite, dim3(nb), dim3(m.tb), 0, st, m, s);
 }
-void chl_launch_massflow(const ChlMap& m, cudaStream_t st, int s, int force) { chl_launch_pdl(k_massflow, dim3(m.n), dim3(256), 0, st, m, s, force); }
+void chl_launch_massflow(const ChlMap& m, int nb, cudaStream_t st, int s, int force) { chl_launch_pdl(k_massflow, dim3(nb), dim3(256), 0, st, m, s, force); }
 void chl_launch_shift(const ChlMap& m, int nb, int s, cudaStream_t st) { chl_launch_pdl(k_shift, dim3(nb), dim3(m.tb), 0, st, m, s); }
 void chl_launch_tadvance(const ChlMap& m, cudaStream_t st) { chl_launch_pdl(k_tadvance, dim3(m.n), dim3(32), 0, st, m); }
 void chl_launch_divmax(const ChlMap& planes, int nplanes, int s, double* out, cudaStream_t st) {

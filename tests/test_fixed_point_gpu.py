@@ -122,3 +122,22 @@ def test_a_non_finite_value_reaches_the_result():
         ch.compute_projection_step()
         assert not np.isfinite(ch.pseudo_pressure()).all()
         ch.close()
+
+
+# the mass-flow sum's blocks: one, several, as many as the partials have room for
+@pytest.mark.parametrize("Nx,Nz", ((32, 16), (64, 32), (48, 64), (1024, 4), (2304, 4)))
+def test_mass_flow_is_kept(Nx, Nz):
+    from channel_rl_gb300.host import Channel
+    case = replace(C.smaller(C.c1_small(), Nx, 8, Nz), LES_model=C.LES_NONE)
+    U, V, W = C.initial_fields(case)
+    o = oracle_for(case)
+    o.set_fields(U, V, W)
+    ch = Channel(case)
+    ch.upload(U, V, W)
+    reg = regions(o.g)["U"]
+    for _ in range(2):                       # the second finds the block counter as the first left it
+        o.step()
+        ch.step(1)
+        assert rel(ch.download(fields=("U",))["U"][reg], o.U[1:, 1:, 1:][reg]) < FIELD_RTOL
+        assert abs(ch.compute_dPx_for_constant_mass_flow()) < 1e-12
+    ch.close()
