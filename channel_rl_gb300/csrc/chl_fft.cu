@@ -262,6 +262,9 @@ __device__ __forceinline__ unsigned abshi2(double2 v) { return max(chl_abshi(v.x
 //         the pressure BC planes and the BC source terms of pressure.f90:138-139.
 // mode 2: mode 0 without a velocity correction to follow (the tuner).  Mode 0
 //         clears the set's largest velocities, which k_project forms anew.
+// Two of the six differences of a pair of planes go to the integer pipe, beside
+// the FP64 one: 88 -> 82 us at 256x96x192 (one, two, three, four, six of them
+// 86, 82, 84, 86, 94 us).
 __global__ void __launch_bounds__(256)
 k_div_fftx(ChlMap map, int s_in, int mode, int xmb) {
   chl_pdl_wait();
@@ -298,8 +301,9 @@ k_div_fftx(ChlMap map, int s_in, int mode, int xmb) {
         if (jc == 1) vlo = I.bc[(size_t)k * Nx + i];
         if (jc == Ny) vhi = I.bc[(size_t)Nx * Nz + (size_t)k * Nx + i];
       }
-      double d = (LDG(U + cidx(I, i, jc, k)) - LDG(U + cidx(I, im, jc, k))) * LDG(I.rdxc + i)
-               + (vhi - vlo) * LDG(I.rdyc + jc)
+      const double uhi = LDG(U + cidx(I, i, jc, k)), ulo = LDG(U + cidx(I, im, jc, k));
+      double d = (h == 0 ? fx_sub(uhi, ulo) : uhi - ulo) * LDG(I.rdxc + i)
+               + (h == 0 ? fx_sub(vhi, vlo) : vhi - vlo) * LDG(I.rdyc + jc)
                + (LDG(W + cidx(I, i, jc, k)) - LDG(W + cidx(I, i, jc, km))) * LDG(I.rdzc + k);
       if (mode == 1) {
         if (jc == 1) d += I.cbc1 * I.bc[(size_t)k * Nx + i];
@@ -777,6 +781,9 @@ k_fftx_inv(ChlMap map, int dst, int xmb) {
 // ------------------------------------------------------------ velocity correction
 // project_velocity (projection.f90:192-214) + Dirichlet ghost rows; folds
 // the set's largest velocities (cleared by k_div_fftx) for its fixed-point copies.
+// The FP64 pipe bounds it (6 instructions per point, 71 % busy), so two of a
+// pair's six differences are formed on the integer pipe: 60 -> 55 us at
+// 256x96x192 (one, two, three, four, six of them 57, 55, 55, 61, 64 us; HBM floor 39).
 __global__ void __launch_bounds__(256)
 k_project(ChlMap map, int s) {
   chl_pdl_wait();
@@ -801,7 +808,7 @@ k_project(ChlMap map, int s) {
     const double px = LDG(p + cidx(I, wrap(i + 2, Nx), jc, k));
     const double2 u = at(U, c), w = at(W, c), v = at(V, e);
     const double rx0 = LDG(I.rdxf + i), rx1 = LDG(I.rdxf + i + 1), ry = LDG(I.rdyf + jc), rz = LDG(I.rdzf + k);
-    const double2 un = make_double2(u.x - (p0.y - p0.x) * rx0, u.y - (px - p0.y) * rx1);
+    const double2 un = make_double2(u.x - fx_sub(p0.y, p0.x) * rx0, u.y - fx_sub(px, p0.y) * rx1);
     const double2 wn = make_double2(w.x - (pz.x - p0.x) * rz, w.y - (pz.y - p0.y) * rz);
     put(U, c, un); put(W, c, wn);
     hi[0] = top(un); hi[2] = top(wn);

@@ -56,6 +56,14 @@ __device__ __forceinline__ double fx_to(fx f, int e) {
   if (lz == 64) rh = 0u;
   return __hiloint2double((int)(rh | ((unsigned)sign & 0x80000000u)), (int)(unsigned)r);
 }
+// a - b on the integer pipe: exact like the FP64 subtraction where that is
+// (magnitudes within 2^8 of each other keep all their bits), else within 2^-61
+// of the larger before its one rounding; NaN if a or b is not finite.
+__device__ __forceinline__ double fx_sub(double a, double b) {
+  const int m = max(__double2hiint(a) >> 20 & 0x7FF, __double2hiint(b) >> 20 & 0x7FF);
+  const double d = fx_to<true>(fx_from(a, m - 1084) - fx_from(b, m - 1084), m - 1084);
+  return m == 0x7FF ? __longlong_as_double(0x7FF8000000000000LL) : d;
+}
 // F as a double, on the FP64 pipe (64 clocks, no other) or the integer pipe
 template <bool HW>
 __device__ __forceinline__ double fx_raw(fx f) { return HW ? __ll2double_rn(f) : fx_to(f, 0); }
