@@ -755,7 +755,7 @@ static void enqueue_rhs_only(chl_handle* h) {
 static void enqueue_dt(chl_handle* h, cudaStream_t st) {
   bool fixed = true;   // every instance on a fixed step: only the non-finite check
   for (auto& I : h->in) fixed = fixed && I.d.CFL < 0.0;
-  if (fixed) KL("dt_minabs", chl_launch_nonfinite(h->map(M_PT), h->nblk[M_PT], 0, st));
+  if (fixed) KL("dt_minabs", chl_launch_nonfinite(h->map(M_PT2), h->nblk[M_PT2], 0, st));
   else KL("dt_minabs", chl_launch_minabs(h->map(M_MINABS), h->nblk[M_MINABS], 0, st));
 }
 

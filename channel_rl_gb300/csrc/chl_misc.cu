@@ -266,25 +266,25 @@ k_minabs(ChlMap map, int s) {
 
 // With a fixed time step the minima are not needed (compute_dt reduces them
 // and then replaces dt by -CFL, time_integration.f90:146-148); what the pass
-// must still do is flag non-finite velocities.  One thread per centre
-// (i, jc, k), jc = 1..Ny, reading the same U, V, W entries as k_minabs.
+// must still do is flag non-finite velocities.  One thread per pair of centres
+// (i, jc, k), jc = 1..Ny, reading the same U, V, W entries as k_minabs; 32-bit
+// index arithmetic (a 64-bit division takes FP64 instructions, six per point).
 __global__ void __launch_bounds__(256)
 k_nonfinite(ChlMap map, int s) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
-  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
-  const long t = (long)lb * blockDim.x + threadIdx.x;
+  const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
   if (t == 0) chl_put_dt(I.scal, -I.CFL);   // fixed step (compute_dt, time_integration.f90:146-148)
   bool bad = false;
-  if (t < (long)Nx * Ny * Nz) {
-    const int i = (int)(t % Nx);
-    const int jc = 1 + (int)((t / Nx) % Ny);
-    const int k = (int)(t / ((long)Nx * Ny));
-    const unsigned long long bu = absbits(I.U[s][cidx(I, i, jc, k)]);
-    const unsigned long long bv = absbits(I.V[s][vidx(I, i, jc, k)]);
-    const unsigned long long bw = absbits(I.W[s][cidx(I, i, jc, k)]);
-    bad = (bu >= CHL_BIG_BITS) | (bv >= CHL_BIG_BITS) | (bw >= CHL_BIG_BITS);
+  if (t < (unsigned)(I.Nx / 2 * I.Ny * I.Nz)) {
+    const ChlIdx p = chl_split(t, I.Nx / 2, I.Ny);
+    const int i = 2 * p.i, jc = 1 + p.j, k = p.k;
+    auto inf = [](const double* f) {
+      const double2 v = __ldg(reinterpret_cast<const double2*>(f));
+      return absbits(v.x) >= CHL_BIG_BITS || absbits(v.y) >= CHL_BIG_BITS;
+    };
+    bad = inf(I.U[s] + cidx(I, i, jc, k)) | inf(I.V[s] + vidx(I, i, jc, k)) | inf(I.W[s] + cidx(I, i, jc, k));
   }
   if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(I.status, CHL_STATUS_NONFINITE);
 }
