@@ -56,13 +56,12 @@ UNIT = "grid-point-steps/s"
 # Algorithmic HBM bytes per grid point per launch of each kernel (compulsory
 # 8-byte streams; spectral arrays count their half-spectrum share).
 KERNEL_BYTES = {
+    "fix": 8 * 6.0,              # U, V, W and their fixed-point copies
     "rhs_flux": 8 * 13.0,        # U, V, W, nu+nu_t in; 9 face fluxes out
     "rhs_update": 8 * 18.0,      # 9 fluxes + 3 base (+3 F1) in; 3 (+3 F1) out
-    # 15 components in + out (the 3 centre velocities on the wall rows only)
-    "filter_y": 8 * 30.0, "filter_x": 8 * 30.0, "filter_z": 8 * 30.0,
-    "centre_strain": 8 * 19.0,   # U,V,W + 3 edge fields in, |S| + 12 filter inputs out
-    "edges": 8 * 6.0,
-    "dsm_LM_MM": 8 * 18.0,       # 12 filtered centre fields, 3 filtered faces, 3 edge fields
+    "strain": 8 * 16.0,          # U, V, W in, |S| + 12 filter inputs out
+    "filter": 8 * 30.0,          # 12 centre and 3 face fields in + out
+    "dsm_LM_MM": 8 * 15.0,       # 12 filtered centre fields, 3 filtered faces
     "nut": 8 * 2.0,
     "div_fft_x": 8 * 4.0,        # U,V,W in, half spectrum out
     "fft_z": 8 * 2.0,
@@ -72,9 +71,10 @@ KERNEL_BYTES = {
     "massflow_shift": 8 * 2.0,
     "dt_minabs": 8 * 3.0,
     "z_solve": 8 * 3.5,          # half spectrum in and out (8 B per point each), tridiagonal factors (12 B)
-    "amd": 8 * 4.0,              # U, V, W in, nu_t out
-    "vreman": 8 * 4.0,           # U, V, W in, nu_t out
+    "amd": 8 * 5.0,              # U, V, W in, nu_t and nu + nu_t out
+    "vreman": 8 * 5.0,           # U, V, W in, nu_t and nu + nu_t out
 }
+STATIC_STRAIN_BYTES = 8 * 5.0    # the static model's: U, V, W in, |S| and nu + nu_t out
 # Compulsory traffic of an ideally fused step (8-byte streams per point):
 # 107 with the dynamic model, 101 with static Smagorinsky.
 STEP_STREAMS = {"dsm": 107, "smag": 101}
@@ -343,13 +343,13 @@ def roofline_of(args, prof, points, step_ms, workload_name, rank=0, dev_index=0)
     fp64 = (live_fp64_peak(dev_index) if rank == 0 else None) or \
         load_json(os.path.join(HERE, "profiles", "fp64_peak.json"), {})
     traffic = load_json(os.path.join(HERE, "profiles", "kernel_traffic.json"), {})
-    byt = KERNEL_BYTES.get(dom, 0.0) * points
+    sgs = "dsm" if args.sgs == C.LES_DSM else "smag"
+    byt = (STATIC_STRAIN_BYTES if dom == "strain" and sgs == "smag" else KERNEL_BYTES.get(dom, 0.0)) * points
     ach = byt / per_launch_s / 1e9
     hbm = {"bound": "hbm", "kernel": dom, "achieved": ach, "peak": hbm_peak, "unit": "GB/s",
            "frac": ach / hbm_peak, "peak_source": hbm_src,
            "traffic": (traffic.get(workload_name, {}).get(dom) if traffic else None),
            "algorithmic_bytes_per_launch": byt, "launch_ms": per_launch_s * 1e3}
-    sgs = "dsm" if args.sgs == C.LES_DSM else "smag"
     hbm["step_hbm_gbs_vs_fused_minimum"] = 8 * STEP_STREAMS[sgs] * points / (step_ms * 1e-3) / 1e9
     fl = (traffic or {}).get("fp64_instr_per_point", {}).get(workload_name, {})
     peak_gops = fp64.get("fp64_peak_gops")

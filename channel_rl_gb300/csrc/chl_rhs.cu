@@ -21,7 +21,7 @@
 //
 // Both kernels work in 64-bit fixed point (chl_fix.cuh): as FP64 code they
 // were bound by the FP64 pipe (52 and 24 instructions per point, 457 and 201
-// us per launch at 256x96x192).  The velocities come as the fixed-point
+// us per launch at 256x96x192; 172 and 147 now).  The velocities come as the fixed-point
 // copies k_fix made of the stage's input, the fluxes are kept as integers,
 // and only the three components of F and the two FMAs of the stage update
 // are FP64.  Halves and quarters of the averages are exponents.  The y-face

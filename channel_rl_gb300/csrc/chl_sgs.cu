@@ -10,7 +10,7 @@
 //
 // The strain, the filter and L are formed in fixed point (chl_fix.cuh,
 // chl_strain.cuh): as FP64 code the dynamic model took 212 FP64 instructions
-// per point and stage, which the FP64 pipe bounds; 30 are left.
+// per point and stage, which the FP64 pipe bounds; 43 are left.
 //
 // Static Smagorinsky with van Driest damping (subgrid.f90:563-612, which
 // aborts in the reference) is written from its formula.  The stress wall
@@ -77,7 +77,7 @@ k_strain(ChlMap map, int s_in, int use_wm) {
 // (4, 2)/6 at its first and last row.  Three separable FP64 passes took 2
 // instructions of 64 clocks per pass, field and point and moved every field
 // three times: 247 us per pass at 256x96x192.  Here a tap is an integer
-// shift and two additions.
+// shift and two additions, and the three passes take 236 us together.
 //
 // A pass forms (a + 4 b + c) >> 3, so that a field starts and ends below 2^60
 // and a filtered value is 512/216 times its integer.  A thread holds two

@@ -97,12 +97,12 @@ struct GradColumn {
 }  // namespace
 
 // AMD in fixed point.  As FP64 code this kernel issued 114 FP64 instructions
-// per point (0.97 ms per launch at 256x96x192, the FP64 pipe 90 % busy).  The
+// per point (0.97 ms per launch at 256x96x192, the FP64 pipe 90 % busy; 0.28 ms now).  The
 // edge differences are exact integers from the fixed-point copies (k_fix);
 // each point scales its fifteen by their largest, so that the products keep
 // 54 bits or more of the largest product, and forms the derivatives, D and
 // the a_ij there.  N and the division are FP64 (17 instructions).
-__global__ void __launch_bounds__(CHL_FLUX_THREADS, 5)   // 102 registers: 2, 3, 4, 5, 6 blocks per SM take 417, 321, 289, 288, 290 us
+__global__ void __launch_bounds__(CHL_FLUX_THREADS, 5)   // 2, 3, 4, 5, 6 blocks per SM took 417, 321, 289, 288, 290 us (283 now)
 k_amd(ChlMap map, int s_in, int use_wm) {
   chl_pdl_wait();
   int lb;

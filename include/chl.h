@@ -286,8 +286,8 @@ const char* chl_noalloc_last_error(void);
  * w0(1:ny), dxmin, dymin, dzmin, coef_bc_1, coef_bc_2]. */
 int chl_grid_constants_size(const chl_grid_desc* desc);
 int chl_grid_constants(const chl_grid_desc* desc, double* out);
-/* Host-only: the pass table of the length-N transform that chl_create
- * stages for the x (N = nx-2) and z (N = nz-2) transforms.  Per pass with
+/* Host-only: the FP64 pass table of a length-N Stockham transform in tangent
+ * form (the library's own transforms use fixed-point twiddles).  Per pass with
  * twiddles (radix R = 4 while the remaining length allows, then 3, then 2;
  * sub-transform size Ns > 1) 7 fields of Ns doubles, entry jm for the
  * twiddles w_r = exp(-2 pi i jm r/(Ns R)), r = 1..R-1, each kept as a scale
