@@ -71,7 +71,7 @@ namespace {
 constexpr double RK_T[3] = {8.0 / 15.0, 2.0 / 3.0, 1.0};
 
 enum { M_PT, M_PT2, M_FULL2, M_DSMF, M_WALL, M_PLANE, M_FFTX, M_FFTZ, M_TRI, M_MINABS, M_ROWS, M_MLP, M_WALLN,
-       M_ZPLANE, M_ZSOLVE, M_FLUX, M_MARCH, M_FILTER, M_MASS, NMAP };
+       M_ZPLANE, M_ZSOLVE, M_FLUX, M_MARCH, M_FILTER, M_MASS, M_NUT, NMAP };
 constexpr int MLP_NPARAM = 4545;
 
 // Grid constants of one instance (host, FP64), in the device index
@@ -367,7 +367,7 @@ struct chl_handle {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   ChlMap map(int which) const {
-    const bool pt = which == M_PT || which == M_PT2 || which == M_FULL2;
+    const bool pt = which == M_PT || which == M_PT2 || which == M_FULL2 || which == M_NUT;
     return ChlMap{d_inst, d_off[which], (int)in.size(), pt ? tb_pt : 256, planes, fplanes};
   }
 };
@@ -648,6 +648,7 @@ static int build_maps(chl_handle* h) {
         case M_MLP: b = cdiv(2L * Nx * Nz, 128); break;
         case M_WALLN: b = cdiv(2L * Nx * Nz, CHL_WALL_THREADS); break;
         case M_ZPLANE: b = Nz; break;
+        case M_NUT: b = cdiv((long)(Nx / 2) * (Ny + 2) * cdiv(Nz, h->planes), h->tb_pt); break;
         case M_MASS: b = chl_mass_blocks(Nx, Nz); break;
         case M_ZSOLVE: b = Nxh * h->zlanes; break;
       }
@@ -714,7 +715,7 @@ static int enqueue_sgs(chl_handle* h, int s, bool with_wm, int stage = 0, bool w
   }
   if (!fused) {
     CK(join_mlp());
-    KL("nut", chl_launch_nut(h->map(M_FULL2), h->nblk[M_FULL2], wm ? 1 : 0, st));
+    KL("nut", chl_launch_nut(h->map(M_NUT), h->nblk[M_NUT], wm ? 1 : 0, st));
   }
   if (fork && wm && !mlp) CK(cudaStreamWaitEvent(st, h->side.wall, 0));
   LAUNCHED();
@@ -1453,7 +1454,7 @@ int chl_compute_wall_model(chl_handle* h) {
   if (h->wall_model >= CHL_WM_EQLOG) chl_launch_eqwm(h->map(M_WALLN), h->nblk[M_WALLN], 0, h->st);
   if (h->wall_model == CHL_WM_MLP) chl_launch_mlp(h->map(M_MLP), h->nblk[M_MLP], 0, 0, h->d_mlp_status, h->st);
   if (h->wall_model != CHL_WM_NONE) chl_launch_wall_rows(h->map(M_WALL), h->nblk[M_WALL], 0, h->st);
-  chl_launch_nut(h->map(M_FULL2), h->nblk[M_FULL2], h->wall_model != CHL_WM_NONE ? 1 : 0, h->st);
+  chl_launch_nut(h->map(M_NUT), h->nblk[M_NUT], h->wall_model != CHL_WM_NONE ? 1 : 0, h->st);
   LAUNCHED();
   return finish(h);
 }

@@ -465,39 +465,50 @@ static __device__ __noinline__ double nut_other(const ChlInst& I, int i, int jc,
   }
   return I.nu + chl_pos(I.S[cidx(I, i, jc, k)]);
 }
-// One thread per pair of x points of a row (jc, k), jc = 0..Ny+1 (with one
-// point per thread this kernel took 52 us at 256x96x192 for 11 us of HBM
-// traffic: blocks too short-lived for their start-up).  With the wall model on,
+// One thread per pair of x points of a row jc = 0..Ny+1 and `planes` planes: a
+// stream of 16 bytes in and out per pair, 11 us of HBM at 256x96x192.  With one
+// point per thread it took 52 us, with one pair 30 (blocks too short-lived for
+// their start-up and their fold of the maximum), now 22.  With the wall model on,
 // rows 0, 1 and Ny, Ny+1 are k_wall_rows's.
 __global__ void __launch_bounds__(256)
 k_nut(ChlMap map, int use_wm) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
-  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz, nxp = Nx / 2;
-  const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  const bool valid = t < (unsigned)(nxp * (Ny + 2) * Nz);
-  // lanes past the end repeat the last pair and write nothing
-  const ChlIdx p = chl_split(valid ? t : (unsigned)(nxp * (Ny + 2) * Nz) - 1u, nxp, Ny + 2);
-  const int i = 2 * p.i, jc = p.j, k = p.k;
+  const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz, nxp = Nx / 2, M = map.planes, nk = (Nz + M - 1) / M;
+  const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x, n = (unsigned)(nxp * (Ny + 2) * nk);
+  const bool valid = t < n;
+  // lanes past the end repeat the last column and write nothing
+  const ChlIdx p = chl_split(valid ? t : n - 1u, nxp, Ny + 2);
+  const int i = 2 * p.i, jc = p.j, k0 = p.k * M, k1 = min(Nz, k0 + M);
   const bool wm = use_wm && I.wall_model != 0 && (jc <= 1 || jc >= Ny);
-  double2 v = make_double2(0.0, 0.0);
+  unsigned hi = 0u;
   if (valid && !wm) {
     // stored as nu + nu_t: every consumer adds nu (equations.f90:139-155)
     const double nu = I.nu;
-    const size_t c = cidx(I, i, jc, k) / 2;
+    double2* nut = reinterpret_cast<double2*>(I.nut);
     if (I.LES_model == 0 || I.LES_model >= 3 || jc == 0 || jc == Ny + 1) {
-      v = make_double2(nut_other(I, i, jc, k), nut_other(I, i + 1, jc, k));
+      for (int k = k0; k < k1; ++k) {
+        const double2 v = make_double2(nut_other(I, i, jc, k), nut_other(I, i + 1, jc, k));
+        nut[cidx(I, i, jc, k) / 2] = v;
+        hi = max(hi, max(chl_abshi(v.x), chl_abshi(v.y)));
+      }
     } else {
       // nu + max(0, c |S|) as one FMA, nu + c |S|, clipped below at nu by the
       // bit patterns (both positive; a NaN, for which max gives 0, gives nu)
       const double cj = I.coef[jc];
-      const double2 S = __ldg(reinterpret_cast<const double2*>(I.S) + c);
-      v = make_double2(chl_atleast(fma(cj, S.x, nu), nu), chl_atleast(fma(cj, S.y, nu), nu));
+      const double2* S = reinterpret_cast<const double2*>(I.S);
+#pragma unroll 4
+      for (int k = k0; k < k1; ++k) {
+        const size_t c = cidx(I, i, jc, k) / 2;
+        const double2 s = __ldg(S + c);
+        const double2 v = make_double2(chl_atleast(fma(cj, s.x, nu), nu), chl_atleast(fma(cj, s.y, nu), nu));
+        nut[c] = v;
+        hi = max(hi, max(chl_abshi(v.x), chl_abshi(v.y)));
+      }
     }
-    reinterpret_cast<double2*>(I.nut)[c] = v;
   }
-  chl_line_max(I.nmax, (unsigned)(k * (Ny + 2) + jc), Ny + 2, 0, max(chl_abshi(v.x), chl_abshi(v.y)));
+  chl_line_max(I.nmax, (unsigned)(p.k * (Ny + 2) + jc), Ny + 2, 0, hi);
 }
 
 // nu + nu_t on the wall-model rows, jc = 0, 1 and Ny, Ny+1: nu_t is the mean
