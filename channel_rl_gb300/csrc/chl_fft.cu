@@ -13,7 +13,7 @@
 //    the rows;
 //  * z: complex columns of the half-spectrum, staged up to 8 kx-columns at a time
 //    in shared memory;
-//  * y: one thread per mode runs the Thomas elimination with factors
+//  * y: one thread per real column of a mode runs the Thomas elimination with factors
 //    precomputed once per grid (the matrix of a mode never changes between
 //    steps), into which the 1/(Nx*Nz) of the inverse transform and the 2 of
 //    the real-row packing are folded; the mode's column is staged in shared

@@ -26,8 +26,8 @@
 // largest per row.
 // With DSM = false (the static model, whose row coefficients do not depend on
 // the strain) nu + nu_t instead, so that no pass reads |S| back: 143 -> 157 us
-// at 256x96x192 for the 37 of k_nut and the launch of the coefficients' own
-// kernel.
+// at 256x96x192 for the 37 that k_nut then took and the launch of the
+// coefficients' own kernel.
 template <bool DSM>
 __global__ void __launch_bounds__(CHL_FLUX_THREADS, 7)
 k_strain(ChlMap map, int s_in, int use_wm) {
