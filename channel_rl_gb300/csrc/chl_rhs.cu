@@ -101,6 +101,89 @@ k_fix(ChlMap map, int s, int prep) {
   if (t < nv) put(I.X[1], v, ev);
 }
 
+// Fluxes next to a wall whose nu + nu_t the wall model sets (y-faces 0, 1 and
+// Ny-1, Ny, centre rows 1 and Ny).  It is tau dyw/du there, without a bound where
+// the wall shear passes zero, and with one unit per row the largest of a row takes
+// the digits of all its points: one with 1e-9 of the others' shear left 7 of them,
+// one with none left NaN.  So each of these fluxes has a unit of its own, from the
+// nu + nu_t of its edge, and is stored as a double.
+__device__ __forceinline__ bool wall_face(const ChlInst& I, int j) { return I.wall_model != 0 && (j <= 1 || j >= I.Ny - 1); }
+__device__ __forceinline__ bool wall_centre(const ChlInst& I, int j) { return I.wall_model != 0 && (j == 1 || j == I.Ny); }
+
+// x as m 2^e, |m| < 2^61 (0 for a subnormal x)
+struct Norm {
+  fx m; int e; bool bad;
+  __device__ __forceinline__ explicit Norm(double x) {
+    const long long b = __double_as_longlong(x);
+    const int x11 = (int)(b >> 52) & 0x7FF;
+    const fx f = (fx)(((unsigned long long)b << 12 >> 4) | (1ULL << 60));
+    m = x11 == 0 ? 0 : (b < 0 ? -f : f);
+    e = x11 - 1083;
+    bad = x11 == 0x7FF;
+  }
+};
+
+// These fluxes of column i, planes k0..k1-1: of y-face jf (on a wall only those
+// that a row takes) and of centre row jc (0: none).  A call, for the registers.
+// The averages of nu + nu_t are its only FP64 instructions, 13 per point (52 with
+// the fluxes in FP64 as well, which cost the 128x40x64 channel 6 % of a step).
+static __device__ __noinline__ void flux_wall(const ChlInst& I, int sin, int i, int jf, int jc, int k0, int k1) {
+  const int Nx = I.Nx, Nz = I.Nz, ip = wrap(i + 1, Nx), im = wrap(i - 1, Nx);
+  const unsigned* vm = chl_vmax(I, sin);
+  const int eu = fx_exp<61>(vm[0]), ev = fx_exp<61>(vm[1]), ew = fx_exp<61>(vm[2]);
+  const bool bad = fx_bad(vm[0]) || fx_bad(vm[1]) || fx_bad(vm[2]), wall = jf == 0 || jf == I.Ny;
+  auto u = [&](int a, int b, int k) { return LDG(I.X[0] + cidx(I, a, b, k)); };
+  auto v = [&](int a, int b, int k) { return LDG(I.X[1] + vidx(I, a, b, k)); };
+  auto w = [&](int a, int b, int k) { return LDG(I.X[2] + cidx(I, a, b, k)); };
+  auto n = [&](int a, int b, int k) { return LDG(I.nut + cidx(I, a, b, k)); };
+  // viscous less advective part: vis 2^ev less adv 2^ea
+  auto put = [&](int m, size_t q, fx adv, int ea, const Norm& nu, fx grad, int ev) {
+    ev += nu.e;
+    const int g = max(ea, ev) + 1;
+    const double f = fx_to((fx_mul_shr<61>(nu.m, grad) >> min(63, g - ev)) - (adv >> min(63, g - ea)), g);
+    reinterpret_cast<double*>(I.G[m])[q] = bad || nu.bad ? __longlong_as_double(0x7FF8000000000000LL) : f;
+  };
+  const fx rxf = LDG(I.fxrxf + i);
+#pragma unroll 1
+  for (int k = k0; k < k1; ++k) {
+    const int kp = wrap(k + 1, Nz);
+    const fx rzf = LDG(I.fxrzf + k);
+    {
+      const int j = jf, jp = j + 1, eyf = I.eyf[j];
+      const fx ryf = LDG(I.fxryf + j), w1 = LDG(I.fxw1 + j);
+      const double w0x2 = LDG(I.w0x2 + j), w1x2 = LDG(I.w1x2 + j);
+      const fx ua = u(i, j, k), du = u(i, jp, k) - ua, wa = w(i, j, k), dw = w(i, jp, k) - wa;
+      const fx v0 = v(i, j, k), vz = v(i, j, kp), vp = v(ip, j, k);
+      const double na = n(i, j, k), nb = n(i, jp, k);
+      const size_t e = vidx(I, i, j, k);
+      // yz edge: 2 v w, 4 nu; xy edge: 2 u v, 4 nu
+      const fx vw = fx_mul_shr<62>(wa + 2 * fx_mul(dw, w1), v0 + vz), uv = fx_mul_shr<62>(ua + 2 * fx_mul(du, w1), v0 + vp);
+      const Norm nyz(fma(w0x2, na + n(i, j, kp), w1x2 * (nb + n(i, jp, kp))));
+      const Norm nxy(fma(w0x2, na + n(ip, j, k), w1x2 * (nb + n(ip, jp, k))));
+      put(G_WY, e, vw, ev + ew + 61, nyz, fx_mul(dw, ryf), ew + eyf + 123);
+      put(G_UY, e, uv, eu + ev + 61, nxy, fx_mul(du, ryf), eu + eyf + 123);
+      if (!wall) {
+        put(G_VZ, e, vw, ev + ew + 61, nyz, fx_mul(vz - v0, rzf), ev + I.ezf + 123);
+        put(G_VX, e, uv, eu + ev + 61, nxy, fx_mul(vp - v0, rxf), ev + I.exf + 123);
+      }
+    }
+    if (jc == 0) continue;
+    const int j = jc;
+    const size_t c = cidx(I, i, j, k);
+    const fx ua = u(i, j, k), wa = w(i, j, k), v0 = v(i, j, k);
+    const fx um = u(im, j, k), vm_ = v(i, j - 1, k), wm = w(i, j, wrap(k - 1, Nz)), su = um + ua, sv = vm_ + v0, sw = wm + wa;
+    const fx uz = u(i, j, kp), wp = w(ip, j, k), uw = fx_mul_shr<62>(ua + uz, wa + wp);
+    const double na = n(i, j, k);
+    // xz edge: 4 u w, 4 nu; cell centre: u u with both halves in the exponent, nu
+    const Norm nxz((na + n(ip, j, k)) + (n(i, j, kp) + n(ip, j, kp))), nu(na);
+    put(G_UX, c, fx_mul_shr<62>(su, su), 2 * eu + 60, nu, fx_mul(ua - um, LDG(I.fxrxc + i)), eu + I.exc + 125);
+    put(G_VY, c, fx_mul_shr<62>(sv, sv), 2 * ev + 60, nu, fx_mul(v0 - vm_, LDG(I.fxryc + j)), ev + I.eyc[j] + 125);
+    put(G_WZ, c, fx_mul_shr<62>(sw, sw), 2 * ew + 60, nu, fx_mul(wa - wm, LDG(I.fxrzc + k)), ew + I.ezc + 125);
+    put(G_UZ, c, uw, eu + ew + 60, nxz, fx_mul(uz - ua, rzf), eu + I.ezf + 123);
+    put(G_WX, c, uw, eu + ew + 60, nxz, fx_mul(wp - wa, rxf), ew + I.exf + 123);
+  }
+}
+
 // 28 products and 4 conversions of nu + nu_t per point on the integer pipe,
 // no FP64 instruction; 104 bytes per point.  A thread marches through
 // a few planes at its (i, j), so that what the next plane shares (U, V,
@@ -133,6 +216,14 @@ k_flux(ChlMap map, int sin) {
     dn_a = LDG(nt + cidx(I, i, j, k0)); dn_b = LDG(nt + cidx(I, i, jp, k0)); dn_p = LDG(nt + cidx(I, ip, j, k0));
   }
   if (!valid) return;
+  // the wall model's rows: the threads of row 0 take both walls' faces, those of
+  // rows 1 and Ny a face and a centre row each, those of Ny-1 its centre row below
+  const bool own = wall_face(I, j);
+  if (own && j != Ny - 1) {
+    if (j == 0) { flux_wall(I, sin, i, 0, 0, k0, k1); flux_wall(I, sin, i, Ny, 0, k0, k1); }
+    else flux_wall(I, sin, i, j == 1 ? 1 : Ny - 1, j, k0, k1);
+    return;
+  }
   int sa[9], sv_[9];          // right shifts of the advective and viscous parts
   int en;
   {
@@ -160,7 +251,7 @@ k_flux(ChlMap map, int sin) {
     const fx n_pz = fx_from(LDG(nt + cidx(I, ip, j, kp)), en), n_bp = fx_from(LDG(nt + cidx(I, ip, jp, k)), en);
     const fx rzf = LDG(I.fxrzf + k);
     const fx nx_a = n_a + n_p;             // x pair of row j: the xy and xz edges share it
-    {  // yz edge (x-centre i, y-face j, z-face k): vw, nu -> GVz, GWy
+    if (!own) {  // yz edge (x-centre i, y-face j, z-face k): vw, nu -> GVz, GWy
       const fx dw = w_b - w_a;
       const fx vw = ADV(w_a + 2 * MUL(dw, w1), v_0 + v_z);                            // 2 v w
       const fx na = n_a + n_az;
@@ -168,7 +259,7 @@ k_flux(ChlMap map, int sin) {
       PUT(G_VZ, e, vw, VIS(nyz, MUL(v_z - v_0, rzf)));
       PUT(G_WY, e, vw, VIS(nyz, MUL(dw, ryf)));
     }
-    {  // xy edge (x-face i, y-face j, z-centre k): uv, nu -> GUy, GVx
+    if (!own) {  // xy edge (x-face i, y-face j, z-centre k): uv, nu -> GUy, GVx
       const fx du = u_b - u_a;
       const fx uv = ADV(u_a + 2 * MUL(du, w1), v_0 + v_p);                            // 2 u v
       const fx nxy = nx_a + 2 * MUL(n_b + n_bp - nx_a, w1);                           // 2 nu
@@ -211,76 +302,92 @@ __device__ __forceinline__ double row_diff(fx hi, int eh, fx lo, int el) {
   return fx_to<true>((hi >> min(63, m - eh)) - (lo >> min(63, m - el)), m);
 }
 
-// The flux differences are exact integers; each is rounded once to a double
-// and multiplied by its reciprocal spacing there (with the products in
-// integers as well, F lost two to four bits to their common exponent).  One
-// thread per pair of x points: 16-byte loads, and the pair shares the fluxes
-// between its points.
-__global__ void __launch_bounds__(256)
-k_rhs_update(ChlMap map, RhsArgs a) {
-  chl_pdl_wait();
-  int lb;
-  const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
+// A flux as a double: stored so (next to a modelled wall) or in its row's unit 2^e.
+__device__ __forceinline__ double flux_val(fx f, bool dbl, int e) { return dbl ? __longlong_as_double(f) : fx_to<true>(f, e); }
+
+// F at x points i (even) and i + 1 of row jc, plane k.  WALL: a row next to a
+// modelled wall, where some of the fluxes are doubles.
+struct Rhs { double2 u, v, w; };
+template <bool WALL>
+__device__ __forceinline__ Rhs rhs_pair(const ChlInst& I, int i, int jc, int k) {
   const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
-  const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  if (t >= (unsigned)(Nx / 2 * Ny * Nz)) return;
-  const ChlIdx p = chl_split(t, Nx / 2, Ny);
-  const int i = 2 * p.i, jc = 1 + p.j, k = p.k;
   const int im = wrap(i - 1, Nx), ip = wrap(i + 2, Nx);
   const int km = wrap(k - 1, Nz), kp = wrap(k + 1, Nz);
   const fx* const* G = I.G;
   const bool hasv = jc <= Ny - 1;
   const size_t c = cidx(I, i, jc, k), e = vidx(I, i, jc, k), em = vidx(I, i, jc - 1, k);
   auto g2 = [](const fx* f, size_t q) { return __ldg(reinterpret_cast<const longlong2*>(f + q)); };
-  auto d2 = [](const double* f, size_t q) { return *reinterpret_cast<const double2*>(f + q); };
-  auto put = [](double* f, size_t q, double2 v) { *reinterpret_cast<double2*>(f + q) = v; };
-  auto neg = [](double2 v) { return make_double2(chl_neg(v.x), chl_neg(v.y)); };
   const double rxc0 = LDG(I.rdxc + i), rxc1 = LDG(I.rdxc + i + 1), rxf0 = LDG(I.rdxf + i), rxf1 = LDG(I.rdxf + i + 1);
   const double ryc = LDG(I.rdyc + jc), ryf = LDG(I.rdyf + jc);
   const double rzc = LDG(I.rdzc + k), rzf = LDG(I.rdzf + k), dpdx = I.scal[CHL_S_DPDX];
   // exponents of the fluxes of rows jc - 1, jc, jc + 1
   const int4 e0 = LDG(I.upd + jc), el = LDG(I.upd + jc - 1), eh = LDG(I.upd + min(jc + 1, Ny));
-  double2 Fu, Fv = make_double2(0.0, 0.0), Fw;
+  // stored as doubles: y-faces jc - 1 and jc, centre rows jc and jc + 1
+  const bool dl = WALL && wall_face(I, jc - 1), dh = WALL && wall_face(I, jc), dc = WALL && wall_centre(I, jc);
+  const bool dn = WALL && wall_centre(I, jc + 1);
+  // difference of two fluxes of one row, and of two rows
+  auto diff = [](fx hi, fx lo, bool d, int x) {
+    return WALL && d ? __longlong_as_double(hi) - __longlong_as_double(lo) : fx_to<true>(hi - lo, x);
+  };
+  auto ydiff = [](fx hi, bool dhi, int ehi, fx lo, bool dlo, int elo) {
+    return WALL ? flux_val(hi, dhi, ehi) - flux_val(lo, dlo, elo) : row_diff(hi, ehi, lo, elo);
+  };
+  Rhs F;
+  F.v = make_double2(0.0, 0.0);
   {  // u at (x-face i, row jc, z-centre k)
     const longlong2 x = g2(G[G_UX], c), yh = g2(G[G_UY], e), yl = g2(G[G_UY], em);
     const longlong2 zh = g2(G[G_UZ], c), zl = g2(G[G_UZ], cidx(I, i, jc, km));
     const fx xp = LDG(G[G_UX] + cidx(I, ip, jc, k));
-    Fu.x = fma(fx_to<true>(x.y - x.x, e0.x), rxf0, dpdx);
-    Fu.y = fma(fx_to<true>(xp - x.y, e0.x), rxf1, dpdx);
-    Fu.x = fma(row_diff(yh.x, e0.x, yl.x, el.x), ryc, Fu.x);
-    Fu.y = fma(row_diff(yh.y, e0.x, yl.y, el.x), ryc, Fu.y);
-    Fu.x = fma(fx_to<true>(zh.x - zl.x, e0.x), rzc, Fu.x);
-    Fu.y = fma(fx_to<true>(zh.y - zl.y, e0.x), rzc, Fu.y);
+    F.u.x = fma(diff(x.y, x.x, dc, e0.x), rxf0, dpdx);
+    F.u.y = fma(diff(xp, x.y, dc, e0.x), rxf1, dpdx);
+    F.u.x = fma(ydiff(yh.x, dh, e0.x, yl.x, dl, el.x), ryc, F.u.x);
+    F.u.y = fma(ydiff(yh.y, dh, e0.x, yl.y, dl, el.x), ryc, F.u.y);
+    F.u.x = fma(diff(zh.x, zl.x, dc, e0.x), rzc, F.u.x);
+    F.u.y = fma(diff(zh.y, zl.y, dc, e0.x), rzc, F.u.y);
   }
   {  // w at (x-centre i, row jc, z-face k)
     const longlong2 x = g2(G[G_WX], c), yh = g2(G[G_WY], e), yl = g2(G[G_WY], em);
     const longlong2 zl = g2(G[G_WZ], c), zh = g2(G[G_WZ], cidx(I, i, jc, kp));
     const fx xm = LDG(G[G_WX] + cidx(I, im, jc, k));
-    Fw.x = fx_to<true>(x.x - xm, e0.z) * rxc0;
-    Fw.y = fx_to<true>(x.y - x.x, e0.z) * rxc1;
-    Fw.x = fma(row_diff(yh.x, e0.z, yl.x, el.z), ryc, Fw.x);
-    Fw.y = fma(row_diff(yh.y, e0.z, yl.y, el.z), ryc, Fw.y);
-    Fw.x = fma(fx_to<true>(zh.x - zl.x, e0.z), rzf, Fw.x);
-    Fw.y = fma(fx_to<true>(zh.y - zl.y, e0.z), rzf, Fw.y);
+    F.w.x = diff(x.x, xm, dc, e0.z) * rxc0;
+    F.w.y = diff(x.y, x.x, dc, e0.z) * rxc1;
+    F.w.x = fma(ydiff(yh.x, dh, e0.z, yl.x, dl, el.z), ryc, F.w.x);
+    F.w.y = fma(ydiff(yh.y, dh, e0.z, yl.y, dl, el.z), ryc, F.w.y);
+    F.w.x = fma(diff(zh.x, zl.x, dc, e0.z), rzf, F.w.x);
+    F.w.y = fma(diff(zh.y, zl.y, dc, e0.z), rzf, F.w.y);
   }
   if (hasv) {  // v at (x-centre i, y-face jv = jc, z-centre k)
     const longlong2 x = g2(G[G_VX], e), yl = g2(G[G_VY], c), yh = g2(G[G_VY], cidx(I, i, jc + 1, k));
     const longlong2 zh = g2(G[G_VZ], e), zl = g2(G[G_VZ], vidx(I, i, jc, km));
     const fx xm = LDG(G[G_VX] + vidx(I, im, jc, k));
-    Fv.x = fx_to<true>(x.x - xm, e0.y) * rxc0;
-    Fv.y = fx_to<true>(x.y - x.x, e0.y) * rxc1;
-    Fv.x = fma(row_diff(yh.x, eh.y, yl.x, e0.y), ryf, Fv.x);
-    Fv.y = fma(row_diff(yh.y, eh.y, yl.y, e0.y), ryf, Fv.y);
-    Fv.x = fma(fx_to<true>(zh.x - zl.x, e0.y), rzc, Fv.x);
-    Fv.y = fma(fx_to<true>(zh.y - zl.y, e0.y), rzc, Fv.y);
+    F.v.x = diff(x.x, xm, dh, e0.y) * rxc0;
+    F.v.y = diff(x.y, x.x, dh, e0.y) * rxc1;
+    F.v.x = fma(ydiff(yh.x, dn, eh.y, yl.x, dc, e0.y), ryf, F.v.x);
+    F.v.y = fma(ydiff(yh.y, dn, eh.y, yl.y, dc, e0.y), ryf, F.v.y);
+    F.v.x = fma(diff(zh.x, zl.x, dh, e0.y), rzc, F.v.x);
+    F.v.y = fma(diff(zh.y, zl.y, dh, e0.y), rzc, F.v.y);
   }
-  if (e0.w | el.w | eh.w) {
+  // a row marked non-finite by its maxima (none where its fluxes are doubles)
+  const int bad = WALL ? (dc ? 0 : e0.w) | (dl ? 0 : el.w) | (dn ? 0 : eh.w) : e0.w | el.w | eh.w;
+  if (bad) {
     const double q = __longlong_as_double(0x7FF8000000000000LL);
-    Fu = Fv = Fw = make_double2(q, q);
+    F.u = F.v = F.w = make_double2(q, q);
   }
+  return F;
+}
+// F and the stage update at x points i (even) and i + 1 of row jc, plane k.
+template <bool WALL>
+__device__ __forceinline__ void update_pair(const ChlInst& I, const RhsArgs& a, int i, int jc, int k) {
+  const int Ny = I.Ny;
+  const bool hasv = jc <= Ny - 1;
+  const size_t c = cidx(I, i, jc, k), e = vidx(I, i, jc, k);
+  auto d2 = [](const double* f, size_t q) { return *reinterpret_cast<const double2*>(f + q); };
+  auto put = [](double* f, size_t q, double2 v) { *reinterpret_cast<double2*>(f + q) = v; };
+  auto neg = [](double2 v) { return make_double2(chl_neg(v.x), chl_neg(v.y)); };
+  const Rhs F = rhs_pair<WALL>(I, i, jc, k);
   if (a.mode == 2) {           // actual-pressure RHS: keep F only
-    put(I.Fp[0], c, Fu); put(I.Fp[2], c, Fw);
-    if (hasv) put(I.Fp[1], e, Fv);
+    put(I.Fp[0], c, F.u); put(I.Fp[2], c, F.w);
+    if (hasv) put(I.Fp[1], e, F.v);
     return;
   }
   // out = base + dt (c1 F1 + c2 F) as two FMAs per component; the products
@@ -288,11 +395,11 @@ k_rhs_update(ChlMap map, RhsArgs a) {
   const double dc1 = I.scal[CHL_S_DC + 2 * a.stage], dc2 = I.scal[CHL_S_DC + 2 * a.stage + 1];
   double* Uo = I.U[a.sout]; double* Vo = I.V[a.sout]; double* Wo = I.W[a.sout];
   auto axpy = [](double s, double2 x, double2 y) { return make_double2(fma(s, x.x, y.x), fma(s, x.y, y.y)); };
-  double2 un = axpy(dc2, Fu, d2(I.U[a.sbase], c)), wn = axpy(dc2, Fw, d2(I.W[a.sbase], c)), vn;
-  if (hasv) vn = axpy(dc2, Fv, d2(I.V[a.sbase], e));
+  double2 un = axpy(dc2, F.u, d2(I.U[a.sbase], c)), wn = axpy(dc2, F.w, d2(I.W[a.sbase], c)), vn;
+  if (hasv) vn = axpy(dc2, F.v, d2(I.V[a.sbase], e));
   if (a.mode == 0) {
-    put(I.F1[0], c, Fu); put(I.F1[2], c, Fw);
-    if (hasv) put(I.F1[1], e, Fv);
+    put(I.F1[0], c, F.u); put(I.F1[2], c, F.w);
+    if (hasv) put(I.F1[1], e, F.v);
   } else {
     un = axpy(dc1, d2(I.F1[0], c), un);
     wn = axpy(dc1, d2(I.F1[2], c), wn);
@@ -302,6 +409,28 @@ k_rhs_update(ChlMap map, RhsArgs a) {
   if (hasv) put(Vo, e, vn);
   if (jc == 1) { put(Uo, cidx(I, i, 0, k), neg(un)); put(Wo, cidx(I, i, 0, k), neg(wn)); }
   if (jc == Ny) { put(Uo, cidx(I, i, Ny + 1, k), neg(un)); put(Wo, cidx(I, i, Ny + 1, k), neg(wn)); }
+}
+// a call: its FP64 instructions would be predicated into every row
+static __device__ __noinline__ void update_pair_wall(const ChlInst& I, const RhsArgs& a, int i, int jc, int k) {
+  update_pair<true>(I, a, i, jc, k);
+}
+
+// The flux differences are exact integers; each is rounded once to a double
+// and multiplied by its reciprocal spacing there (with the products in
+// integers as well, F lost two to four bits to their common exponent).  One
+// thread per pair of x points: 16-byte loads, and the pair shares the fluxes
+// between its points.
+__global__ void __launch_bounds__(256, 4)
+k_rhs_update(ChlMap map, RhsArgs a) {
+  chl_pdl_wait();
+  int lb;
+  const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
+  const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
+  if (t >= (unsigned)(I.Nx / 2 * I.Ny * I.Nz)) return;
+  const ChlIdx p = chl_split(t, I.Nx / 2, I.Ny);
+  const int i = 2 * p.i, jc = 1 + p.j;
+  if (I.wall_model != 0 && (jc <= 2 || jc >= I.Ny - 1)) update_pair_wall(I, a, i, jc, p.k);
+  else update_pair<false>(I, a, i, jc, p.k);
 }
 
 extern "C" {

@@ -514,8 +514,9 @@ k_nut(ChlMap map, int use_wm) {
 // nu + nu_t on the wall-model rows, jc = 0, 1 and Ny, Ny+1: nu_t is the mean
 // of the face values at x faces i-1 and i, the same in both rows of a wall.
 // One thread per wall point; face i-1 comes from the lane to the left when
-// that lane is on the same row, so no thread returns before the shuffle.  A
-// kernel of its own, beside the model's (300 -> 283 us of k_amd and 166 -> 157
+// that lane is on the same row, so no thread returns before the shuffle.  The
+// values, which have no bound, stay out of the rows' largest (chl_rhs.cu:
+// wall_face).  A kernel of its own, beside the model's (300 -> 283 us of k_amd and 166 -> 157
 // of k_strain<false> at 256x96x192 where they did these rows, whose divisions
 // the whole block waits for).
 __global__ void __launch_bounds__(256)
@@ -534,12 +535,6 @@ k_wall_rows(ChlMap map, int s_in) {
   const double fl = ((threadIdx.x & 31) > 0 && i > 0) ? f_left : wm_face(I, U, wrap(i - 1, Nx), k, wall);
   const double v = I.nu + 0.5 * (fl + f);
   if (valid) I.nut[cidx(I, i, wall == 0 ? 0 : Ny, k)] = I.nut[cidx(I, i, wall == 0 ? 1 : Ny + 1, k)] = v;
-  const unsigned hi = valid ? chl_abshi(v) : 0u;
-  const unsigned m0 = __reduce_max_sync(0xffffffffu, wall == 0 ? hi : 0u), m1 = __reduce_max_sync(0xffffffffu, wall == 0 ? 0u : hi);
-  if ((threadIdx.x & 31) == 0) {
-    if (m0 > __ldcg(I.nmax + 1)) atomicMax(I.nmax + 1, m0);
-    if (m1 > __ldcg(I.nmax + Ny)) atomicMax(I.nmax + Ny, m1);
-  }
 }
 
 // ------------------------------------------------------------ launchers
