@@ -101,6 +101,11 @@ __host__ __device__ inline int chl_fft_threads(int lines, int n) {
   int t = (lines * n / 4 + 31) & ~31;
   return t < 64 ? 64 : (t > 256 ? 256 : t);
 }
+#define CHL_FLUX_THREADS 128   // block of the kernels that march (flux, strain, AMD)
+// blocks of k_flux for the walls' own fluxes: six rows of points (chl_rhs.cu)
+__host__ __device__ inline int chl_wall_flux_blocks(int Nx, int Nz) {
+  return (int)((6L * Nx * Nz + CHL_FLUX_THREADS - 1) / CHL_FLUX_THREADS);
+}
 // blocks of the mass-flow sum of an Nx x Nz plane (partials in red, 2 Nz long)
 #define CHL_MASS_POINTS 1024
 __host__ __device__ inline int chl_mass_blocks(int Nx, int Nz) {
@@ -154,6 +159,7 @@ struct ChlInst {
   const long long *fxhyl, *fxhyh; // h_y/dy of the y spacings below and above a centre row, 2^-62 (Vreman)
   const int *eyc, *eyf;
   int exc, exf, ezc, ezf;
+  int4 *vexp;                     // per row: exponents of the velocities that its fluxes take (chl_rhs.cu)
   int4 *upd;                      // per row, from the flux kernel to the update: exponents (chl_rhs.cu)
   unsigned *nmax, *smax;          // largest |nu + nu_t| and largest of the six |S| S_ij of every centre row (chl_fix.cuh)
   double *q[CHL_NQ], *r[CHL_NQ];  // DSM: filter inputs 3..14 and filtered fields 0..17 (chl_sgs.cu; products and r are integers)
@@ -277,7 +283,10 @@ struct ChlField1 {
 };
 struct ChlFields3 {
   ChlField1 f[3];
-  unsigned* vmax;   // where unpacking folds the largest |U|, |V|, |W| (zeroed before)
+  // where unpacking folds the largest |U|, |V|, |W| and those of every row
+  // (CHL_ROW_COPIES times three fields of `pitch` words); zeroed before
+  unsigned *vmax, *vrow;
+  int pitch;
 };
 
 struct ChlMap {
@@ -311,7 +320,6 @@ __device__ __forceinline__ int chl_find(const ChlMap& m, int b, int& local) {
 // unsigned arithmetic (an instance has fewer than 2^31 points, checked at
 // creation): the 64-bit divisions this replaces were long integer sequences
 // ahead of every kernel's first load.
-#define CHL_FLUX_THREADS 128   // block of the kernels that march (flux, strain, AMD)
 struct ChlIdx { int i, j, k; };
 __device__ __forceinline__ ChlIdx chl_split(unsigned t, unsigned Nx, unsigned rows) {
   const unsigned q = t / Nx, k = q / rows;
@@ -331,6 +339,10 @@ __device__ __forceinline__ int wrap(int i, int n) { return i < 0 ? i + n : (i >=
 // clears both at once.
 #define CHL_ST_VMAX0 1
 #define CHL_ST_VMAX12 5
+// behind the 16 words of the status area: the same of every row of the set written
+// last, CHL_ROW_COPIES times U, V, W with Ny + 2 words each (chl_fix.cuh)
+#define CHL_ROW_COPIES 8
+#define CHL_ST_ROWS 16
 
 // The bounds-checked build (-DCHL_BOUNDS_CHECK, build.build(variant="bounds"))
 // records an out-of-range index in the status word and clamps it, so the

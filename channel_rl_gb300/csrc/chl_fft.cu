@@ -282,7 +282,12 @@ k_div_fftx(ChlMap map, int s_in, int mode, int xmb) {
   for (int r = threadIdx.x; r < CR; r += blockDim.x) hi[r] = 0u;
   __syncthreads();
   const double *U, *V, *W;
-  if (mode == 0 && lb == 0 && threadIdx.x < 3) chl_vmax(I, s_in)[threadIdx.x] = 0u;
+  if (mode == 0) {
+    if (lb == 0 && threadIdx.x < 3) chl_vmax(I, s_in)[threadIdx.x] = 0u;
+    const int nb = (nrow + CR - 1) / CR;
+    for (int w = lb * (int)blockDim.x + threadIdx.x; w < 3 * CHL_ROW_COPIES * (Ny + 2); w += nb * (int)blockDim.x)
+      chl_row_copy(I, 0)[w] = 0u;
+  }
   if (mode != 1) { U = I.U[s_in]; V = I.V[s_in]; W = I.W[s_in]; }
   else { U = I.Fp[0]; V = I.Fp[1]; W = I.Fp[2]; }
   const SmallDiv byNx(Nx);
@@ -780,7 +785,7 @@ k_fftx_inv(ChlMap map, int dst, int xmb) {
 
 // ------------------------------------------------------------ velocity correction
 // project_velocity (projection.f90:192-214) + Dirichlet ghost rows; folds
-// the set's largest velocities (cleared by k_div_fftx) for its fixed-point copies.
+// the largest velocities of the set and its rows (cleared by k_div_fftx).
 // The FP64 pipe bounds it (6 instructions per point, 71 % busy), so two of a
 // pair's six differences are formed on the integer pipe: 60 -> 55 us at
 // 256x96x192 (one, two, three, four, six of them 57, 55, 55, 61, 64 us; HBM floor 39).
@@ -792,8 +797,8 @@ k_project(ChlMap map, int s) {
   const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
   unsigned hi[3] = {0u, 0u, 0u};
+  const ChlIdx ix = chl_split(t, Nx / 2, Ny);
   if (t < (unsigned)(Nx / 2 * Ny * Nz)) {     // pairs of points
-    const ChlIdx ix = chl_split(t, Nx / 2, Ny);
     const int i = 2 * ix.i, jc = 1 + ix.j, k = ix.k;
     const bool hasv = jc <= Ny - 1;
     auto at = [](const double* f, size_t c) { return *reinterpret_cast<const double2*>(f + c); };
@@ -820,7 +825,7 @@ k_project(ChlMap map, int s) {
     if (jc == 1) { put(U, cidx(I, i, 0, k), neg(un)); put(W, cidx(I, i, 0, k), neg(wn)); }
     if (jc == Ny) { put(U, cidx(I, i, Ny + 1, k), neg(un)); put(W, cidx(I, i, Ny + 1, k), neg(wn)); }
   }
-  chl_block_max(chl_vmax(I, s), hi);
+  chl_set_max(I, s, (unsigned)(ix.k * Ny + ix.j), 1 + ix.j, hi);
 }
 
 // ------------------------------------------------------------ actual pressure: wall BC planes

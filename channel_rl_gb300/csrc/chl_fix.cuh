@@ -10,7 +10,7 @@
 // double.  A field is scaled by its own largest magnitude (kept with the
 // velocity set, ChlInst::status), so that |F| < 2^61: eight bits finer than
 // a double's last bit at that magnitude, and exact for every double down to
-// 2^-8 of it.  Sums and differences are exact; a product keeps 60 bits or
+// 2^-8 of it (k_flux, whose rows differ by more, scales every row by its own).  Sums and differences are exact; a product keeps 60 bits or
 // more of its largest possible value.
 #pragma once
 #include "chl_common.cuh"
@@ -28,6 +28,9 @@ __device__ __forceinline__ int fx_exp(unsigned hi) {
 __device__ __forceinline__ int fx_line_exp(unsigned hi, int bits) { return max((int)(hi >> 20), 64) - 1022 - bits; }
 __device__ __forceinline__ bool fx_bad(unsigned hi) { return hi >= 0x7FF00000u; }
 
+// 2^e as a double, -1022 <= e <= 1023
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+
 // x as F 2^e, rounded toward zero
 __device__ __forceinline__ fx fx_from(double x, int e) {
   const long long b = __double_as_longlong(x);
@@ -37,6 +40,18 @@ __device__ __forceinline__ fx fx_from(double x, int e) {
   asm("shr.u64 %0, %1, %2;" : "=l"(f) : "l"(((unsigned long long)b << 11) | 0x8000000000000000ULL), "r"(r));
   return b < 0 ? -(fx)f : (fx)f;
 }
+
+// The same for |x| < 2^(61+e) on the FP64 pipe (one conversion; the scaling is an
+// addition to the exponent, clamped at zero so that zeros and tiny x stay below one
+// unit), for kernels that leave it idle.
+struct FxConv {
+  int d;
+  __device__ __forceinline__ explicit FxConv(int e) : d(-e * (1 << 20)) {}
+  __device__ __forceinline__ fx operator()(double x) const {
+    const int h = __double2hiint(x), a = max((int)((unsigned)(h & 0x7FFFFFFF) + (unsigned)d), 0);
+    return __double2ll_rz(__hiloint2double(a | (h & (int)0x80000000), __double2loint(x)));
+  }
+};
 
 // F 2^e as a double, rounded to nearest; exponents beyond a double's give its
 // smallest and largest magnitudes.  EXACT = false takes the magnitude of a
@@ -72,8 +87,6 @@ __device__ __forceinline__ double scale_exp(double x, int e) {
   return __hiloint2double(__double2hiint(x) + (e << 20), __double2loint(x));
 }
 
-// 2^e as a double, -1022 <= e <= 1023
-__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
 
 // (a b) >> 64, low by less than three units, for |a| < 2^62 and |b| < 2^63 (or
 // |a| < 2^63 and 0 <= b < 2^63):
@@ -96,37 +109,31 @@ __device__ __forceinline__ fx fx_mul_shr(fx a, fx b) {
   return (fx)((unsigned long long)((long long)ah * bh) << (64 - S)) + (t >> (S - 33));
 }
 
-// High words of the largest |U|, |V|, |W| of a velocity set, and of the
-// largest |nu + nu_t| of every centre row.  Written with the fields by every
-// kernel that leaves a velocity set behind (upload, projection, mass-flow
-// shift) or nu + nu_t.
+// High words of the largest |U|, |V|, |W| of a velocity set and of the largest
+// |nu + nu_t| of every centre row.  Written with the fields by every kernel that
+// leaves a velocity set behind (upload, projection, mass-flow shift) or nu + nu_t.
 __device__ __forceinline__ unsigned* chl_vmax(const ChlInst& I, int set) {
   return reinterpret_cast<unsigned*>(I.status) + (set == 0 ? CHL_ST_VMAX0 : CHL_ST_VMAX12 + 3 * (set - 1));
 }
+// The same of every row of the set that was written last (U and W: centre rows
+// 1..Ny, whose mirrors the ghost rows are; V: faces 0..Ny), [3][Ny + 2] words, of
+// which only the exponent counts.  The writers fold them into one of
+// CHL_ROW_COPIES arrays each, from which k_fix forms the rows' exponents: all warps
+// reading and raising the words of one array made k_project 55 -> 69 us at
+// 256x96x192.
+__device__ __forceinline__ unsigned* chl_row_copy(const ChlInst& I, int copy) {
+  return reinterpret_cast<unsigned*>(I.status) + CHL_ST_ROWS + copy * 3 * (I.Ny + 2);
+}
+// raises *g to x where x has the larger exponent
+__device__ __forceinline__ void chl_raise_exp(unsigned* g, unsigned x) {
+  if ((x >> 20) > (__ldcg(g) >> 20)) atomicMax(g, x);
+}
 __device__ __forceinline__ unsigned chl_abshi(double x) { return (unsigned)__double2hiint(x) & 0x7FFFFFFFu; }
 
-// Folds each thread's N values into g[0..N) (whole block; every thread
-// calls).  The global word is read first: only blocks that raise it issue an
-// atomic, or the tens of thousands of same-address atomics would take longer
-// than the kernels.
-template <int N>
-__device__ __forceinline__ void chl_block_max(unsigned* g, const unsigned (&v)[N]) {
-  __shared__ unsigned sm[N];
-  if (threadIdx.x < N) sm[threadIdx.x] = 0u;
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < N; ++q) {
-    const unsigned m = __reduce_max_sync(0xffffffffu, v[q]);
-    if ((threadIdx.x & 31) == 0) atomicMax(sm + q, m);
-  }
-  __syncthreads();
-  if (threadIdx.x < N && sm[threadIdx.x] > __ldcg(g + threadIdx.x)) atomicMax(g + threadIdx.x, sm[threadIdx.x]);
-}
-
+#define CHL_BLOCK_LINES 130
 // Folds each thread's v into g[off + j], j = q mod rows the row of its x-line
 // q = k rows + j (whole block, at most 256 threads; x-lines are numbered
 // upwards through the block and hold two threads or more).
-#define CHL_BLOCK_LINES 130
 __device__ __forceinline__ void chl_line_max(unsigned* g, unsigned q, int rows, int off, unsigned v) {
   __shared__ unsigned sm[CHL_BLOCK_LINES];
   __shared__ unsigned q0;
@@ -144,6 +151,47 @@ __device__ __forceinline__ void chl_line_max(unsigned* g, unsigned q, int rows, 
   for (unsigned w = threadIdx.x; w < CHL_BLOCK_LINES; w += blockDim.x) {
     unsigned* d = g + off + (q0 + w) % (unsigned)rows;
     if (sm[w] && sm[w] > __ldcg(d)) atomicMax(d, sm[w]);
+  }
+}
+
+// Folds the magnitudes of each thread's U, V, W (of U alone with N = 1) in row j
+// into the set's largest and the row's (whole block; x-line q).  The global words
+// are read first: only blocks, and warps for the rows, that raise one issue an
+// atomic, or the tens of thousands of same-address atomics would take longer than
+// the kernels.
+template <int N>
+__device__ __forceinline__ void chl_set_max(const ChlInst& I, int set, unsigned q, int j, const unsigned (&v)[N]) {
+  __shared__ unsigned sm[N][8], line[8], row[8];      // per warp
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const bool one = __all_sync(0xffffffffu, q == __shfl_sync(0xffffffffu, q, 0));     // the warp is in one x-line
+  unsigned mine = 0u;
+#pragma unroll
+  for (int c = 0; c < N; ++c) {
+    const unsigned x = __reduce_max_sync(0xffffffffu, v[c]);
+    if (lane == c) mine = x;
+  }
+  if (lane < N) sm[lane][warp] = mine;
+  if (lane == 0) { line[warp] = one ? q : 0xFFFFFFFFu; row[warp] = j; }
+  __syncthreads();
+  unsigned* rows = chl_row_copy(I, (int)(blockIdx.x % CHL_ROW_COPIES));
+  // thread (c, w): the warps from w on that share its x-line
+  if (threadIdx.x < 8 * N) {
+    const unsigned c = threadIdx.x >> 3, w = threadIdx.x & 7;
+    if (w < nw && line[w] != 0xFFFFFFFFu && (w == 0 || line[w - 1] != line[w])) {
+      unsigned x = sm[c][w];
+      for (unsigned k = w + 1; k < nw && line[k] == line[w]; ++k) x = max(x, sm[c][k]);
+      chl_raise_exp(rows + c * (I.Ny + 2) + row[w], x);
+    }
+    if (w == 7) {
+      unsigned x = sm[c][0];
+      for (unsigned k = 1; k < nw; ++k) x = max(x, sm[c][k]);
+      unsigned* all = chl_vmax(I, set) + c;
+      if (x > __ldcg(all)) atomicMax(all, x);
+    }
+  }
+  if (!one) {
+#pragma unroll
+    for (int c = 0; c < N; ++c) chl_raise_exp(rows + c * (I.Ny + 2) + j, v[c]);
   }
 }
 

@@ -399,7 +399,7 @@ static int upload_consts(chl_handle* h, Inst& I) {
   size_t o_w0 = A.take(8 * (Ny + 2)), o_w1 = A.take(8 * (Ny + 2)), o_ygc = A.take(8 * (Ny + 2));
   size_t o_fxrxc = A.take(8 * (Nx + 3)), o_fxryc = A.take(8 * (Ny + 2)), o_fxrzc = A.take(8 * (Nz + 3));
   size_t o_fxrxf = A.take(8 * (Nx + 3)), o_fxryf = A.take(8 * (Ny + 2)), o_fxrzf = A.take(8 * (Nz + 3));
-  size_t o_fxw1 = A.take(8 * (Ny + 2)), o_upd = A.take(16 * (Ny + 2));
+  size_t o_fxw1 = A.take(8 * (Ny + 2)), o_upd = A.take(16 * (Ny + 2)), o_vexp = A.take(16 * (Ny + 2));
   size_t o_eyc = A.take(4 * (Ny + 2)), o_eyf = A.take(4 * (Ny + 2)), o_nmax = A.take(4 * (Ny + 2)), o_smax = A.take(4 * (Ny + 2));
   size_t o_csd = A.take(8 * (Ny + 2)), o_dw = A.take(8 * (Ny + 2));
   size_t o_twx = A.take(16 * (size_t)chl_twf_len(Nx)), o_twz = A.take(16 * (size_t)chl_twf_len(Nz));
@@ -419,7 +419,7 @@ static int upload_consts(chl_handle* h, Inst& I) {
   size_t o_alpha = A.take(8 * 2 * (size_t)Nx * Nz), o_bc = A.take(8 * 2 * (size_t)Nx * Nz);
   size_t o_part = A.take(8 * 2 * (size_t)(Ny + 2) * npart * CHL_DSMF_THREADS);   // one partial per DSM thread
   size_t o_coef = A.take(8 * (Ny + 2)), o_scal = A.take(8 * CHL_S_NSCAL);
-  size_t o_min = A.take(8 * (size_t)(Nx + Ny + 1 + Nz)), o_status = A.take(64);
+  size_t o_min = A.take(8 * (size_t)(Nx + Ny + 1 + Nz)), o_status = A.take(4 * (CHL_ST_ROWS + 3 * CHL_ROW_COPIES * (size_t)(Ny + 2)));
   size_t o_dcnt = A.take(4 * (size_t)(Ny + 2));
   size_t o_red = A.take(8 * 2 * (size_t)Nz);
   size_t o_trace = A.take(4 * (size_t)MLP_NPARAM);
@@ -466,7 +466,7 @@ static int upload_consts(chl_handle* h, Inst& I) {
   auto L = [&](size_t o) { return (long long*)(base + o); };
   D.fxrxc = L(o_fxrxc) + 1; D.fxryc = L(o_fxryc); D.fxrzc = L(o_fxrzc) + 1;
   D.fxrxf = L(o_fxrxf) + 1; D.fxryf = L(o_fxryf); D.fxrzf = L(o_fxrzf) + 1;
-  D.fxw1 = L(o_fxw1); D.fxhyl = L(o_hyl); D.fxhyh = L(o_hyh); D.upd = (int4*)(base + o_upd);
+  D.fxw1 = L(o_fxw1); D.fxhyl = L(o_hyl); D.fxhyh = L(o_hyh); D.upd = (int4*)(base + o_upd); D.vexp = (int4*)(base + o_vexp);
   D.eyc = (const int*)(base + o_eyc); D.eyf = (const int*)(base + o_eyf); D.nmax = (unsigned*)(base + o_nmax);
   D.smax = (unsigned*)(base + o_smax);
   D.smag_csdelta = P(o_csd); D.smag_dwall = P(o_dw);
@@ -634,7 +634,12 @@ static int build_maps(chl_handle* h) {
         case M_PT2: b = cdiv((long)(Nx / 2) * Ny * Nz, h->tb_pt); break;         // pairs of x points (Nx even)
         case M_FULL2: b = cdiv((long)(Nx / 2) * (Ny + 2) * Nz, h->tb_pt); break;
         case M_FILTER: b = chl_filter_blocks(Nx, Ny, Nz, h->tb_filter, h->fplanes); break;
-        case M_FLUX: b = cdiv((long)Nx * (Ny + 1) * cdiv(Nz, h->planes), CHL_FLUX_THREADS); break;
+        case M_FLUX: {
+          const bool wm = h->wall_model != CHL_WM_NONE;
+          b = cdiv((long)Nx * (wm ? Ny - 2 : Ny + 1) * cdiv(Nz, h->planes), CHL_FLUX_THREADS);
+          if (wm) b += chl_wall_flux_blocks(Nx, Nz);
+          break;
+        }
         case M_MARCH: b = cdiv((long)Nx * Ny * cdiv(Nz, h->planes), CHL_FLUX_THREADS); break;
         case M_DSMF: b = Ny * dsm_npart(Nx, Ny, Nz); break;
         case M_WALL: b = cdiv(2L * Nx * Nz, 256); break;
@@ -744,7 +749,7 @@ static int enqueue_projection(chl_handle* h, int s, int mode) {
 }
 
 // The momentum RHS of velocity set 0 into Fp (chl_compute_rhs, the actual
-// pressure, the tuner); the set's fixed-point copies are in place.
+// pressure, the tuner); k_fix has run on it.
 static void enqueue_rhs_only(chl_handle* h) {
   chl_launch_flux(h->map(M_FLUX), h->nblk[M_FLUX], 0, h->st);
   chl_launch_update(h->map(M_PT2), h->nblk[M_PT2], 0, 0, 0, 2, h->st);
@@ -991,7 +996,15 @@ static ChlFields3 fields3(Inst* I, bool out = false) {
   f.f[1] = ChlField1{s + n, I->dev.V[0], c.nxg, c.ny, c.nzg, c.Ny + 1, 1};
   f.f[2] = ChlField1{s + 2 * n, I->dev.W[0], c.nxg, c.nyg, c.nz, c.Ny + 2, 0};
   f.vmax = (unsigned*)I->dev.status + CHL_ST_VMAX0;
+  f.vrow = (unsigned*)I->dev.status + CHL_ST_ROWS;
+  f.pitch = c.Ny + 2;
   return f;
+}
+
+// Status word, set 0's maxima and the rows'.  The counter and the other sets' maxima between
+// them are zero or formed anew before their next use.
+static cudaError_t clear_set0(chl_handle* h, Inst* I) {
+  return cudaMemsetAsync(I->dev.status, 0, sizeof(int) * (CHL_ST_ROWS + 3 * CHL_ROW_COPIES * (size_t)(I->c.Ny + 2)), h->st);
 }
 
 int chl_upload(chl_handle* h, int inst, const double* U, const double* V, const double* W) {
@@ -1005,7 +1018,7 @@ int chl_upload(chl_handle* h, int inst, const double* U, const double* V, const 
     const ChlField1& d = f3.f[q];
     CK(cudaMemcpyAsync(d.fort, src[q], 8 * (size_t)d.n1 * d.n2 * d.n3, cudaMemcpyHostToDevice, h->st));
   }
-  CK(cudaMemsetAsync(I->dev.status, 0, sizeof(int) * (CHL_ST_VMAX0 + 3), h->st));   // status word, set 0's maxima
+  CK(clear_set0(h, I));
   chl_launch_unpack3(f3, I->c.Nx, I->c.Nz, h->st);
   LAUNCHED();
   const int Nz = I->c.Nz;
@@ -1563,7 +1576,7 @@ int chl_set_fields(chl_handle* h, int inst, const double* U, const double* V, co
   }
   CK(cudaEventRecord(I->ev_h2d, h->st_h2d));
   CK(cudaStreamWaitEvent(h->st, I->ev_h2d, 0));
-  CK(cudaMemsetAsync(I->dev.status, 0, sizeof(int) * (CHL_ST_VMAX0 + 3), h->st));   // status word, set 0's maxima
+  CK(clear_set0(h, I));
   chl_launch_unpack3(f3, I->c.Nx, I->c.Nz, h->st);
   LAUNCHED();
   CK(cudaEventRecord(I->ev_unpacked, h->st));

@@ -36,26 +36,29 @@ __global__ void k_pack(double* __restrict__ F, const double* __restrict__ src, i
 #define CHL_CONV_ROWS 4
 #define CHL_CONV_LANES 64
 #define CHL_CONV_BLOCK_ROWS (4 * CHL_CONV_ROWS)
-// Unpacking also folds the field's largest magnitude into f3.vmax.
+// Unpacking also folds the largest magnitudes of the field and its rows.
 __global__ void __launch_bounds__(CHL_CONV_ROWS * CHL_CONV_LANES)
 k_unpack3(ChlFields3 f3, int Nx, int Nz) {
   const ChlField1& q = f3.f[blockIdx.y];
   const int nrow = q.nrow, last = nrow - 1, rows = nrow * Nz;
   const int r0 = blockIdx.x * CHL_CONV_BLOCK_ROWS + threadIdx.y;      // rows (j, k) of the device field
-  // per row: its source (none: zero), and whether it is a ghost, minus the row next to it
+  // per row: its source (none: zero), whether it is a ghost, minus the row next to
+  // it, and its number
   const double* src[4];
   bool neg[4];
+  int row[4];
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
     const int r = r0 + m * CHL_CONV_ROWS, k = r / nrow, j = r - k * nrow;
     const bool ghost = q.kind == 0 && (j == 0 || j == last);
     const int js = ghost ? (j == 0 ? 1 : last - 1) : j;
     neg[m] = ghost;
+    row[m] = js;
     src[m] = r < rows && !(q.kind == 1 && (j == 0 || j == last))
                  ? q.fort + 1 + (size_t)q.n1 * ((size_t)js + (size_t)q.n2 * (size_t)(k + 1)) : nullptr;
   }
   double* dst = q.dev + (size_t)Nx * r0;
-  unsigned hi = 0u;
+  unsigned hi[4] = {0u, 0u, 0u, 0u};
   for (int i = threadIdx.x; i < Nx; i += CHL_CONV_LANES) {
     double v[4];
 #pragma unroll
@@ -63,15 +66,22 @@ k_unpack3(ChlFields3 f3, int Nx, int Nz) {
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
       if (r0 + m * CHL_CONV_ROWS < rows) dst[(size_t)m * CHL_CONV_ROWS * Nx + i] = neg[m] ? chl_neg(v[m]) : v[m];
-      hi = max(hi, chl_abshi(v[m]));
+      hi[m] = max(hi[m], chl_abshi(v[m]));
     }
+  }
+  unsigned all = 0u;      // a warp has one lane of threadIdx.y
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const unsigned w = __reduce_max_sync(0xffffffffu, hi[m]);
+    unsigned* g = f3.vrow + (3 * (blockIdx.x % CHL_ROW_COPIES) + blockIdx.y) * f3.pitch + row[m];
+    if ((threadIdx.x & 31) == 0 && r0 + m * CHL_CONV_ROWS < rows) chl_raise_exp(g, w);
+    all = max(all, w);
   }
   __shared__ unsigned sm;
   const bool first = threadIdx.x == 0 && threadIdx.y == 0;
   if (first) sm = 0u;
   __syncthreads();
-  hi = __reduce_max_sync(0xffffffffu, hi);
-  if ((threadIdx.x & 31) == 0) atomicMax(&sm, hi);
+  if ((threadIdx.x & 31) == 0) atomicMax(&sm, all);
   __syncthreads();
   if (first && sm > __ldcg(f3.vmax + blockIdx.y)) atomicMax(f3.vmax + blockIdx.y, sm);
 }
@@ -365,10 +375,12 @@ k_massflow(ChlMap map, int s, int force) {
     sum = block_sum256(acc, red);
     if (threadIdx.x == 0) I.dsm_cnt[0] = 0;
   }
+  if (!force)        // k_shift forms the largest |U| anew
+    for (int w = threadIdx.x; w < CHL_ROW_COPIES * (Ny + 2); w += 256) chl_row_copy(I, w / (Ny + 2))[w % (Ny + 2)] = 0u;
   if (threadIdx.x == 0) {
     const double d = I.scal[CHL_S_Q0] - sum / (double)(Nx * Nz);
     I.scal[CHL_S_SHIFT] = d;
-    if (!force) chl_vmax(I, s)[0] = 0u;     // k_shift forms the largest |U| anew
+    if (!force) chl_vmax(I, s)[0] = 0u;
     if (!force) I.scal[CHL_S_DPDX] = 0.0;   // dPdx = 0 after the shift (time_integration.f90:92)
   }
 }
@@ -394,8 +406,8 @@ k_shift(ChlMap map, int s) {
   }
   if (!I.x_mass_cte) return;
   unsigned hi[1] = {0u};
+  const ChlIdx p = chl_split(t, Nx / 2, Ny);
   if (t < (unsigned)(Nx / 2 * Ny * Nz)) {     // pairs of points
-    const ChlIdx p = chl_split(t, Nx / 2, Ny);
     const int i = 2 * p.i, jc = 1 + p.j, k = p.k;
     auto U = [&](int j) -> double2& { return *reinterpret_cast<double2*>(I.U[s] + cidx(I, i, j, k)); };
     const double d = I.scal[CHL_S_SHIFT];
@@ -406,7 +418,7 @@ k_shift(ChlMap map, int s) {
     if (jc == Ny) U(Ny + 1) = make_double2(chl_neg(u.x), chl_neg(u.y));
     hi[0] = max(chl_abshi(u.x), chl_abshi(u.y));
   }
-  chl_block_max(chl_vmax(I, s), hi);
+  chl_set_max(I, s, (unsigned)(p.k * Ny + p.j), 1 + p.j, hi);
 }
 
 // time advance t += dt (compute_time_step_RK3 leaves t = to + rk_t(3)*dt)

@@ -21,10 +21,9 @@
 //
 // Both kernels work in 64-bit fixed point (chl_fix.cuh): as FP64 code they
 // were bound by the FP64 pipe (52 and 24 instructions per point, 457 and 201
-// us per launch at 256x96x192; 172 and 147 now).  The velocities come as the fixed-point
-// copies k_fix made of the stage's input, the fluxes are kept as integers,
-// and only the three components of F and the two FMAs of the stage update
-// are FP64.  Halves and quarters of the averages are exponents.  The y-face
+// us per launch at 256x96x192; 192 and 135 now).  The velocities are scaled by
+// their rows' largest, the fluxes are kept as integers, and only the three
+// components of F and the two FMAs of the stage update are FP64.  Halves and quarters of the averages are exponents.  The y-face
 // value of u (and w) is u_a + w1 (u_b - u_a).
 #include "chl_fix.cuh"
 
@@ -32,21 +31,36 @@
 // V-like (rows 0..Ny): 5 GUy, 6 GVx, 7 GVz, 8 GWy
 enum { G_UX = 0, G_VY, G_WZ, G_UZ, G_WX, G_UY, G_VX, G_VZ, G_WY };
 
-// Exponents of the fluxes of row j (y-face j and centre row j), from the
-// largest |U|, |V|, |W| of the launch's input and the largest |nu + nu_t| of
-// the row and the one above.  Flux m = viscous - advective part: the
+// Exponents of the velocities that the fluxes of y-face j and centre row j take
+// (U and W of rows j and j + 1, V of faces j - 1 and j), from those rows' largest.
+// Next to a resolved wall V is a millionth of its largest and less, U a hundredth:
+// in units of the field's largest the rows there had up to 35 roundings of error
+// (FP64 and this 3), and more the stronger the grid is stretched.  x, y, z are the
+// exponents, w whether a velocity is not finite; left in vexp by k_fix.
+__device__ __forceinline__ int4 vel_exp(const ChlInst& I, int j) {
+  unsigned u = 0u, v = 0u, w = 0u;
+  const int a = max(j, 1), b = min(j + 1, I.Ny), n = I.Ny + 2;
+#pragma unroll
+  for (int c = 0; c < CHL_ROW_COPIES; ++c) {
+    const unsigned* r = chl_row_copy(I, c);
+    u = max(u, max(__ldcg(r + a), __ldcg(r + b)));
+    v = max(v, max(__ldcg(r + n + max(j - 1, 0)), __ldcg(r + n + j)));
+    w = max(w, max(__ldcg(r + 2 * n + a), __ldcg(r + 2 * n + b)));
+  }
+  return make_int4(fx_exp<61>(u), fx_exp<61>(v), fx_exp<61>(w), fx_bad(u) || fx_bad(v) || fx_bad(w));
+}
+
+// Exponents of the fluxes of row j, from those of its velocities and the largest
+// |nu + nu_t| of the row and the one above.  Flux m = viscous - advective part: the
 // advective product has last bit 2^adv[m], the viscous one 2^vis[m]; the
 // fluxes of one momentum component are stored with last bit 2^G, one above
-// the largest, so that |flux| < 2^62.  Rows have their own exponents because
-// the y spacing and nu + nu_t differ by orders of magnitude between the wall
-// and the core.
+// the largest, so that |flux| < 2^62.
 __device__ constexpr int FLUX_A[9] = {0, 1, 2, 0, 2, 0, 1, 1, 2};   // momentum component
 __device__ constexpr int FLUX_B[9] = {0, 1, 2, 2, 0, 1, 0, 2, 1};   // direction
 struct RowExp { int adv[9], vis[9], G[3], n; bool bad; };
-__device__ __forceinline__ RowExp row_exp(const ChlInst& I, int sin, int j) {
-  const unsigned* vm = chl_vmax(I, sin);
+__device__ __forceinline__ RowExp row_exp(const ChlInst& I, int4 x, int j) {
   const unsigned nm = max(I.nmax[j], I.nmax[j + 1]);
-  const int ev[3] = {fx_exp<61>(vm[0]), fx_exp<61>(vm[1]), fx_exp<61>(vm[2])};
+  const int ev[3] = {x.x, x.y, x.z};
   const int ef[3] = {I.exf, I.eyf[j], I.ezf}, ec[3] = {I.exc, I.eyc[j], I.ezc};
   RowExp q;
   q.n = fx_exp<60>(nm);
@@ -60,7 +74,7 @@ __device__ __forceinline__ RowExp row_exp(const ChlInst& I, int sin, int j) {
     q.vis[m] = q.n + ev[a] + (m <= G_WZ ? ec[b] + 125 : m <= G_WX ? ef[b] + 123 : ef[b] + 124);
     q.G[a] = max(q.G[a], max(q.adv[m], q.vis[m]) + 1);
   }
-  q.bad = fx_bad(vm[0]) || fx_bad(vm[1]) || fx_bad(vm[2]) || fx_bad(nm);
+  q.bad = x.w || fx_bad(nm);
   return q;
 }
 
@@ -77,7 +91,8 @@ static __device__ __noinline__ double smag_coef(const ChlInst& I, int jc) {
 // Fixed-point copies of the velocity set that a stage works on (rows as
 // stored, ghosts included).  prep: 1 clears the rows' largest |nu + nu_t|
 // and |S| S_ij ahead of the kernels that form them, + 2 forms the static
-// model's row coefficients.  Moves 48 bytes per point: HBM-bound.
+// model's row coefficients.  Also forms the exponents of the rows' velocities for
+// k_flux, from what the set's writer folded.  Moves 48 bytes per point: HBM-bound.
 __global__ void __launch_bounds__(256)
 k_fix(ChlMap map, int s, int prep) {
   chl_pdl_wait();
@@ -99,6 +114,7 @@ k_fix(ChlMap map, int s, int prep) {
   if (t < nv) v = get(I.V[s]);
   if (t < nc) { put(I.X[0], u, eu); put(I.X[2], w, ew); }
   if (t < nv) put(I.X[1], v, ev);
+  if (t <= (unsigned)I.Ny) I.vexp[t] = vel_exp(I, t);
 }
 
 // Fluxes next to a wall whose nu + nu_t the wall model sets (y-faces 0, 1 and
@@ -123,71 +139,66 @@ struct Norm {
   }
 };
 
-// These fluxes of column i, planes k0..k1-1: of y-face jf (on a wall only those
-// that a row takes) and of centre row jc (0: none).  A call, for the registers.
-// The averages of nu + nu_t are its only FP64 instructions, 13 per point (52 with
-// the fluxes in FP64 as well, which cost the 128x40x64 channel 6 % of a step).
-static __device__ __noinline__ void flux_wall(const ChlInst& I, int sin, int i, int jf, int jc, int k0, int k1) {
-  const int Nx = I.Nx, Nz = I.Nz, ip = wrap(i + 1, Nx), im = wrap(i - 1, Nx);
-  const unsigned* vm = chl_vmax(I, sin);
-  const int eu = fx_exp<61>(vm[0]), ev = fx_exp<61>(vm[1]), ew = fx_exp<61>(vm[2]);
-  const bool bad = fx_bad(vm[0]) || fx_bad(vm[1]) || fx_bad(vm[2]), wall = jf == 0 || jf == I.Ny;
-  auto u = [&](int a, int b, int k) { return LDG(I.X[0] + cidx(I, a, b, k)); };
-  auto v = [&](int a, int b, int k) { return LDG(I.X[1] + vidx(I, a, b, k)); };
-  auto w = [&](int a, int b, int k) { return LDG(I.X[2] + cidx(I, a, b, k)); };
-  auto n = [&](int a, int b, int k) { return LDG(I.nut + cidx(I, a, b, k)); };
+// One of these: of y-face j (of a wall's only those that a row takes) or of centre
+// row j at (i, k).  The averages of nu + nu_t are its only FP64 instructions, 4 and 3
+// per point (in FP64 throughout, 28 and 24, they cost the 128x40x64 channel 6 % of a
+// step).  A call, for the registers.
+static __device__ __noinline__ void flux_wall(const ChlInst& I, int sin, int i, int j, int k, bool centre) {
+  const int Nx = I.Nx, Nz = I.Nz, ip = wrap(i + 1, Nx), kp = wrap(k + 1, Nz);
+  const int4 x = LDG(I.vexp + j);
+  const int eu = x.x, ev = x.y, ew = x.z;
+  auto u = [&](int a, int b, int kk) { return fx_from(LDG(I.U[sin] + cidx(I, a, b, kk)), eu); };
+  auto v = [&](int a, int b, int kk) { return fx_from(LDG(I.V[sin] + vidx(I, a, b, kk)), ev); };
+  auto w = [&](int a, int b, int kk) { return fx_from(LDG(I.W[sin] + cidx(I, a, b, kk)), ew); };
+  auto n = [&](int a, int b, int kk) { return LDG(I.nut + cidx(I, a, b, kk)); };
   // viscous less advective part: vis 2^ev less adv 2^ea
   auto put = [&](int m, size_t q, fx adv, int ea, const Norm& nu, fx grad, int ev) {
     ev += nu.e;
     const int g = max(ea, ev) + 1;
     const double f = fx_to((fx_mul_shr<61>(nu.m, grad) >> min(63, g - ev)) - (adv >> min(63, g - ea)), g);
-    reinterpret_cast<double*>(I.G[m])[q] = bad || nu.bad ? __longlong_as_double(0x7FF8000000000000LL) : f;
+    reinterpret_cast<double*>(I.G[m])[q] = x.w || nu.bad ? __longlong_as_double(0x7FF8000000000000LL) : f;
   };
-  const fx rxf = LDG(I.fxrxf + i);
-#pragma unroll 1
-  for (int k = k0; k < k1; ++k) {
-    const int kp = wrap(k + 1, Nz);
-    const fx rzf = LDG(I.fxrzf + k);
-    {
-      const int j = jf, jp = j + 1, eyf = I.eyf[j];
-      const fx ryf = LDG(I.fxryf + j), w1 = LDG(I.fxw1 + j);
-      const double w0x2 = LDG(I.w0x2 + j), w1x2 = LDG(I.w1x2 + j);
-      const fx ua = u(i, j, k), du = u(i, jp, k) - ua, wa = w(i, j, k), dw = w(i, jp, k) - wa;
-      const fx v0 = v(i, j, k), vz = v(i, j, kp), vp = v(ip, j, k);
-      const double na = n(i, j, k), nb = n(i, jp, k);
-      const size_t e = vidx(I, i, j, k);
-      // yz edge: 2 v w, 4 nu; xy edge: 2 u v, 4 nu
-      const fx vw = fx_mul_shr<62>(wa + 2 * fx_mul(dw, w1), v0 + vz), uv = fx_mul_shr<62>(ua + 2 * fx_mul(du, w1), v0 + vp);
-      const Norm nyz(fma(w0x2, na + n(i, j, kp), w1x2 * (nb + n(i, jp, kp))));
-      const Norm nxy(fma(w0x2, na + n(ip, j, k), w1x2 * (nb + n(ip, jp, k))));
-      put(G_WY, e, vw, ev + ew + 61, nyz, fx_mul(dw, ryf), ew + eyf + 123);
-      put(G_UY, e, uv, eu + ev + 61, nxy, fx_mul(du, ryf), eu + eyf + 123);
-      if (!wall) {
-        put(G_VZ, e, vw, ev + ew + 61, nyz, fx_mul(vz - v0, rzf), ev + I.ezf + 123);
-        put(G_VX, e, uv, eu + ev + 61, nxy, fx_mul(vp - v0, rxf), ev + I.exf + 123);
-      }
+  const fx rxf = LDG(I.fxrxf + i), rzf = LDG(I.fxrzf + k);
+  const fx ua = u(i, j, k), wa = w(i, j, k), v0 = v(i, j, k);
+  const double na = n(i, j, k), nx = n(ip, j, k), nz = n(i, j, kp);
+  if (!centre) {
+    const int jp = j + 1, eyf = I.eyf[j];
+    const fx ryf = LDG(I.fxryf + j), w1 = LDG(I.fxw1 + j);
+    const double w0x2 = LDG(I.w0x2 + j), w1x2 = LDG(I.w1x2 + j);
+    const fx du = u(i, jp, k) - ua, dw = w(i, jp, k) - wa, vz = v(i, j, kp), vp = v(ip, j, k);
+    const double nb = n(i, jp, k);
+    const size_t e = vidx(I, i, j, k);
+    // yz edge: 2 v w, 4 nu; xy edge: 2 u v, 4 nu
+    const fx vw = fx_mul_shr<62>(wa + 2 * fx_mul(dw, w1), v0 + vz), uv = fx_mul_shr<62>(ua + 2 * fx_mul(du, w1), v0 + vp);
+    const Norm nyz(fma(w0x2, na + nz, w1x2 * (nb + n(i, jp, kp))));
+    const Norm nxy(fma(w0x2, na + nx, w1x2 * (nb + n(ip, jp, k))));
+    put(G_WY, e, vw, ev + ew + 61, nyz, fx_mul(dw, ryf), ew + eyf + 123);
+    put(G_UY, e, uv, eu + ev + 61, nxy, fx_mul(du, ryf), eu + eyf + 123);
+    if (j != 0 && j != I.Ny) {
+      put(G_VZ, e, vw, ev + ew + 61, nyz, fx_mul(vz - v0, rzf), ev + I.ezf + 123);
+      put(G_VX, e, uv, eu + ev + 61, nxy, fx_mul(vp - v0, rxf), ev + I.exf + 123);
     }
-    if (jc == 0) continue;
-    const int j = jc;
-    const size_t c = cidx(I, i, j, k);
-    const fx ua = u(i, j, k), wa = w(i, j, k), v0 = v(i, j, k);
-    const fx um = u(im, j, k), vm_ = v(i, j - 1, k), wm = w(i, j, wrap(k - 1, Nz)), su = um + ua, sv = vm_ + v0, sw = wm + wa;
-    const fx uz = u(i, j, kp), wp = w(ip, j, k), uw = fx_mul_shr<62>(ua + uz, wa + wp);
-    const double na = n(i, j, k);
-    // xz edge: 4 u w, 4 nu; cell centre: u u with both halves in the exponent, nu
-    const Norm nxz((na + n(ip, j, k)) + (n(i, j, kp) + n(ip, j, kp))), nu(na);
-    put(G_UX, c, fx_mul_shr<62>(su, su), 2 * eu + 60, nu, fx_mul(ua - um, LDG(I.fxrxc + i)), eu + I.exc + 125);
-    put(G_VY, c, fx_mul_shr<62>(sv, sv), 2 * ev + 60, nu, fx_mul(v0 - vm_, LDG(I.fxryc + j)), ev + I.eyc[j] + 125);
-    put(G_WZ, c, fx_mul_shr<62>(sw, sw), 2 * ew + 60, nu, fx_mul(wa - wm, LDG(I.fxrzc + k)), ew + I.ezc + 125);
-    put(G_UZ, c, uw, eu + ew + 60, nxz, fx_mul(uz - ua, rzf), eu + I.ezf + 123);
-    put(G_WX, c, uw, eu + ew + 60, nxz, fx_mul(wp - wa, rxf), ew + I.exf + 123);
+    return;
   }
+  const size_t c = cidx(I, i, j, k);
+  const fx um = u(wrap(i - 1, Nx), j, k), vm = v(i, j - 1, k), wm = w(i, j, wrap(k - 1, Nz));
+  const fx su = um + ua, sv = vm + v0, sw = wm + wa;
+  const fx uz = u(i, j, kp), wp = w(ip, j, k), uw = fx_mul_shr<62>(ua + uz, wa + wp);
+  // xz edge: 4 u w, 4 nu; cell centre: u u with both halves in the exponent, nu
+  const Norm nxz((na + nx) + (nz + n(ip, j, kp))), nu(na);
+  put(G_UX, c, fx_mul_shr<62>(su, su), 2 * eu + 60, nu, fx_mul(ua - um, LDG(I.fxrxc + i)), eu + I.exc + 125);
+  put(G_VY, c, fx_mul_shr<62>(sv, sv), 2 * ev + 60, nu, fx_mul(v0 - vm, LDG(I.fxryc + j)), ev + I.eyc[j] + 125);
+  put(G_WZ, c, fx_mul_shr<62>(sw, sw), 2 * ew + 60, nu, fx_mul(wa - wm, LDG(I.fxrzc + k)), ew + I.ezc + 125);
+  put(G_UZ, c, uw, eu + ew + 60, nxz, fx_mul(uz - ua, rzf), eu + I.ezf + 123);
+  put(G_WX, c, uw, eu + ew + 60, nxz, fx_mul(wp - wa, rxf), ew + I.exf + 123);
 }
 
-// 28 products and 4 conversions of nu + nu_t per point on the integer pipe,
-// no FP64 instruction; 104 bytes per point.  A thread marches through
-// a few planes at its (i, j), so that what the next plane shares (U, V,
-// nu + nu_t one plane up, W one down) is loaded and converted once.
+// 28 products and 4 conversions of nu + nu_t per point on the integer pipe, 9
+// conversions of velocities: 7 on the FP64 pipe, which nothing else here uses, 2 on
+// the integer pipe (9 and 0, 8 and 1, 4 and 5, 0 and 9: 2 to 4 % more); 104 bytes
+// per point.  A thread marches through a few planes at its (i, j), so that what
+// the next plane shares (U, V, nu + nu_t one plane up, W one down) is loaded and
+// converted once.
 __global__ void __launch_bounds__(CHL_FLUX_THREADS, 6)
 k_flux(ChlMap map, int sin) {
   chl_pdl_wait();
@@ -195,39 +206,46 @@ k_flux(ChlMap map, int sin) {
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
   const int Nx = I.Nx, Ny = I.Ny, Nz = I.Nz;
   const int M = map.planes;
-  const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  const ChlIdx p = chl_split(t, Nx, Ny + 1);
-  const int i = p.i, j = p.j, k0 = p.k * M, k1 = min(Nz, k0 + M);
-  const fx* __restrict__ U = I.X[0];
-  const fx* __restrict__ V = I.X[1];
-  const fx* __restrict__ W = I.X[2];
+  // with a wall model the first blocks form the walls' own fluxes, a point each,
+  // and the others leave out rows 0, 1 and Ny
+  const bool wm = I.wall_model != 0;
+  const int nw = wm ? chl_wall_flux_blocks(Nx, Nz) : 0;
+  if (lb < nw) {
+    const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
+    if (t >= (unsigned)(6 * Nx * Nz)) return;
+    const ChlIdx p = chl_split(t, Nx, 6);       // centre rows 1, Ny; y-faces 1, Ny-1, 0, Ny
+    flux_wall(I, sin, p.i, p.j == 4 ? 0 : ((p.j & 1) == 0 ? 1 : (p.j == 3 ? Ny - 1 : Ny)), p.k, p.j < 2);
+    return;
+  }
+  const unsigned t = (unsigned)(lb - nw) * blockDim.x + threadIdx.x;
+  const ChlIdx p = chl_split(t, Nx, wm ? Ny - 2 : Ny + 1);
+  const int i = p.i, j = p.j + (wm ? 2 : 0), k0 = p.k * M, k1 = min(Nz, k0 + M);
+  const double* __restrict__ U = I.U[sin];
+  const double* __restrict__ V = I.V[sin];
+  const double* __restrict__ W = I.W[sin];
   const double* __restrict__ nt = I.nut;   // nu + nu_t
   const bool valid = k0 < Nz;
+  const int4 x = LDG(I.vexp + j);
   const fx w1 = LDG(I.fxw1 + j), rxf = LDG(I.fxrxf + i), ryf = LDG(I.fxryf + j);
   const fx rxc = LDG(I.fxrxc + i), ryc = LDG(I.fxryc + j);
   const int ip = wrap(i + 1, Nx), im = wrap(i - 1, Nx);
   const int jp = min(j + 1, Ny + 1), jm = max(j - 1, 0);
-  fx u_a = 0, v_0 = 0, w_m = 0;
+  double u_a0 = 0.0, v_00 = 0.0, w_m0 = 0.0;
   double dn_a = 0.0, dn_b = 0.0, dn_p = 0.0;
   if (valid) {
-    u_a = LDG(U + cidx(I, i, j, k0));
-    v_0 = LDG(V + vidx(I, i, j, k0));
-    w_m = LDG(W + cidx(I, i, j, k0 == 0 ? Nz - 1 : k0 - 1));
+    u_a0 = LDG(U + cidx(I, i, j, k0));
+    v_00 = LDG(V + vidx(I, i, j, k0));
+    w_m0 = LDG(W + cidx(I, i, j, k0 == 0 ? Nz - 1 : k0 - 1));
     dn_a = LDG(nt + cidx(I, i, j, k0)); dn_b = LDG(nt + cidx(I, i, jp, k0)); dn_p = LDG(nt + cidx(I, ip, j, k0));
   }
   if (!valid) return;
-  // the wall model's rows: the threads of row 0 take both walls' faces, those of
-  // rows 1 and Ny a face and a centre row each, those of Ny-1 its centre row below
-  const bool own = wall_face(I, j);
-  if (own && j != Ny - 1) {
-    if (j == 0) { flux_wall(I, sin, i, 0, 0, k0, k1); flux_wall(I, sin, i, Ny, 0, k0, k1); }
-    else flux_wall(I, sin, i, j == 1 ? 1 : Ny - 1, j, k0, k1);
-    return;
-  }
+  const bool own = wm && j == Ny - 1;        // the face above this centre row is the wall's
+  const FxConv cu(x.x), cv(x.y), cw(x.z);
+  fx u_a = cu(u_a0), v_0 = cv(v_00), w_m = cw(w_m0);
   int sa[9], sv_[9];          // right shifts of the advective and viscous parts
   int en;
   {
-    const RowExp q = row_exp(I, sin, j);
+    const RowExp q = row_exp(I, x, j);
     en = q.n;
 #pragma unroll
     for (int m = 0; m < 9; ++m) {
@@ -244,9 +262,9 @@ k_flux(ChlMap map, int sin) {
   for (int k = k0; k < k1; ++k) {
     const int kp = k + 1 == Nz ? 0 : k + 1;
     const size_t c = cidx(I, i, j, k), e = vidx(I, i, j, k);
-    const fx u_b = LDG(U + cidx(I, i, jp, k)), w_b = LDG(W + cidx(I, i, jp, k));
-    const fx w_a = LDG(W + c);
-    const fx u_z = LDG(U + cidx(I, i, j, kp)), v_z = LDG(V + vidx(I, i, j, kp)), v_p = LDG(V + vidx(I, ip, j, k));
+    const fx u_b = cu(LDG(U + cidx(I, i, jp, k))), w_b = cw(LDG(W + cidx(I, i, jp, k)));
+    const fx w_a = cw(LDG(W + c));
+    const fx u_z = fx_from(LDG(U + cidx(I, i, j, kp)), x.x), v_z = cv(LDG(V + vidx(I, i, j, kp))), v_p = cv(LDG(V + vidx(I, ip, j, k)));
     const fx n_az = fx_from(LDG(nt + cidx(I, i, j, kp)), en), n_bz = fx_from(LDG(nt + cidx(I, i, jp, kp)), en);
     const fx n_pz = fx_from(LDG(nt + cidx(I, ip, j, kp)), en), n_bp = fx_from(LDG(nt + cidx(I, ip, jp, k)), en);
     const fx rzf = LDG(I.fxrzf + k);
@@ -268,14 +286,14 @@ k_flux(ChlMap map, int sin) {
     }
     if (j >= 1) {
       {  // cell centre: diagonal fluxes
-        const fx u_m = LDG(U + cidx(I, im, j, k)), v_m = LDG(V + vidx(I, i, jm, k));
+        const fx u_m = cu(LDG(U + cidx(I, im, j, k))), v_m = fx_from(LDG(V + vidx(I, i, jm, k)), x.y);
         const fx su = u_m + u_a, sv = v_m + v_0, sw = w_m + w_a;
         PUT(G_UX, c, ADV(su, su), VIS(n_a, MUL(u_a - u_m, rxc)));
         PUT(G_VY, c, ADV(sv, sv), VIS(n_a, MUL(v_0 - v_m, ryc)));
         PUT(G_WZ, c, ADV(sw, sw), VIS(n_a, MUL(w_a - w_m, LDG(I.fxrzc + k))));
       }
       {  // xz edge (x-face i, y-centre jc, z-face k): uw, nu -> GUz, GWx
-        const fx w_p = LDG(W + cidx(I, ip, j, k));
+        const fx w_p = cw(LDG(W + cidx(I, ip, j, k)));
         const fx uw = ADV(u_a + u_z, w_a + w_p);                                      // 4 u w
         const fx nxz = nx_a + (n_az + n_pz);                                          // 4 nu
         PUT(G_UZ, c, uw, VIS(nxz, MUL(u_z - u_a, rzf)));
@@ -325,9 +343,11 @@ __device__ __forceinline__ Rhs rhs_pair(const ChlInst& I, int i, int jc, int k) 
   // stored as doubles: y-faces jc - 1 and jc, centre rows jc and jc + 1
   const bool dl = WALL && wall_face(I, jc - 1), dh = WALL && wall_face(I, jc), dc = WALL && wall_centre(I, jc);
   const bool dn = WALL && wall_centre(I, jc + 1);
-  // difference of two fluxes of one row, and of two rows
-  auto diff = [](fx hi, fx lo, bool d, int x) {
-    return WALL && d ? __longlong_as_double(hi) - __longlong_as_double(lo) : fx_to<true>(hi - lo, x);
+  // difference of two fluxes of one row (of doubles the first of a pair on the
+  // integer pipe, beside the second) and of two rows
+  auto diff = [](fx hi, fx lo, bool d, int x, bool first) {
+    const double a = __longlong_as_double(hi), b = __longlong_as_double(lo);
+    return WALL && d ? (first ? fx_sub(a, b) : a - b) : fx_to<true>(hi - lo, x);
   };
   auto ydiff = [](fx hi, bool dhi, int ehi, fx lo, bool dlo, int elo) {
     return WALL ? flux_val(hi, dhi, ehi) - flux_val(lo, dlo, elo) : row_diff(hi, ehi, lo, elo);
@@ -338,34 +358,34 @@ __device__ __forceinline__ Rhs rhs_pair(const ChlInst& I, int i, int jc, int k) 
     const longlong2 x = g2(G[G_UX], c), yh = g2(G[G_UY], e), yl = g2(G[G_UY], em);
     const longlong2 zh = g2(G[G_UZ], c), zl = g2(G[G_UZ], cidx(I, i, jc, km));
     const fx xp = LDG(G[G_UX] + cidx(I, ip, jc, k));
-    F.u.x = fma(diff(x.y, x.x, dc, e0.x), rxf0, dpdx);
-    F.u.y = fma(diff(xp, x.y, dc, e0.x), rxf1, dpdx);
+    F.u.x = fma(diff(x.y, x.x, dc, e0.x, true), rxf0, dpdx);
+    F.u.y = fma(diff(xp, x.y, dc, e0.x, false), rxf1, dpdx);
     F.u.x = fma(ydiff(yh.x, dh, e0.x, yl.x, dl, el.x), ryc, F.u.x);
     F.u.y = fma(ydiff(yh.y, dh, e0.x, yl.y, dl, el.x), ryc, F.u.y);
-    F.u.x = fma(diff(zh.x, zl.x, dc, e0.x), rzc, F.u.x);
-    F.u.y = fma(diff(zh.y, zl.y, dc, e0.x), rzc, F.u.y);
+    F.u.x = fma(diff(zh.x, zl.x, dc, e0.x, true), rzc, F.u.x);
+    F.u.y = fma(diff(zh.y, zl.y, dc, e0.x, false), rzc, F.u.y);
   }
   {  // w at (x-centre i, row jc, z-face k)
     const longlong2 x = g2(G[G_WX], c), yh = g2(G[G_WY], e), yl = g2(G[G_WY], em);
     const longlong2 zl = g2(G[G_WZ], c), zh = g2(G[G_WZ], cidx(I, i, jc, kp));
     const fx xm = LDG(G[G_WX] + cidx(I, im, jc, k));
-    F.w.x = diff(x.x, xm, dc, e0.z) * rxc0;
-    F.w.y = diff(x.y, x.x, dc, e0.z) * rxc1;
+    F.w.x = diff(x.x, xm, dc, e0.z, true) * rxc0;
+    F.w.y = diff(x.y, x.x, dc, e0.z, false) * rxc1;
     F.w.x = fma(ydiff(yh.x, dh, e0.z, yl.x, dl, el.z), ryc, F.w.x);
     F.w.y = fma(ydiff(yh.y, dh, e0.z, yl.y, dl, el.z), ryc, F.w.y);
-    F.w.x = fma(diff(zh.x, zl.x, dc, e0.z), rzf, F.w.x);
-    F.w.y = fma(diff(zh.y, zl.y, dc, e0.z), rzf, F.w.y);
+    F.w.x = fma(diff(zh.x, zl.x, dc, e0.z, true), rzf, F.w.x);
+    F.w.y = fma(diff(zh.y, zl.y, dc, e0.z, false), rzf, F.w.y);
   }
   if (hasv) {  // v at (x-centre i, y-face jv = jc, z-centre k)
     const longlong2 x = g2(G[G_VX], e), yl = g2(G[G_VY], c), yh = g2(G[G_VY], cidx(I, i, jc + 1, k));
     const longlong2 zh = g2(G[G_VZ], e), zl = g2(G[G_VZ], vidx(I, i, jc, km));
     const fx xm = LDG(G[G_VX] + vidx(I, im, jc, k));
-    F.v.x = diff(x.x, xm, dh, e0.y) * rxc0;
-    F.v.y = diff(x.y, x.x, dh, e0.y) * rxc1;
+    F.v.x = diff(x.x, xm, dh, e0.y, true) * rxc0;
+    F.v.y = diff(x.y, x.x, dh, e0.y, false) * rxc1;
     F.v.x = fma(ydiff(yh.x, dn, eh.y, yl.x, dc, e0.y), ryf, F.v.x);
     F.v.y = fma(ydiff(yh.y, dn, eh.y, yl.y, dc, e0.y), ryf, F.v.y);
-    F.v.x = fma(diff(zh.x, zl.x, dh, e0.y), rzc, F.v.x);
-    F.v.y = fma(diff(zh.y, zl.y, dh, e0.y), rzc, F.v.y);
+    F.v.x = fma(diff(zh.x, zl.x, dh, e0.y, true), rzc, F.v.x);
+    F.v.y = fma(diff(zh.y, zl.y, dh, e0.y, false), rzc, F.v.y);
   }
   // a row marked non-finite by its maxima (none where its fluxes are doubles)
   const int bad = WALL ? (dc ? 0 : e0.w) | (dl ? 0 : el.w) | (dn ? 0 : eh.w) : e0.w | el.w | eh.w;
