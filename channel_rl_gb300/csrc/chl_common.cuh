@@ -284,7 +284,7 @@ struct ChlField1 {
 struct ChlFields3 {
   ChlField1 f[3];
   // where unpacking folds the largest |U|, |V|, |W| and those of every row
-  // (CHL_ROW_COPIES times three fields of `pitch` words); zeroed before
+  // (CHL_ROW_COPIES words each, `pitch` rows per field); zeroed before
   unsigned *vmax, *vrow;
   int pitch;
 };
@@ -340,7 +340,7 @@ __device__ __forceinline__ int wrap(int i, int n) { return i < 0 ? i + n : (i >=
 #define CHL_ST_VMAX0 1
 #define CHL_ST_VMAX12 5
 // behind the 16 words of the status area: the same of every row of the set written
-// last, CHL_ROW_COPIES times U, V, W with Ny + 2 words each (chl_fix.cuh)
+// last, CHL_ROW_COPIES words for each of the Ny + 2 rows of U, V, W (chl_fix.cuh)
 #define CHL_ROW_COPIES 8
 #define CHL_ST_ROWS 16
 

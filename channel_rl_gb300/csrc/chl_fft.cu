@@ -286,7 +286,7 @@ k_div_fftx(ChlMap map, int s_in, int mode, int xmb) {
     if (lb == 0 && threadIdx.x < 3) chl_vmax(I, s_in)[threadIdx.x] = 0u;
     const int nb = (nrow + CR - 1) / CR;
     for (int w = lb * (int)blockDim.x + threadIdx.x; w < 3 * CHL_ROW_COPIES * (Ny + 2); w += nb * (int)blockDim.x)
-      chl_row_copy(I, 0)[w] = 0u;
+      chl_row_words(I, 0, 0)[w] = 0u;
   }
   if (mode != 1) { U = I.U[s_in]; V = I.V[s_in]; W = I.W[s_in]; }
   else { U = I.Fp[0]; V = I.Fp[1]; W = I.Fp[2]; }

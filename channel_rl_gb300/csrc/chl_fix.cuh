@@ -116,13 +116,17 @@ __device__ __forceinline__ unsigned* chl_vmax(const ChlInst& I, int set) {
   return reinterpret_cast<unsigned*>(I.status) + (set == 0 ? CHL_ST_VMAX0 : CHL_ST_VMAX12 + 3 * (set - 1));
 }
 // The same of every row of the set that was written last (U and W: centre rows
-// 1..Ny, whose mirrors the ghost rows are; V: faces 0..Ny), [3][Ny + 2] words, of
-// which only the exponent counts.  The writers fold them into one of
-// CHL_ROW_COPIES arrays each, from which k_fix forms the rows' exponents: all warps
-// reading and raising the words of one array made k_project 55 -> 69 us at
-// 256x96x192.
-__device__ __forceinline__ unsigned* chl_row_copy(const ChlInst& I, int copy) {
-  return reinterpret_cast<unsigned*>(I.status) + CHL_ST_ROWS + copy * 3 * (I.Ny + 2);
+// 1..Ny, whose mirrors the ghost rows are; V: faces 0..Ny), of which only the
+// exponent counts.  The writers fold them into one of CHL_ROW_COPIES words each,
+// from which k_fix forms the rows' exponents: all warps reading and raising one
+// word per row made k_project 55 -> 69 us at 256x96x192.
+__device__ __forceinline__ unsigned* chl_row_words(const ChlInst& I, int comp, int row) {
+  return reinterpret_cast<unsigned*>(I.status) + CHL_ST_ROWS + CHL_ROW_COPIES * (comp * (I.Ny + 2) + row);
+}
+__device__ __forceinline__ unsigned chl_row_max(const ChlInst& I, int comp, int row) {
+  const uint4* p = reinterpret_cast<const uint4*>(chl_row_words(I, comp, row));
+  const uint4 a = __ldcg(p), b = __ldcg(p + 1);
+  return max(max(max(a.x, a.y), max(a.z, a.w)), max(max(b.x, b.y), max(b.z, b.w)));
 }
 // raises *g to x where x has the larger exponent
 __device__ __forceinline__ void chl_raise_exp(unsigned* g, unsigned x) {
@@ -155,32 +159,33 @@ __device__ __forceinline__ void chl_line_max(unsigned* g, unsigned q, int rows, 
 }
 
 // Folds the magnitudes of each thread's U, V, W (of U alone with N = 1) in row j
-// into the set's largest and the row's (whole block; x-line q).  The global words
-// are read first: only blocks, and warps for the rows, that raise one issue an
-// atomic, or the tens of thousands of same-address atomics would take longer than
-// the kernels.
+// into the set's largest and the row's (whole block, at most 256 threads; x-line
+// q = k Ny + j - 1, numbered upwards through the block, of Nx/2 threads).  The
+// global words are read first: only blocks that raise one issue an atomic, or the
+// tens of thousands of same-address atomics would take longer than the kernels.
 template <int N>
 __device__ __forceinline__ void chl_set_max(const ChlInst& I, int set, unsigned q, int j, const unsigned (&v)[N]) {
-  __shared__ unsigned sm[N][8], line[8], row[8];      // per warp
-  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const bool one = __all_sync(0xffffffffu, q == __shfl_sync(0xffffffffu, q, 0));     // the warp is in one x-line
-  unsigned mine = 0u;
+  __shared__ unsigned sm[N][CHL_BLOCK_LINES];
+  __shared__ unsigned line[8], row[8], q0;
+  const unsigned copy = blockIdx.x % CHL_ROW_COPIES;
+  if (I.Nx % 64 == 0) {       // every warp is in one x-line
+    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    unsigned mine = 0u;
 #pragma unroll
-  for (int c = 0; c < N; ++c) {
-    const unsigned x = __reduce_max_sync(0xffffffffu, v[c]);
-    if (lane == c) mine = x;
-  }
-  if (lane < N) sm[lane][warp] = mine;
-  if (lane == 0) { line[warp] = one ? q : 0xFFFFFFFFu; row[warp] = j; }
-  __syncthreads();
-  unsigned* rows = chl_row_copy(I, (int)(blockIdx.x % CHL_ROW_COPIES));
-  // thread (c, w): the warps from w on that share its x-line
-  if (threadIdx.x < 8 * N) {
+    for (int c = 0; c < N; ++c) {
+      const unsigned x = __reduce_max_sync(0xffffffffu, v[c]);
+      if (lane == c) mine = x;
+    }
+    if (lane < N) sm[lane][warp] = mine;
+    if (lane == 0) { line[warp] = q; row[warp] = j; }
+    __syncthreads();
+    if (threadIdx.x >= 8 * N) return;
+    // thread (c, w): the warps from w on that share its x-line; w = 7 all of them
     const unsigned c = threadIdx.x >> 3, w = threadIdx.x & 7;
-    if (w < nw && line[w] != 0xFFFFFFFFu && (w == 0 || line[w - 1] != line[w])) {
+    if (w < nw && (w == 0 || line[w - 1] != line[w])) {
       unsigned x = sm[c][w];
       for (unsigned k = w + 1; k < nw && line[k] == line[w]; ++k) x = max(x, sm[c][k]);
-      chl_raise_exp(rows + c * (I.Ny + 2) + row[w], x);
+      chl_raise_exp(chl_row_words(I, c, row[w]) + copy, x);
     }
     if (w == 7) {
       unsigned x = sm[c][0];
@@ -188,10 +193,22 @@ __device__ __forceinline__ void chl_set_max(const ChlInst& I, int set, unsigned 
       unsigned* all = chl_vmax(I, set) + c;
       if (x > __ldcg(all)) atomicMax(all, x);
     }
+    return;
   }
-  if (!one) {
+  const unsigned nl = min((unsigned)CHL_BLOCK_LINES, blockDim.x / (unsigned)(I.Nx / 2) + 2u);   // lines of the block
+  for (unsigned t = threadIdx.x; t < N * nl; t += blockDim.x) sm[t / nl][t % nl] = 0u;
+  if (threadIdx.x == 0) q0 = q;
+  __syncthreads();
+  const unsigned l = q - q0;
 #pragma unroll
-    for (int c = 0; c < N; ++c) chl_raise_exp(rows + c * (I.Ny + 2) + j, v[c]);
+  for (int c = 0; c < N; ++c) atomicMax(&sm[c][l], v[c]);
+  __syncthreads();
+  for (unsigned t = threadIdx.x; t < N * nl; t += blockDim.x) {
+    const unsigned c = t / nl, w = t - c * nl, x = sm[c][w];
+    if (x == 0u) continue;
+    chl_raise_exp(chl_row_words(I, c, 1 + (q0 + w) % (unsigned)I.Ny) + copy, x);
+    unsigned* all = chl_vmax(I, set) + c;
+    if (x > __ldcg(all)) atomicMax(all, x);
   }
 }
 

@@ -73,7 +73,7 @@ k_unpack3(ChlFields3 f3, int Nx, int Nz) {
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
     const unsigned w = __reduce_max_sync(0xffffffffu, hi[m]);
-    unsigned* g = f3.vrow + (3 * (blockIdx.x % CHL_ROW_COPIES) + blockIdx.y) * f3.pitch + row[m];
+    unsigned* g = f3.vrow + CHL_ROW_COPIES * (blockIdx.y * f3.pitch + row[m]) + blockIdx.x % CHL_ROW_COPIES;
     if ((threadIdx.x & 31) == 0 && r0 + m * CHL_CONV_ROWS < rows) chl_raise_exp(g, w);
     all = max(all, w);
   }
@@ -376,7 +376,7 @@ k_massflow(ChlMap map, int s, int force) {
     if (threadIdx.x == 0) I.dsm_cnt[0] = 0;
   }
   if (!force)        // k_shift forms the largest |U| anew
-    for (int w = threadIdx.x; w < CHL_ROW_COPIES * (Ny + 2); w += 256) chl_row_copy(I, w / (Ny + 2))[w % (Ny + 2)] = 0u;
+    for (int w = threadIdx.x; w < CHL_ROW_COPIES * (Ny + 2); w += 256) chl_row_words(I, 0, 0)[w] = 0u;
   if (threadIdx.x == 0) {
     const double d = I.scal[CHL_S_Q0] - sum / (double)(Nx * Nz);
     I.scal[CHL_S_SHIFT] = d;

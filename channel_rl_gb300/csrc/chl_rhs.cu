@@ -38,15 +38,10 @@ enum { G_UX = 0, G_VY, G_WZ, G_UZ, G_WX, G_UY, G_VX, G_VZ, G_WY };
 // (FP64 and this 3), and more the stronger the grid is stretched.  x, y, z are the
 // exponents, w whether a velocity is not finite; left in vexp by k_fix.
 __device__ __forceinline__ int4 vel_exp(const ChlInst& I, int j) {
-  unsigned u = 0u, v = 0u, w = 0u;
-  const int a = max(j, 1), b = min(j + 1, I.Ny), n = I.Ny + 2;
-#pragma unroll
-  for (int c = 0; c < CHL_ROW_COPIES; ++c) {
-    const unsigned* r = chl_row_copy(I, c);
-    u = max(u, max(__ldcg(r + a), __ldcg(r + b)));
-    v = max(v, max(__ldcg(r + n + max(j - 1, 0)), __ldcg(r + n + j)));
-    w = max(w, max(__ldcg(r + 2 * n + a), __ldcg(r + 2 * n + b)));
-  }
+  const int a = max(j, 1), b = min(j + 1, I.Ny);
+  const unsigned u = max(chl_row_max(I, 0, a), chl_row_max(I, 0, b));
+  const unsigned v = max(chl_row_max(I, 1, max(j - 1, 0)), chl_row_max(I, 1, j));
+  const unsigned w = max(chl_row_max(I, 2, a), chl_row_max(I, 2, b));
   return make_int4(fx_exp<61>(u), fx_exp<61>(v), fx_exp<61>(w), fx_bad(u) || fx_bad(v) || fx_bad(w));
 }
 
