@@ -156,10 +156,16 @@ struct ChlInst {
   // for r 2^e, r < 2^63, one exponent for a table along x or z and one per
   // row along y; the weight's is -63 (chl_fix.cuh)
   const long long *fxrxc, *fxrxf, *fxryc, *fxryf, *fxrzc, *fxrzf, *fxw1;
+  // what a grid that is uniform only to the accepted tolerance adds: the difference
+  // of the reciprocal face spacings at i-1 and i, 2^(exf+3) (k: 2^(ezf+3)), and, with
+  // h the centre's width, h/d - 1 at faces i-1 (x) and i (y), 2^-59 (Vreman)
+  const int *dxr, *dzr;
+  const int2 *hxe, *hze;
   const long long *fxhyl, *fxhyh; // h_y/dy of the y spacings below and above a centre row, 2^-62 (Vreman)
   const int *eyc, *eyf;
   int exc, exf, ezc, ezf;
   int4 *vexp;                     // per row: exponents of the velocities that its fluxes take (chl_rhs.cu)
+  int4 *slack;                    // per row: bits that the copies X have above the row's velocities (dynamic model)
   int4 *upd;                      // per row, from the flux kernel to the update: exponents (chl_rhs.cu)
   unsigned *nmax, *smax;          // largest |nu + nu_t| and largest of the six |S| S_ij of every centre row (chl_fix.cuh)
   double *q[CHL_NQ], *r[CHL_NQ];  // DSM: filter inputs 3..14 and filtered fields 0..17 (chl_sgs.cu; products and r are integers)

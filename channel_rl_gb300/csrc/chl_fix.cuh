@@ -220,3 +220,8 @@ __device__ __forceinline__ void top_or(unsigned& m, fx a) {
 }
 // a 2^s for s of either sign (toward minus infinity)
 __device__ __forceinline__ fx scale2(fx a, int s) { return (a << max(s, 0)) >> max(-s, 0); }
+// its high word, for s <= 31
+__device__ __forceinline__ int scale2_hi(fx a, int s) {
+  const int h = __funnelshift_l((unsigned)a, (unsigned)(a >> 32), (unsigned)max(s, 0));
+  return h >> min(31, max(-s, 0));
+}

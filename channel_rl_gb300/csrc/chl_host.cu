@@ -80,8 +80,8 @@ constexpr int MLP_NPARAM = 4545;
 struct Consts {
   int nx, ny, nz, nxg, nyg, nzg, Nx, Ny, Nz, Nxh;
   std::vector<double> xf, yf, zf, xg, yg, zg;   // 1-based Fortran copies (index 0 unused)
-  std::vector<double> rdxc, rdxf, dxf, rdzc, rdzf, dzf;   // offset 1, length N+3
-  std::vector<double> rdyc, rdyf, dyf, w0, w1;            // length Ny+2
+  std::vector<double> rdxc, rdxf, dxc, dxf, rdzc, rdzf, dzc, dzf;   // offset 1, length N+3
+  std::vector<double> rdyc, rdyf, dyc, dyf, w0, w1;                 // length Ny+2
   std::vector<double> csdelta, dwall;                     // length Ny+2
   std::vector<double> kxx, kzz;
   std::vector<double> Dd, Du, Dl;                          // 1-based by j_f
@@ -145,17 +145,17 @@ int make_consts(const chl_grid_desc& d, Consts& c, std::string& err) {
   c.dxmin = dmin(c.xg, c.nxg); c.dymin = dmin(c.yg, c.nyg); c.dzmin = dmin(c.zg, c.nzg);
   // x/z spacings (device index i <-> Fortran i+2), stored with offset 1
   auto periodic = [&](const std::vector<double>& f, const std::vector<double>& g, int N,
-                      std::vector<double>& rc, std::vector<double>& rf, std::vector<double>& df) {
-    rc.assign(N + 3, NaN); rf.assign(N + 3, NaN); df.assign(N + 3, NaN);
-    for (int i = 0; i <= N; ++i) rc[i + 1] = 1.0 / (f[i + 2] - f[i + 1]);
+                      std::vector<double>& rc, std::vector<double>& rf, std::vector<double>& dc, std::vector<double>& df) {
+    rc.assign(N + 3, NaN); rf.assign(N + 3, NaN); dc.assign(N + 3, NaN); df.assign(N + 3, NaN);
+    for (int i = 0; i <= N; ++i) { dc[i + 1] = f[i + 2] - f[i + 1]; rc[i + 1] = 1.0 / dc[i + 1]; }
     for (int i = -1; i <= N; ++i) { df[i + 1] = g[i + 3] - g[i + 2]; rf[i + 1] = 1.0 / df[i + 1]; }
   };
-  periodic(c.xf, c.xg, c.Nx, c.rdxc, c.rdxf, c.dxf);
-  periodic(c.zf, c.zg, c.Nz, c.rdzc, c.rdzf, c.dzf);
+  periodic(c.xf, c.xg, c.Nx, c.rdxc, c.rdxf, c.dxc, c.dxf);
+  periodic(c.zf, c.zg, c.Nz, c.rdzc, c.rdzf, c.dzc, c.dzf);
   const int Ny = c.Ny;
-  c.rdyc.assign(Ny + 2, NaN); c.rdyf.assign(Ny + 2, NaN); c.dyf.assign(Ny + 2, NaN);
+  c.rdyc.assign(Ny + 2, NaN); c.rdyf.assign(Ny + 2, NaN); c.dyc.assign(Ny + 2, NaN); c.dyf.assign(Ny + 2, NaN);
   c.w0.assign(Ny + 2, NaN); c.w1.assign(Ny + 2, NaN);
-  for (int jc = 1; jc <= Ny; ++jc) c.rdyc[jc] = 1.0 / (c.yf[jc + 1] - c.yf[jc]);
+  for (int jc = 1; jc <= Ny; ++jc) { c.dyc[jc] = c.yf[jc + 1] - c.yf[jc]; c.rdyc[jc] = 1.0 / c.dyc[jc]; }
   for (int jv = 0; jv <= Ny; ++jv) {
     c.dyf[jv] = c.yg[jv + 2] - c.yg[jv + 1];
     c.rdyf[jv] = 1.0 / c.dyf[jv];
@@ -399,8 +399,9 @@ static int upload_consts(chl_handle* h, Inst& I) {
   size_t o_w0 = A.take(8 * (Ny + 2)), o_w1 = A.take(8 * (Ny + 2)), o_ygc = A.take(8 * (Ny + 2));
   size_t o_fxrxc = A.take(8 * (Nx + 3)), o_fxryc = A.take(8 * (Ny + 2)), o_fxrzc = A.take(8 * (Nz + 3));
   size_t o_fxrxf = A.take(8 * (Nx + 3)), o_fxryf = A.take(8 * (Ny + 2)), o_fxrzf = A.take(8 * (Nz + 3));
-  size_t o_fxw1 = A.take(8 * (Ny + 2)), o_upd = A.take(16 * (Ny + 2)), o_vexp = A.take(16 * (Ny + 2));
+  size_t o_fxw1 = A.take(8 * (Ny + 2)), o_upd = A.take(16 * (Ny + 2)), o_vexp = A.take(16 * (Ny + 2)), o_slack = A.take(16 * (Ny + 2));
   size_t o_eyc = A.take(4 * (Ny + 2)), o_eyf = A.take(4 * (Ny + 2)), o_nmax = A.take(4 * (Ny + 2)), o_smax = A.take(4 * (Ny + 2));
+  size_t o_dxr = A.take(4 * (Nx + 3)), o_dzr = A.take(4 * (Nz + 3)), o_hxe = A.take(8 * (Nx + 3)), o_hze = A.take(8 * (Nz + 3));
   size_t o_csd = A.take(8 * (Ny + 2)), o_dw = A.take(8 * (Ny + 2));
   size_t o_twx = A.take(16 * (size_t)chl_twf_len(Nx)), o_twz = A.take(16 * (size_t)chl_twf_len(Nz));
   size_t o_ti = A.take(8 * ntri), o_tm = A.take(8 * ntri), o_tc = A.take(8 * ntri);
@@ -466,9 +467,11 @@ static int upload_consts(chl_handle* h, Inst& I) {
   auto L = [&](size_t o) { return (long long*)(base + o); };
   D.fxrxc = L(o_fxrxc) + 1; D.fxryc = L(o_fxryc); D.fxrzc = L(o_fxrzc) + 1;
   D.fxrxf = L(o_fxrxf) + 1; D.fxryf = L(o_fxryf); D.fxrzf = L(o_fxrzf) + 1;
-  D.fxw1 = L(o_fxw1); D.fxhyl = L(o_hyl); D.fxhyh = L(o_hyh); D.upd = (int4*)(base + o_upd); D.vexp = (int4*)(base + o_vexp);
+  D.fxw1 = L(o_fxw1); D.fxhyl = L(o_hyl); D.fxhyh = L(o_hyh); D.upd = (int4*)(base + o_upd); D.vexp = (int4*)(base + o_vexp); D.slack = (int4*)(base + o_slack);
   D.eyc = (const int*)(base + o_eyc); D.eyf = (const int*)(base + o_eyf); D.nmax = (unsigned*)(base + o_nmax);
   D.smax = (unsigned*)(base + o_smax);
+  D.dxr = (const int*)(base + o_dxr) + 1; D.dzr = (const int*)(base + o_dzr) + 1;
+  D.hxe = (const int2*)(base + o_hxe) + 1; D.hze = (const int2*)(base + o_hze) + 1;
   D.smag_csdelta = P(o_csd); D.smag_dwall = P(o_dw);
   D.twx = (const int4*)(base + o_twx); D.twz = (const int4*)(base + o_twz);
   D.lenx = chl_twf_len(Nx); D.lenz = chl_twf_len(Nz); D.passx = chl_fft_passes(Nx); D.passz = chl_fft_passes(Nz);
@@ -512,28 +515,49 @@ static int upload_consts(chl_handle* h, Inst& I) {
   std::vector<std::vector<int>> fixede;
   fixed.reserve(8); fixede.reserve(2);
   auto exponent = [](double m) { int k = 0; std::frexp(m, &k); return k - 63; };   // m 2^-e < 2^63
-  auto fixtab = [&](size_t o, const std::vector<double>& v, const std::vector<int>& e) {
+  // d: the spacings whose reciprocals v are, for the ten bits that v has no room for
+  auto fixtab = [&](size_t o, const std::vector<double>& v, const std::vector<int>& e, const std::vector<double>* d = nullptr) {
     fixed.emplace_back(v.size(), 0LL);
     for (size_t q = 0; q < v.size(); ++q)
-      if (std::isfinite(v[q])) fixed.back()[q] = std::llrint(std::ldexp(v[q], -e[e.size() == 1 ? 0 : q]));
+      if (std::isfinite(v[q])) {
+        const int x = -e[e.size() == 1 ? 0 : q];
+        fixed.back()[q] = std::llrint(std::ldexp(v[q], x));
+        if (d) fixed.back()[q] += std::llrint(std::ldexp(v[q] * std::fma(-v[q], (*d)[q], 1.0), x));
+      }
     return cudaMemcpyAsync(base + o, fixed.back().data(), 8 * v.size(), cudaMemcpyHostToDevice, h->st);
   };
-  auto uniform = [&](size_t o, const std::vector<double>& v, int& e) {
+  auto uniform = [&](size_t o, const std::vector<double>& v, const std::vector<double>& d, int& e) {
     double m = 0.0;
     for (double x : v) if (std::isfinite(x)) m = std::max(m, x);
-    e = exponent(m);
-    return fixtab(o, v, {e});
+    e = exponent(m * (1.0 + 1e-12));       // room for the correction
+    return fixtab(o, v, {e}, &d);
   };
-  auto perrow = [&](size_t o, size_t oe, const std::vector<double>& v) {
+  auto perrow = [&](size_t o, size_t oe, const std::vector<double>& v, const std::vector<double>& d) {
     fixede.emplace_back(v.size(), -4096);   // undefined entries: below every other exponent
-    for (size_t q = 0; q < v.size(); ++q) if (std::isfinite(v[q])) fixede.back()[q] = exponent(v[q]);
+    for (size_t q = 0; q < v.size(); ++q) if (std::isfinite(v[q])) fixede.back()[q] = exponent(v[q] * (1.0 + 1e-12));
     cudaError_t e = cudaMemcpyAsync(base + oe, fixede.back().data(), 4 * v.size(), cudaMemcpyHostToDevice, h->st);
-    return e == cudaSuccess ? fixtab(o, v, fixede.back()) : e;
+    return e == cudaSuccess ? fixtab(o, v, fixede.back(), &d) : e;
   };
-  CK(uniform(o_fxrxc, c.rdxc, D.exc)); CK(uniform(o_fxrxf, c.rdxf, D.exf));
-  CK(uniform(o_fxrzc, c.rdzc, D.ezc)); CK(uniform(o_fxrzf, c.rdzf, D.ezf));
-  CK(perrow(o_fxryc, o_eyc, c.rdyc)); CK(perrow(o_fxryf, o_eyf, c.rdyf));
+  CK(uniform(o_fxrxc, c.rdxc, c.dxc, D.exc)); CK(uniform(o_fxrxf, c.rdxf, c.dxf, D.exf));
+  CK(uniform(o_fxrzc, c.rdzc, c.dzc, D.ezc)); CK(uniform(o_fxrzf, c.rdzf, c.dzf, D.ezf));
+  CK(perrow(o_fxryc, o_eyc, c.rdyc, c.dyc)); CK(perrow(o_fxryf, o_eyf, c.rdyf, c.dyf));
   CK(fixtab(o_fxw1, c.w1, {-63}));
+  // differences of the neighbouring spacings of x and z, at most 2e-9 of them
+  auto nonuniform = [&](size_t o_d, size_t o_h, const std::vector<double>& dc, const std::vector<double>& df,
+                        const std::vector<double>& rf, int N, int e) -> cudaError_t {
+    std::vector<int> d(N + 3, 0);
+    std::vector<int2> h(N + 3, make_int2(0, 0));
+    for (int i = 0; i < N; ++i) {          // faces i - 1 and i of centre i, at i and i + 1 in the tables
+      const double w = dc[i + 1];
+      const int l = i == 0 ? N : i;        // periodic
+      d[i + 1] = (int)std::llrint(std::ldexp((df[i + 1] - df[l]) * rf[l] * rf[i + 1], -e - 3));
+      h[i + 1] = make_int2((int)std::llrint(std::ldexp((w - df[i]) * rf[i], 59)), (int)std::llrint(std::ldexp((w - df[i + 1]) * rf[i + 1], 59)));
+    }
+    cudaError_t err = cudaMemcpy(base + o_d, d.data(), 4 * d.size(), cudaMemcpyHostToDevice);
+    return err == cudaSuccess ? cudaMemcpy(base + o_h, h.data(), 8 * h.size(), cudaMemcpyHostToDevice) : err;
+  };
+  CK(nonuniform(o_dxr, o_hxe, c.dxc, c.dxf, c.rdxf, Nx, D.exf));
+  CK(nonuniform(o_dzr, o_hze, c.dzc, c.dzf, c.rdzf, Nz, D.ezf));
   {
     // both below 2: a centre row is at most twice its distance to the next centre
     std::vector<double> hl(Ny + 2, NaN), hh(Ny + 2, NaN);

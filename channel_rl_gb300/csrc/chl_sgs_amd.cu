@@ -180,9 +180,9 @@ k_amd(ChlMap map, int s_in, int use_wm) {
 // Vreman in fixed point (124 FP64 instructions per point before, 25 now).
 // b_ij sums products of the grid-scaled differences h_m a_mi and h_m a_mj of
 // components i and j, so each component is scaled by its own largest: b_22 of
-// a weak V keeps its digits beside b_11.  Along the uniform x and z the
-// grid-scaled difference is the mean edge difference itself, along y the edge
-// differences times h_y/dy of their spacings.  B_b, which cancels, and the
+// a weak V keeps its digits beside b_11.  The grid-scaled difference is the mean
+// of the edge differences times h/d of their spacings (in x and z 1 but for the
+// tolerance of a uniform grid).  B_b, which cancels, and the
 // quotient are FP64.
 __global__ void __launch_bounds__(CHL_FLUX_THREADS, 5)
 k_vreman(ChlMap map, int s_in, int use_wm) {
@@ -214,8 +214,14 @@ k_vreman(ChlMap map, int s_in, int use_wm) {
     const fx xu = 4 * scale2(d.dux, su), yv = 4 * scale2(d.dvy, sv), zw = 4 * scale2(d.dwz, sw);
     const fx yu = 4 * (fx_mul(scale2(d.uyL, su), wl) + fx_mul(scale2(d.uyH, su), wh));
     const fx yw = 4 * (fx_mul(scale2(d.wyL, sw), wl) + fx_mul(scale2(d.wyH, sw), wh));
-    const fx zu = scale2(d.uzL, su) + scale2(d.uzH, su), zv = scale2(d.vzL, sv) + scale2(d.vzH, sv);
-    const fx xv = scale2(d.vxL, sv) + scale2(d.vxR, sv), xw = scale2(d.wxL, sw) + scale2(d.wxR, sw);
+    // (in x and z h/dx is 1 to the 1e-9 that a grid may be off uniform)
+    const int2 hx = LDG(I.hxe + i), hz = LDG(I.hze + k);
+    auto mean = [](fx lo, fx hi, int s, int2 e) {
+      lo = scale2(lo, s); hi = scale2(hi, s);
+      return lo + hi + ((long long)(int)(lo >> 32) * e.x + (long long)(int)(hi >> 32) * e.y >> 27);
+    };
+    const fx zu = mean(d.uzL, d.uzH, su, hz), zv = mean(d.vzL, d.vzH, sv, hz);
+    const fx xv = mean(d.vxL, d.vxR, sv, hx), xw = mean(d.wxL, d.wxR, sw, hx);
     // b_ij, 16 x, 2^64 units
     const double b11 = fx_to(fx_mul(xu, xu) + fx_mul(yu, yu) + fx_mul(zu, zu) + 4, 0);
     const double b22 = fx_to(fx_mul(xv, xv) + fx_mul(yv, yv) + fx_mul(zv, zv) + 4, 0);
@@ -229,11 +235,11 @@ k_vreman(ChlMap map, int s_in, int use_wm) {
     const int n12 = max(-900, 2 * (eU + eV - 2 * em)), n13 = max(-900, 2 * (eU + eW - 2 * em)), n23 = max(-900, 2 * (eV + eW - 2 * em));
     const double Bb = fma(q12, pow2(n12), fma(q13, pow2(n13), q23 * pow2(n23)));
     // derivatives, 4 x, in units of 2^(em + er + 64), then scaled by their largest
-    const fx rzf = col.rzf(k), rxf = col.rxf;
+    const fx rzc = col.rzc(k), rxc = col.rxc;
     const int du = eU - em, dv = eV - em, dw = eW - em;
-    fx a1 = fx_mul(xu, col.rxc) >> min(63, -du), a7 = fx_mul(yu, col.ryc) >> min(63, -du), a8 = fx_mul(zu, rzf) >> min(63, -du);
-    fx a4 = fx_mul(xv, rxf) >> min(63, -dv), a2 = fx_mul(yv, col.ryc) >> min(63, -dv), a9 = fx_mul(zv, rzf) >> min(63, -dv);
-    fx a5 = fx_mul(xw, rxf) >> min(63, -dw), a6 = fx_mul(yw, col.ryc) >> min(63, -dw), a3 = fx_mul(zw, col.rzc(k)) >> min(63, -dw);
+    fx a1 = fx_mul(xu, rxc) >> min(63, -du), a7 = fx_mul(yu, col.ryc) >> min(63, -du), a8 = fx_mul(zu, rzc) >> min(63, -du);
+    fx a4 = fx_mul(xv, rxc) >> min(63, -dv), a2 = fx_mul(yv, col.ryc) >> min(63, -dv), a9 = fx_mul(zv, rzc) >> min(63, -dv);
+    fx a5 = fx_mul(xw, rxc) >> min(63, -dw), a6 = fx_mul(yw, col.ryc) >> min(63, -dw), a3 = fx_mul(zw, rzc) >> min(63, -dw);
     unsigned md = 0u;
     top_or(md, a1); top_or(md, a2); top_or(md, a3); top_or(md, a4); top_or(md, a5);
     top_or(md, a6); top_or(md, a7); top_or(md, a8); top_or(md, a9);

@@ -2,16 +2,19 @@
 // column of planes, from fixed-point velocities.
 //
 // The four edge strains around a centre are sums of differences of four faces
-// each; on the uniform x and z they collapse to
-//   8 S12 = ry(jc-1) A + ry(jc) B + rx C,  A, B the y differences of
+// each, collected per spacing:
+//   8 S12 = ry(jc-1) A + ry(jc) B + rx(i) C,  A, B the y differences of
 //     U(i-1) + U(i) below and above, C = V(i+1) - V(i-1) on both y faces,
-//   8 S13 = rz D + rx E,  D = U(k+1) - U(k-1) on both x faces,
+//   8 S13 = rz(k) D + rx(i) E,  D = U(k+1) - U(k-1) on both x faces,
 //     E = W(i+1) - W(i-1) on both z faces,
-//   8 S23 = ry(jc-1) G + ry(jc) H + rz K,  likewise of W and V,
-// sums and differences that are exact in integers.  Each centre scales its
-// eleven differences by their largest and its six strain rates by theirs, so
-// that the products keep 54 bits or more of the largest.  A thread marches
-// through planes and carries what they share: 17 loads per centre.
+//   8 S23 = ry(jc-1) G + ry(jc) H + rz(k) K,  likewise of W and V,
+// sums and differences that are exact in integers.  x and z are uniform only
+// within 1e-9 (chl_create), and the edges below i and k have spacings of their
+// own: the lower half of C, D, E, K takes the difference of the reciprocals,
+// (rx(i-1) - rx(i)) C_lo, for which 32 bits of either are enough.  Each centre
+// scales its fifteen differences by their largest and its six strain rates by
+// theirs, so that the products keep 54 bits or more of the largest.  A thread
+// marches through planes and carries what they share: 17 loads per centre.
 #pragma once
 #include "chl_fix.cuh"
 
@@ -24,9 +27,10 @@ struct StrainColumn {
   int eu, ev, ew;               // exponents of U, V, W
   int i, im, ip, jc, er;
   fx rx, rxc, ryl, ryh, ryc;    // reciprocal spacings, last bit 2^er
+  int dx, sz;                   // rx(i-1) - rx(i), last bit 2^(er+3); shift of its like along z
   fx um, u0, us, usb;           // plane k: U at both x faces and their sum, the sum on plane k-1
   fx vm, v0, vs, vsb;           // V at both y faces
-  fx wb, xwb, ylb, yhb;         // plane k-1: W and its x and y differences
+  fx wb, xwb, xlb, ylb, yhb;    // plane k-1: W and its x (whole, lower half) and y differences
   fx w0;                        // plane k: W (valid after point())
 
   __device__ __forceinline__ fx u(int a, int j, int k) const { return LDG(U + cidx(I, a, j, k)); }
@@ -45,11 +49,14 @@ struct StrainColumn {
     ryc = LDG(I.fxryc + jc) >> min(63, er - ec);
     rx = LDG(I.fxrxf + i) >> min(63, er - I.exf);
     rxc = LDG(I.fxrxc + i) >> min(63, er - I.exc);
+    dx = LDG(I.dxr + i) >> min(31, er - I.exf);
+    sz = min(31, er - I.ezf);
     const int kb = k == 0 ? I.Nz - 1 : k - 1;
     um = u(im, jc, k); u0 = u(i, jc, k); us = um + u0; usb = u(im, jc, kb) + u(i, jc, kb);
     vm = v(i, jc - 1, k); v0 = v(i, jc, k); vs = vm + v0; vsb = v(i, jc - 1, kb) + v(i, jc, kb);
     wb = w(i, jc, kb);
-    xwb = w(ip, jc, kb) - w(im, jc, kb);
+    const fx wl = w(im, jc, kb);
+    xwb = w(ip, jc, kb) - wl; xlb = wb - wl;
     ylb = wb - w(i, jc - 1, kb); yhb = w(i, jc + 1, kb) - wb;
   }
 
@@ -58,30 +65,35 @@ struct StrainColumn {
     const int kp = k + 1 == I.Nz ? 0 : k + 1;
     const fx ump = u(im, jc, kp), u0p = u(i, jc, kp), vmp = v(i, jc - 1, kp), v0p = v(i, jc, kp);
     w0 = w(i, jc, k);
-    const fx xw = w(ip, jc, k) - w(im, jc, k), yl = w0 - w(i, jc - 1, k), yh = w(i, jc + 1, k) - w0;
+    const fx wl = w(im, jc, k), xw = w(ip, jc, k) - wl, xl = w0 - wl, yl = w0 - w(i, jc - 1, k), yh = w(i, jc + 1, k) - w0;
     const fx usp = ump + u0p, vsp = vmp + v0p;
     fx A = us - (u(im, jc - 1, k) + u(i, jc - 1, k)), B = (u(im, jc + 1, k) + u(i, jc + 1, k)) - us;
     fx D = usp - usb, K = vsp - vsb;
-    fx C = (v(ip, jc - 1, k) - v(im, jc - 1, k)) + (v(ip, jc, k) - v(im, jc, k));
+    const fx vl = v(im, jc - 1, k) + v(im, jc, k);
+    fx C = (v(ip, jc - 1, k) + v(ip, jc, k)) - vl;
+    // the lower halves of C, D, E, K
+    const fx Cl = vs - vl, Dl = us - usb, El = xlb + xl, Kl = vs - vsb;
     fx E = xwb + xw, G = ylb + yl, H = yhb + yh;
     fx d1 = u0 - um, d2 = v0 - vm, d3 = w0 - wb;
     c[0] = us; c[1] = vs; c[2] = wb + w0;
     usb = us; us = usp; um = ump; u0 = u0p;
     vsb = vs; vs = vsp; vm = vmp; v0 = v0p;
-    wb = w0; xwb = xw; ylb = yl; yhb = yh;
+    wb = w0; xwb = xw; xlb = xl; ylb = yl; yhb = yh;
     // |difference| < 2^60 in units of 2^et
     unsigned mu = 0u, mv = 0u, mw = 0u;
-    top_or(mu, d1); top_or(mu, A); top_or(mu, B); top_or(mu, D);
-    top_or(mv, d2); top_or(mv, C); top_or(mv, K);
-    top_or(mw, d3); top_or(mw, E); top_or(mw, G); top_or(mw, H);
+    top_or(mu, d1); top_or(mu, A); top_or(mu, B); top_or(mu, D); top_or(mu, Dl);
+    top_or(mv, d2); top_or(mv, C); top_or(mv, K); top_or(mv, Cl); top_or(mv, Kl);
+    top_or(mw, d3); top_or(mw, E); top_or(mw, G); top_or(mw, H); top_or(mw, El);
     const int et = max(max(eu + 64 - __clz((int)mu), ev + 64 - __clz((int)mv)), ew + 64 - __clz((int)mw)) - 60;
     const int su = eu - et, sv = ev - et, sw = ew - et;
     const fx rz = LDG(I.fxrzf + k) >> min(63, er - I.ezf), rzc = LDG(I.fxrzc + k) >> min(63, er - I.ezc);
+    const int dz = LDG(I.dzr + k) >> sz;
     // strain rates: 4 S_ii, 8 S_ij, |x| < 2^61
     fx s1 = 4 * fx_mul(scale2(d1, su), rxc), s2 = 4 * fx_mul(scale2(d2, sv), ryc), s3 = 4 * fx_mul(scale2(d3, sw), rzc);
-    fx t1 = fx_mul(scale2(A, su), ryl) + fx_mul(scale2(B, su), ryh) + fx_mul(scale2(C, sv), rx);
-    fx t2 = fx_mul(scale2(D, su), rz) + fx_mul(scale2(E, sw), rx);
-    fx t3 = fx_mul(scale2(G, sw), ryl) + fx_mul(scale2(H, sw), ryh) + fx_mul(scale2(K, sv), rz);
+    fx t1 = fx_mul(scale2(A, su), ryl) + fx_mul(scale2(B, su), ryh) + fx_mul(scale2(C, sv), rx) + ((long long)scale2_hi(Cl, sv) * dx >> 29);
+    fx t2 = fx_mul(scale2(D, su), rz) + fx_mul(scale2(E, sw), rx) +
+            ((long long)scale2_hi(Dl, su) * dz + (long long)scale2_hi(El, sw) * dx >> 29);
+    fx t3 = fx_mul(scale2(G, sw), ryl) + fx_mul(scale2(H, sw), ryh) + fx_mul(scale2(K, sv), rz) + ((long long)scale2_hi(Kl, sv) * dz >> 29);
     unsigned md = 0u;
     top_or(md, s1); top_or(md, s2); top_or(md, s3); top_or(md, t1); top_or(md, t2); top_or(md, t3);
     const int sd = __clz((int)md) - 3;
