@@ -97,12 +97,16 @@ struct GradColumn {
 }  // namespace
 
 // AMD in fixed point.  As FP64 code this kernel issued 114 FP64 instructions
-// per point (0.97 ms per launch at 256x96x192, the FP64 pipe 90 % busy; 0.28 ms now).  The
+// per point (0.97 ms per launch at 256x96x192, the FP64 pipe 90 % busy; 0.30 ms now).  The
 // edge differences are exact integers from the fixed-point copies (k_fix);
-// each point scales its fifteen by their largest, so that the products keep
-// 54 bits or more of the largest product, and forms the derivatives, D and
-// the a_ij there.  N and the division are FP64 (17 instructions).
-__global__ void __launch_bounds__(CHL_FLUX_THREADS, 5)   // 2, 3, 4, 5, 6 blocks per SM took 417, 321, 289, 288, 290 us (283 now)
+// each point scales those of each component by their largest, so that a weak
+// component keeps its digits, and forms the a_ij, the derivatives and D there.  The
+// S_ii, N and the division are FP64 (one scale for the three components and the
+// S_ii in integers beside the largest derivative took 0.28 ms and left nu_t of a
+// nearly parallel flow 9 times as far off as in FP64, of turbulent ones 1.1 to 1.2
+// times).  With three, six and twelve of N's twelve conversions on the FP64 pipe
+// 300, 309 and 359 us: all are on the integer pipe.
+__global__ void __launch_bounds__(CHL_FLUX_THREADS, 5)   // 2, 3, 4, 5, 6 blocks per SM took 417, 321, 289, 288, 290 us (301 now)
 k_amd(ChlMap map, int s_in, int use_wm) {
   chl_pdl_wait();
   int lb;
@@ -123,13 +127,13 @@ k_amd(ChlMap map, int s_in, int use_wm) {
     const Diffs d = col.point(k);
     fx dux = d.dux, dvy = d.dvy, dwz = d.dwz, uyL = d.uyL, uyH = d.uyH, vxL = d.vxL, vxR = d.vxR;
     fx wxL = d.wxL, wxR = d.wxR, wyL = d.wyL, wyH = d.wyH;
-    // scale: |x| < 2^60 in units of 2^et
+    // scale: each component's differences below 2^59 in units of 2^eU, 2^eV, 2^eW
     unsigned mu = 0u, mv = 0u, mw = 0u;
     top_or(mu, dux); top_or(mu, uyL); top_or(mu, uyH); top_or(mu, d.uzL); top_or(mu, d.uzH);
     top_or(mv, dvy); top_or(mv, vxL); top_or(mv, vxR); top_or(mv, d.vzL); top_or(mv, d.vzH);
     top_or(mw, dwz); top_or(mw, wxL); top_or(mw, wxR); top_or(mw, wyL); top_or(mw, wyH);
-    const int et = max(max(eu + 64 - __clz((int)mu), ev + 64 - __clz((int)mv)), ew + 64 - __clz((int)mw)) - 60;
-    const int su = eu - et, sv = ev - et, sw = ew - et;
+    const int su = __clz((int)mu) - 5, sv = __clz((int)mv) - 5, sw = __clz((int)mw) - 5;
+    const int eU = eu - su, eV = ev - sv, eW = ew - sw, em = max(eU, max(eV, eW));
     dux = scale2(dux, su); uyL = scale2(uyL, su); uyH = scale2(uyH, su);
     const fx uL = scale2(d.uzL, su), uH = scale2(d.uzH, su);
     dvy = scale2(dvy, sv); vxL = scale2(vxL, sv); vxR = scale2(vxR, sv);
@@ -137,39 +141,43 @@ k_amd(ChlMap map, int s_in, int use_wm) {
     dwz = scale2(dwz, sw); wxL = scale2(wxL, sw); wxR = scale2(wxR, sw); wyL = scale2(wyL, sw); wyH = scale2(wyH, sw);
     // grid-scaled centre differences, 4 x
     const fx Yu = uyL + uyH, Zu = uL + uH, Xv = vxL + vxR, Zv = vL + vH, Xw = wxL + wxR, Yw = wyL + wyH;
-    // derivatives, 4 x, scaled anew: the spacings differ by up to the
-    // stretching of the grid (units 2^(et + er + 64 - sd))
+    // exponents in N, whose differences are in units of 2^em
+    const int cU = max(-300, eU - em), cV = max(-300, eV - em), cW = max(-300, eW - em);
+    // D, a sum of squares, from the derivatives, 4 x, in units of 2^(em + er + 64 -
+    // sd): scaled anew, as the spacings differ by up to the stretching of the grid
+    const int du = min(63, em - eU), dv = min(63, em - eV), dw = min(63, em - eW);
     const fx rzf = col.rzf(k), rxf = col.rxf, ryl = col.ryl, ryh = col.ryh;
-    fx s11 = 4 * fx_mul(dux, col.rxc), s22 = 4 * fx_mul(dvy, col.ryc), s33 = 4 * fx_mul(dwz, col.rzc(k));
-    fx dUy = fx_mul(uyL, ryl) + fx_mul(uyH, ryh), dWy = fx_mul(wyL, ryl) + fx_mul(wyH, ryh);
-    fx dUz = fx_mul(Zu, rzf), dVz = fx_mul(Zv, rzf), dVx = fx_mul(Xv, rxf), dWx = fx_mul(Xw, rxf);
+    fx s11 = 4 * fx_mul(dux, col.rxc) >> du, s22 = 4 * fx_mul(dvy, col.ryc) >> dv, s33 = 4 * fx_mul(dwz, col.rzc(k)) >> dw;
+    fx dUy = fx_mul(uyL, ryl) + fx_mul(uyH, ryh) >> du, dWy = fx_mul(wyL, ryl) + fx_mul(wyH, ryh) >> dw;
+    fx dUz = fx_mul(Zu, rzf) >> du, dVz = fx_mul(Zv, rzf) >> dv, dVx = fx_mul(Xv, rxf) >> dv, dWx = fx_mul(Xw, rxf) >> dw;
     unsigned md = 0u;
     top_or(md, s11); top_or(md, s22); top_or(md, s33);
     top_or(md, dUy); top_or(md, dUz); top_or(md, dVx); top_or(md, dVz); top_or(md, dWx); top_or(md, dWy);
     const int sd = __clz((int)md) - 3;     // |x| < 2^61; a derivative is below 2^61 already
     s11 <<= sd; s22 <<= sd; s33 <<= sd;
     dUy <<= sd; dUz <<= sd; dVx <<= sd; dVz <<= sd; dWx <<= sd; dWy <<= sd;
-    // D, 16 x (2^64 units of the derivatives' square); 12 makes up for nine products
+    // 16 x (2^64 units of the derivatives' square); 12 makes up for nine products
     const fx D = (fx_mul(s11, s11) + fx_mul(s22, s22) + fx_mul(s33, s33) + 12) +
                  (fx_mul(dUy, dUy) + fx_mul(dUz, dUz) + fx_mul(dVx, dVx)) +
                  (fx_mul(dVz, dVz) + fx_mul(dWx, dWx) + fx_mul(dWy, dWy));
-    // a_ii 16 x in 2^63 units, a_ij 4 x in 2^61 units of the differences' square:
-    // sum_k (d^_k u_i)(d^_k u_j) with the reference's product forms; the third
-    // mixed term of each is the edge product averaged
-#define SQ(a) fx_mul_shr<63>(a, a)
-    const fx a11 = SQ(4 * dux) + SQ(Yu) + SQ(Zu), a22 = SQ(4 * dvy) + SQ(Xv) + SQ(Zv), a33 = SQ(4 * dwz) + SQ(Xw) + SQ(Yw);
-#undef SQ
+    // N = sum a_ij S_ij, 64 x.  a_ii 16 x in 2^63 units, a_ij 4 x in 2^61 units of
+    // the differences' products: sum_k (d^_k u_i)(d^_k u_j) with the reference's
+    // product forms; the third mixed term of each is the edge product averaged.
+    // S_ii 4 x, S_ij 8 x; S_ii in FP64 from the exact differences, because in a nearly
+    // parallel flow a weak one times the largest a_ii is N's largest term.
     const fx a12 = fx_mul_shr<61>(Xv, dux) + fx_mul_shr<61>(Yu, dvy) + fx_mul_shr<62>(uL, vL) + fx_mul_shr<62>(uH, vH);
     const fx a13 = fx_mul_shr<61>(Xw, dux) + fx_mul_shr<61>(Zu, dwz) + fx_mul_shr<62>(uyL, wyL) + fx_mul_shr<62>(uyH, wyH);
     const fx a23 = fx_mul_shr<61>(Yw, dvy) + fx_mul_shr<61>(Zv, dwz) + fx_mul_shr<62>(vxL, wxL) + fx_mul_shr<62>(vxR, wxR);
-    // N = sum a_ij S_ij, 64 x (S_ii 4 x, a_ij 4 x with S_ij 8 x in 2^-2 units of a_ii)
-    double Nd = fx_raw<true>(a11) * fx_raw<false>(s11);
-    Nd = fma(fx_raw<true>(a22), fx_raw<false>(s22), Nd);
-    Nd = fma(fx_raw<false>(a33), fx_raw<false>(s33), Nd);
-    Nd = fma(fx_raw<false>(a12), fx_raw<false>(dUy + dVx), Nd);
-    Nd = fma(fx_raw<false>(a13), fx_raw<false>(dUz + dWx), Nd);
-    Nd = fma(fx_raw<false>(a23), fx_raw<false>(dVz + dWy), Nd);
-    double v = (-0.3 * Nd) / fx_to(D, 0) * pow2(min(1023, max(-1022, et - er - 67 + sd)));
+    double No = fx_to(a12, cU + cV) * fx_raw<false>(dUy + dVx);
+    No = fma(fx_to(a13, cU + cW), fx_raw<false>(dUz + dWx), No);
+    No = fma(fx_to(a23, cV + cW), fx_raw<false>(dVz + dWy), No);
+#define SQ(a) fx_mul_shr<63>(a, a)
+    double Nd = fx_to(SQ(4 * dux) + SQ(Yu) + SQ(Zu), 2 * cU) * (fx_to<true>(d.dux, cU + su + 2) * LDG(I.rdxc + i));
+    Nd = fma(fx_to(SQ(4 * dvy) + SQ(Xv) + SQ(Zv), 2 * cV), fx_to<true>(d.dvy, cV + sv + 2) * LDG(I.rdyc + jc), Nd);
+    Nd = fma(fx_to(SQ(4 * dwz) + SQ(Xw) + SQ(Yw), 2 * cW), fx_to<true>(d.dwz, cW + sw + 2) * LDG(I.rdzc + k), Nd);
+#undef SQ
+    Nd = fma(No, pow2(min(1023, max(-1022, er + 64 - sd))), Nd);
+    double v = (-0.3 * Nd) / fx_to(D, 0) * pow2(min(1023, max(-1022, em - 2 * er - 131 + 2 * sd)));
     if (bad) v = __longlong_as_double(0x7FF8000000000000LL);
     if (valid) I.S[cidx(I, i, jc, k)] = v;
     if (valid) hi = max(hi, write_nut_rows(I, i, jc, k, I.nu + chl_pos(v), [v] { return chl_pos(v); }, use_wm));
