@@ -56,7 +56,7 @@ struct FxConv {
 // F 2^e as a double, rounded to nearest; exponents beyond a double's give its
 // smallest and largest magnitudes.  EXACT = false takes the magnitude of a
 // negative F one unit short, which saves the carry, for values whose last bits
-// are rounding anyway.
+// are rounding anyway and whose sums are not taken (it is a mean error).
 template <bool EXACT = false>
 __device__ __forceinline__ double fx_to(fx f, int e) {
   const int sign = (int)(f >> 63);
@@ -97,6 +97,17 @@ __device__ __forceinline__ fx fx_mul(fx a, fx b) {
   const int al = (int)((unsigned)a >> 1), bl = (int)((unsigned)b >> 1);
   const long long t = (long long)ah * bl + (long long)bh * al;
   return (long long)ah * bh + (t >> 31);
+}
+
+// (a b) >> S for 34 <= S <= 64, without a mean error where low words are random:
+// half a unit for the last shift and a quarter of 2^(64-S) for the low words' product
+// come back with the start of t.  For what sums over many points collect.
+template <int S>
+__device__ __forceinline__ fx fx_mul_mean(fx a, fx b) {
+  const int ah = (int)(a >> 32), bh = (int)(b >> 32);
+  const int al = (int)((unsigned)a >> 1), bl = (int)((unsigned)b >> 1);
+  const long long t = (1LL << (S - 34)) + (1LL << 29) + (long long)ah * bl + (long long)bh * al;
+  return (fx)((unsigned long long)((long long)ah * bh) << (64 - S)) + (t >> (S - 33));
 }
 
 // (a b) >> S for 34 <= S <= 64, |a b| < 2^(62+S): keeps 64 - S more bits of a

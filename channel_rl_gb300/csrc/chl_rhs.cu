@@ -109,7 +109,18 @@ k_fix(ChlMap map, int s, int prep) {
   if (t < nv) v = get(I.V[s]);
   if (t < nc) { put(I.X[0], u, eu); put(I.X[2], w, ew); }
   if (t < nv) put(I.X[1], v, ev);
-  if (t <= (unsigned)I.Ny) I.vexp[t] = vel_exp(I, t);
+  if (t <= (unsigned)I.Ny) {
+    const int j = t;
+    const int4 x = vel_exp(I, j);
+    I.vexp[j] = x;
+    if (j >= 1) {
+      // centre row j with the rows of faces that the test filter brings into it
+      const int a = max(j - 1, 1);
+      const int u = max(x.x, fx_exp<61>(chl_row_max(I, 0, a))), w = max(x.z, fx_exp<61>(chl_row_max(I, 2, a)));
+      const int v = max(x.y, fx_exp<61>(max(chl_row_max(I, 1, max(j - 2, 0)), chl_row_max(I, 1, min(j + 1, I.Ny)))));
+      I.slack[j] = make_int4(min(24, eu - u), min(24, ev - v), min(24, ew - w), 0);
+    }
+  }
 }
 
 // Fluxes next to a wall whose nu + nu_t the wall model sets (y-faces 0, 1 and

@@ -22,7 +22,8 @@
 // ---------------------------------------------------------------- strain
 // Strain magnitude and the DSM filter inputs at centres (rows 1..Ny): q3..8
 // the products of the centre velocities' face sums in fixed point (last bit
-// 2^(e_i + e_j + 64)), q9..14 = |S|*(S_ii, 2 S_ij) / sqrt(2) and their
+// 2^(e_i + e_j + 64), less the row's slack of both: next to a resolved wall the
+// products are 1e-8 of the field's largest and less), q9..14 = |S|*(S_ii, 2 S_ij) / sqrt(2) and their
 // largest per row.
 // With DSM = false (the static model, whose row coefficients do not depend on
 // the strain) nu + nu_t instead, so that no pass reads |S| back: 143 -> 157 us
@@ -44,6 +45,8 @@ k_strain(ChlMap map, int s_in, int use_wm) {
   StrainColumn col(I, I.X[0], I.X[1], I.X[2], fx_exp<61>(vm[0]), fx_exp<61>(vm[1]), fx_exp<61>(vm[2]), i, jc,
                    min(k0, Nz - 1));
   const double cj = DSM ? 0.0 : I.coef[jc], nu = I.nu;
+  int4 sl = make_int4(0, 0, 0, 0);
+  if (DSM) sl = LDG(I.slack + jc);
   for (int k = k0; k < min(Nz, k0 + M); ++k) {
     fx f[3];
     Strain s = col.point(k, f);
@@ -57,8 +60,9 @@ k_strain(ChlMap map, int s_in, int use_wm) {
       continue;
     }
     fx* const* q = reinterpret_cast<fx* const*>(I.q);
-    q[3][c] = fx_mul(f[0], f[0]); q[4][c] = fx_mul(f[1], f[1]); q[5][c] = fx_mul(f[2], f[2]);
-    q[6][c] = fx_mul(f[0], f[1]); q[7][c] = fx_mul(f[0], f[2]); q[8][c] = fx_mul(f[1], f[2]);
+    f[0] <<= sl.x; f[1] <<= sl.y; f[2] <<= sl.z;
+    q[3][c] = fx_mul_mean<64>(f[0], f[0]); q[4][c] = fx_mul_mean<64>(f[1], f[1]); q[5][c] = fx_mul_mean<64>(f[2], f[2]);
+    q[6][c] = fx_mul_mean<64>(f[0], f[1]); q[7][c] = fx_mul_mean<64>(f[0], f[2]); q[8][c] = fx_mul_mean<64>(f[1], f[2]);
     const double se = s.s * pow2(min(1023, max(-1022, s.e)));
     // two of the six conversions on the FP64 pipe, which is the less busy
     const double d[6] = {se * fx_raw<true>(s.t[0]), se * fx_raw<true>(s.t[1]), se * fx_raw<false>(s.t[2]),
@@ -79,7 +83,8 @@ k_strain(ChlMap map, int s_in, int use_wm) {
 // three times: 247 us per pass at 256x96x192.  Here a tap is an integer
 // shift and two additions, and the three passes take 236 us together.
 //
-// A pass forms (a + 4 b + c) >> 3, so that a field starts and ends below 2^60
+// A pass forms (a + 4 b + c) >> 3, rounded (up at a half in y and z, down in x: a
+// mean error of L would not average out of its sums), so that a field starts and ends below 2^60
 // and a filtered value is 512/216 times its integer.  A thread holds two
 // points in x of two rows, filters them in y from the four rows it loads,
 // exchanges with its neighbours in x through shared memory and marches in z,
@@ -110,14 +115,30 @@ __host__ __device__ inline FiltShape filt_shape(int Nx, int Ny, int Nz, int T, i
 
 // the exponent of |S| S_ij in the filter of row group g (rows 1 + 2 g, 2 + 2 g)
 __device__ __forceinline__ int filt_exp(const ChlInst& I, int g) {
-  unsigned m = 0u;
-  for (int j = max(1, 2 * g); j <= min(I.Ny, 2 * g + 3); ++j) m = max(m, I.smax[j]);
+  unsigned m = I.smax[max(1, 2 * g)];
+#pragma unroll
+  for (int r = 1; r < 4; ++r) m = max(m, I.smax[min(I.Ny, 2 * g + r)]);
   return fx_exp<60>(m);
+}
+
+// bits by which the velocities of row group g's centre rows are shifted up
+__device__ __forceinline__ int4 filt_slack(const ChlInst& I, int g) {
+  int4 m = LDG(I.slack + max(1, 2 * g));
+#pragma unroll
+  for (int r = 1; r < 4; ++r) {
+    const int4 s = LDG(I.slack + min(I.Ny, 2 * g + r));
+    m.x = min(m.x, s.x); m.y = min(m.y, s.y); m.z = min(m.z, s.z);
+  }
+  return m;
+}
+// of the product of field 0..5: u u, v v, w w, u v, u w, v w
+__device__ __forceinline__ int product_slack(int4 s, int field) {
+  return (field == 1 || field == 5 ? s.y : field == 2 ? s.z : s.x) + (field == 0 ? s.x : field == 1 || field == 3 ? s.y : s.z);
 }
 
 struct Pair { fx x, y; };
 __device__ __forceinline__ Pair tap(Pair a, Pair b, Pair c) {
-  return Pair{(a.x + 4 * b.x + c.x) >> 3, (a.y + 4 * b.y + c.y) >> 3};
+  return Pair{(a.x + 4 * b.x + c.x + 4) >> 3, (a.y + 4 * b.y + c.y + 4) >> 3};
 }
 __device__ __forceinline__ Pair one_sided(Pair a, Pair b) { return Pair{(a.x >> 1) + (b.x >> 2), (a.y >> 1) + (b.y >> 2)}; }
 
@@ -189,10 +210,9 @@ k_filter(ChlMap map) {
     row[3] = j + 1 >= last ? j : j + 2;
   }
   const int e = conv ? filt_exp(I, min(g, (Ny - 1) / 2)) : 0;
-  const int down = field >= 12 ? 1 : 0;        // the velocities' copies are below 2^61
   const unsigned pitch = (unsigned)f.nxp * (unsigned)nrow;
   const unsigned off0 = f.nxp * row[0] + pi, off1 = f.nxp * row[1] + pi, off2 = f.nxp * row[2] + pi, off3 = f.nxp * row[3] + pi;
-  auto get = [&](longlong2 v) {
+  auto get = [&](longlong2 v, int down) {
     if (conv) return Pair{fx_from(__longlong_as_double(v.x), e), fx_from(__longlong_as_double(v.y), e)};
     return Pair{v.x >> down, v.y >> down};
   };
@@ -200,9 +220,17 @@ k_filter(ChlMap map) {
   int k = k0 == 0 ? Nz - 1 : k0 - 1;
   const longlong2* s = src + (size_t)pitch * k;
   longlong2 n0 = __ldg(s + off0), n1 = __ldg(s + off1), n2 = __ldg(s + off2), n3 = __ldg(s + off3);
+  // right shifts of the four rows: the velocities' copies are below 2^61, products
+  // come in the unit of their row and go in that of the group
+  int4 down = make_int4(1, 1, 1, 1);
+  if (field < 6) {
+    const int to = product_slack(filt_slack(I, min(g, (Ny - 1) / 2)), field);
+    auto by = [&](int r) { return max(0, product_slack(LDG(I.slack + min(max(r, 1), Ny)), field) - to); };
+    down = make_int4(by(row[0]), by(row[1]), by(row[2]), by(row[3]));
+  }
   Pair a0 = {0, 0}, a1 = {0, 0}, b0 = {0, 0}, b1 = {0, 0};      // the planes k - 2 and k - 1 of both rows
   for (int it = 0; it < k1 - k0 + 2; ++it) {
-    const Pair v0 = get(n0), v1 = get(n1), v2 = get(n2), v3 = get(n3);
+    const Pair v0 = get(n0, down.x), v1 = get(n1, down.y), v2 = get(n2, down.z), v3 = get(n3, down.w);
     k = k + 1 == Nz ? 0 : k + 1;
     if (it < k1 - k0 + 1) {
       s = src + (size_t)pitch * k;
@@ -221,8 +249,8 @@ k_filter(ChlMap map) {
     buf[1][tid] = make_longlong2(y1.x, y1.y);
     __syncthreads();
     const fx l0 = buf[0][left].y, r0 = buf[0][right].x, l1 = buf[1][left].y, r1 = buf[1][right].x;
-    const Pair x0 = {(l0 + 4 * y0.x + y0.y) >> 3, (y0.x + 4 * y0.y + r0) >> 3};
-    const Pair x1 = {(l1 + 4 * y1.x + y1.y) >> 3, (y1.x + 4 * y1.y + r1) >> 3};
+    const Pair x0 = {(l0 + 4 * y0.x + y0.y + 3) >> 3, (y0.x + 4 * y0.y + r0 + 3) >> 3};
+    const Pair x1 = {(l1 + 4 * y1.x + y1.y + 3) >> 3, (y1.x + 4 * y1.y + r1 + 3) >> 3};
     if (it >= 2 && out) {
       const Pair z0 = tap(a0, b0, x0), z1 = tap(a1, b1, x1);
       // wall fields go to rows 1 and Ny of a centre-like field
@@ -313,6 +341,8 @@ k_dsm_final(ChlMap map, int s_in) {
     const int es = filt_exp(I, (jc - 1) / 2);
     const fx* const* R = reinterpret_cast<const fx* const*>(I.r);
     StrainColumn c(I, R[15], R[16], R[17], eu, ev, ew, i, jc, k0);
+    const int4 sl = filt_slack(I, (jc - 1) / 2);
+    const int lu = eu - sl.x, lv = ev - sl.y, lw = ew - sl.z;      // exponents in L
     for (int k = k0; k < k1; ++k) {
       fx f[3];
       const Strain h = c.point(k, f);
@@ -329,15 +359,16 @@ k_dsm_final(ChlMap map, int s_in) {
       const double M1 = MIJ(0), M2 = MIJ(1), M3 = MIJ(2), M4 = MIJ(3), M5 = MIJ(4), M6 = MIJ(5);
 #undef MIJ
       // L_ij: f are the filtered face sums, 216/512 of their value and in
-      // units twice the copies'; g = 512/216 f / 8
-      const fx g0 = fx_mul(2 * f[0], DSM_C), g1 = fx_mul(2 * f[1], DSM_C), g2 = fx_mul(2 * f[2], DSM_C);
-#define PROD(g, h) fx_mul_shr<62>(2 * (g), 2 * (h))
-      const double L1 = fx_to(LDG(R[3] + o) - PROD(g0, f[0]), eu + eu + 60);
-      const double L2 = fx_to(LDG(R[4] + o) - PROD(g1, f[1]), ev + ev + 60);
-      const double L3 = fx_to(LDG(R[5] + o) - PROD(g2, f[2]), ew + ew + 60);
-      const double L4 = fx_to(LDG(R[6] + o) - PROD(g0, f[1]), eu + ev + 60);
-      const double L5 = fx_to(LDG(R[7] + o) - PROD(g0, f[2]), eu + ew + 60);
-      const double L6 = fx_to(LDG(R[8] + o) - PROD(g1, f[2]), ev + ew + 60);
+      // units twice the copies', shifted up by the group's slack; g = 512/216 f / 8
+      f[0] <<= sl.x; f[1] <<= sl.y; f[2] <<= sl.z;
+      const fx g0 = fx_mul_mean<64>(2 * f[0], DSM_C), g1 = fx_mul_mean<64>(2 * f[1], DSM_C), g2 = fx_mul_mean<64>(2 * f[2], DSM_C);
+#define PROD(g, h) fx_mul_mean<62>(2 * (g), 2 * (h))
+      const double L1 = fx_to<true>(LDG(R[3] + o) - PROD(g0, f[0]), lu + lu + 60);
+      const double L2 = fx_to<true>(LDG(R[4] + o) - PROD(g1, f[1]), lv + lv + 60);
+      const double L3 = fx_to<true>(LDG(R[5] + o) - PROD(g2, f[2]), lw + lw + 60);
+      const double L4 = fx_to<true>(LDG(R[6] + o) - PROD(g0, f[1]), lu + lv + 60);
+      const double L5 = fx_to<true>(LDG(R[7] + o) - PROD(g0, f[2]), lu + lw + 60);
+      const double L6 = fx_to<true>(LDG(R[8] + o) - PROD(g1, f[2]), lv + lw + 60);
 #undef PROD
       a.ld = fma(L1, M1, a.ld); a.ld = fma(L2, M2, a.ld); a.ld = fma(L3, M3, a.ld);
       a.lo = fma(L4, M4, a.lo); a.lo = fma(L5, M5, a.lo); a.lo = fma(L6, M6, a.lo);
