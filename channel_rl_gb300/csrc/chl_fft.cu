@@ -193,14 +193,16 @@ struct RawLd {
   }
 };
 // a line's result as doubles: the passes with twiddles halved it `halvings`
-// times; a line with a non-finite input is NaN throughout
+// times; a line with a non-finite input is NaN throughout, one without a value of
+// 2^-958 or more zero (the passes round zeros to a unit)
 struct LineOut {
   int bits, halvings; const unsigned* hi;
   __device__ __forceinline__ double2 operator()(int r, fx2 v) const {
     const int x = fx_line_exp(hi[r], bits) + halvings;
-    const double s = fx_bad(hi[r]) ? __longlong_as_double(0x7FF8000000000000LL) : pow2(x);
+    const bool special = hi[r] - (64u << 20) >= 0x7FF00000u - (64u << 20);
+    const double s = !special ? pow2(x) : fx_bad(hi[r]) ? __longlong_as_double(0x7FF8000000000000LL) : 0.0;
     double a = fx_to(v.x, x);
-    if (fx_bad(hi[r])) a = s;
+    if (special) a = s;
     return make_double2(a, __ll2double_rn(v.y) * s);
   }
 };

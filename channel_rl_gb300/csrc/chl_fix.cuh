@@ -73,9 +73,10 @@ __device__ __forceinline__ double fx_to(fx f, int e) {
 }
 // a - b on the integer pipe: exact like the FP64 subtraction where that is
 // (magnitudes within 2^8 of each other keep all their bits), else within 2^-61
-// of the larger before its one rounding; NaN if a or b is not finite.
+// of the larger, 2^-1019 at least, before its one rounding; zeros of either sign
+// are zero; NaN if a or b is not finite.
 __device__ __forceinline__ double fx_sub(double a, double b) {
-  const int m = max(__double2hiint(a) >> 20 & 0x7FF, __double2hiint(b) >> 20 & 0x7FF);
+  const int m = max(max(__double2hiint(a) >> 20 & 0x7FF, __double2hiint(b) >> 20 & 0x7FF), 64);
   const double d = fx_to<true>(fx_from(a, m - 1084) - fx_from(b, m - 1084), m - 1084);
   return m == 0x7FF ? __longlong_as_double(0x7FF8000000000000LL) : d;
 }
