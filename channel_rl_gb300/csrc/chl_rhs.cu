@@ -49,7 +49,9 @@ __device__ __forceinline__ int4 vel_exp(const ChlInst& I, int j) {
 // |nu + nu_t| of the row and the one above.  Flux m = viscous - advective part: the
 // advective product has last bit 2^adv[m], the viscous one 2^vis[m]; the
 // fluxes of one momentum component are stored with last bit 2^G, one above
-// the largest, so that |flux| < 2^62.
+// the largest, so that |flux| < 2^62.  A row whose fluxes may exceed a double's
+// range counts as not finite, as their overflow in FP64 would have it.
+#define FLUX_G_MAX 962
 __device__ constexpr int FLUX_A[9] = {0, 1, 2, 0, 2, 0, 1, 1, 2};   // momentum component
 __device__ constexpr int FLUX_B[9] = {0, 1, 2, 2, 0, 1, 0, 2, 1};   // direction
 struct RowExp { int adv[9], vis[9], G[3], n; bool bad; };
@@ -69,7 +71,7 @@ __device__ __forceinline__ RowExp row_exp(const ChlInst& I, int4 x, int j) {
     q.vis[m] = q.n + ev[a] + (m <= G_WZ ? ec[b] + 125 : m <= G_WX ? ef[b] + 123 : ef[b] + 124);
     q.G[a] = max(q.G[a], max(q.adv[m], q.vis[m]) + 1);
   }
-  q.bad = x.w || fx_bad(nm);
+  q.bad = x.w || fx_bad(nm) || max(q.G[0], max(q.G[1], q.G[2])) > FLUX_G_MAX;
   return q;
 }
 
@@ -162,7 +164,7 @@ static __device__ __noinline__ void flux_wall(const ChlInst& I, int sin, int i, 
     ev += nu.e;
     const int g = max(ea, ev) + 1;
     const double f = fx_to((fx_mul_shr<61>(nu.m, grad) >> min(63, g - ev)) - (adv >> min(63, g - ea)), g);
-    reinterpret_cast<double*>(I.G[m])[q] = x.w || nu.bad ? __longlong_as_double(0x7FF8000000000000LL) : f;
+    reinterpret_cast<double*>(I.G[m])[q] = x.w || nu.bad || g > FLUX_G_MAX ? __longlong_as_double(0x7FF8000000000000LL) : f;
   };
   const fx rxf = LDG(I.fxrxf + i), rzf = LDG(I.fxrzf + k);
   const fx ua = u(i, j, k), wa = w(i, j, k), v0 = v(i, j, k);
