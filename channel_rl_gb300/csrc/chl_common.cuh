@@ -30,7 +30,8 @@
 // about twice the FP64 work, which a batch that fills the GPU would feel.
 // So: 1 for instances of CHL_TRI_SPLIT_MODES modes or more, else doubled
 // up to 8 while the instance has fewer than CHL_MIN_BLOCKS x 32 mode-lanes
-// and every lane keeps at least two rows.  A function of the instance's own
+// and Ny is at least 4 P.  A lane has ceil(Ny / P) rows, the last lanes fewer or
+// none (Ny = 9: 3, 3, 3, 0).  A function of the instance's own
 // extents only, like chl_dsm_ppt.
 #define CHL_TRI_SPLIT_MODES 1024
 __host__ __device__ inline int chl_tri_lanes(long modes, int Ny) {

@@ -115,7 +115,7 @@ __device__ __forceinline__ fx2* smem_fx() { extern __shared__ double2 sm[]; retu
 __device__ __forceinline__ double2* smem_d2() { extern __shared__ double2 sm[]; return sm; }
 __device__ __forceinline__ int4* smem_tw() { extern __shared__ double2 sm[]; return reinterpret_cast<int4*>(sm); }
 
-// n / d for n, d < 2^16 by one multiplication with m = 2^32/d rounded up (0
+// n / d for n < 2^16, 0 < d < 2^16 by one multiplication with m = 2^32/d rounded up (0
 // stands for d = 1)
 __device__ __forceinline__ int small_div(int n, unsigned m) { return m == 0u ? n : (int)__umulhi((unsigned)n, m); }
 struct SmallDiv {
@@ -666,8 +666,10 @@ k_zsolve(ChlMap map) {
   line_max(A, nr, nr, Nz, top);
   const int r0 = fx_last_tile(0, L * Nz, I.passz);
   double2* res = sm + r0;
-  fx_fft<false>(RawLd{0, 1, nr, LineIn{bits, top}}, DoubleTileSt{r0, 1, nr, LineOut{bits, halvings, top}}, 0, L * Nz, nr, 1,
-                nr, Nz, I.passz, T);
+  // (the last CTAs of a cluster may have no rows)
+  if (nr > 0)
+    fx_fft<false>(RawLd{0, 1, nr, LineIn{bits, top}}, DoubleTileSt{r0, 1, nr, LineOut{bits, halvings, top}}, 0, L * Nz, nr, 1,
+                  nr, Nz, I.passz, T);
   __syncthreads();
   // column w = 2 kz + part of this CTA's rows: element l at rows + 2 l (kz nr of them before)
   double* const rows = reinterpret_cast<double*>(res);
@@ -719,8 +721,9 @@ k_zsolve(ChlMap map) {
     tri_backward<4, false, true>(column(w), 2, column(w), 2, factor(I.tri_c, w), ps, 0, nr, P > 1 ? in[w] : 0.0, none);
   __syncthreads();
   line_max(res, nr, nr, Nz, top);
-  fx_fft<true>(RawLd{r0, 1, nr, LineIn{bits, top}}, RowSt{spec + (size_t)lo * ps, ps, (size_t)Nxh, LineOut{bits, halvings, top}},
-               r0, L * Nz - r0, nr, 1, nr, Nz, I.passz, T);
+  if (nr > 0)
+    fx_fft<true>(RawLd{r0, 1, nr, LineIn{bits, top}}, RowSt{spec + (size_t)lo * ps, ps, (size_t)Nxh, LineOut{bits, halvings, top}},
+                 r0, L * Nz - r0, nr, 1, nr, Nz, I.passz, T);
   cl.sync();   // no CTA leaves while another may still read its lane values
 }
 
