@@ -31,8 +31,10 @@ def sources():
     return sorted(os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cu"))
 
 
-# variants: None (the library) or "bounds" (every field index checked and
-# clamped, violations recorded in the instance's status word)
+# variants: None (the library) or "bounds" (the field indices of every kernel
+# that forms them from x, y and z checked and clamped, violations recorded in the
+# instance's status word; tests/test_kernel_sources_cpu.py lists the kernels that
+# run over whole arrays, lines or columns by a flat index instead)
 VARIANTS = {None: (OUT, LIB, []),
             "bounds": (os.path.join(OUT, "bounds"), os.path.join(OUT, "libchl_bounds.so"), ["-DCHL_BOUNDS_CHECK"])}
 

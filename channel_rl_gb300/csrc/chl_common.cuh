@@ -365,6 +365,18 @@ __device__ __forceinline__ void chl_clamp(const ChlInst& I, int& i, int& j, int&
 #endif
 }
 
+// an index of [0, n)
+__device__ __forceinline__ void chl_clamp_to(const ChlInst& I, int& i, int n) {
+#ifdef CHL_BOUNDS_CHECK
+  if (i < 0 || i >= n) {
+    atomicOr(I.status, CHL_STATUS_BOUNDS);
+    i = min(max(i, 0), n - 1);
+  }
+#else
+  (void)I; (void)i; (void)n;
+#endif
+}
+
 // element of a centre-like and of a V-like field (an instance has fewer than
 // 2^31 points, so 32-bit arithmetic)
 __device__ __forceinline__ size_t cidx(const ChlInst& I, int i, int jc, int k) {

@@ -210,6 +210,13 @@ k_filter(ChlMap map) {
     row[3] = j + 1 >= last ? j : j + 2;
   }
   const int e = conv ? filt_exp(I, min(g, (Ny - 1) / 2)) : 0;
+  // the field indices of this kernel are offsets; the bounds-checked build checks
+  // what they are made of (and the neighbours in shared memory as x and y of a block)
+  int xi = 2 * pi, kz = zc * f.M;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) chl_clamp(I, xi, row[q], kz, nrow - 1);
+  pi = xi >> 1;
+  chl_clamp_to(I, left, (int)blockDim.x); chl_clamp_to(I, right, (int)blockDim.x);
   const unsigned pitch = (unsigned)f.nxp * (unsigned)nrow;
   const unsigned off0 = f.nxp * row[0] + pi, off1 = f.nxp * row[1] + pi, off2 = f.nxp * row[2] + pi, off3 = f.nxp * row[3] + pi;
   auto get = [&](longlong2 v, int down) {
@@ -233,6 +240,7 @@ k_filter(ChlMap map) {
     const Pair v0 = get(n0, down.x), v1 = get(n1, down.y), v2 = get(n2, down.z), v3 = get(n3, down.w);
     k = k + 1 == Nz ? 0 : k + 1;
     if (it < k1 - k0 + 1) {
+      chl_clamp_to(I, k, Nz);
       s = src + (size_t)pitch * k;
       n0 = __ldg(s + off0); n1 = __ldg(s + off1); n2 = __ldg(s + off2); n3 = __ldg(s + off3);
     }
@@ -254,8 +262,11 @@ k_filter(ChlMap map) {
     if (it >= 2 && out) {
       const Pair z0 = tap(a0, b0, x0), z1 = tap(a1, b1, x1);
       // wall fields go to rows 1 and Ny of a centre-like field
-      const int nr = wall ? Ny + 2 : nrow, ra = wall ? 1 : j0, rc = wall ? Ny : j0 + 1;
-      longlong2* d = dst + (size_t)f.nxp * ((size_t)nr * (k0 + it - 2)) + pi;
+      const int nr = wall ? Ny + 2 : nrow;
+      int ra = wall ? 1 : j0, rc = wall ? Ny : j0 + 1, ko = k0 + it - 2;
+      chl_clamp(I, xi, ra, ko, nr - 1);
+      if (two) chl_clamp_to(I, rc, nr);
+      longlong2* d = dst + (size_t)f.nxp * ((size_t)nr * ko) + pi;
       d[(size_t)f.nxp * ra] = make_longlong2(z0.x, z0.y);
       if (two) d[(size_t)f.nxp * rc] = make_longlong2(z1.x, z1.y);
     }
