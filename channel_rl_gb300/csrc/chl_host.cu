@@ -240,8 +240,8 @@ std::vector<int4> fft_table(int N) {
   return t;
 }
 
-// FP64 pass table of a length-N Stockham FFT in tangent form
-// (chl_fft_pass_table): per pass with twiddles and butterfly class jm, the
+// FP64 pass table of a length-N Stockham FFT in tangent form, for callers of
+// chl_fft_pass_table (the library's transforms use fft_table's): per pass with twiddles and butterfly class jm, the
 // twiddles w_r = C + iS = exp(-2 pi i m/N), m = jm r N/(Ns R), each as sigma
 // (C or S, the larger in magnitude) and m (S/C or C/S), and the butterfly's
 // combined scales.
@@ -899,13 +899,27 @@ int chl_grid_constants(const chl_grid_desc* d, double* out) {
   return CHL_OK;
 }
 
+// N = 2^a 3^b
+static bool fft_length(int N) {
+  while (N > 1 && N % 2 == 0) N /= 2;
+  while (N > 1 && N % 3 == 0) N /= 3;
+  return N == 1;
+}
+
+int chl_fft_table(int N, int* out, int cap) {
+  if (!fft_length(N)) return -1;
+  const std::vector<int4> t = fft_table(N);
+  const int len = 1 + 4 * (int)t.size();
+  if (out) {
+    if (cap < len) return -2;
+    out[0] = chl_fft_bits(N);
+    std::memcpy(out + 1, t.data(), 16 * t.size());
+  }
+  return len;
+}
+
 int chl_fft_pass_table(int N, double* out, int cap) {
-  if (N < 1) return -1;
-  int r = N;
-  while (r % 4 == 0) r /= 4;
-  while (r % 3 == 0) r /= 3;
-  while (r % 2 == 0) r /= 2;
-  if (r != 1) return -1;
+  if (!fft_length(N)) return -1;
   const std::vector<double> t = fft_pass_table(N);
   if (out) {
     if (cap < (int)t.size()) return -2;

@@ -71,7 +71,7 @@ EXPORTS = (
     "chl_compute_wall_model", "chl_compute_rhs", "chl_compute_projection_step",
     "chl_compute_dPx_for_constant_mass_flow", "chl_compute_pressure", "chl_check_divergence",
     "chl_stats", "chl_stats_profiles", "chl_synchronize", "chl_grid_constants_size",
-    "chl_grid_constants", "chl_fft_pass_table", "chl_set_fields", "chl_download_async", "chl_time_steps",
+    "chl_grid_constants", "chl_fft_pass_table", "chl_fft_table", "chl_set_fields", "chl_download_async", "chl_time_steps",
     "chl_graph_kernel_count", "chl_profile_step",
     "chl_autotune", "chl_get_tile_shapes", "chl_set_tile_shapes",
     "chl_check_divergence_noalloc", "chl_noalloc_last_error", "chl_device_reset",
@@ -271,8 +271,22 @@ def sqrt_selftest(a):
     return y
 
 
+def fft_table(N):
+    """Starting bits and table entries (n, 4) of the length-N transform
+    (chl_fft_table; no GPU needed)."""
+    f = load().chl_fft_table
+    f.argtypes = [C.c_int, C.POINTER(C.c_int), C.c_int]
+    n = f(int(N), None, 0)
+    if n < 0:
+        raise ChlError(f"chl_fft_table: no table for length {N} ({n})", n)
+    out = np.zeros(n, dtype=np.int32)
+    f(int(N), out.ctypes.data_as(C.POINTER(C.c_int)), n)
+    return int(out[0]), out[1:].reshape(-1, 4)
+
+
 def fft_pass_table(N):
-    """The length-N transform's pass table (chl_fft_pass_table; no GPU needed)."""
+    """The pass table of a length-N FP64 transform in tangent form
+    (chl_fft_pass_table; no GPU needed; the library's transforms use fft_table's)."""
     lib = load()
     n = lib.chl_fft_pass_table(int(N), None, 0)
     if n < 0:

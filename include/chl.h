@@ -301,6 +301,16 @@ int chl_grid_constants(const chl_grid_desc* desc, double* out);
  * too small. */
 int chl_fft_pass_table(int N, double* out, int cap);
 
+/* The table that the library's own transforms of length N use, in 64-bit fixed
+ * point (host only, no GPU needed): out[0] the bits that a line's largest
+ * component may have at the start, then entries of four words: per pass {R, Ns,
+ * 2^32/Ns, 2^32/(N/R)} (reciprocals rounded up, 0 for 1), then per pass after
+ * the first and r = 1..R-1 the twiddles exp(-2 pi i jm r/(Ns R)), jm =
+ * 0..Ns-1, as the words (high, low >> 1) of cos 2^63 and of sin 2^63.  Returns
+ * the length in words and fills out when out is not NULL and cap holds it; -1
+ * and -2 as above. */
+int chl_fft_table(int N, int* out, int cap);
+
 /* ---- files in the reference's formats (host only, no GPU needed) ----------
  * Snapshot: the stream layout of output_data / read_input_data
  * (input_output.f90:390-730), as scripts/check_file.m reads it: int32 n and
