@@ -131,7 +131,6 @@ struct ChlInst {
   double dy1;                   // y(2)-y(1) (nu_t ghost rule 2 of AMD and Vreman)
   double gb1, gb2, gt1, gt2;    // pressure-BC metric factors g, g2 (pressure.f90:282-316)
   double dygb, dygt;            // yg(2)-yg(1), yg(nyg)-yg(nyg-1)
-  double mass_norm;             // 1/(Nx*Nz)
   // geometry (reciprocal spacings; see chl_host.cpp for the exact list)
   const double *rdxc, *rdxf, *rdyc, *rdyf, *rdzc, *rdzf;
   const double *dxf, *dyf, *dzf;  // raw spacings (dt)

@@ -460,7 +460,6 @@ static int upload_consts(chl_handle* h, Inst& I) {
   D.gt1 = (3.0 * y[c.ny] - 4.0 * y[c.ny - 1] + y[c.ny - 2]) / 2.0;
   D.gt2 = 2.0 * y[c.ny] - 5.0 * y[c.ny - 1] + 4.0 * y[c.ny - 2] - 1.0 * y[c.ny - 3];
   D.dygb = c.yg[2] - c.yg[1]; D.dygt = c.yg[c.nyg] - c.yg[c.nyg - 1];
-  D.mass_norm = 1.0 / ((double)Nx * Nz);
   D.rdxc = P(o_rdxc) + 1; D.rdxf = P(o_rdxf) + 1; D.dxf = P(o_dxf) + 1;
   D.rdzc = P(o_rdzc) + 1; D.rdzf = P(o_rdzf) + 1; D.dzf = P(o_dzf) + 1;
   D.rdyc = P(o_rdyc); D.rdyf = P(o_rdyf); D.dyf = P(o_dyf); D.w0x2 = P(o_w0); D.w1x2 = P(o_w1); D.ygc = P(o_ygc);
