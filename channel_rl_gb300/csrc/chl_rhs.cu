@@ -351,11 +351,10 @@ __device__ __forceinline__ Rhs rhs_pair(const ChlInst& I, int i, int jc, int k) 
   // stored as doubles: y-faces jc - 1 and jc, centre rows jc and jc + 1
   const bool dl = WALL && wall_face(I, jc - 1), dh = WALL && wall_face(I, jc), dc = WALL && wall_centre(I, jc);
   const bool dn = WALL && wall_centre(I, jc + 1);
-  // difference of two fluxes of one row (of doubles the first of a pair on the
-  // integer pipe, beside the second) and of two rows
-  auto diff = [](fx hi, fx lo, bool d, int x, bool first) {
-    const double a = __longlong_as_double(hi), b = __longlong_as_double(lo);
-    return WALL && d ? (first ? fx_sub(a, b) : a - b) : fx_to<true>(hi - lo, x);
+  // difference of two fluxes of one row (of doubles on the integer pipe: the FP64
+  // pipe has the products) and of two rows
+  auto diff = [](fx hi, fx lo, bool d, int x) {
+    return WALL && d ? fx_sub(__longlong_as_double(hi), __longlong_as_double(lo)) : fx_to<true>(hi - lo, x);
   };
   auto ydiff = [](fx hi, bool dhi, int ehi, fx lo, bool dlo, int elo) {
     return WALL ? flux_val(hi, dhi, ehi) - flux_val(lo, dlo, elo) : row_diff(hi, ehi, lo, elo);
@@ -366,34 +365,34 @@ __device__ __forceinline__ Rhs rhs_pair(const ChlInst& I, int i, int jc, int k) 
     const longlong2 x = g2(G[G_UX], c), yh = g2(G[G_UY], e), yl = g2(G[G_UY], em);
     const longlong2 zh = g2(G[G_UZ], c), zl = g2(G[G_UZ], cidx(I, i, jc, km));
     const fx xp = LDG(G[G_UX] + cidx(I, ip, jc, k));
-    F.u.x = fma(diff(x.y, x.x, dc, e0.x, true), rxf0, dpdx);
-    F.u.y = fma(diff(xp, x.y, dc, e0.x, false), rxf1, dpdx);
+    F.u.x = fma(diff(x.y, x.x, dc, e0.x), rxf0, dpdx);
+    F.u.y = fma(diff(xp, x.y, dc, e0.x), rxf1, dpdx);
     F.u.x = fma(ydiff(yh.x, dh, e0.x, yl.x, dl, el.x), ryc, F.u.x);
     F.u.y = fma(ydiff(yh.y, dh, e0.x, yl.y, dl, el.x), ryc, F.u.y);
-    F.u.x = fma(diff(zh.x, zl.x, dc, e0.x, true), rzc, F.u.x);
-    F.u.y = fma(diff(zh.y, zl.y, dc, e0.x, false), rzc, F.u.y);
+    F.u.x = fma(diff(zh.x, zl.x, dc, e0.x), rzc, F.u.x);
+    F.u.y = fma(diff(zh.y, zl.y, dc, e0.x), rzc, F.u.y);
   }
   {  // w at (x-centre i, row jc, z-face k)
     const longlong2 x = g2(G[G_WX], c), yh = g2(G[G_WY], e), yl = g2(G[G_WY], em);
     const longlong2 zl = g2(G[G_WZ], c), zh = g2(G[G_WZ], cidx(I, i, jc, kp));
     const fx xm = LDG(G[G_WX] + cidx(I, im, jc, k));
-    F.w.x = diff(x.x, xm, dc, e0.z, true) * rxc0;
-    F.w.y = diff(x.y, x.x, dc, e0.z, false) * rxc1;
+    F.w.x = diff(x.x, xm, dc, e0.z) * rxc0;
+    F.w.y = diff(x.y, x.x, dc, e0.z) * rxc1;
     F.w.x = fma(ydiff(yh.x, dh, e0.z, yl.x, dl, el.z), ryc, F.w.x);
     F.w.y = fma(ydiff(yh.y, dh, e0.z, yl.y, dl, el.z), ryc, F.w.y);
-    F.w.x = fma(diff(zh.x, zl.x, dc, e0.z, true), rzf, F.w.x);
-    F.w.y = fma(diff(zh.y, zl.y, dc, e0.z, false), rzf, F.w.y);
+    F.w.x = fma(diff(zh.x, zl.x, dc, e0.z), rzf, F.w.x);
+    F.w.y = fma(diff(zh.y, zl.y, dc, e0.z), rzf, F.w.y);
   }
   if (hasv) {  // v at (x-centre i, y-face jv = jc, z-centre k)
     const longlong2 x = g2(G[G_VX], e), yl = g2(G[G_VY], c), yh = g2(G[G_VY], cidx(I, i, jc + 1, k));
     const longlong2 zh = g2(G[G_VZ], e), zl = g2(G[G_VZ], vidx(I, i, jc, km));
     const fx xm = LDG(G[G_VX] + vidx(I, im, jc, k));
-    F.v.x = diff(x.x, xm, dh, e0.y, true) * rxc0;
-    F.v.y = diff(x.y, x.x, dh, e0.y, false) * rxc1;
+    F.v.x = diff(x.x, xm, dh, e0.y) * rxc0;
+    F.v.y = diff(x.y, x.x, dh, e0.y) * rxc1;
     F.v.x = fma(ydiff(yh.x, dn, eh.y, yl.x, dc, e0.y), ryf, F.v.x);
     F.v.y = fma(ydiff(yh.y, dn, eh.y, yl.y, dc, e0.y), ryf, F.v.y);
-    F.v.x = fma(diff(zh.x, zl.x, dh, e0.y, true), rzc, F.v.x);
-    F.v.y = fma(diff(zh.y, zl.y, dh, e0.y, false), rzc, F.v.y);
+    F.v.x = fma(diff(zh.x, zl.x, dh, e0.y), rzc, F.v.x);
+    F.v.y = fma(diff(zh.y, zl.y, dh, e0.y), rzc, F.v.y);
   }
   // a row marked non-finite by its maxima (none where its fluxes are doubles)
   const int bad = WALL ? (dc ? 0 : e0.w) | (dl ? 0 : el.w) | (dn ? 0 : eh.w) : e0.w | el.w | eh.w;
