@@ -292,25 +292,30 @@ k_minabs(ChlMap map, int s) {
   }
 }
 
+// chl_put_dt as a call: its products would be predicated into every thread
+static __device__ __noinline__ void put_dt(double* scal, double dt) { chl_put_dt(scal, dt); }
+
 // With a fixed time step the minima are not needed (compute_dt reduces them
 // and then replaces dt by -CFL, time_integration.f90:146-148); what the pass
 // must still do is flag non-finite velocities.  One thread per pair of centres
 // (i, jc, k), jc = 1..Ny, reading the same U, V, W entries as k_minabs; 32-bit
-// index arithmetic (a 64-bit division takes FP64 instructions, six per point).
+// index arithmetic (a 64-bit division takes FP64 instructions), and the words are
+// read as integers: of a comparison of doubles' bit patterns the compiler makes
+// FP64 comparisons, six per point.
 __global__ void __launch_bounds__(256)
 k_nonfinite(ChlMap map, int s) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
   const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  if (t == 0) chl_put_dt(I.scal, -I.CFL);   // fixed step (compute_dt, time_integration.f90:146-148)
+  if (t == 0) put_dt(I.scal, -I.CFL);   // fixed step (compute_dt, time_integration.f90:146-148)
   bool bad = false;
   if (t < (unsigned)(I.Nx / 2 * I.Ny * I.Nz)) {
     const ChlIdx p = chl_split(t, I.Nx / 2, I.Ny);
     const int i = 2 * p.i, jc = 1 + p.j, k = p.k;
     auto inf = [](const double* f) {
-      const double2 v = __ldg(reinterpret_cast<const double2*>(f));
-      return absbits(v.x) >= CHL_BIG_BITS || absbits(v.y) >= CHL_BIG_BITS;
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(f));
+      return max(v.y & 0x7FFFFFFFu, v.w & 0x7FFFFFFFu) >= 0x7FF00000u;
     };
     bad = inf(I.U[s] + cidx(I, i, jc, k)) | inf(I.V[s] + vidx(I, i, jc, k)) | inf(I.W[s] + cidx(I, i, jc, k));
   }
@@ -534,7 +539,7 @@ void chl_launch_minabs_init(const ChlMap& m, cudaStream_t st) {
 void chl_launch_minabs(const ChlMap& m, int nb, int s, cudaStream_t st) {
   chl_launch_pdl(k_minabs, dim3(nb), dim3(256), 0, st, m, s);
 }
-// nb: blocks of 256 centres (the point map)
+// nb: blocks of the map of point pairs
 void chl_launch_nonfinite(const ChlMap& m, int nb, int s, cudaStream_t st) {
   chl_launch_pdl(k_nonfinite, dim3(nb), dim3(m.tb), 0, st, m, s);
 }
