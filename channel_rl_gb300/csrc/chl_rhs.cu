@@ -115,7 +115,7 @@ k_fix(ChlMap map, int s, int prep) {
     const int j = t;
     const int4 x = vel_exp(I, j);
     I.vexp[j] = x;
-    if (j >= 1) {
+    if (j >= 1 && I.LES_model == 2) {      // dynamic model
       // centre row j with the rows of faces that the test filter brings into it
       const int a = max(j - 1, 1);
       const int u = max(x.x, fx_exp<61>(chl_row_max(I, 0, a))), w = max(x.z, fx_exp<61>(chl_row_max(I, 2, a)));
