@@ -87,9 +87,9 @@ __host__ __device__ inline int chl_dsm_planes(int Nx, int Ny, int Nz) {
   return m;
 }
 // complex rows (pairs of real x lines) per x-transform block: up to
-// 512/Nx (at 256x96x192 the two x transforms take 95 + 54 us per launch with
-// 1024 points, 89 + 51 with 512, 91 + 52 with 256), halved while the instance's grid would have fewer than
-// min_blocks blocks (CHL_FFT_MIN_BLOCKS unless the tuner chose another)
+// 512/Nx (at 256x96x192 the two x transforms take 88 + 51 us per launch with
+// 1024 points, 82 + 49 with 512, 84 + 49 with 256), halved while the instance's
+// grid would have fewer than min_blocks blocks (CHL_FFT_MIN_BLOCKS unless the tuner chose another)
 __host__ __device__ inline int chl_fftx_rows(int Nx, int nrow, int min_blocks) {
   int cr = 512 / Nx;
   if (cr < 1) cr = 1;
@@ -415,7 +415,7 @@ __device__ __forceinline__ double nut_ghost(const ChlInst& I, double v) {
 // until that kernel has finished and its writes are visible.  Without the
 // launch attribute the wait returns at once.  (No kernel triggers its
 // successor early: with a trigger ahead of or behind the wait the 32x48x32
-// step took 324 or 296 us instead of 252, the 256x96x192 one 1-5 % more.)
+// step took 29 or 17 % longer, the 256x96x192 one 1-5 %.)
 __device__ __forceinline__ void chl_pdl_wait() {
 #if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ >= 900)
   cudaGridDependencySynchronize();

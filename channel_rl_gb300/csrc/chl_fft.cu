@@ -793,7 +793,8 @@ k_fftx_inv(ChlMap map, int dst, int xmb) {
 // the largest velocities of the set and its rows (cleared by k_div_fftx).
 // The FP64 pipe bounds it (6 instructions per point, 71 % busy), so two of a
 // pair's six differences are formed on the integer pipe: 60 -> 55 us at
-// 256x96x192 (one, two, three, four, six of them 57, 55, 55, 61, 64 us; HBM floor 39).
+// 256x96x192 (one, two, three, four, six of them 57, 55, 55, 61, 64 us; HBM floor
+// 39), 61 since it folds the rows' largest too.
 __global__ void __launch_bounds__(256)
 k_project(ChlMap map, int s) {
   chl_pdl_wait();

@@ -10,8 +10,9 @@
 // double.  A field is scaled by its own largest magnitude (kept with the
 // velocity set, ChlInst::status), so that |F| < 2^61: eight bits finer than
 // a double's last bit at that magnitude, and exact for every double down to
-// 2^-8 of it (k_flux, whose rows differ by more, scales every row by its own).  Sums and differences are exact; a product keeps 60 bits or
-// more of its largest possible value.
+// 2^-8 of it (k_flux, whose rows differ by more, scales every row by its own).
+// Sums and differences are exact; a product keeps 60 bits or more of its largest
+// possible value.
 #pragma once
 #include "chl_common.cuh"
 

@@ -348,8 +348,8 @@ struct chl_handle {
   int twz = 0;                        // longest z transform table of the instances
   // planes per thread of the marching kernels: 4, halved while the batch has
   // fewer than 4 x 256 threads per SM (at 256x96x192 one, two, four, eight and
-  // sixteen planes: k_flux 211, 181, 172, 174, 181 us, k_strain -, 238, 200,
-  // 202, 204 us); of the test filter: 16, halved while it has fewer than 8
+  // sixteen planes took k_flux 211, 181, 172, 174, 181 us and k_strain -, 238, 200,
+  // 202, 204 us when chosen; 193 and 218 with four now); of the test filter: 16, halved while it has fewer than 8
   // blocks per SM
   int planes = 4, fplanes = 16;
   int tb_filter = 128;                // threads of the test filter's blocks: a whole x-line of point pairs where it fits

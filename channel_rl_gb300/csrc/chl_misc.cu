@@ -335,8 +335,9 @@ __global__ void k_minabs_init(ChlMap map) {
 // (time_integration.f90:89-94).  A block per CHL_MASS_POINTS points of a plane
 // writes its sum to red, the instance's last block to finish (counter
 // dsm_cnt[0]; rows count from 1) adds them in order.  One block for the whole
-// plane is bound by its loads' latency: 94 us at 256x192, 12 like this; k_shift over pairs of
-// points 27 -> 18.
+// plane is bound by its loads' latency: 94 us at 256x192, 12 like this; k_shift
+// takes 22 us over pairs of points (18 before it folded the rows' largest, 27 over
+// single points).
 __device__ __forceinline__ double block_sum256(double v, double* red) {
   red[threadIdx.x] = v;
   __syncthreads();

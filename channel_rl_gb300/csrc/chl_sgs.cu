@@ -23,12 +23,13 @@
 // Strain magnitude and the DSM filter inputs at centres (rows 1..Ny): q3..8
 // the products of the centre velocities' face sums in fixed point (last bit
 // 2^(e_i + e_j + 64), less the row's slack of both: next to a resolved wall the
-// products are 1e-8 of the field's largest and less), q9..14 = |S|*(S_ii, 2 S_ij) / sqrt(2) and their
-// largest per row.
+// products are 1e-8 of the field's largest and less), q9..14 = |S|*(S_ii, 2 S_ij)
+// / sqrt(2) and their largest per row.
 // With DSM = false (the static model, whose row coefficients do not depend on
-// the strain) nu + nu_t instead, so that no pass reads |S| back: 143 -> 157 us
-// at 256x96x192 for the 37 that k_nut then took and the launch of the
-// coefficients' own kernel.
+// the strain) nu + nu_t instead, so that no pass reads |S| back: 14 us at
+// 256x96x192 for the 37 that k_nut then took and the launch of the coefficients'
+// own kernel.  218 and 170 us there (202 and 157 with one x and z spacing for both
+// edges of a centre).
 template <bool DSM>
 __global__ void __launch_bounds__(CHL_FLUX_THREADS, 7)
 k_strain(ChlMap map, int s_in, int use_wm) {
@@ -81,7 +82,7 @@ k_strain(ChlMap map, int s_in, int use_wm) {
 // (4, 2)/6 at its first and last row.  Three separable FP64 passes took 2
 // instructions of 64 clocks per pass, field and point and moved every field
 // three times: 247 us per pass at 256x96x192.  Here a tap is an integer
-// shift and two additions, and the three passes take 236 us together.
+// shift and two additions, and the three passes take 239 us together.
 //
 // A pass forms (a + 4 b + c) >> 3, rounded (up at a half in y and z, down in x: a
 // mean error of L would not average out of its sums), so that a field starts and ends below 2^60
@@ -558,9 +559,9 @@ k_nut(ChlMap map, int use_wm) {
 // One thread per wall point; face i-1 comes from the lane to the left when
 // that lane is on the same row, so no thread returns before the shuffle.  The
 // values, which have no bound, stay out of the rows' largest (chl_rhs.cu:
-// wall_face).  A kernel of its own, beside the model's (300 -> 283 us of k_amd and 166 -> 157
-// of k_strain<false> at 256x96x192 where they did these rows, whose divisions
-// the whole block waits for).
+// wall_face).  A kernel of its own, beside the model's: where k_amd and
+// k_strain<false> did these rows, whose divisions the whole block waits for, they
+// took 17 and 9 us more at 256x96x192.
 __global__ void __launch_bounds__(256)
 k_wall_rows(ChlMap map, int s_in) {
   chl_pdl_wait();

@@ -1,5 +1,6 @@
 // Anisotropic minimum-dissipation (AMD) and Vreman eddy viscosities, one
-// fused kernel each, one thread per interior centre (rows 1..Ny).  Both write
+// fused kernel each, a thread per column of a few planes at an interior centre
+// (rows 1..Ny).  Both write
 // the unclipped nu_t into S and, in the same pass, nu + nu_t with k_nut's
 // rules for these models (write_nut_rows): max(., 0) and the ghost-row rule of
 // Dirichlet_nu_t - so there is no separate nu_t pass.
@@ -13,8 +14,7 @@
 // the three mixed products of each S_ij row are formed as written: two from
 // centre values, one interpolated after the product.  S_ij is compute_Sij's
 // (subgrid.f90:1014-1072), formed from the same edge sums.  The halves and
-// quarters of the interpolations are folded into constants (0.0625,
-// 0.03125): the FP64 pipe bounds these kernels.
+// quarters of the interpolations are exponents of the fixed-point values.
 //
 // Vreman (subgrid.f90:897-1004):
 //   nu_t = C sqrt(B_b / a_ij a_ij),  C = 2.5 * 0.1^2,
@@ -97,16 +97,16 @@ struct GradColumn {
 }  // namespace
 
 // AMD in fixed point.  As FP64 code this kernel issued 114 FP64 instructions
-// per point (0.97 ms per launch at 256x96x192, the FP64 pipe 90 % busy; 0.30 ms now).  The
+// per point (0.97 ms per launch at 256x96x192, the FP64 pipe 90 % busy; 0.31 ms now).  The
 // edge differences are exact integers from the fixed-point copies (k_fix);
 // each point scales those of each component by their largest, so that a weak
 // component keeps its digits, and forms the a_ij, the derivatives and D there.  The
 // S_ii, N and the division are FP64 (one scale for the three components and the
 // S_ii in integers beside the largest derivative took 0.28 ms and left nu_t of a
 // nearly parallel flow 9 times as far off as in FP64, of turbulent ones 1.1 to 1.2
-// times).  With three, six and twelve of N's twelve conversions on the FP64 pipe
-// 300, 309 and 359 us: all are on the integer pipe.
-__global__ void __launch_bounds__(CHL_FLUX_THREADS, 5)   // 2, 3, 4, 5, 6 blocks per SM took 417, 321, 289, 288, 290 us (301 now)
+// times).  With none, three, six and twelve of N's twelve conversions on the FP64
+// pipe 301, 300, 309 and 359 us (before the exact S_ii): all are on the integer pipe.
+__global__ void __launch_bounds__(CHL_FLUX_THREADS, 5)   // 2, 3, 4, 5, 6 blocks per SM took 417, 321, 289, 288, 290 us (312 now)
 k_amd(ChlMap map, int s_in, int use_wm) {
   chl_pdl_wait();
   int lb;
