@@ -655,7 +655,7 @@ static int build_maps(chl_handle* h) {
       switch (m) {
         case M_PT: b = cdiv((long)Nx * Ny * Nz, h->tb_pt); break;
         case M_PT2: b = cdiv((long)(Nx / 2) * Ny * Nz, h->tb_pt); break;         // pairs of x points (Nx even)
-        case M_FULL2: b = cdiv((long)(Nx / 2) * (Ny + 2) * Nz, h->tb_pt); break;
+        case M_FULL2: b = cdiv((long)(Nx / 2) * (Ny + 2) * Nz, h->tb_pt) + cdiv(Ny + 2, h->tb_pt); break;   // and rows
         case M_FILTER: b = chl_filter_blocks(Nx, Ny, Nz, h->tb_filter, h->fplanes); break;
         case M_FLUX: {
           const bool wm = h->wall_model != CHL_WM_NONE;

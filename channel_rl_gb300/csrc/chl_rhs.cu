@@ -85,24 +85,48 @@ static __device__ __noinline__ double smag_coef(const ChlInst& I, int jc) {
   return cd * cd * 1.41421356237309504880;    // (Cs Delta f)^2 |S| with S holding |S|/sqrt(2)
 }
 
+// k_fix's work for row j.  A call, for the registers.
+static __device__ __noinline__ void fix_row(const ChlInst& I, int s, int j, int prep) {
+  if (prep) {
+    I.nmax[j] = I.smax[j] = 0u;
+    if (prep & 2) I.coef[j] = j >= 1 && j <= I.Ny ? smag_coef(I, j) : 0.0;
+  }
+  if (j > I.Ny) return;
+  const int4 x = vel_exp(I, j);
+  I.vexp[j] = x;
+  if (j >= 1 && I.LES_model == 2) {      // dynamic model
+    // centre row j with the rows of faces that the test filter brings into it
+    const int a = max(j - 1, 1);
+    const int u = max(x.x, fx_exp<61>(chl_row_max(I, 0, a))), w = max(x.z, fx_exp<61>(chl_row_max(I, 2, a)));
+    const int v = max(x.y, fx_exp<61>(max(chl_row_max(I, 1, max(j - 2, 0)), chl_row_max(I, 1, min(j + 1, I.Ny)))));
+    const unsigned* vm = chl_vmax(I, s);
+    I.slack[j] = make_int4(min(24, fx_exp<61>(vm[0]) - u), min(24, fx_exp<61>(vm[1]) - v), min(24, fx_exp<61>(vm[2]) - w), 0);
+  }
+}
+
 // Fixed-point copies of the velocity set that a stage works on (rows as
 // stored, ghosts included).  prep: 1 clears the rows' largest |nu + nu_t|
 // and |S| S_ij ahead of the kernels that form them, + 2 forms the static
 // model's row coefficients.  Also forms the exponents of the rows' velocities for
 // k_flux, from what the set's writer folded.  Moves 48 bytes per point: HBM-bound.
+// An instance's first blocks do what goes by rows (a thread per row), beside the
+// others: in blocks that also copy it added 1 us to a launch of 8.
 __global__ void __launch_bounds__(256)
 k_fix(ChlMap map, int s, int prep) {
   chl_pdl_wait();
   int lb;
   const ChlInst& I = map.inst[chl_find(map, blockIdx.x, lb)];
-  const unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
-  if (prep && t < (unsigned)(I.Ny + 2)) {
-    I.nmax[t] = I.smax[t] = 0u;
-    if (prep & 2) I.coef[t] = t >= 1 && (int)t <= I.Ny ? smag_coef(I, t) : 0.0;
-  }
-  const unsigned* vm = chl_vmax(I, s);
   // pairs of points (Nx is even)
   const unsigned nc = (unsigned)(I.Nx * (I.Ny + 2) * I.Nz) / 2, nv = (unsigned)(I.Nx * (I.Ny + 1) * I.Nz) / 2;
+  // threads of the blocks of rows (blockDim is a power of two)
+  const unsigned rows = ((unsigned)I.Ny + 1u + blockDim.x) & ~(blockDim.x - 1u);
+  unsigned t = (unsigned)lb * blockDim.x + threadIdx.x;
+  if (t < rows) {
+    if ((int)t <= I.Ny + 1) fix_row(I, s, (int)t, prep);
+    return;
+  }
+  t -= rows;
+  const unsigned* vm = chl_vmax(I, s);
   const int eu = fx_exp<61>(vm[0]), ev = fx_exp<61>(vm[1]), ew = fx_exp<61>(vm[2]);
   auto put = [t](fx* x, double2 v, int e) { reinterpret_cast<longlong2*>(x)[t] = make_longlong2(fx_from(v.x, e), fx_from(v.y, e)); };
   auto get = [t](const double* x) { return __ldg(reinterpret_cast<const double2*>(x) + t); };
@@ -111,18 +135,6 @@ k_fix(ChlMap map, int s, int prep) {
   if (t < nv) v = get(I.V[s]);
   if (t < nc) { put(I.X[0], u, eu); put(I.X[2], w, ew); }
   if (t < nv) put(I.X[1], v, ev);
-  if (t <= (unsigned)I.Ny) {
-    const int j = t;
-    const int4 x = vel_exp(I, j);
-    I.vexp[j] = x;
-    if (j >= 1 && I.LES_model == 2) {      // dynamic model
-      // centre row j with the rows of faces that the test filter brings into it
-      const int a = max(j - 1, 1);
-      const int u = max(x.x, fx_exp<61>(chl_row_max(I, 0, a))), w = max(x.z, fx_exp<61>(chl_row_max(I, 2, a)));
-      const int v = max(x.y, fx_exp<61>(max(chl_row_max(I, 1, max(j - 2, 0)), chl_row_max(I, 1, min(j + 1, I.Ny)))));
-      I.slack[j] = make_int4(min(24, eu - u), min(24, ev - v), min(24, ew - w), 0);
-    }
-  }
 }
 
 // Fluxes next to a wall whose nu + nu_t the wall model sets (y-faces 0, 1 and
